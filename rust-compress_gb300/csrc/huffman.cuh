@@ -10,6 +10,7 @@ namespace rcg {
 constexpr int kHuffSyms = 257;
 
 struct HuffScratch {
+  uint4 key[(kHuffSyms + 3) / 4];  // the counts, an unused symbol's as the largest value
   int order[kHuffSyms];  // sorted position -> symbol
   unsigned long long weight[2 * kHuffSyms];
   int parent[2 * kHuffSyms];
@@ -28,14 +29,26 @@ __device__ inline void huff_lengths(const unsigned* freq, unsigned char* lens, H
   if (t < kHuffSyms) lens[t] = 0;
   if (t == 0) s.n_used = 0;
   if (t < 17) s.count[t] = 0;
+  const unsigned mine = t < kHuffSyms ? freq[t] : 0u;
+  if (t < 4 * ((kHuffSyms + 3) / 4)) reinterpret_cast<unsigned*>(s.key)[t] = mine > 0 ? mine : 0xffffffffu;
   __syncthreads();
-  if (t < kHuffSyms && freq[t] > 0) {
-    unsigned f = freq[t];
+  if (mine > 0) {
+    // Rank among the used symbols in the order (count, descending symbol): those before t must be smaller, those
+    // after t smaller or equal. Four counts per shared-memory load; 0xffffffff never counts.
+    const unsigned f = mine;
+    const int own = t >> 2;
     int r = 0;
-    for (int j = 0; j < kHuffSyms; j++) {
-      unsigned g = freq[j];
-      if (g > 0 && (g < f || (g == f && j > t))) r++;
-    }
+    auto below = [&](const uint4 g, unsigned lim) {
+      r += (g.x < lim) + (g.y < lim) + (g.z < lim) + (g.w < lim);
+    };
+#pragma unroll 4
+    for (int j = 0; j < own; j++) below(s.key[j], f);
+    const uint4 g = s.key[own];
+    const unsigned o[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++) r += (e < (t & 3) && o[e] < f) || (e > (t & 3) && o[e] <= f);
+#pragma unroll 4
+    for (int j = own + 1; j < (kHuffSyms + 3) / 4; j++) below(s.key[j], f + 1);
     s.order[r] = t;
     s.weight[r] = f;
     atomicAdd(&s.n_used, 1);
