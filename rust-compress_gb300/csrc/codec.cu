@@ -446,8 +446,7 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
   huff_lengths(freq, lens, scratch);
   // optimal_table sizes of the 256 real symbols; an empty table gets symbol 0 at length 1. Rdo: 0 -> 18 bits.
   if (t < 256) {
-    bool any = false;
-    for (int s = 0; s < 256; s++) any |= lens[s] > 0;
+    const bool any = scratch.n_used > 1;  // a used symbol besides the dummy
     unsigned size = lens[t];
     if (!any && t == 0) size = 1;
     len[t] = size == 0 ? 18.0f : (float)size;
@@ -459,6 +458,19 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
     int run = i / 16, size = i % 16;
     float rate = fadd(fadd(fmul((float)(run / 16), len[0xF0]), len[((run % 16) << 4) | size]), (float)size);
     st->lr[comp][i] = fmul(lambda, rate);
+  }
+  // Per size, the least entry over all runs (the trellis's scan bound): 16 lanes of 4 runs each per size. The products
+  // are those of the table and rounding is monotone, so the minimum is one of its entries.
+  if (t < 256) {
+    const int size = t >> 4;
+    float least = 3.0e38f;
+    for (int run = t & 15; run < 64; run += 16) {
+      float rate = fadd(fadd(fmul((float)(run / 16), len[0xF0]), len[((run % 16) << 4) | size]), (float)size);
+      least = fminf(least, fmul(lambda, rate));
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, off));
+    if ((t & 15) == 0) st->lrmin[comp][size] = least;
   }
   if (t == 0) st->eob[comp] = fmul(lambda, len[0]);
 }
@@ -479,22 +491,34 @@ int rate_tables(rcg_ctx* ctx, StepDesc* d_step) {
 // own position, so no 64-entry zd table is needed.
 // kWeighted: the perceptual mode. Each coefficient's distortion weight becomes rw[k] * pweights[block][k] (one f32
 // product, then the same squared-error product as the plain weight); the plain instantiation reads no weights.
-// 8 CTAs per SM (64 registers; the weighted instantiation spills 8 bytes and is still faster, 20.9 against 24.1 us
-// per candidate of a 3 MP perceptual search). The DP is latency-bound (one block's positions are serial); measured per
-// 12 MP candidate: 16-coefficient chunks at 6 CTAs per SM 75.6 us, 8-coefficient chunks at 8 CTAs 72.1 us. A rolled
-// DP loop over cp.async-staged shared-memory coefficients, (cost, zd) node pairs and an unrolled node scan were all
-// slower or no faster (80-92, 74.2 and 72.3-76.6 us). So was a work-list: at the qualities a search visits most
-// blocks have no position with a candidate (72% at q74, 96% at q62, yet only 3% of 32-block warps are all such
-// blocks), so the quantize kernel wrote those blocks' results (DC only) and listed the rest for the trellis: the
-// trellis went 70 -> 61 us but the quantize kernel 29 -> 40 us (the extra test per coefficient and the writes it
-// took over); listing the blocks in buckets by their count of candidates, heaviest first, scattered each warp's
-// blocks and cost 78 + 41 us. Sorting each CTA's blocks by that count, heaviest first, after a counting pass (the
-// DC-only blocks written there) gave the same 70.6 us: the cost is the per-position work every lane runs, not the
-// lanes that wait for a heavy neighbour. Cutting that work did help: each position's scale, step and weight are one
-// 16-byte shared-memory entry, and a node keeps its value with its sign instead of a 64-bit sign mask updated at
-// every position: 70.7 -> 66.8 us, the same coefficients. The pass then waits on its coefficient loads, yet deeper
-// prefetches measured slower: two chunks ahead 68.5 us, 16-position chunks 71.2 us (7 CTAs per SM), two or three
-// chunks staged ahead in shared memory by 4-byte cp.async copies 79-81 us.
+// One block per thread: the DP of a block is serial, so the kernel is bound by the latency of one position and, at
+// large sizes, by the per-position work every lane runs (sorting or listing blocks by their number of candidates
+// measured no better). What counts is therefore the length of a position's dependency chain and the bytes a block
+// keeps outside registers. Measured per candidate, full scans over nodes in local memory against the form below:
+// 240x180 4:4:4 35 -> 19 us (a search's mean), 1283x857 69 -> 25, 1653x2339 gray 77 -> 38, 4000x3000 65.5 -> 55,
+// a 3000x2000 requantization 154 -> 100 (its source rows as 16-byte loads among that), weighted 1620x1080 54 -> 32.
+// 7 CTAs per SM (72 registers): 8 spill (58 us at 12 MP), 6 leave too few warps (68 us with 4 nodes in registers);
+// the window at 2 nodes: 1, 3, 4 and 6 measured 53, 64, 66 and 71 us at 12 MP and 42, -, -, - against 38 us gray; 64
+// threads a CTA 62 us. Coefficients arrive 8 at a time, the next chunk's loads in flight (deeper prefetches, through
+// registers or shared memory, measured slower); scale, step and weight of a position are one 16-byte entry.
+//
+// The scan over earlier nodes goes from the newest to the oldest and stops when no older node can win. Keeping a
+// coefficient of magnitude >= 1 lowers cost - zd (the cost relative to dropping everything so far) by far more than
+// any code length differs, so the best predecessor is nearly always one of the last few nodes, where a full scan
+// costs as many steps as the block has candidates so far. The bound is exact, so the coefficients are those of the
+// full scan: npmin is the least cost - zd of a node and all before it, rounded down; every node's base is at least
+// (npmin + zprev)(1 - 2^-23) by the two roundings of its own computation (costs and zd are sums of non-negative terms
+// and zd never falls), scan_floor stays below that, and the two additions after it are the node's own, with the
+// least rate of the table in place of the node's: rounding is monotone, so a bound above the best rules out every
+// older node. Ties: a full ascending scan with strict < keeps the start of the block over any node and the lowest
+// node of equal cost, which descending is <= among nodes and < against the start. Weights of a caller may be negative
+// or NaN: such a block scans in full from there on.
+__device__ __forceinline__ float scan_floor(float pmin, float zprev) {
+  return __fmul_rd(__fadd_rd(pmin, zprev), 1.0f - 0x1p-22f);
+}
+
+constexpr int kWin = 2;  // nodes of the trellis scan held in registers
+
 template <bool kWeighted>
 __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const CacheSet& cs, long long bx) {
   // The per-position tables of every component and the lambda*rate tables of the components this CTA's blocks
@@ -523,30 +547,46 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
   const int16_t* src = requant ? st->coef_src + gb * 64 : nullptr;
   const float4* tab = s_tab[c];
   const float* lrc = lr[c];
+  const float* lmin = st->lrmin[c];
   const float* pw = kWeighted ? st->pweights + gb * 64 : nullptr;  // 16-byte aligned rows of 64 floats
 
-  float ncost[128], nzd[128];
-  unsigned char npos[128];
-  short nv[128];
-  signed char nprev[128];
+  // Every node as (cost, zd, the least cost - zd up to it, packed position | value | predecessor): written once, read
+  // by the few scans that go past the window and by the final walk back.
+  float4 nodes[126];
+  // The newest kWin nodes, newest first (cost infinity: none yet), and the bound for the nodes older than they.
+  float wcost[kWin], wzd[kWin];
+  int wrow[kWin];  // (position + 1) * 16: the rate row of position i is i * 16 - wrow
+#pragma unroll
+  for (int n = 0; n < kWin; n++) {
+    wcost[n] = __int_as_float(0x7f800000);
+    wzd[n] = 0.0f;
+    wrow[n] = 16;
+  }
+  float pm_all = __int_as_float(0x7f800000), pm_old = pm_all;
+  bool prune = true;
   int nn = 0;
   int dc = 0;
   float zprev = 0.0f;  // zd[i-1]
 
   // The coefficients arrive 8 at a time: the next chunk's loads are in flight while this chunk's DP steps run.
   constexpr int kChunk = 8;
-  auto load = [&](int k) -> float {
-    return requant ? (float)__ldg(src + k) : __ldg(cache + (long long)k * nb);
+  // A requantization's chunk is one 16-byte load of the block's row.
+  auto load_chunk = [&](int c0, float* to) {
+    if (requant) {
+      const int4 p = __ldg(reinterpret_cast<const int4*>(src + c0));
+      const int w4[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+      for (int j = 0; j < kChunk; j++) to[j] = (float)(short)((w4[j >> 1] >> (16 * (j & 1))) & 0xFFFF);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kChunk; j++) to[j] = __ldg(cache + (long long)(c0 + j) * nb);
+    }
   };
   float cur[kChunk], nxt[kChunk];
-#pragma unroll
-  for (int j = 0; j < kChunk; j++) cur[j] = load(j);
+  load_chunk(0, cur);
 #pragma unroll 1
   for (int c0 = 0; c0 < 64; c0 += kChunk) {
-    if (c0 + kChunk < 64) {
-#pragma unroll
-      for (int j = 0; j < kChunk; j++) nxt[j] = load(c0 + kChunk + j);
-    }
+    if (c0 + kChunk < 64) load_chunk(c0 + kChunk, nxt);
     float wv[kChunk];
     if constexpr (kWeighted) {
       const float4* p4 = reinterpret_cast<const float4*>(pw + c0);
@@ -569,11 +609,14 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
         continue;
       }
       float q = tb.y, w = kWeighted ? fmul(tb.z, wv[j]) : tb.z;
+      if constexpr (kWeighted) prune = prune && w >= 0.0f;
       const bool neg = a < 0.0f;  // a node keeps its value with this sign
       float m = fabsf(a);
-      unsigned v0 = (unsigned)fadd(m, 0.5f);
-      int pushed = 0;
-      if (v0 != 0) {
+      const float rounded = fadd(m, 0.5f);
+      int pushed = 0, packed[2] = {0, 0};
+      float best[2] = {0.0f, 0.0f};
+      if (rounded >= 1.0f) {
+        const unsigned v0 = (unsigned)rounded;
         unsigned lo = v0 > 1 ? v0 - 1 : v0;
         bool two = lo != v0;
         // candidate lo (first) and v0 (second, if distinct)
@@ -585,40 +628,63 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
         float best_lo = fadd(fadd(zprev, lrc[(i - 1) * 16 + s_lo]), dnz_lo);
         float best_hi = fadd(fadd(zprev, lrc[(i - 1) * 16 + s_hi]), dnz_hi);
         int prev_lo = -1, prev_hi = -1;
-        for (int ni = 0; ni < nn; ni++) {
-          float base = fadd(ncost[ni], fsub(zprev, nzd[ni]));
-          int ridx = (i - npos[ni] - 1) * 16;
-          float c_lo = fadd(fadd(base, lrc[ridx + s_lo]), dnz_lo);
-          float c_hi = fadd(fadd(base, lrc[ridx + s_hi]), dnz_hi);
-          if (c_lo < best_lo) {
+        auto offer = [&](float cost, float zd, int row, int ni) {
+          const float base = fadd(cost, fsub(zprev, zd));
+          const float* lrow = lrc + (i * 16 - row);
+          const float c_lo = fadd(fadd(base, lrow[s_lo]), dnz_lo);
+          const float c_hi = fadd(fadd(base, lrow[s_hi]), dnz_hi);
+          if (c_lo < best_lo || (c_lo == best_lo && prev_lo >= 0)) {
             best_lo = c_lo;
             prev_lo = ni;
           }
-          if (c_hi < best_hi) {
+          if (c_hi < best_hi || (c_hi == best_hi && prev_hi >= 0)) {
             best_hi = c_hi;
             prev_hi = ni;
           }
+        };
+#pragma unroll
+        for (int n = 0; n < kWin; n++) offer(wcost[n], wzd[n], wrow[n], nn - 1 - n);
+        // No node from here down can win once both bounds lie above the best (see the note on the scan above).
+        auto settled = [&](float pm) {
+          const float floor_base = scan_floor(pm, zprev);
+          return prune && fadd(fadd(floor_base, lmin[s_lo]), dnz_lo) > best_lo &&
+                 fadd(fadd(floor_base, lmin[s_hi]), dnz_hi) > best_hi;
+        };
+        if (nn > kWin && !settled(pm_old)) {
+          for (int ni = nn - 1 - kWin; ni >= 0; ni--) {
+            const float4 nd = nodes[ni];
+            if (settled(nd.z)) break;
+            offer(nd.x, nd.y, ((__float_as_int(nd.w) & 63) + 1) * 16, ni);
+          }
         }
-        ncost[nn] = best_lo;
-        npos[nn] = (unsigned char)i;
-        nv[nn] = (short)(neg ? -(int)lo : (int)lo);
-        nprev[nn] = (signed char)prev_lo;
-        nn++;
-        pushed = 1;
-        if (two) {
-          ncost[nn] = best_hi;
-          npos[nn] = (unsigned char)i;
-          nv[nn] = (short)(neg ? -(int)v0 : (int)v0);
-          nprev[nn] = (signed char)prev_hi;
-          nn++;
-          pushed = 2;
-        }
+        best[0] = best_lo;
+        best[1] = best_hi;
+        const int sign = neg ? -1 : 1;
+        packed[0] = i | (prev_lo & 0xff) << 6 | (sign * (int)lo) << 14;
+        packed[1] = i | (prev_hi & 0xff) << 6 | (sign * (int)v0) << 14;
+        pushed = two ? 2 : 1;
       }
       // zd[i] = zd[i-1] + (a*q)^2 * w; a node at position i keeps zd[i] (the reference reads zd[n.pos]).
       float e = fmul(a, q);
       float zcur = fadd(zprev, fmul(fmul(e, e), w));
-      if (pushed >= 1) nzd[nn - 1] = zcur;
-      if (pushed == 2) nzd[nn - 2] = zcur;
+#pragma unroll
+      for (int n = 0; n < 2; n++) {
+        if (n < pushed) {
+          pm_all = fminf(pm_all, __fsub_rd(best[n], zcur));
+          nodes[nn] = make_float4(best[n], zcur, pm_all, __int_as_float(packed[n]));
+          nn++;
+          pm_old = fminf(pm_old, __fsub_rd(wcost[kWin - 1], wzd[kWin - 1]));
+#pragma unroll
+          for (int k = kWin - 1; k > 0; k--) {
+            wcost[k] = wcost[k - 1];
+            wzd[k] = wzd[k - 1];
+            wrow[k] = wrow[k - 1];
+          }
+          wcost[0] = best[n];
+          wzd[0] = zcur;
+          wrow[0] = (i + 1) * 16;
+        }
+      }
       zprev = zcur;
     }
 #pragma unroll
@@ -628,9 +694,13 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
   const float eob = st->eob[c];
   float best_cost = fadd(zprev, eob);
   int best_end = -1;
-  for (int ni = 0; ni < nn; ni++) {
-    float cst = fadd(fadd(ncost[ni], fsub(zprev, nzd[ni])), npos[ni] < 63 ? eob : 0.0f);
-    if (cst < best_cost) {
+  for (int ni = nn - 1; ni >= 0; ni--) {
+    // Positions ascend, so once a node lies below 63 all before it do and pay the end-of-block code.
+    const float4 nd = nodes[ni];
+    const bool pays = (__float_as_int(nd.w) & 63) < 63;
+    if (prune && pays && fadd(scan_floor(nd.z, zprev), eob) > best_cost) break;
+    float cst = fadd(fadd(nd.x, fsub(zprev, nd.y)), pays ? eob : 0.0f);
+    if (cst < best_cost || (cst == best_cost && best_end >= 0)) {
       best_cost = cst;
       best_end = ni;
     }
@@ -646,15 +716,14 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
   for (int g = 1; g < 8; g++) reinterpret_cast<int4*>(out)[g] = z;
   int node = best_end;
   while (node >= 0) {
-    int p = npos[node];
-    short v = nv[node];
-    out[p] = (int16_t)v;
-    node = nprev[node];
+    const int pk = __float_as_int(nodes[node].w);
+    out[pk & 63] = (int16_t)(pk >> 14);
+    node = (int)(signed char)(pk >> 6);
   }
 }
 
 template <bool kWeighted>
-__global__ void __launch_bounds__(128, 8) k_trellis(StepDesc* __restrict__ st, CacheSet cs) {
+__global__ void __launch_bounds__(128, 7) k_trellis(StepDesc* __restrict__ st, CacheSet cs) {
   trellis_body<kWeighted>(st, cs, blockIdx.x);
 }
 
@@ -1029,7 +1098,7 @@ __global__ void __launch_bounds__(288) k_rate_tables_lock(const LockItem* __rest
   rate_tables_body(items[blockIdx.y].st, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(128, 8) k_trellis_lock(const LockItem* __restrict__ items, int n) {
+__global__ void __launch_bounds__(128, 7) k_trellis_lock(const LockItem* __restrict__ items, int n) {
   const int i = lock_find<&LockItem::q0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   trellis_body<false>(it.st, lock_caches(it), (long long)blockIdx.x - it.q0);

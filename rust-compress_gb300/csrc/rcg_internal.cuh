@@ -77,6 +77,7 @@ struct StepDesc {
   float lambda[3];
   float eob[3];          // lambda * len[0x00]
   float lr[3][64 * 16];  // lambda * rate(run, v) for run 0..63, size 0..15 (index run*16 + size)
+  float lrmin[3][16];    // least lr over the runs, per size
   unsigned int hist[2][256];  // AC symbol histogram of the plain pass, per class (jpeg/src/encode.rs:223-227)
   // Requantization of existing coefficients (jpeg/src/encode.rs:107-172)
   int requant;           // 1: the candidate requantizes coef_src instead of quantizing the FDCT cache
