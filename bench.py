@@ -248,12 +248,12 @@ def scorer_batch_workload(ctx, torch, dev, timed, n=64, steps=5):
     mpx = sum(w * h for w, h in sizes) / 1e6
     ctx.set_profiling(True)
     batch()
-    kb = {k: ctx.kernel_time(k)[1] for k in ("to_linear_batch", "pyramid_batch", "ssim2_tiles_batch",
+    kb = {k: ctx.kernel_time(k)[1] for k in ("build_batch", "ssim2_tiles_batch",
                                              "ssim2_reduce_batch")}
     ctx.set_profiling(False)
     ctx.set_profiling(True)
     one_by_one()
-    kp = {k: ctx.kernel_time(k)[1] for k in ("to_linear", "pyramid", "ssim2_tiles", "ssim2_reduce")}
+    kp = {k: ctx.kernel_time(k)[1] for k in ("build_pair", "ssim2_tiles", "ssim2_reduce")}
     ctx.set_profiling(False)
     del d_r, d_d
     torch.cuda.empty_cache()
@@ -262,8 +262,8 @@ def scorer_batch_workload(ctx, torch, dev, timed, n=64, steps=5):
             "pairs": n, "megapixels": mpx, "batch_ms": ms_b, "one_by_one_ms": ms_p,
             "batch_mpx_per_s": mpx / (ms_b / 1000.0), "one_by_one_mpx_per_s": mpx / (ms_p / 1000.0),
             "batch_vs_one_by_one": ms_p / ms_b, "identical_scores": [float(x) for x in sb] == sp,
-            "batch_kernels_ms": kb, "one_by_one_kernels_ms": kp, "launches_per_batch": 4,
-            "launches_one_by_one": 6 * n, "clocks": clocks}
+            "batch_kernels_ms": kb, "one_by_one_kernels_ms": kp, "launches_per_batch": 3,
+            "launches_one_by_one": 3 * n, "clocks": clocks}
 
 
 def sweep_workload(ctx, img, steps=3):
@@ -795,9 +795,8 @@ def main():
         step_device()
     prof = {}
     for k in ("ssim2_tiles_cached", "ssim2_tiles_store", "ssim2_tiles", "trellis", "quantize", "dequant_idct",
-              "upsample_color", "pyramid", "upsample_pyramid", "ssim2_reduce", "rate_tables", "step_tables",
-              "fdct_cache", "color_pad",
-              "chroma_down", "to_linear"):
+              "build_diff", "build_reference", "ssim2_reduce", "rate_tables", "step_tables",
+              "fdct_cache", "color_pad", "chroma_down"):
         n, ms = ctx.kernel_time(k)
         prof[k] = {"launches": n, "ms": ms}
     ctx.set_profiling(False)

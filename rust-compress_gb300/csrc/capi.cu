@@ -650,15 +650,12 @@ int rcg_ctx_band_chunks(rcg_ctx* ctx, uint32_t width, uint32_t height) {
 static int score_device_images(rcg_ctx* ctx, const uint8_t* d_ref, const uint8_t* d_dist, int w, int h, int channels,
                                int depth, double* score) {
   PyramidDesc pd = make_pyramid(w, h);
-  float* ref_pyr = (float*)workspace(ctx, "ref_pyr", (size_t)pd.floats * sizeof(float));
+  float* ref_pyr = (float*)workspace(ctx, "ref_xyb", (size_t)pd.floats * sizeof(float));
   float* dist_pyr = (float*)workspace(ctx, "dist_pyr", (size_t)pd.floats * sizeof(float));
   double* d_score = (double*)workspace(ctx, "score", sizeof(double));
   if (!ref_pyr || !dist_pyr || !d_score) return RCG_NO_MEMORY;
   int rc;
-  if ((rc = to_linear(ctx, d_ref, w, h, channels, depth, ref_pyr)) != RCG_OK) return rc;
-  if ((rc = to_linear(ctx, d_dist, w, h, channels, depth, dist_pyr)) != RCG_OK) return rc;
-  build_pyramid(ctx, pd, ref_pyr);
-  build_pyramid(ctx, pd, dist_pyr);
+  if ((rc = build_pair(ctx, pd, d_ref, d_dist, channels, depth, ref_pyr, dist_pyr)) != RCG_OK) return rc;
   score_pyramids(ctx, pd, ref_pyr, dist_pyr, d_score, nullptr, nullptr);
   double s = 0.0;
   cudaMemcpyAsync(&s, d_score, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
@@ -706,8 +703,8 @@ int rcg_ssimulacra2_exact(rcg_ctx* ctx, const uint8_t* reference, const uint8_t*
   int rc;
   if ((rc = copy_to_device(ctx, d_a, reference, bytes)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_b, distorted, bytes)) != RCG_OK) return rc;
-  if ((rc = to_linear(ctx, d_a, w, h, channels, depth, lin)) != RCG_OK) return rc;
-  if ((rc = to_linear(ctx, d_b, w, h, channels, depth, lin + np)) != RCG_OK) return rc;
+  if ((rc = to_linear(ctx, d_a, w, h, w, channels, depth, lin)) != RCG_OK) return rc;
+  if ((rc = to_linear(ctx, d_b, w, h, w, channels, depth, lin + np)) != RCG_OK) return rc;
   if ((rc = exact_score(ctx, lin, lin + np, w, h, d_score)) != RCG_OK) return rc;
   double s = 0.0;
   cudaMemcpyAsync(&s, d_score, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
@@ -1176,25 +1173,29 @@ int rcg_reconstruct_tables(rcg_ctx* ctx, uint32_t width, uint32_t height, const 
 
 // ---- search
 
-// Per-candidate scorer of the device searches: SSIMULACRA2 from the candidate's linear pyramid against the
-// reference's, or SSIM from the candidate's 8-bit pixels against the reference's.
+// Per-candidate scorer of the device searches: SSIMULACRA2 from the candidate's XYB differences against the reference's
+// linear pyramid and the reference's XYB, or SSIM from the candidate's 8-bit pixels against the reference's.
 struct SearchScorer {
   int metric;
   PyramidDesc pd;
-  float* ref_pyr = nullptr;
+  float* ref_pyr = nullptr;   // linear
+  float* ref_xyb = nullptr;
   float* dist_pyr = nullptr;
   float2* ref_moments = nullptr;  // the reference's blurred a', a'^2 per pyramid pixel (null: the cache is off)
   const uint8_t* ref_px = nullptr;
   uint8_t* cand_px = nullptr;
   double* d_score = nullptr;
-  bool fuse420 = false;  // every candidate has the 4:2:0 layout of upsample_pyramid (set by the search's setup)
+  bool direct = true;  // every candidate's layout is one build_decoded reads directly (an encoder's always are)
 };
 
-// Whether a host-side layout is the 4:2:0 case of upsample_pyramid.
-static bool layout_fast420(const StepDesc* st, int w) {
+// Whether a layout is one that build_decoded reads directly: luma at full resolution, chroma halved across, both ways or
+// not at all.
+static bool layout_direct(const StepDesc* st) {
   const CompDesc& c0 = st->comp[0];
-  return st->ncomp == 3 && st->hmax == 2 && st->vmax == 2 && c0.h == 2 && c0.v == 2 && st->comp[1].h == 1 &&
-         st->comp[1].v == 1 && st->comp[2].h == 1 && st->comp[2].v == 1 && w % 4 == 0;
+  if (c0.h != st->hmax || c0.v != st->vmax) return false;
+  if (st->ncomp == 1) return true;
+  return st->ncomp == 3 && st->hmax <= 2 && st->vmax <= st->hmax && st->comp[1].h == 1 && st->comp[1].v == 1 &&
+         st->comp[2].h == 1 && st->comp[2].v == 1;
 }
 
 // Every buffer the per-candidate scoring uses is allocated here, before the step loop: the loop itself never
@@ -1212,8 +1213,9 @@ static int scorer_setup(rcg_ctx* ctx, int metric, int w, int h, int channels, Se
   }
   sc->pd = make_pyramid(w, h);
   sc->ref_pyr = (float*)workspace(ctx, "ref_pyr", (size_t)sc->pd.floats * sizeof(float));
+  sc->ref_xyb = (float*)workspace(ctx, "ref_xyb", (size_t)sc->pd.floats * sizeof(float));
   sc->dist_pyr = (float*)workspace(ctx, "dist_pyr", (size_t)sc->pd.floats * sizeof(float));
-  if (!sc->ref_pyr || !sc->dist_pyr) return RCG_NO_MEMORY;
+  if (!sc->ref_pyr || !sc->ref_xyb || !sc->dist_pyr) return RCG_NO_MEMORY;
   if (ctx->ref_cache) {
     // Sized for the band layout the scorer will run (the same plan_bands call score_pyramids makes).
     sc->ref_moments = (float2*)workspace(ctx, "ref_moments", ref_moment_bytes(plan_bands(ctx, sc->pd)));
@@ -1231,29 +1233,43 @@ static void score_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st
     ssim_score(ctx, sc.ref_px, sc.cand_px, w, h, channels, sc.d_score, d_ss, d_st);
     return;
   }
-  if (sc.fuse420) {
-    upsample_pyramid(ctx, d_st, planes, w, h, sc.pd, sc.dist_pyr);
-  } else {
-    upsample_color(ctx, d_st, planes, w, h, nullptr, sc.dist_pyr);
-    build_pyramid_gated(ctx, sc.pd, sc.dist_pyr, d_st);
-  }
-  score_pyramids(ctx, sc.pd, sc.ref_pyr, sc.dist_pyr, sc.d_score, d_ss, d_st, sc.ref_moments,
+  build_decoded(ctx, sc.pd, d_st, planes, sc.direct, sc.dist_pyr, nullptr, sc.ref_pyr);
+  score_pyramids(ctx, sc.pd, sc.ref_xyb, sc.dist_pyr, sc.d_score, d_ss, d_st, sc.ref_moments,
                  s == 0 ? kRefWrite : kRefRead);
+}
+
+// The reference-order FP64 score of a paused search's candidate to d_exact. Its planes are still the paused candidate's
+// (every later step was inactive), so its linear samples are made again from them, and the reference's are copied out
+// of its pyramid: both in rows without padding, as exact_score reads them.
+static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st, const uint8_t* planes, int w, int h,
+                           double* d_exact) {
+  const size_t np = (size_t)w * h;
+  float* lin = (float*)workspace(ctx, "x_lin", 6 * np * sizeof(float), false);
+  if (!lin) return RCG_NO_MEMORY;
+  const ScaleDesc& s0 = sc.pd.s[0];
+  cudaError_t e = cudaMemcpy2DAsync(lin, (size_t)w * sizeof(float), sc.ref_pyr + s0.off, (size_t)s0.pitch * sizeof(float),
+                                    (size_t)w * sizeof(float), (size_t)3 * h, cudaMemcpyDeviceToDevice, ctx->stream);
+  static const int kActive = 1;  // the later steps' tables cleared it; the next step's set it again
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&d_st->active, &kActive, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "near-tie rescore");
+  upsample_color(ctx, d_st, planes, w, h, nullptr, lin + 3 * np, w);
+  return exact_score(ctx, lin, lin + 3 * np, w, h, d_exact);
 }
 
 // Near ties. jpeg/src/target.rs:48 accepts a candidate on s >= target; the fast scorer is within about 1e-6 of the
 // reference, so a candidate scored within ctx->tie_band of the target paused the device bisection (search_record,
-// done = 2) with its decoded linear planes still at scale 0 of the candidate pyramid (every later step was
-// inactive). Here it is rescored in the reference's f64 arithmetic and order on the GPU (exact_score), the bisection
+// done = 2) with its decoded planes still in place (every later step was
+// inactive). Here it is rescored in the reference's f64 arithmetic and order on the GPU (exact_candidate), the bisection
 // records that score and goes on, and the remaining steps run as plain launches; repeated while a later candidate
 // pauses again. `issue_step(s)` issues step s's kernels.
-static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, SearchState* hs, int max_steps,
-                       int w, int h, const std::function<void(int)>& issue_step) {
+static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, SearchState* hs, StepDesc* d_st,
+                       const uint8_t* planes, int max_steps, int w, int h, const std::function<void(int)>& issue_step) {
   while (hs->done == 2) {
     if (sc.metric != RCG_METRIC_SSIMULACRA2) return fail(ctx, RCG_INVALID, "paused search without a rescorer");
     double* d_exact = (double*)workspace(ctx, "x_score", sizeof(double), false);
     if (!d_exact) return RCG_NO_MEMORY;
-    int rc = exact_score(ctx, sc.ref_pyr, sc.dist_pyr, w, h, d_exact);
+    int rc = exact_candidate(ctx, sc, d_st, planes, w, h, d_exact);
     if (rc != RCG_OK) return rc;
     search_resume(ctx, d_ss, d_exact);
     ctx->tie_rescores++;
@@ -1294,12 +1310,8 @@ static int search_prepare(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int 
   if (metric == RCG_METRIC_SSIM) {
     sc.ref_px = d_src;
   } else {
-    if ((rc = to_linear(ctx, d_src, w, h, channels, 8, sc.ref_pyr)) != RCG_OK) return rc;
-    build_pyramid(ctx, sc.pd, sc.ref_pyr);
+    if ((rc = build_reference(ctx, sc.pd, d_src, channels, sc.ref_pyr, sc.ref_xyb)) != RCG_OK) return rc;
   }
-  // Every candidate of an explicit 4:2:0 colour search has the fused layout (the sampling factors of
-  // jpeg/src/encode.rs:428-439 do not depend on the quality then).
-  sc.fuse420 = metric == RCG_METRIC_SSIMULACRA2 && channels != 1 && subsampling == RCG_SUB_420 && w % 4 == 0;
   if ((rc = setup_encoder(ctx, d_src, w, h, channels, subsampling, &run->es)) != RCG_OK) return rc;
   int max_steps = 1;
   for (int span = max_q; span > 1; span = (span + 1) / 2) max_steps++;
@@ -1391,7 +1403,7 @@ static int search_impl(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int cha
   SearchState hs;
   cudaMemcpyAsync(&hs, d_ss, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
   if ((rc = finish(ctx, "search")) != RCG_OK) return rc;
-  if ((rc = settle_ties(ctx, sc, d_ss, &hs, nsteps, w, h, issue_step)) != RCG_OK) return rc;
+  if ((rc = settle_ties(ctx, sc, d_ss, &hs, d_st, run.planes, nsteps, w, h, issue_step)) != RCG_OK) return rc;
   if (nsteps < run.max_steps && !hs.done) {
     // A probe: the evaluated candidates only (not the next one the bisection has chosen), and as its result the
     // candidate whose score is closest to the target, from either side.
@@ -1586,7 +1598,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
   }
   // The work-lists: per image its StepDesc, search state, buffers and first CTA in each stage's grid.
   std::vector<LockItem> items((size_t)n);
-  long long q_total = 0, u_total = 0, p_total = 0, t_total = 0;
+  long long q_total = 0, p_total = 0, t_total = 0;
   int max_scales = 1, max_steps = 1;
   for (int i = 0; i < n; i++) {
     const SearchRun& r = runs[(size_t)i];
@@ -1602,6 +1614,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     it.w = r.w;
     it.h = r.h;
     it.ref_pyr = r.sc.ref_pyr;
+    it.ref_xyb = r.sc.ref_xyb;
     it.refm = r.sc.ref_moments;
     it.dist_pyr = r.sc.dist_pyr;
     it.partials = (double*)sub->bufs["score_partials"].ptr;
@@ -1611,10 +1624,6 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     it.pd = plan_bands(ctx, r.sc.pd);
     it.q0 = q_total;
     q_total += (r.es.max_blocks + 127) / 128;
-    it.ux = ((r.w + 3) / 4 + 127) / 128;
-    it.uy = std::min(((r.h + 1) / 2 + 3) / 4, 65535);  // four chroma rows per CTA, as upsample_color
-    it.u0 = u_total;
-    u_total += (long long)it.ux * it.uy;
     it.p0 = p_total;
     p_total += pyramid_ctas(it.pd);
     it.t0 = t_total;
@@ -1622,19 +1631,19 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     max_scales = std::max(max_scales, it.pd.nscales);
     max_steps = std::max(max_steps, r.max_steps);
   }
-  if (q_total > INT32_MAX || u_total > INT32_MAX || p_total > INT32_MAX || t_total > INT32_MAX)
+  if (q_total > INT32_MAX || p_total > INT32_MAX || t_total > INT32_MAX)
     return fail(ctx, RCG_INVALID, "batch too large for one launch");
   LockItem* d_items = (LockItem*)workspace(ctx, "lock_items", sizeof(LockItem) * (size_t)n);
   double* d_exact = (double*)workspace(ctx, "x_score", sizeof(double), false);
   if (!d_items || !d_exact) return RCG_NO_MEMORY;
   cudaMemcpyAsync(d_items, items.data(), sizeof(LockItem) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
   auto issue_step = [&](int s) {
-    lock_step_codec(ctx, d_items, n, q_total, u_total);
+    lock_step_codec(ctx, d_items, n, q_total);
     lock_step_score(ctx, d_items, n, p_total, t_total, max_scales,
                     ctx->ref_cache ? (s == 0 ? kRefWrite : kRefRead) : kRefNone);
   };
   // The grids follow from the totals; the images' buffers come in through the work-list uploaded above.
-  const std::vector<long long> key = {5, n, max_steps, q_total, u_total, p_total, t_total, max_scales};
+  const std::vector<long long> key = {5, n, max_steps, q_total, p_total, t_total, max_scales};
   rc = run_step_loop(ctx, key, [&]() {
     for (int s = 0; s < max_steps; s++) issue_step(s);
   });
@@ -1653,7 +1662,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     for (int i = 0; i < n; i++) {
       if (hs[(size_t)i].done != 2) continue;
       const SearchRun& r = runs[(size_t)i];
-      if ((rc = exact_score(ctx, r.sc.ref_pyr, r.sc.dist_pyr, r.w, r.h, d_exact)) != RCG_OK) return rc;
+      if ((rc = exact_candidate(ctx, r.sc, r.d_st, r.planes, r.w, r.h, d_exact)) != RCG_OK) return rc;
       search_resume(ctx, r.d_ss, d_exact);
       ctx->tie_rescores++;
       from = std::min(from, hs[(size_t)i].step + 1);
@@ -1779,15 +1788,11 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
   dequant_idct(ctx, d_st, d_src, planes, nblocks);
   // A requantized candidate keeps the source's block layout.
-  sc.fuse420 = metric == RCG_METRIC_SSIMULACRA2 && layout_fast420(st, w);
-  if (metric == RCG_METRIC_SSIM) {
+  sc.direct = layout_direct(st);
+  if (metric == RCG_METRIC_SSIM)
     upsample_color(ctx, d_st, planes, w, h, ref_px, nullptr);
-  } else if (sc.fuse420) {
-    upsample_pyramid(ctx, d_st, planes, w, h, sc.pd, sc.ref_pyr);
-  } else {
-    upsample_color(ctx, d_st, planes, w, h, nullptr, sc.ref_pyr);
-    build_pyramid(ctx, sc.pd, sc.ref_pyr);
-  }
+  else
+    build_decoded(ctx, sc.pd, d_st, planes, sc.direct, sc.ref_pyr, sc.ref_xyb, nullptr);
   SearchState hs;
   std::memset(&hs, 0, sizeof hs);
   hs.lo = 1;
@@ -1824,7 +1829,7 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   }
   cudaMemcpyAsync(&hs, d_ss, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
   if ((rc = finish(ctx, "search_requantize")) != RCG_OK ||
-      (rc = settle_ties(ctx, sc, d_ss, &hs, max_steps, w, h, issue_step)) != RCG_OK) {
+      (rc = settle_ties(ctx, sc, d_ss, &hs, d_st, planes, max_steps, w, h, issue_step)) != RCG_OK) {
     delete st;
     return rc;
   }

@@ -20,7 +20,6 @@
 
 #include "rcg_internal.cuh"
 #include "huffman.cuh"
-#include "upsample420.cuh"
 
 namespace rcg {
 
@@ -860,27 +859,6 @@ __device__ __forceinline__ int up_sample(const uint8_t* p, int stride, int cw, i
   return px(x / fx, y / fy);
 }
 
-// The search's common case (upsample420.cuh): one thread = 4 columns x 2 rows (output rows 2j, 2j+1 of chroma row
-// j), stored as one 16-byte write per row and plane. Same arithmetic as the general path below
-// (jpeg/src/decode.rs:1806-1818, :1438-1441).
-__device__ __forceinline__ void upsample_420(const StepDesc* __restrict__ st, const uint8_t* __restrict__ planes,
-                                             int w, int h, float* __restrict__ lin, const float* lut, int x0,
-                                             int j) {
-  float l[2][3][4];
-  upsample_420_rows(st, planes, w, h, lut, x0, j, l);
-  const size_t np = (size_t)w * h;
-#pragma unroll
-  for (int par = 0; par < 2; par++) {
-    const int y = 2 * j + par;
-    if (y >= h) break;
-    const size_t o = (size_t)y * w + x0;
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      *reinterpret_cast<float4*>(lin + c * np + o) = make_float4(l[par][c][0], l[par][c][1], l[par][c][2],
-                                                                 l[par][c][3]);
-  }
-}
-
 // Decoder::finish for an 8-bit YCbCr or Gray CoefImage (jpeg/src/decode.rs:1404-1444): upsample every component to
 // full resolution, then the fixed-point YCbCr->RGB of :1438-1441. Writes interleaved pixels and/or the linear-light
 // planes the scorer starts from (core/src/ssimulacra2.rs:192-203: Gray is replicated to three channels).
@@ -889,13 +867,10 @@ __device__ __forceinline__ void upsample_420(const StepDesc* __restrict__ st, co
 __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__ st,
                                                     const uint8_t* __restrict__ planes, int w, int h,
                                                     uint8_t* __restrict__ rgb, float* __restrict__ lin,
-                                                    const unsigned bx, const unsigned by, const unsigned gy) {
+                                                    const int pitch, const unsigned bx, const unsigned by, const unsigned gy) {
   if (!st->active) return;
   const int ncomp = st->ncomp, hmax = st->hmax, vmax = st->vmax;
   const CompDesc c0 = st->comp[0];
-  // 4:2:0 linear planes for the scorer: the two-row path, over chroma rows (half the grid's rows)
-  const bool fast420 = !rgb && lin && layout_is_fast420(st, w);
-  if (fast420 && (int)by >= (h + 1) / 2) return;
   // The sRGB table lives in shared memory: per-thread indices differ, which would serialize constant-memory reads.
   __shared__ float lut[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = c_lut8[i];
@@ -903,12 +878,8 @@ __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__
   // Four consecutive pixels of one row per thread, so each thread moves enough bytes per request.
   const int x0 = 4 * (bx * blockDim.x + threadIdx.x);
   if (x0 >= w) return;
-  if (fast420) {
-    for (int j = by; j < (h + 1) / 2; j += gy) upsample_420(st, planes, w, h, lin, lut, x0, j);
-    return;
-  }
-  const size_t np = (size_t)w * h;
-  const bool vec_out = (w % 4 == 0) && (np % 4 == 0) && (x0 + 4 <= w);
+  const size_t np = (size_t)pitch * h;  // a plane of lin
+  const bool vec_out = pitch % 4 == 0;    // whole quads: the last one may run into the row's padding
   for (int y = by; y < h; y += gy) {
     int yv[4], cbv[4], crv[4];
     // Luma: full resolution when it carries the maximum sampling factors (always, for this encoder's layouts).
@@ -982,7 +953,7 @@ __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__
       }
     }
     if (lin) {
-      size_t i = (size_t)y * w + x0;
+      size_t i = (size_t)y * pitch + x0;
       if (vec_out) {
 #pragma unroll
         for (int c = 0; c < 3; c++)
@@ -998,17 +969,16 @@ __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__
 
 __global__ void __launch_bounds__(128, 10) k_upsample_color(const StepDesc* __restrict__ st,
                                                              const uint8_t* __restrict__ planes, int w, int h,
-                                                             uint8_t* __restrict__ rgb, float* __restrict__ lin) {
-  upsample_color_body(st, planes, w, h, rgb, lin, blockIdx.x, blockIdx.y, gridDim.y);
+                                                             uint8_t* __restrict__ rgb, float* __restrict__ lin,
+                                                             int pitch) {
+  upsample_color_body(st, planes, w, h, rgb, lin, pitch, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, uint8_t* d_rgb,
-                   float* d_lin) {
-  // (h + 1) / 8 rows of CTAs: the 4:2:0 path writes two rows per chroma row and each CTA takes four chroma rows (its
-  // shared-memory table filled once for 8 output rows: 46.5 -> 40.7 us per 12 MP candidate against one chroma row
-  // per CTA); the general path strides over the rows by the grid height, so every layout is covered.
+                   float* d_lin, int pitch) {
+  // A CTA takes every (h + 1) / 8-th row, eight in all, so that it fills its shared-memory table once for them.
   dim3 grid(((w + 3) / 4 + 127) / 128, std::min(((h + 1) / 2 + 3) / 4, 65535));
-  RCG_LAUNCH(ctx, "upsample_color", k_upsample_color, grid, 128, 0, d_step, d_planes, w, h, d_rgb, d_lin);
+  RCG_LAUNCH(ctx, "upsample_color", k_upsample_color, grid, 128, 0, d_step, d_planes, w, h, d_rgb, d_lin, pitch);
   return RCG_OK;
 }
 
@@ -1110,21 +1080,12 @@ __global__ void __launch_bounds__(128) k_dequant_idct_lock(const LockItem* __res
   dequant_idct_body(it.st, nullptr, it.planes, (long long)blockIdx.x - it.q0);
 }
 
-__global__ void __launch_bounds__(128, 10) k_upsample_color_lock(const LockItem* __restrict__ items, int n) {
-  const int i = lock_find<&LockItem::u0>(items, n, blockIdx.x);
-  const LockItem& it = items[i];
-  const long long local = (long long)blockIdx.x - it.u0;
-  const unsigned bx = (unsigned)(local % it.ux), by = (unsigned)(local / it.ux);
-  upsample_color_body(it.st, it.planes, it.w, it.h, nullptr, it.dist_pyr, bx, by, (unsigned)it.uy);
-}
-
-void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total, long long u_total) {
+void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total) {
   RCG_LAUNCH(ctx, "step_tables_lock", k_step_tables_lock, n, 192, 0, d_items);
   RCG_LAUNCH(ctx, "quantize_lock", k_quantize_lock, (unsigned)q_total, 128, 0, d_items, n);
   RCG_LAUNCH(ctx, "rate_tables_lock", k_rate_tables_lock, dim3(3, n), 288, 0, d_items);
   RCG_LAUNCH(ctx, "trellis_lock", k_trellis_lock, (unsigned)q_total, 128, 0, d_items, n);
   RCG_LAUNCH(ctx, "dequant_idct_lock", k_dequant_idct_lock, (unsigned)q_total, 128, 0, d_items, n);
-  RCG_LAUNCH(ctx, "upsample_color_lock", k_upsample_color_lock, (unsigned)u_total, 128, 0, d_items, n);
 }
 
 int codec_upload_lut(const float* lut8) {

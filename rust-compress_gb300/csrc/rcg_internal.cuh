@@ -24,13 +24,17 @@ constexpr int kScoreSums = 18;    // 3 channels x 6 sums (core/src/ssimulacra2.r
 constexpr int kRadius = 5;
 constexpr int kTileW = 32;
 constexpr int kTileH = 32;
-constexpr int kTileThreads = 256;
+constexpr int kTileThreads = 128;
+constexpr int kTileCtas = 4, kTileCtasRead = 6;  // per SM: the scorer's form with five blurred moments, with three
 
 // ------------------------------------------------------------------------------------------------ descriptors
 
-// One scale of the scorer's pyramid: planes are channel-planar f32, [3][h][w], at `off` (floats) in a pyramid buffer.
+// One scale of the scorer's pyramid: planes are channel-planar f32, [3][h][pitch], at `off` (floats) in a pyramid
+// buffer. Rows are padded to whole 16-byte quads (pitch = w rounded up to 4), so every row of every width takes vector
+// loads and stores; the padding's values are never used.
 struct ScaleDesc {
   int w, h;
+  int pitch;
   int tiles_x, tiles_y;  // CTAs across and down (32-column bands of nch chunks of 32 rows; nch = 1: 32x32 tiles)
   int tile0;        // first CTA of this scale in the multi-scale launch
   int nch;          // 32-row chunks per CTA (ssim2.cu, ssim2_band)
@@ -161,7 +165,8 @@ struct LockItem {
   uint8_t* planes;         // decoded component planes
   int w, h;
   float* ref_pyr;          // the reference's linear pyramid
-  float* dist_pyr;         // the candidate's (scale 0 written by the upsampling)
+  float* ref_xyb;          // its XYB
+  float* dist_pyr;         // the candidate's XYB differences
   double* partials;        // scorer scratch: per-CTA sums, per-scale sums, completion counter, score
   double* scale_sums;
   unsigned* counter;
@@ -169,8 +174,6 @@ struct LockItem {
   PyramidDesc pd;          // the scorer's CTA layout (bands)
   float2* refm;            // the reference moments (null: the store is off)
   long long q0;            // first CTA in the block grids (quantize, trellis, dequantize: 128 blocks a CTA)
-  long long u0;            // first CTA in the upsampling grid (ux x uy CTAs)
-  int ux, uy;
   long long p0;            // first CTA in the pyramid grid
   long long t0;            // first CTA in the scorer's grid (pd.total_tiles)
 };
@@ -304,28 +307,31 @@ PyramidDesc make_pyramid(int w, int h);
 // ---- scorer (ssim2.cu)
 // Upload the 8-bit LUT to constant memory once per device.
 int scorer_init(rcg_ctx* ctx);
-// Interleaved 8-bit Gray/Rgb (or GrayAlpha/Rgba, or 16-bit) image -> linear planes at scale 0 of `pyr`.
-int to_linear(rcg_ctx* ctx, const uint8_t* d_img, int w, int h, int channels, int depth, float* d_pyr);
-// Fill scales 1.. of a pyramid from scale 0 (core/src/ssimulacra2.rs:225-247).
-int build_pyramid(rcg_ctx* ctx, const PyramidDesc& pd, float* d_pyr);
-// The same, skipped on the device when the search step is inactive.
-int build_pyramid_gated(rcg_ctx* ctx, const PyramidDesc& pd, float* d_pyr, const StepDesc* st);
-// CTAs of one pyramid launch (k_pyramid and the work-list forms): one per scale-1 tile, 0 for a single scale.
+// Interleaved 8-bit Gray/Rgb (or GrayAlpha/Rgba, or 16-bit) image -> linear planes [3][h][pitch].
+int to_linear(rcg_ctx* ctx, const uint8_t* d_img, int w, int h, int pitch, int channels, int depth, float* d_lin);
+// CTAs of one pyramid builder launch: one per 64x64 block of scale 0.
 int pyramid_ctas(const PyramidDesc& pd);
-// upsample_color's linear planes and build_pyramid_gated in one launch, for a step whose layout is the 4:2:0 case of
-// upsample420.cuh (the caller's promise: 3 components, luma 2x2 and chroma 1x1 sampling, w % 4 == 0).
-int upsample_pyramid(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, const PyramidDesc& pd,
-                     float* d_pyr);
+// Pyramids for the scorer in one launch each. A pair of images: the XYB of the first, the XYB differences of the two.
+int build_pair(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_ref, const uint8_t* d_dist, int channels, int depth,
+               float* d_xyb, float* d_diff);
+// A search's 8-bit reference image: its linear pyramid (which candidates are compared with) and its XYB.
+int build_reference(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_img, int channels, float* d_lin, float* d_xyb);
+// Decoded planes of a step (skipped on the device when it is inactive). d_ref null: a reference (d_out linear, d_xyb its
+// XYB); else a candidate: d_out its differences against the linear pyramid d_ref. `direct`: the layout is Gray, 4:4:4,
+// 4:2:2 or 4:2:0 with full-resolution luma (layout_direct); others go through upsample_color first.
+int build_decoded(rcg_ctx* ctx, const PyramidDesc& pd, StepDesc* d_step, const uint8_t* d_planes, bool direct,
+                  float* d_out, float* d_xyb, const float* d_ref);
 // Reference moments of the tile kernel: kRefNone computes every blurred moment; kRefWrite also stores the
 // reference-only ones (blur a', blur a'^2) for later candidates against the same reference; kRefRead reads them
 // instead of blurring them. Same scores in every mode. The store is chunk-major: per 32x32 chunk of the banded
 // layout the scorer runs (plan_bands), kRefChunk float2 as [channel][row][column], ref_moment_bytes() in all.
 constexpr int kRefChunk = 3 * kTileH * kTileW;
 constexpr int kRefNone = 0, kRefWrite = 1, kRefRead = 2;
-// Score: per-tile sums of every scale, then the final mapping. `d_score` receives the score (f64); when
+// Score of a reference's XYB pyramid and a candidate's XYB differences: per-tile sums of every scale, then the final
+// mapping. `d_score` receives the score (f64); when
 // `search` is non-null the final kernel also advances the device-side bisection. `refm`/`ref_mode`: the reference
 // moments (nullptr / kRefNone: none).
-int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, const float* d_dist, double* d_score,
+int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_xyb, const float* d_diff, double* d_score,
                    SearchState* search, StepDesc* step, float2* refm = nullptr, int ref_mode = kRefNone);
 // The reference-order FP64 score (exact.cu) of two images given as scale-0 linear planes ([3][h][w] f32, as
 // to_linear writes them): to d_score (NaN for the reference's non-finite Err), queued on the context stream.
@@ -353,7 +359,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
                 double** d_scores);
 
 // ---- lockstep batch (work-list launches over the LockItems of a batch; totals are the grids' CTA counts)
-void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total, long long u_total);
+void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total);
 void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_total, long long t_total,
                      int max_scales, int ref_mode = kRefNone);
 
@@ -375,9 +381,9 @@ int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long l
 // d_coefs null: decode the candidate's own coefficients (d_step->coefs).
 int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks);
 // Upsample + YCbCr->RGB (jpeg/src/decode.rs:1404-1444). Writes interleaved 8-bit pixels to d_rgb (nullable)
-// and/or linear planes to d_lin (nullable).
+// and/or linear planes [3][h][pitch] to d_lin (nullable).
 int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, uint8_t* d_rgb,
-                   float* d_lin);
+                   float* d_lin, int pitch = 0);
 // Host-side table setup of one quality into a host StepDesc (no device work).
 void host_step_tables(StepDesc* st, int quality, int subsampling, int channels, int trellis, int w, int h);
 // core/src/metrics.rs on device images: ssim (score to d_score; with ss, one bisection step; gated by st), the

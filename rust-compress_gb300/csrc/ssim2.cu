@@ -35,7 +35,7 @@
 #include <vector>
 
 #include "rcg_internal.cuh"
-#include "upsample420.cuh"
+#include "planes_quad.cuh"
 
 namespace rcg {
 
@@ -69,65 +69,88 @@ __device__ __forceinline__ float fdiv_ftz(float a, float b) {
   return r;
 }
 
-// x^2 + x*y + y^2: cbrt(u) - cbrt(v) = (u - v) / D(cbrt(u), cbrt(v)).
-__device__ __forceinline__ float dsq(float x, float y) { return fmaf(x, x, fmaf(x, y, y * y)); }
+// x^2 + x*y + y^2 = D(x, y): cbrt(u) - cbrt(v) = (u - v) / D(cbrt(u), cbrt(v)).
+// Per pixel the scorer needs the reference image's XYB without its constants (`a`, core/src/ssimulacra2.rs:249-258 less
+// kXyb0*) and XYB(reference) - XYB(distorted) (`d`). Every quantity that is a small difference of nearly equal cube
+// roots is formed from the identity above, so it keeps its relative precision in f32: X - 0.42 = 7 (c0 - c1), B - 0.55 =
+// ((c2 - c0) + (c2 - c1)) / 2, each c_i - c_j from the difference of two opsin-matrix rows applied to (r, g, b); and
+// the per-pixel differences between the two images from the linear differences (r_a - r_b, ...).
+// The constants of X, Y and B that `a` leaves out.
+constexpr float kXyb0X = 0.42f, kXyb0Y = 0.01f, kXyb0B = 0.55f;
 
-// q_a/D_a - q_b/D_b without cancellation: (dq*D_b - q_b*dD) / (D_a*D_b), dq = q_a - q_b and dD = D_a - D_b given.
-__device__ __forceinline__ float qdiff(float qb, float dq, float Da, float Db, float dD) {
-  return fdiv_ftz(fmaf(dq, Db, -qb * dD), Da * Db);
+// Two pixels at a time, every step one packed two-lane operation: the conversion is bound by instruction issue, and this
+// halves it but for the special functions. A difference a - b is fma(b, -1, a), which rounds once, as it does. The opsin
+// sums are at least the bias: linear samples and the rows are not negative.
+__device__ __forceinline__ float2 two(float k) { return make_float2(k, k); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, two(-1.0f), a); }
+__device__ __forceinline__ float2 cbrt2(float2 x) {
+  float2 l, y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l.x) : "f"(x.x));
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l.y) : "f"(x.y));
+  l = __fmul2_rn(l, two(1.0f / 3.0f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(l.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(l.y));
+  return y;
+}
+__device__ __forceinline__ float2 div2(float2 a, float2 b) { return make_float2(fdiv_ftz(a.x, b.x), fdiv_ftz(a.y, b.y)); }
+__device__ __forceinline__ float2 dsq2(float2 x, float2 y) {
+  return __ffma2_rn(x, x, __ffma2_rn(x, y, __fmul2_rn(y, y)));
+}
+// m0 r + m1 g + m2 b + c, and without c.
+__device__ __forceinline__ float2 row2(float m0, float m1, float m2, float2 r, float2 g, float2 b, float c) {
+  return __ffma2_rn(two(m0), r, __ffma2_rn(two(m1), g, __ffma2_rn(two(m2), b, two(c))));
+}
+__device__ __forceinline__ float2 row2(float m0, float m1, float m2, float2 r, float2 g, float2 b) {
+  return __ffma2_rn(two(m0), r, __ffma2_rn(two(m1), g, __fmul2_rn(two(m2), b)));
 }
 
-// One pixel of the tile: the reference image's XYB minus the tile offsets (`a`, core/src/ssimulacra2.rs:249-258)
-// and XYB(reference) - XYB(distorted) minus the tile's difference offsets (`d`). Every quantity that is a small
-// difference of nearly equal cube roots is formed from the identity above, so it keeps its relative precision in
-// f32: X - 0.42 = 7 (c0 - c1), B - 0.55 = ((c2 - c0) + (c2 - c1)) / 2, each c_i - c_j from the difference of two
-// opsin-matrix rows applied to (r, g, b); and the per-pixel differences between the two images from the linear
-// differences (r_a - r_b, ...).
-struct Pix {
-  float a[3], d[3];
-};
+// The three opsin rows and the exact differences of rows, rounded once.
+constexpr float M00 = (float)kM00, M01 = (float)kM01, M02 = (float)kM02;
+constexpr float M10 = (float)kM10, M11 = (float)kM11, M12 = (float)kM12;
+constexpr float M20 = (float)kM20, M21 = (float)kM21, M22 = (float)kM22;
+constexpr float L20r = (float)(kM20 - kM00), L20g = (float)(kM21 - kM01), L20b = (float)(kM22 - kM02);
+constexpr float L21r = (float)(kM20 - kM10), L21g = (float)(kM21 - kM11), L21b = (float)(kM22 - kM12);
 
-__device__ __forceinline__ Pix pix(float ra, float ga, float ba, float rb, float gb, float bb, const float* oa,
-                                   const float* od, float cbrt_bias) {
+// `a` of two pixels.
+__device__ __forceinline__ void pix_xyb2(float2 r, float2 g, float2 b, float2 (&a)[3]) {
   const float bias = (float)kBias;
-  // opsin rows (f32) and the exact differences of rows, rounded once
-  const float M00 = (float)kM00, M01 = (float)kM01, M02 = (float)kM02;
-  const float M10 = (float)kM10, M11 = (float)kM11, M12 = (float)kM12;
-  const float M20 = (float)kM20, M21 = (float)kM21, M22 = (float)kM22;
-  const float L20r = (float)(kM20 - kM00), L20g = (float)(kM21 - kM01), L20b = (float)(kM22 - kM02);
-  const float L21r = (float)(kM20 - kM10), L21g = (float)(kM21 - kM11), L21b = (float)(kM22 - kM12);
-  float ca[3], cb[3];
-  ca[0] = cbrt_fast(fmaxf(fmaf(M00, ra, fmaf(M01, ga, fmaf(M02, ba, bias))), 0.0f));
-  ca[1] = cbrt_fast(fmaxf(fmaf(M10, ra, fmaf(M11, ga, fmaf(M12, ba, bias))), 0.0f));
-  ca[2] = cbrt_fast(fmaxf(fmaf(M20, ra, fmaf(M21, ga, fmaf(M22, ba, bias))), 0.0f));
-  cb[0] = cbrt_fast(fmaxf(fmaf(M00, rb, fmaf(M01, gb, fmaf(M02, bb, bias))), 0.0f));
-  cb[1] = cbrt_fast(fmaxf(fmaf(M10, rb, fmaf(M11, gb, fmaf(M12, bb, bias))), 0.0f));
-  cb[2] = cbrt_fast(fmaxf(fmaf(M20, rb, fmaf(M21, gb, fmaf(M22, bb, bias))), 0.0f));
-  float q01a = 0.07f * (ra - ga), q01b = 0.07f * (rb - gb);
-  float q20a = fmaf(L20r, ra, fmaf(L20g, ga, L20b * ba)), q20b = fmaf(L20r, rb, fmaf(L20g, gb, L20b * bb));
-  float q21a = fmaf(L21r, ra, fmaf(L21g, ga, L21b * ba)), q21b = fmaf(L21r, rb, fmaf(L21g, gb, L21b * bb));
-  float D01a = dsq(ca[0], ca[1]), D20a = dsq(ca[2], ca[0]), D21a = dsq(ca[2], ca[1]);
-  float D01b = dsq(cb[0], cb[1]), D20b = dsq(cb[2], cb[0]), D21b = dsq(cb[2], cb[1]);
-  Pix o;
-  float ya = 0.5f * (ca[0] + ca[1]);
-  o.a[0] = fmaf(7.0f, fdiv_ftz(q01a, D01a), 0.42f - oa[0]);
-  o.a[1] = (ya - cbrt_bias) + (0.01f - oa[1]);
-  o.a[2] = 0.5f * (fdiv_ftz(q20a, D20a) + fdiv_ftz(q21a, D21a)) + (0.55f - oa[2]);
-  float dr = ra - rb, dg = ga - gb, db = ba - bb;
-  float dc0 = fdiv_ftz(fmaf(M00, dr, fmaf(M01, dg, M02 * db)), dsq(ca[0], cb[0]));
-  float dc1 = fdiv_ftz(fmaf(M10, dr, fmaf(M11, dg, M12 * db)), dsq(ca[1], cb[1]));
-  float dc2 = fdiv_ftz(fmaf(M20, dr, fmaf(M21, dg, M22 * db)), dsq(ca[2], cb[2]));
-  // D(x, y) of image a minus of image b: dx (xa + xb) + dx ya + xb dy + dy (ya + yb)
-  float dD01 = fmaf(dc0, ca[0] + cb[0], fmaf(dc0, ca[1], fmaf(cb[0], dc1, dc1 * (ca[1] + cb[1]))));
-  float dD20 = fmaf(dc2, ca[2] + cb[2], fmaf(dc2, ca[0], fmaf(cb[2], dc0, dc0 * (ca[0] + cb[0]))));
-  float dD21 = fmaf(dc2, ca[2] + cb[2], fmaf(dc2, ca[1], fmaf(cb[2], dc1, dc1 * (ca[1] + cb[1]))));
-  float dq01 = 0.07f * (dr - dg);
-  float dq20 = fmaf(L20r, dr, fmaf(L20g, dg, L20b * db));
-  float dq21 = fmaf(L21r, dr, fmaf(L21g, dg, L21b * db));
-  o.d[0] = 7.0f * qdiff(q01b, dq01, D01a, D01b, dD01) - od[0];
-  o.d[1] = 0.5f * (dc0 + dc1) - od[1];
-  o.d[2] = 0.5f * (qdiff(q20b, dq20, D20a, D20b, dD20) + qdiff(q21b, dq21, D21a, D21b, dD21)) - od[2];
-  return o;
+  const float2 c0 = cbrt2(row2(M00, M01, M02, r, g, b, bias)), c1 = cbrt2(row2(M10, M11, M12, r, g, b, bias)),
+               c2 = cbrt2(row2(M20, M21, M22, r, g, b, bias));
+  a[0] = __fmul2_rn(two(7.0f), div2(__fmul2_rn(two(0.07f), sub2(r, g)), dsq2(c0, c1)));
+  a[1] = sub2(__fmul2_rn(two(0.5f), __fadd2_rn(c0, c1)), two(cbrt_fast(bias)));
+  a[2] = __fmul2_rn(two(0.5f), __fadd2_rn(div2(row2(L20r, L20g, L20b, r, g, b), dsq2(c2, c0)),
+                                          div2(row2(L21r, L21g, L21b, r, g, b), dsq2(c2, c1))));
+}
+
+// `d` of two pixels. The quotient difference q_a/D_a - q_b/D_b of a row pair is formed without cancellation as
+// (dq D_b - q_b dD) / (D_a D_b), dq = q_a - q_b and dD = D_a - D_b from the cube roots' differences.
+__device__ __forceinline__ void pix_diff2(float2 ra, float2 ga, float2 ba, float2 rb, float2 gb, float2 bb,
+                                          float2 (&d)[3]) {
+  const float bias = (float)kBias;
+  const float2 ca0 = cbrt2(row2(M00, M01, M02, ra, ga, ba, bias)), cb0 = cbrt2(row2(M00, M01, M02, rb, gb, bb, bias));
+  const float2 ca1 = cbrt2(row2(M10, M11, M12, ra, ga, ba, bias)), cb1 = cbrt2(row2(M10, M11, M12, rb, gb, bb, bias));
+  const float2 ca2 = cbrt2(row2(M20, M21, M22, ra, ga, ba, bias)), cb2 = cbrt2(row2(M20, M21, M22, rb, gb, bb, bias));
+  const float2 dr = sub2(ra, rb), dg = sub2(ga, gb), db = sub2(ba, bb);
+  const float2 dc0 = div2(row2(M00, M01, M02, dr, dg, db), dsq2(ca0, cb0));
+  const float2 dc1 = div2(row2(M10, M11, M12, dr, dg, db), dsq2(ca1, cb1));
+  const float2 dc2 = div2(row2(M20, M21, M22, dr, dg, db), dsq2(ca2, cb2));
+  d[1] = __fmul2_rn(two(0.5f), __fadd2_rn(dc0, dc1));
+  const float2 s0 = __fadd2_rn(ca0, cb0), s1 = __fadd2_rn(ca1, cb1), s2 = __fadd2_rn(ca2, cb2);
+  // nq = -q of image b; D(x, y) of image a minus of image b: dx (xa + xb) + dx ya + xb dy + dy (ya + yb)
+  auto qd = [&](float2 nq, float2 dq, float2 cax, float2 cbx, float2 dcx, float2 sx, float2 cay, float2 cby, float2 dcy,
+                float2 sy) {
+    const float2 Da = dsq2(cax, cay), Db = dsq2(cbx, cby);
+    const float2 dD = __ffma2_rn(dcx, sx, __ffma2_rn(dcx, cay, __ffma2_rn(cbx, dcy, __fmul2_rn(dcy, sy))));
+    return div2(__ffma2_rn(dq, Db, __fmul2_rn(nq, dD)), __fmul2_rn(Da, Db));
+  };
+  const float2 q01 = qd(__fmul2_rn(two(0.07f), sub2(gb, rb)), __fmul2_rn(two(0.07f), sub2(dr, dg)), ca0, cb0, dc0, s0, ca1,
+                        cb1, dc1, s1);
+  d[0] = __fmul2_rn(two(7.0f), q01);
+  const float2 q20 = qd(row2(-L20r, -L20g, -L20b, rb, gb, bb), row2(L20r, L20g, L20b, dr, dg, db), ca2, cb2, dc2, s2, ca0,
+                        cb0, dc0, s0);
+  const float2 q21 = qd(row2(-L21r, -L21g, -L21b, rb, gb, bb), row2(L21r, L21g, L21b, dr, dg, db), ca2, cb2, dc2, s2, ca1,
+                        cb1, dc1, s1);
+  d[2] = __fmul2_rn(two(0.5f), __fadd2_rn(q20, q21));
 }
 
 // Row index under the top/bottom mirror rule (core/src/ssimulacra2.rs:385-397); -1 for rows no valid output reads.
@@ -138,91 +161,84 @@ __device__ __forceinline__ int mirror_row(int yy, int h) {
   return yy;
 }
 
-// Row pitch 45 pairs (>= 42 columns): a horizontal-pass item reads 8-byte (a', d') pairs at a stride of 4 pairs,
-// and 2 * 45 = 26 mod 32 shifts each of the 4 rows a half-warp covers to its own bank class, so its 16 loads hit
-// 32 distinct banks.
-constexpr int kIW = 45;
+// Shared-memory layout of one channel of a chunk: its `a` and its `d` samples of the 42 halo rows, columns x0 - 8 ..
+// x0 + 39 (whole quads around the 42 that count). A row is 52 floats, 13 16-byte slots: odd, so the two rows that eight
+// lanes of the horizontal pass read (16 bytes each, 32 apart) fall in each other's gaps.
+constexpr int kIW = 52;
 constexpr int kIH = kTileH + 2 * kRadius;  // 42
-constexpr int kHx = 4;                     // horizontal-pass outputs per item
-constexpr size_t kTileSmem = (size_t)(6 * kIH * kIW + 5 * kIH * kTileW) * sizeof(float);
+constexpr int kLead = 8;                   // columns left of x0 in a row
+constexpr int kQuads = (kLead + kTileW + 8) / 4;  // 12 quads per row
+constexpr int kXs = kIH * kIW;                    // floats of one of the two
+// Blurred moments: the reading form keeps three per sample (one plane of pairs, one of singles), the others five.
+constexpr int pair_planes(int ref_mode) { return ref_mode == kRefRead ? 1 : 2; }
+constexpr size_t tile_smem(int ref_mode) {
+  return (size_t)(2 * kXs + (2 * pair_planes(ref_mode) + 1) * kIH * kTileW) * sizeof(float);
+}
+constexpr int tile_ctas(int ref_mode) { return ref_mode == kRefRead ? kTileCtasRead : kTileCtas; }  // per SM
+constexpr int kVy = kTileH / (kTileThreads / 32);  // vertical-pass outputs per thread
 
-// One CTA = one band of 32 output columns and nch chunks of 32 output rows of one scale, walked top to bottom.
-// Shared memory: per channel the (a', d') pairs of the chunk plus its 5-pixel halo (42 x 42); then per channel the
-// horizontally blurred five moments of the 42 halo rows. Between chunks the 10 halo rows that the next chunk shares
-// with this one (its top halo and first output rows) move to the top of the buffer instead of being converted to XYB
-// again, so a band pays the vertical halo's XYB once: 42 x (32 nch + 10) conversions for 32 x 32 nch outputs where
-// nch separate tiles pay 42 x 42 x nch. The blurs run the moment pairs that share a tap weight ((a', d'),
-// (a'^2, d'^2)) as packed two-lane f32 FMAs, each lane exactly fmaf, so the results are those of scalar FMAs in the
-// same order.
-// Offsets: every chunk takes the XYB and XYB difference at its own centre, as a 32 x 32 tile does; the carried rows
-// are re-offset by the change (one f32 subtraction each). With nch = 1 the band is exactly the single tile.
-// Band `local` of scale `sd` (sd.tiles_x bands across; sd.nch chunks each) of a pyramid pair; the band's 18 sums go to
-// out[i * stride], i < 18.
-// Reference moments (kRef). The offsets a chunk subtracts come from the reference alone (its XYB at the chunk
-// centre), so the blurred a' and a'^2 of every output pixel depend on the reference and the band layout only. A
-// search scores every candidate against one reference: its first candidate runs kRef = kRefWrite, which also stores
-// (blur a', blur a'^2) per output pixel and channel; the later ones run kRef = kRefRead, which blur only (b'^2, d'^2)
-// as a packed pair and d', and read the other two. Each blurred moment is the same chain of per-lane fmaf in every
-// mode, so the scores are bit-identical to kRefNone. The store keeps each chunk's 3 x 32 x 32 pairs contiguous
-// (24 KB, [channel][row][column]); a reading CTA asks for the whole block in L2 with one bulk prefetch per channel
-// as the chunk starts and reads it in its vertical pass. Measured per 12 MP score: 584.7 us without the store,
-// 612.7 us writing it, 547.0 us reading it (before the flush-to-zero forms and packed squares: 651.5 / 680.0 /
-// 608.9, and 603 us with the two moments left out altogether); with the store indexed like the pyramid planes and
-// no bulk prefetch the read mode took 645 us, and staging each channel's block in shared memory with cp.async 629.
+// Where the blurred planes' rows keep a column (a multiple of 4 and the three after it stay together): the permutation
+// that puts the 16-byte stores of eight lanes (four items of each of two rows) in distinct banks.
+__device__ __forceinline__ constexpr int hb_pair(int c, int r) { return c ^ (c >> 3 & 2) ^ (4 * (r & 1)); }
+__device__ __forceinline__ constexpr int hb_one(int c, int r) { return c ^ (4 * (r & 1)); }
 
+// 16 bytes from global to shared memory without passing through registers.
+__device__ __forceinline__ void copy_quad(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// One tap of a blur chain; the first is the product alone (what fma gives with a zero sum).
+__device__ __forceinline__ void tap_pair(float2& s, float2 k, float2 v, bool first) {
+  s = first ? __fmul2_rn(k, v) : __ffma2_rn(k, v, s);
+}
+__device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) {
+  s = first ? __fmul_rn(k, v) : fmaf(k, v, s);
+}
+
+// One CTA = one band of 32 output columns and nch chunks of 32 output rows of one scale, walked top to bottom, from the
+// reference's XYB planes (Pix::a) and the XYB differences (Pix::d). Per chunk and channel: the halo's samples are copied
+// to shared memory asynchronously, the horizontal pass takes off the chunk's offsets and blurs the 42 halo rows, the
+// vertical pass blurs the columns and evaluates the error maps while the next halo is on its way. The blurs run the
+// moment pairs that share a tap weight as packed two-lane f32 FMAs, each lane exactly fmaf.
+// Offsets: every chunk takes the XYB and XYB difference at its own centre.
+// Band `local` of scale `sd` (sd.tiles_x bands across; sd.nch chunks each); the band's 18 sums go to out[i * stride],
+// i < 18.
+// Reference moments (kRef). The offsets a chunk subtracts from `a` come from the reference alone, so the blurred a' and
+// a'^2 of every output pixel depend on the reference and the band layout only. A search scores every candidate against
+// one reference: its first candidate runs kRef = kRefWrite, which also stores (blur a', blur a'^2) per output pixel and
+// channel; the later ones run kRef = kRefRead, which blur only (b'^2, d'^2) as a packed pair and d', and read the other
+// two. Each blurred moment is the same chain of per-lane fmaf in every mode, so the scores are bit-identical to
+// kRefNone. The store keeps each chunk's 3 x 32 x 32 pairs contiguous (24 KB, [channel][row][column]); a reading CTA
+// asks for the whole block in L2 with one bulk prefetch per channel as the chunk starts and reads it in its vertical
+// pass.
+// What bounds it: instruction issue (79% active, the FP32 pipes 62%). Measured per 12 MP score, against a kernel that
+// read both linear pyramids and converted every halo sample to XYB itself (1.5 conversions per pixel and half of its
+// instructions): reading form 538 -> 276 us, storing 597 -> 354; plain 4K score 397 -> 238. Of that, the planes of XYB
+// alone gave 420; loads by quads with the next channel's in registers beside the passes, and the maps without their edge
+// cases inside the image, 349; eight outputs per thread in both passes with the halo copied asynchronously into one
+// buffer 276 (387 with two buffers of converted pairs, which left room for 16 warps per SM). CTAs per SM: 6 reading (5
+// measured 282, 4 287), 4 for the other forms (5 faster at 4K by 1%, slower in a batch by 4%). Quad offsets kept over a
+// chunk's channels measured 278, the maps of two rows as packed operations 273 but 242 plain: neither was kept.
 template <int kRef>
-__device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, const float* __restrict__ ref,
-                                           const float* __restrict__ dist, double* __restrict__ out,
+__device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, const float* __restrict__ xa,
+                                           const float* __restrict__ xd, double* __restrict__ out,
                                            const size_t stride, float2* __restrict__ refm) {
-  extern __shared__ float smem[];
-  float2* xs = reinterpret_cast<float2*>(smem);  // [3][kIH][kIW] pairs (a', d') per channel
-  float* hb = smem + 6 * kIH * kIW;              // pair planes (m0, m1), (m2, m3) then m4, [kIH][kTileW] each
+  extern __shared__ float4 smem4[];
+  float* const xs = reinterpret_cast<float*>(smem4);  // the channel's a, then its d
+  // Horizontally blurred moments, [kIH][kTileW]: one plane of pairs (reading form) or two, then one of singles.
+  float* const hb = xs + 2 * kXs;
+  constexpr int kOnes = 2 * pair_planes(kRef) * kIH * kTileW;  // where the plane of singles starts
   __shared__ float s_red[kTileThreads / 32][kScoreSums];
-  __shared__ float s_oa[3], s_od[3], s_noa[3], s_nod[3];
 
   const int tx = local % sd.tiles_x, ty = local / sd.tiles_x;
   const int nch = sd.nch;
   const int x0 = tx * kTileW, ybeg = ty * kTileH * nch;
-  const int w = sd.w, h = sd.h;
-  const size_t np = (size_t)w * h;
-  const float* ra = ref + sd.off;
-  const float* rb = dist + sd.off;
-  const float cb_bias = cbrt_fast((float)kBias);
-  const int tid = threadIdx.x;
-  constexpr int kCols = kTileW + 2 * kRadius;  // 42 real columns of the kIW-pitched rows
-  constexpr int kCarry = 2 * kRadius;          // rows a chunk hands to the next
-
-  // The six plane values of halo pixel e of the chunk at y0 (rows from r0 on), with the mirror rule for rows.
-  auto load6 = [&](int e, int y0, int r0, float* v) -> bool {
-    int r = r0 + e / kCols, c = e - (r - r0) * kCols;
-    int gy = mirror_row(y0 - kRadius + r, h);
-    int gx = x0 - kRadius + c;
-    if (r < kIH && gy >= 0 && gx >= 0 && gx < w) {
-      size_t i = (size_t)gy * w + gx;
-      v[0] = __ldg(ra + i);
-      v[1] = __ldg(ra + np + i);
-      v[2] = __ldg(ra + 2 * np + i);
-      v[3] = __ldg(rb + i);
-      v[4] = __ldg(rb + np + i);
-      v[5] = __ldg(rb + 2 * np + i);
-      return true;
-    }
-    return false;
-  };
-  // Per-chunk offsets: the reference's XYB and the XYB difference at the centre of the chunk at y0. Stored values
-  // are a' = a - oa and d' = (a - b) - od inside the image and 0 outside (the zero border). Every moment the maps
-  // need is recovered exactly from the blurred primed values and the in-image tap sum K of the column (K = 1 away
-  // from the left/right edges, where the offsets cancel outright).
-  auto centre = [&](int y0, float* oa_out, float* od_out) {
-    int cx = min(x0 + kTileW / 2, w - 1), cy = min(y0 + kTileH / 2, h - 1);
-    size_t i = (size_t)cy * w + cx;
-    const float z[3] = {0.f, 0.f, 0.f};
-    Pix c = pix(ra[i], ra[np + i], ra[2 * np + i], rb[i], rb[np + i], rb[2 * np + i], z, z, cb_bias);
-    for (int k = 0; k < 3; k++) {
-      oa_out[k] = c.a[k];
-      od_out[k] = c.d[k];
-    }
-  };
+  const int w = sd.w, h = sd.h, pitch = sd.pitch;
+  const size_t np = (size_t)pitch * h;
+  const float* pa = xa + sd.off;
+  const float* pd = xd + sd.off;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   float sums[kScoreSums];
 #pragma unroll
@@ -232,8 +248,9 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
   float2 g2[kRadius + 1];
 #pragma unroll
   for (int t = 0; t <= kRadius; t++) g2[t] = make_float2(c_gauss[t], c_gauss[t]);
+  auto tap = [&](int t) { return g2[t <= kRadius ? t : 2 * kRadius - t]; };
 
-  const int col = tid & 31, rg = tid >> 5;  // vertical pass: column, group of 4 output rows
+  const int col = lane, rg = warp;  // vertical pass: column, group of kVy output rows
   const int gx = x0 + col;
   // In-image tap sum of this column (1 except within kRadius of the left/right edge).
   const bool edge = gx < kRadius || gx >= w - kRadius;
@@ -248,289 +265,214 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
   }
   const float omk = 1.0f - K;
 
-#pragma unroll 1
-  for (int chunk = 0; chunk < nch; chunk++) {
-    const int y0 = ybeg + chunk * kTileH;
-    if (y0 >= h) break;
-    // Rows of the halo buffer converted in this chunk: all 42 in the first, the 32 below the carried ones after.
-    const int r0 = chunk == 0 ? 0 : kCarry;
-    float cur[6], nxt[6];
-    bool cur_ok;
-    if (chunk == 0) {
-      // The first pixel's loads go out before the offsets are settled (they do not depend on them).
-      cur_ok = load6(tid, y0, r0, cur);
-      if (tid == 0) centre(y0, s_oa, s_od);
-      __syncthreads();
-    } else {
-      __syncthreads();  // the previous chunk's passes are done with xs and hb; s_noa/s_nod are visible
-      cur_ok = load6(tid, y0, r0, cur);
-      // Carried rows: rows 32..41 of the previous chunk become rows 0..9, re-offset from the previous chunk's
-      // offsets to this one's (s_noa/s_nod, computed during the previous chunk).
-      float da[3], dd[3];
+  const int nrun = min(nch, (h - ybeg + kTileH - 1) / kTileH);  // chunks of this band that lie in the image
+  // The halo of one channel of a chunk: 42 rows x 12 quads. Rows follow the mirror rule; outside the left and right
+  // border a' and d' are zero, so those samples hold the offsets themselves.
+  auto centre_of = [&](int y0) {  // a plane has fewer than 2^32 samples
+    return (unsigned)min(y0 + kTileH / 2, h - 1) * (unsigned)pitch + (unsigned)min(x0 + kTileW / 2, w - 1);
+  };
+  auto fetch = [&](int ch, int y0, float oa, float od) {
+    const float* ca = pa + ch * np;
+    const float* cd = pd + ch * np;
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        da[k] = s_noa[k] - s_oa[k];
-        dd[k] = s_nod[k] - s_od[k];
-      }
-      constexpr int kCarried = kCarry * kCols * 3, kPer = (kCarried + kTileThreads - 1) / kTileThreads;
-      float2 keep[kPer];
+    for (int it = 0; it < (kIH * kQuads + kTileThreads - 1) / kTileThreads; it++) {
+      const int e = tid + it * kTileThreads;
+      if (e >= kIH * kQuads) break;
+      const int r = e / kQuads, q = e - r * kQuads;
+      const int gy = mirror_row(y0 - kRadius + r, h), gq = x0 - kLead + 4 * q;
+      float* dst = xs + r * kIW + 4 * q;
+      const unsigned at = (unsigned)gy * (unsigned)pitch + (unsigned)gq;
+      if (gy >= 0 && gq >= 0 && gq + 4 <= w) {
+        copy_quad(dst, ca + at);
+        copy_quad(dst + kXs, cd + at);
+      } else {
 #pragma unroll
-      for (int j = 0; j < kPer; j++) {
-        const int e = tid + j * kTileThreads;
-        if (e < kCarried) {
-          const int k = e / (kCarry * kCols), rem = e - k * (kCarry * kCols);
-          const int r = rem / kCols, c = rem - r * kCols;
-          float2 v = xs[k * kIH * kIW + (r + kTileH) * kIW + c];
-          // inside the image the stored values move with the offsets; outside they stay 0 (the zero border)
-          const int gy = mirror_row(y0 - kRadius + r, h), gxx = x0 - kRadius + c;
-          if (gy >= 0 && gxx >= 0 && gxx < w) {
-            const float dak = k == 0 ? da[0] : (k == 1 ? da[1] : da[2]);
-            const float ddk = k == 0 ? dd[0] : (k == 1 ? dd[1] : dd[2]);
-            v = make_float2(v.x - dak, v.y - ddk);
-          }
-          keep[j] = v;
+        for (int k = 0; k < 4; k++) {
+          const bool in = gy >= 0 && gq >= 0 && gq + k < w;
+          dst[k] = in ? __ldg(ca + at + k) : oa;
+          dst[kXs + k] = in ? __ldg(cd + at + k) : od;
         }
       }
-      __syncthreads();  // every carried value is read before rows 32..41 are overwritten
-#pragma unroll
-      for (int j = 0; j < kPer; j++) {
-        const int e = tid + j * kTileThreads;
-        if (e < kCarried) {
-          const int k = e / (kCarry * kCols), rem = e - k * (kCarry * kCols);
-          const int r = rem / kCols, c = rem - r * kCols;
-          xs[k * kIH * kIW + r * kIW + c] = keep[j];
-        }
-      }
-      if (tid < 3) {
-        s_oa[tid] = s_noa[tid];
-        s_od[tid] = s_nod[tid];
-      }
-      __syncthreads();
     }
-    float oa[3] = {s_oa[0], s_oa[1], s_oa[2]}, od[3] = {s_od[0], s_od[1], s_od[2]};
-    // This chunk's block of reference moments (kRefChunk float2).
-    float2* rchunk = nullptr;
+  };
+
+  float oa = __ldg(pa + centre_of(ybeg)), od = __ldg(pd + centre_of(ybeg));
+  fetch(0, ybeg, oa, od);
+#pragma unroll 1
+  for (int chunk = 0; chunk < nrun; chunk++) {
+    const int y0 = ybeg + chunk * kTileH;
+    const unsigned centre = centre_of(y0);
+    // Chunks whose halo and outputs all lie inside the image take the maps without their edge cases.
+    const bool inner = x0 >= kRadius && x0 + kTileW + kRadius <= w && y0 + kTileH <= h;
+    float2* rchunk = nullptr;  // this chunk's block of reference moments (kRefChunk float2)
     if constexpr (kRef != kRefNone) rchunk = refm + (size_t)(sd.chunk0 + local * nch + chunk) * kRefChunk;
     if constexpr (kRef == kRefRead) {
-      // Into L2 while this chunk's XYB and horizontal passes run: 8 KB per channel (16-byte aligned, as the bulk
-      // prefetch requires: blocks are 24 KB apart from an aligned base).
+      // 8 KB per channel (16-byte aligned, as the bulk prefetch requires: blocks are 24 KB apart from an aligned base).
       if (tid < 3) {
         const float2* p = rchunk + tid * kTileH * kTileW;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(kTileH * kTileW * 8) : "memory");
       }
     }
-
-    // XYB of the chunk's new rows; the six plane values of the next pixel are loaded before the current one is
-    // converted, so the global loads overlap the arithmetic. Two halo pixels per trip: the measured best unroll.
-    const int nconv = (kIH - r0) * kCols;
-#pragma unroll 2
-    for (int e = tid; e < nconv; e += kTileThreads) {
-      bool nxt_ok = load6(e + kTileThreads, y0, r0, nxt);
-      float v[6] = {0, 0, 0, 0, 0, 0};
-      if (cur_ok) {
-        Pix p = pix(cur[0], cur[1], cur[2], cur[3], cur[4], cur[5], oa, od, cb_bias);
-        v[0] = p.a[0]; v[1] = p.a[1]; v[2] = p.a[2];
-        v[3] = p.d[0]; v[4] = p.d[1]; v[5] = p.d[2];
-      }
-      const int r = r0 + e / kCols, idx = r * kIW + (e - (r - r0) * kCols);
-#pragma unroll
-      for (int k = 0; k < 3; k++) xs[k * kIH * kIW + idx] = make_float2(v[k], v[3 + k]);
-#pragma unroll
-      for (int k = 0; k < 6; k++) cur[k] = nxt[k];
-      cur_ok = nxt_ok;
-    }
-    // The next chunk's offsets, while the other threads finish their conversions.
-    if (tid == 0 && chunk + 1 < nch && y0 + kTileH < h) centre(y0 + kTileH, s_noa, s_nod);
-
 #pragma unroll 1
     for (int ch = 0; ch < 3; ch++) {
-      __syncthreads();  // xs complete (ch 0) / previous channel's vertical pass done with hb
-      const float2* X = xs + ch * kIH * kIW;
-      // Horizontal pass: kHx adjacent outputs per item; moments a', d', a'^2, b'^2 (b' = a' - d'), d'^2. The pairs
-      // (a', d') and (a'^2, d'^2) share every tap weight and run as packed two-lane FMAs (per lane exactly fmaf);
-      // the squares of a loaded (a', d') pair are one packed multiply.
-      // Items: each half-warp takes 4 rows x 4 items, so its 64-bit loads (row pitch 45 pairs = 26 banks mod 32)
-      // fall in distinct banks.
-      static_assert(kTileThreads == 256 && kTileH == 32 && kTileW == 32 && kIH - kTileH == 10, "item layout");
-      // One item: NX adjacent outputs of row r from column c0 on.
+      // The next halo: the next channel's, or the next chunk's first.
+      const bool more = ch < 2 || chunk + 1 < nrun;
+      const int nch_ = ch < 2 ? ch + 1 : 0, ny0 = ch < 2 ? y0 : y0 + kTileH;
+      float noa = 0.f, nod = 0.f;
+      if (more) {
+        const unsigned nc = centre_of(ny0);
+        noa = __ldg(pa + nch_ * np + nc);
+        nod = __ldg(pd + nch_ * np + nc);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();  // this halo is in place; the previous vertical pass is done with hb
+      // Horizontal pass: NX adjacent outputs of row r from column c0 on. Moments a', d', a'^2, b'^2 (b' = a' - d'), d'^2
+      // (reading form: (b'^2, d'^2) and d'). The row's pairs come in as 16-byte loads of two; every output's chain
+      // takes its taps in ascending order.
       auto hitem = [&](auto nx, const int r, const int c0) {
-        constexpr int NX = decltype(nx)::value;
-        const float2* xr = X + r * kIW + c0;
-        if constexpr (kRef == kRefRead) {
-          // (b'^2, d'^2) pairs and d'; the first plane of hb holds (blur b'^2, blur d'^2). b' replaces a' in its
-          // pair, so one packed multiply squares both.
-          float2 vsq[NX + 2 * kRadius];
-          float vd[NX + 2 * kRadius];
+        // Quads of columns c0 - 8 .. : tap position t (output o takes it as tap t - o) is sample t + 3.
+        constexpr int NX = decltype(nx)::value, NT = NX + 2 * kRadius;
+        static_assert(kLead - kRadius == 3, "samples before the first tap");
+        const float4* xr = reinterpret_cast<const float4*>(xs + r * kIW + c0);
+        [[maybe_unused]] float2 s0[NX];
+        float2 s1[NX];
+        float s4[NX];
 #pragma unroll
-          for (int t = 0; t < NX + 2 * kRadius; t++) {
-            float2 bd = xr[t];
-            vd[t] = bd.y;
-            bd.x = __fsub_rn(bd.x, bd.y);
-            vsq[t] = __fmul2_rn(bd, bd);
-          }
-          float2 m13[NX];
-          float m4[NX];
+        for (int g = 0; g < (NT + 3 + 3) / 4; g++) {
+          const float4 qa = xr[g], qd = xr[kXs / 4 + g];
+          const float va[4] = {qa.x, qa.y, qa.z, qa.w}, vd[4] = {qd.x, qd.y, qd.z, qd.w};
 #pragma unroll
-          for (int o = 0; o < NX; o++) {
-            float2 s13 = make_float2(0.f, 0.f);
-            float sd = 0.f;
-#pragma unroll
-            for (int t = 0; t < 2 * kRadius + 1; t++) {
-              const float2 kk = g2[t <= kRadius ? t : 2 * kRadius - t];
-              s13 = __ffma2_rn(kk, vsq[o + t], s13);
-              sd = fmaf(kk.x, vd[o + t], sd);
+          for (int k = 0; k < 4; k++) {
+            const int t = 4 * g + k - 3;
+            if (t < 0 || t >= NT) continue;
+            const float2 ad = make_float2(__fsub_rn(va[k], oa), __fsub_rn(vd[k], od));
+            const float bp = __fsub_rn(ad.x, ad.y);
+            float2 sq;
+            [[maybe_unused]] float bb = 0.f;
+            if constexpr (kRef == kRefRead) {
+              sq = __fmul2_rn(make_float2(bp, ad.y), make_float2(bp, ad.y));
+            } else {
+              sq = __fmul2_rn(ad, ad);
+              bb = __fmul_rn(bp, bp);
             }
-            m13[o] = s13;
-            m4[o] = sd;
+#pragma unroll
+            for (int o = 0; o < NX; o++) {
+              if (t - o < 0 || t - o > 2 * kRadius) continue;
+              const float2 kk = tap(t - o);
+              tap_pair(s1[o], kk, sq, t == o);
+              if constexpr (kRef == kRefRead) {
+                tap_one(s4[o], kk.x, ad.y, t == o);
+              } else {
+                tap_pair(s0[o], kk, ad, t == o);
+                tap_one(s4[o], kk.x, bb, t == o);
+              }
+            }
           }
-          float* h13 = hb + (r * kTileW + c0) * 2;
-          float* h4 = hb + 4 * kIH * kTileW + r * kTileW + c0;
+        }
+        auto put_pairs = [&](float* plane, const float2* s) {
+          float* d = plane + r * kTileW * 2;
 #pragma unroll
           for (int o = 0; o < NX; o += 2)
-            reinterpret_cast<float4*>(h13)[o / 2] = make_float4(m13[o].x, m13[o].y, m13[o + 1].x, m13[o + 1].y);
-          if constexpr (NX == 4) *reinterpret_cast<float4*>(h4) = make_float4(m4[0], m4[1], m4[2], m4[3]);
-          else *reinterpret_cast<float2*>(h4) = make_float2(m4[0], m4[1]);
+            *reinterpret_cast<float4*>(d + 2 * hb_pair(c0 + o, r)) = make_float4(s[o].x, s[o].y, s[o + 1].x, s[o + 1].y);
+        };
+        if constexpr (kRef == kRefRead) {
+          put_pairs(hb, s1);
         } else {
-          // Pairs (a', d') and (a'^2, d'^2) (one packed multiply of the loaded pair), b'^2 alone.
-          float2 vad[NX + 2 * kRadius], vsq[NX + 2 * kRadius];
-          float vbb[NX + 2 * kRadius];
-#pragma unroll
-          for (int t = 0; t < NX + 2 * kRadius; t++) {
-            const float2 ad = xr[t];
-            const float bb = __fsub_rn(ad.x, ad.y);
-            vad[t] = ad;
-            vsq[t] = __fmul2_rn(ad, ad);
-            vbb[t] = __fmul_rn(bb, bb);
-          }
-          float2 m01[NX], m23[NX];
-          float m4[NX];
-#pragma unroll
-          for (int o = 0; o < NX; o++) {
-            float2 s01 = make_float2(0.f, 0.f), s24 = make_float2(0.f, 0.f);
-            float sbb = 0.f;
-#pragma unroll
-            for (int t = 0; t < 2 * kRadius + 1; t++) {
-              const float2 kk = g2[t <= kRadius ? t : 2 * kRadius - t];
-              s01 = __ffma2_rn(kk, vad[o + t], s01);
-              s24 = __ffma2_rn(kk, vsq[o + t], s24);
-              sbb = fmaf(kk.x, vbb[o + t], sbb);
-            }
-            m01[o] = s01;
-            m23[o] = s24;
-            m4[o] = sbb;
-          }
-          // hb: two planes of (moment 0, moment 1) and (moment 2, moment 4) pairs, then moment 3
-          float* h01 = hb + (r * kTileW + c0) * 2;
-          float* h23 = hb + (kIH * kTileW + r * kTileW + c0) * 2;
-          float* h4 = hb + 4 * kIH * kTileW + r * kTileW + c0;
-#pragma unroll
-          for (int o = 0; o < NX; o += 2) {
-            reinterpret_cast<float4*>(h01)[o / 2] = make_float4(m01[o].x, m01[o].y, m01[o + 1].x, m01[o + 1].y);
-            reinterpret_cast<float4*>(h23)[o / 2] = make_float4(m23[o].x, m23[o].y, m23[o + 1].x, m23[o + 1].y);
-          }
-          if constexpr (NX == 4) *reinterpret_cast<float4*>(h4) = make_float4(m4[0], m4[1], m4[2], m4[3]);
-          else *reinterpret_cast<float2*>(h4) = make_float2(m4[0], m4[1]);
+          put_pairs(hb, s0);
+          put_pairs(hb + 2 * kIH * kTileW, s1);
         }
+        float* h4 = hb + kOnes + r * kTileW;
+#pragma unroll
+        for (int o = 0; o < NX; o += 4)
+          *reinterpret_cast<float4*>(h4 + hb_one(c0 + o, r)) = make_float4(s4[o], s4[o + 1], s4[o + 2], s4[o + 3]);
       };
-      // Rows 0..31: one item of kHx = 4 outputs per thread; each half-warp takes 4 rows x 4 items, so its 64-bit
-      // loads (row pitch 45 pairs = 26 banks mod 32) fall in distinct banks.
-      {
-        const int hw = tid >> 4, j = tid & 15;
-        hitem(std::integral_constant<int, kHx>(), (hw >> 1) * 4 + (j >> 2), kHx * ((j & 3) + 4 * (hw & 1)));
-      }
-      // The 10 halo rows below: 160 items of 2 outputs (a half-warp takes 2 rows x 8 items, again distinct banks),
-      // so this round costs about half an item of 4 and runs on 5 warps instead of 2.5 (measured per 12 MP launch:
-      // reading form 547 -> 537 us, storing form 615 -> 596 us, same bits).
-      if (tid < (kIH - kTileH) * (kTileW / 2)) {
-        const int hw = tid >> 4, j = tid & 15;
-        hitem(std::integral_constant<int, 2>(), kTileH + (hw >> 1) * 2 + (j >> 3), 2 * ((j & 7) + 8 * (hw & 1)));
+      static_assert(kTileThreads == 128 && kTileH == 32 && kTileW == 32 && kIH - kTileH == 10, "item layout");
+      // Rows 0..31: one item of 8 outputs per thread; eight lanes take the 4 items of each of 2 rows.
+      hitem(std::integral_constant<int, 8>(), warp * 8 + (lane >> 2), 8 * (lane & 3));
+      // The 10 halo rows below: 80 items of 4 outputs (eight lanes take 4 items of each of 2 rows).
+      if (tid < (kIH - kTileH) * (kTileW / 4))
+        hitem(std::integral_constant<int, 4>(), kTileH + warp * 4 + ((lane >> 2) & 1) + 2 * (lane >> 4),
+              4 * ((lane & 3) + 4 * ((lane >> 3) & 1)));
+      float ca0[kVy], cd0[kVy];  // this thread's samples, for the edge maps
+#pragma unroll
+      for (int o = 0; o < kVy; o++) {
+        const float* x = xs + (rg * kVy + o + kRadius) * kIW + col + kLead;
+        ca0[o] = __fsub_rn(x[0], oa);
+        cd0[o] = __fsub_rn(x[kXs], od);
       }
       __syncthreads();
-      // Vertical pass + error maps: 4 output rows of one column per thread, the same pairs packed.
-      float mu[5][4];
+      if (more) fetch(nch_, ny0, noa, nod);
+      // Vertical pass + error maps: kVy output rows of one column per thread, the same pairs packed.
       float2* rrow = nullptr;  // this thread's row 0 in the chunk's block
-      if constexpr (kRef != kRefNone) rrow = rchunk + (ch * kTileH + rg * 4) * kTileW + col;
+      if constexpr (kRef != kRefNone) rrow = rchunk + (ch * kTileH + rg * kVy) * kTileW + col;
+      float2 rm[kVy];  // the reference moments: their loads overlap the blur
       if constexpr (kRef == kRefRead) {
-        // The reference moments first (their loads overlap the blur), then (blur b'^2, blur d'^2) and blur d'.
 #pragma unroll
-        for (int o = 0; o < 4; o++) {
-          float2 rm = make_float2(0.f, 0.f);
-          if (gx < w && y0 + rg * 4 + o < h) rm = __ldg(rrow + o * kTileW);
-          mu[0][o] = rm.x;
-          mu[2][o] = rm.y;
-        }
-        const float2* h13 = reinterpret_cast<const float2*>(hb);
-        const float* h4 = hb + 4 * kIH * kTileW;
-        float2 v13[4 + 2 * kRadius];
-        float v4[4 + 2 * kRadius];
-#pragma unroll
-        for (int t = 0; t < 4 + 2 * kRadius; t++) {
-          const int i = (rg * 4 + t) * kTileW + col;
-          v13[t] = h13[i];
-          v4[t] = h4[i];
-        }
-#pragma unroll
-        for (int o = 0; o < 4; o++) {
-          float2 a13 = make_float2(0.f, 0.f);
-          float a4 = 0.f;
-#pragma unroll
-          for (int t = 0; t < 2 * kRadius + 1; t++) {
-            const float2 kk = g2[t <= kRadius ? t : 2 * kRadius - t];
-            a13 = __ffma2_rn(kk, v13[o + t], a13);
-            a4 = fmaf(kk.x, v4[o + t], a4);
-          }
-          mu[3][o] = a13.x;
-          mu[4][o] = a13.y;
-          mu[1][o] = a4;
-        }
-      } else {
-        const float2* h01 = reinterpret_cast<const float2*>(hb);
-        const float2* h23 = reinterpret_cast<const float2*>(hb) + kIH * kTileW;
-        const float* h4 = hb + 4 * kIH * kTileW;
-        float2 v01[4 + 2 * kRadius], v23[4 + 2 * kRadius];
-        float v4[4 + 2 * kRadius];
-#pragma unroll
-        for (int t = 0; t < 4 + 2 * kRadius; t++) {
-          const int i = (rg * 4 + t) * kTileW + col;
-          v01[t] = h01[i];
-          v23[t] = h23[i];
-          v4[t] = h4[i];
-        }
-#pragma unroll
-        for (int o = 0; o < 4; o++) {
-          float2 a01 = make_float2(0.f, 0.f), a23 = make_float2(0.f, 0.f);
-          float a4 = 0.f;
-#pragma unroll
-          for (int t = 0; t < 2 * kRadius + 1; t++) {
-            const float2 kk = g2[t <= kRadius ? t : 2 * kRadius - t];
-            a01 = __ffma2_rn(kk, v01[o + t], a01);
-            a23 = __ffma2_rn(kk, v23[o + t], a23);
-            a4 = fmaf(kk.x, v4[o + t], a4);
-          }
-          mu[0][o] = a01.x;
-          mu[1][o] = a01.y;
-          mu[2][o] = a23.x;
-          mu[4][o] = a23.y;
-          mu[3][o] = a4;
-          if constexpr (kRef == kRefWrite) {
-            if (gx < w && y0 + rg * 4 + o < h) rrow[o * kTileW] = make_float2(a01.x, a23.x);
-          }
+        for (int o = 0; o < kVy; o++) {
+          rm[o] = make_float2(0.f, 0.f);
+          if (inner || (gx < w && y0 + rg * kVy + o < h)) rm[o] = __ldg(rrow + o * kTileW);
         }
       }
-      const float ca = s_oa[ch], cd = s_od[ch], cbv = ca - cd;
-      float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      [[maybe_unused]] float2 s0[kVy];
+      float2 s1[kVy];
+      float s4[kVy];
+      {
+        const float2* hp = reinterpret_cast<const float2*>(hb) + rg * kVy * kTileW;
+        const float* h4 = hb + kOnes + rg * kVy * kTileW;
 #pragma unroll
-      for (int o = 0; o < 4; o++) {
-        int ry = rg * 4 + o;
+        for (int t = 0; t < kVy + 2 * kRadius; t++) {
+          const float2* row = hp + t * kTileW + hb_pair(col, t);  // rg * kVy is even
+          const float2 v0 = row[0];
+          float2 v1 = v0;
+          if constexpr (kRef != kRefRead) v1 = row[kIH * kTileW];
+          const float v4 = h4[t * kTileW + hb_one(col, t)];
+#pragma unroll
+          for (int o = 0; o < kVy; o++) {
+            if (t - o < 0 || t - o > 2 * kRadius) continue;
+            const float2 kk = tap(t - o);
+            tap_pair(s1[o], kk, v1, t == o);
+            if constexpr (kRef != kRefRead) tap_pair(s0[o], kk, v0, t == o);
+            tap_one(s4[o], kk.x, v4, t == o);
+          }
+        }
+        if constexpr (kRef == kRefWrite) {
+#pragma unroll
+          for (int o = 0; o < kVy; o++)
+            if (inner || (gx < w && y0 + rg * kVy + o < h)) rrow[o * kTileW] = make_float2(s0[o].x, s1[o].x);
+        }
+      }
+      // The chunk's offsets with the constants of the channel (kXyb0*), for the corrections at the zero border.
+      const float cd = od;
+      const float ca = oa + (ch == 0 ? kXyb0X : ch == 1 ? kXyb0Y : kXyb0B), cbv = ca - cd;
+      float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      auto maps = [&](auto inside) {
+        constexpr bool kInside = decltype(inside)::value;
+#pragma unroll
+      for (int o = 0; o < kVy; o++) {
+        int ry = rg * kVy + o;
         int gy = y0 + ry;
-        if (gx < w && gy < h) {
+        if (kInside || (gx < w && gy < h)) {
           // Blurred primed moments -> sigma_1^2, sigma_2^2, sigma_(a-b)^2, mu1 - mu2 (exactly, given K).
-          float m1 = mu[0][o], dmp = mu[1][o], m2 = m1 - dmp;
-          float v1 = fmaf(-m1, m1, mu[2][o]);
-          float v2 = fmaf(-m2, m2, mu[3][o]);
-          float vd = fmaf(-dmp, dmp, mu[4][o]);
+          float m1, dmp, e11, e22, edd;
+          if constexpr (kRef == kRefRead) {
+            m1 = rm[o].x;
+            e11 = rm[o].y;
+            dmp = s4[o];
+            e22 = s1[o].x;
+            edd = s1[o].y;
+          } else {
+            m1 = s0[o].x;
+            dmp = s0[o].y;
+            e11 = s1[o].x;
+            edd = s1[o].y;
+            e22 = s4[o];
+          }
+          const float m2 = m1 - dmp;
+          float v1 = fmaf(-m1, m1, e11);
+          float v2 = fmaf(-m2, m2, e22);
+          float vd = fmaf(-dmp, dmp, edd);
           float dmu;
-          if (edge) {
+          if (!kInside && edge) {
             v1 = fmaf(omk * ca, fmaf(ca, K, 2.0f * m1), v1);
             v2 = fmaf(omk * cbv, fmaf(cbv, K, 2.0f * m2), v2);
             vd = fmaf(omk * cd, fmaf(cd, K, 2.0f * dmp), vd);
@@ -544,10 +486,8 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
           float num_s = den - vd;
           float d = fmaxf(fdiv_ftz(fmaf(dmu * dmu, num_s, vd), den), 0.0f);
           // Edge maps (:431-433): d1 = (|r2| - |r1|) / (1 + |r1|) with r1 = a - mu1, r2 = b - mu2 = r1 - rd.
-          const float2 c0 = X[(ry + kRadius) * kIW + col + kRadius];
-          float a0 = c0.x, d0 = c0.y;
-          float r1 = a0 - m1, rd = d0 - dmp;
-          if (edge) {
+          float r1 = ca0[o] - m1, rd = cd0[o] - dmp;
+          if (!kInside && edge) {
             r1 = fmaf(ca, omk, r1);
             rd = fmaf(cd, omk, rd);
           }
@@ -565,16 +505,20 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
           acc[5] += e2 * e2;
         }
       }
+      };
+      if (inner) maps(std::true_type());
+      else maps(std::false_type());
 #pragma unroll
       for (int i = 0; i < 6; i++) sums[ch * 6 + i] += acc[i];
+      oa = noa;
+      od = nod;
     }
   }
-  // Warp sums (f32, 32 threads x 4 pixels), then the 8 warps in f64 in a fixed order. Sums 0..15 by a reduce-scatter
+  // Warp sums (f32, 32 threads x kVy pixels per chunk), then the warps in f64 in a fixed order. Sums 0..15 by a reduce-scatter
   // butterfly: at each exchange (lane distance 16, 8, 4, 2) a lane keeps half of the values it carries and adds its
   // partner's copy of that half, then distance 1 adds the pair; lane l ends with sum l >> 1. The additions are those
   // of a full butterfly per sum, so every sum has the same bits, in 16 shuffles instead of 80. Sums 16 and 17 by full
   // butterflies.
-  const int lane = tid & 31, warp = tid >> 5;
   {
     float a[16];
 #pragma unroll
@@ -608,7 +552,7 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
 }
 
 template <int kRef>
-__global__ void __launch_bounds__(kTileThreads, 3)
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
     k_ssim2_tiles(PyramidDesc pd, const float* __restrict__ ref, const float* __restrict__ dist,
                   double* __restrict__ partials, const StepDesc* __restrict__ st, float2* __restrict__ refm) {
   if (st && !st->active) return;
@@ -689,23 +633,37 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce(PyramidDesc pd, const doub
 
 // ------------------------------------------------------------------------------------------------ planes, pyramid
 
-// Linear planes of an interleaved image (core/src/ssimulacra2.rs:177-221, with core/src/image.rs:143-190 for alpha:
-// 16-bit samples rounded to 8 bits, then composited onto mid-grey 128). Four consecutive pixels per thread (in
-// row-major order; the planes are contiguous [3][h][w]) so each thread moves enough bytes per request.
-// CTA `cta` of an image's 4-pixel groups; lut8: the 8-bit table in shared memory.
-__device__ __forceinline__ void to_linear_groups(const uint8_t* __restrict__ img, int w, int h, int channels, int depth,
-                                                 const float* __restrict__ lut16, float* __restrict__ out,
-                                                 size_t cta, const float* lut8) {
-  const size_t np = (size_t)w * h;
-  const size_t i0 = 4 * (cta * blockDim.x + threadIdx.x);
-  if (i0 >= np) return;
-  const int n = (int)min((size_t)4, np - i0);
-  float v[3][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+// An interleaved image's samples (core/src/ssimulacra2.rs:177-221, with core/src/image.rs:143-190 for alpha: 16-bit
+// samples rounded to 8 bits, then composited onto mid-grey 128).
+struct ImageSrc {
+  const uint8_t* img;
+  int w, h, channels, depth;
+  const float* lut16;  // 65536-entry table for 16-bit samples without alpha
+};
+
+// Linear light of four consecutive pixels of row y (columns x0 .. x0+3, zero beyond the row). lut8: the 8-bit table in
+// shared memory.
+__device__ __forceinline__ void image_quad(const ImageSrc& im, int x0, int y, const float* lut8, float (&v)[3][4]) {
+  const uint8_t* img = im.img;
+  const int w = im.w, channels = im.channels, depth = im.depth;
+  const float* lut16 = im.lut16;
+  const size_t i0 = (size_t)y * w + x0;
+  const int n = min(4, w - x0);
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[c][k] = 0.f;
   const bool alpha = channels == 2 || channels == 4;
-  if (depth == 8 && channels == 3 && n == 4 && ((uintptr_t)img & 3) == 0) {
-    // 12 bytes at 12 * (i0/4): 4-byte aligned when the image is (callers may pass any device pointer)
-    const uint32_t* p = reinterpret_cast<const uint32_t*>(img + i0 * 3);
-    uint32_t q0 = p[0], q1 = p[1], q2 = p[2];
+  const uintptr_t at = (uintptr_t)(img + i0 * 3);
+  const int mis = (int)(at & 3);
+  // 12 bytes of any alignment: the aligned words that hold them and a funnel shift; the fourth word only where the
+  // image goes on past it (the image may end, or start, at any byte of a caller's buffer).
+  if (depth == 8 && channels == 3 && n == 4 && i0 * 3 >= (size_t)mis &&
+      (mis == 0 || i0 * 3 + 16 - mis <= (size_t)w * im.h * 3)) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(at - mis);
+    const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = mis ? p[3] : 0u;
+    const uint32_t q0 = __funnelshift_r(w0, w1, 8 * mis), q1 = __funnelshift_r(w1, w2, 8 * mis),
+                   q2 = __funnelshift_r(w2, w3, 8 * mis);
     uint32_t b[12] = {q0 & 0xFF, (q0 >> 8) & 0xFF, (q0 >> 16) & 0xFF, q0 >> 24, q1 & 0xFF, (q1 >> 8) & 0xFF,
                       (q1 >> 16) & 0xFF, q1 >> 24, q2 & 0xFF, (q2 >> 8) & 0xFF, (q2 >> 16) & 0xFF, q2 >> 24};
 #pragma unroll
@@ -758,24 +716,26 @@ __device__ __forceinline__ void to_linear_groups(const uint8_t* __restrict__ img
       }
     }
   }
-  if (n == 4 && np % 4 == 0 && ((uintptr_t)out & 15) == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      *reinterpret_cast<float4*>(out + c * np + i0) = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
-  } else {
-    for (int k = 0; k < n; k++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) out[c * np + i0 + k] = v[c][k];
-  }
 }
 
-__global__ void k_to_linear(const uint8_t* __restrict__ img, int w, int h, int channels, int depth,
-                            const float* __restrict__ lut16, float* __restrict__ out) {
+// Linear planes [3][h][pitch] of an image (the reference-order scorer's input).
+__global__ void __launch_bounds__(256) k_to_linear(const ImageSrc im, int pitch, float* __restrict__ out) {
   // The table lives in shared memory: per-thread indices differ, which would serialize constant-memory reads.
   __shared__ float lut8[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) lut8[i] = c_lut8s[i];
+  lut8[threadIdx.x] = c_lut8s[threadIdx.x];
   __syncthreads();
-  to_linear_groups(img, w, h, channels, depth, lut16, out, blockIdx.x, lut8);
+  const int groups = (im.w + 3) / 4;
+  const long long g = (long long)blockIdx.x * 256 + threadIdx.x, y = g / groups;
+  if (y >= im.h) return;
+  const int x0 = 4 * (int)(g - y * groups);
+  float v[3][4];
+  image_quad(im, x0, (int)y, lut8, v);
+  const size_t np = (size_t)pitch * im.h, o = (size_t)y * pitch + x0;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (x0 + k < im.w)
+#pragma unroll
+      for (int c = 0; c < 3; c++) out[c * np + o + k] = v[c][k];
 }
 
 // Error-free transform: s + e == a + b exactly (Knuth's TwoSum).
@@ -786,375 +746,305 @@ __device__ __forceinline__ float two_sum(float a, float b, float& e) {
   return s;
 }
 
-// Mean of the 2x2 block at output (ox, oy) of a plane of w x h (fewer samples at odd edges), as downsample
-// (core/src/ssimulacra2.rs:223-247) computes it: the reference sums in f64, which is exact for these inputs, then
-// rounds once to f32; the compensated sum here (TwoSum) rounds the same exact sum once, so the planes agree with the
-// reference's except in rare double-rounding cases.
-// kFresh: the plane was written earlier in the same kernel (the fused upsample + pyramid), so loads go through L2
-// (ld.global.cg) and never through the read-only data path, which need not see this kernel's own writes.
-template <bool kFresh>
-__device__ __forceinline__ float ldp(const float* p) {
-  if constexpr (kFresh) return __ldcg(p);
-  else return *p;
-}
-template <bool kFresh>
-__device__ __forceinline__ float4 ldp4(const float4* p) {
-  if constexpr (kFresh) return __ldcg(p);
-  else return *p;
+// Mean of a 2x2 block (q0 q1 above q2 q3) of which the right column and the lower row may lie outside the image, as
+// downsample (core/src/ssimulacra2.rs:223-247) computes it: the reference sums in f64, which is exact for these inputs,
+// then rounds once to f32; the compensated sum here (TwoSum, in the reference's order) rounds the same exact sum once, so
+// the planes agree with the reference's except in rare double-rounding cases. The scaling is exact.
+__device__ __forceinline__ float block_mean(float q0, float q1, float q2, float q3, bool right, bool below) {
+  float e0 = 0.f, e1 = 0.f, e2 = 0.f;
+  float s = q0;
+  if (right) s = two_sum(s, q1, e0);
+  if (below) s = two_sum(s, q2, e1);
+  if (right && below) s = two_sum(s, q3, e2);
+  return __fadd_rn(s, (e0 + e1) + e2) * (right ? (below ? 0.25f : 0.5f) : (below ? 0.5f : 1.0f));
 }
 
-template <bool kFresh = false>
-__device__ __forceinline__ float mean2x2(const float* p, int stride, int w, int h, int ox, int oy) {
-  int x0 = ox * 2, x1 = min(ox * 2 + 2, w), y0 = oy * 2, y1 = min(oy * 2 + 2, h);
-  float s = 0.0f, err = 0.0f;
-  for (int y = y0; y < y1; y++)
-    for (int x = x0; x < x1; x++) {
-      float e;
-      s = two_sum(s, ldp<kFresh>(p + (size_t)y * stride + x), e);
-      err += e;
-    }
-  // count is 1, 2 or 4: the scaling is exact.
-  return __fadd_rn(s, err) * (1.0f / (float)((y1 - y0) * (x1 - x0)));
-}
+// ---- pyramid builder
+//
+// One launch takes an image (or two) from its source to everything the scorer reads, at every scale: one CTA per 64x64
+// block of scale 0 and the 32x32 .. 2x2 blocks of scales 1-5 below it, which nest exactly because each level halves the
+// one above. Sixteen rows of the block at a time, each thread converts a quad (four samples of a row) to linear light,
+// writes what the scorer needs of it and passes the linear samples on: a row pair sits in one warp, whose halves exchange
+// two samples per channel and make one scale-1 sample each, kept in shared memory. Every coarser level is made from the
+// one above in shared memory and written by quads. Linear planes exist in memory only where a later launch reads them
+// (a search's reference).
+// What bounds it: instruction issue in the colour conversion (69% active; packed in pairs of pixels), then the latency of
+// a quad's loads. Measured per 12 MP candidate of a 4:2:0 search: 133 us, the tile kernel then 276 (62 us when this step
+// wrote linear planes and the tile kernel converted them to XYB in every halo, 538); 154 us with one thread per 4x4
+// block converting its four rows in turn, each waiting for the reference's samples; 168 us with each level written as it
+// was made, its few threads' loads between two barriers; 142 us at 3 CTAs per SM instead of 4. A 4K pair: 130 us where
+// linear planes, pyramids and their conversion took 228 (two launches each of the first two); 151 us at 2 CTAs per SM
+// instead of 3. Layouts other than 4:2:0 with a width divisible by 4 took two launches: 1283x857, mostly 4:4:4,
+// 44 -> 24 us per candidate, gray 1653x2339 76 -> 55.
+enum BuildSrc { kFromPlanes, kFromLinear, kFromImage };
+enum BuildOut {
+  kOutDiff,  // differences against ref (linear) -> out
+  kOutRef,   // linear -> out, XYB -> xyb
+  kOutPair   // two images: XYB of the first -> xyb, differences -> out
+};
+struct BuildArgs {
+  float* out;
+  float* xyb;
+  const float* ref;
+  const uint8_t* planes;  // kFromPlanes: decoded components of the layout in st
+  const StepDesc* st;
+  ImageSrc im[2];         // kFromImage
+};
 
-// Every coarser scale of a pyramid from scale 0 in one launch. One CTA owns a kPyrTW x kPyrTH tile of scale 1 (a
-// block of scale 0 twice as wide and tall) and the tiles of scales 2-5 below it, each half the one above, kept in
-// shared memory between levels: tiles nest exactly because each level halves the previous one, and odd edges occur
-// only in the last tile of a row or column, where mean2x2 clips to the level's size. The scale-5 tile is
-// kPyrTW/16 x kPyrTH/16.
-constexpr int kPyrTW = 32, kPyrTH = 32;
-constexpr int kPyrThreads = 256;  // every pyramid launch
-static_assert(kPyrTH % 16 == 0 && kPyrTW % 32 == 0 && kPyrTW * kPyrTH % (2 * kPyrThreads) == 0, "pyramid tile");
+constexpr int kPyrT = 64;         // scale-0 block of a CTA
+constexpr int kPyrThreads = 256;
+// Rows of a level's block in shared memory, padded so that quads stay 16-byte aligned; where each level starts.
+__device__ __forceinline__ constexpr int lev_pitch(int L) { return (kPyrT >> L) + 4; }
+__device__ __forceinline__ constexpr int lev_off(int L) {
+  int o = 0;
+  for (int k = 1; k < L; k++) o += lev_pitch(k) * (kPyrT >> k);
+  return o;
+}
+constexpr int kLevFloats = 36 * 32 + 20 * 16 + 12 * 8 + 8 * 4 + 6 * 2;  // one channel's levels 1-5
 
 int pyramid_ctas(const PyramidDesc& pd) {
-  if (pd.nscales < 2) return 0;
-  return ((pd.s[1].w + kPyrTW - 1) / kPyrTW) * ((pd.s[1].h + kPyrTH - 1) / kPyrTH);
+  return ((pd.s[0].w + kPyrT - 1) / kPyrT) * ((pd.s[0].h + kPyrT - 1) / kPyrT);
 }
 
-// Scale-1 tile (tx, ty) from scale 0 into `out` (shared) and dst1 (global). Each thread takes pairs of adjacent
-// outputs, whose 2x4 source samples per channel are two aligned 16-byte loads when the scale-0 rows are (width a
-// multiple of 4, planes 16-byte aligned; the usual case); each output sums its four samples in mean2x2's order.
-// Partial blocks (the last odd column or row) and unaligned planes take the general path. Source and destination
-// are separate restricted pointers, so the loads of later outputs may be issued before the stores of earlier ones.
-__device__ __forceinline__ float quad_mean(float q0, float q1, float q2, float q3) {
-  float e0, e1, e2;
-  float t = two_sum(q0, q1, e0);  // 0 + q0 is exact, so this matches mean2x2's first steps
-  t = two_sum(t, q2, e1);
-  t = two_sum(t, q3, e2);
-  return __fadd_rn(t, (e0 + e1) + e2) * 0.25f;
+__device__ __forceinline__ void put4(float* __restrict__ p, size_t np, const float2 (&v)[2][3]) {
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    *reinterpret_cast<float4*>(p + c * np) = make_float4(v[0][c].x, v[0][c].y, v[1][c].x, v[1][c].y);
 }
 
-template <bool kFresh>
-__device__ __forceinline__ void scale1_tile(const float* __restrict__ src0, float* __restrict__ dst1,
-                                            const ScaleDesc& s0, const ScaleDesc& s1, int tx, int ty,
-                                            float (*out)[kPyrTH][kPyrTW + 1]) {
-  const size_t np0 = (size_t)s0.w * s0.h, np1 = (size_t)s1.w * s1.h;
-  const bool vec = (s0.w & 3) == 0 && ((uintptr_t)src0 & 15) == 0;
+// The reference's linear samples of quad (x, y) of a scale (kOutDiff), asked for before the image's own are converted.
+template <int kOut>
+__device__ __forceinline__ void ref_quad(const BuildArgs& g, const ScaleDesc& sd, int x, int y, float4 (&r)[3]) {
+  if constexpr (kOut == kOutDiff) {
+    const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
 #pragma unroll
-  for (int k = 0; k < kPyrTW * kPyrTH / (2 * kPyrThreads); k++) {
-    const int i = threadIdx.x + k * kPyrThreads;
-    const int lx = 2 * (i % (kPyrTW / 2)), ly = i / (kPyrTW / 2);
-    const int ox = tx * kPyrTW + lx, oy = ty * kPyrTH + ly;
-    if (ox >= s1.w || oy >= s1.h) continue;
-    float v[2][3];
-    const bool two = ox + 1 < s1.w;
-    if (vec && 2 * ox + 3 < s0.w && 2 * oy + 1 < s0.h) {
-      float4 r0[3], r1[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float4* p = reinterpret_cast<const float4*>(src0 + c * np0 + (size_t)(2 * oy) * s0.w + 2 * ox);
-        r0[c] = ldp4<kFresh>(p);
-        r1[c] = ldp4<kFresh>(p + s0.w / 4);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        v[0][c] = quad_mean(r0[c].x, r0[c].y, r1[c].x, r1[c].y);
-        v[1][c] = quad_mean(r0[c].z, r0[c].w, r1[c].z, r1[c].w);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int x = ox + j;
-        if (j == 1 && !two) break;
-        const bool full = 2 * x + 1 < s0.w && 2 * oy + 1 < s0.h;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          if (full) {
-            const float* p = src0 + c * np0 + (size_t)(2 * oy) * s0.w + 2 * x;
-            v[j][c] = quad_mean(ldp<kFresh>(p), ldp<kFresh>(p + 1), ldp<kFresh>(p + s0.w), ldp<kFresh>(p + s0.w + 1));
-          } else {
-            v[j][c] = mean2x2<kFresh>(src0 + c * np0, s0.w, s0.w, s0.h, x, oy);
-          }
-        }
-      }
-    }
+    for (int c = 0; c < 3; c++) r[c] = __ldg(reinterpret_cast<const float4*>(g.ref + c * np + i));
+  }
+}
+
+// Write quad (x, y) of a scale: l the linear samples of the image (kOutPair: of the first, l2 of the second), rq its
+// ref_quad.
+template <int kOut>
+__device__ __forceinline__ void emit_quad(const BuildArgs& g, const ScaleDesc& sd, int x, int y, const float4 (&rq)[3],
+                                          const float (&l)[3][4], const float (&l2)[3][4]) {
+  const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
+  auto at = [](const float (&v)[3][4], int c, int k) { return make_float2(v[c][2 * k], v[c][2 * k + 1]); };
+  float2 o[2][3];
+  if constexpr (kOut == kOutDiff) {
+    float r[3][4];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      out[c][ly][lx] = v[0][c];
-      float* d = dst1 + c * np1 + (size_t)oy * s1.w + ox;
-      d[0] = v[0][c];
-      if (two) {
-        out[c][ly][lx + 1] = v[1][c];
-        d[1] = v[1][c];
-      }
-    }
-  }
-}
-
-// Every output of every level of tile (tx, ty) is a full 2x2 mean (no clipped block at an odd edge).
-__device__ __forceinline__ bool pyramid_interior(const PyramidDesc& pd, int tx, int ty) {
-  int tw = kPyrTW, th = kPyrTH;
-  for (int L = 1; L < pd.nscales; L++) {
-    if (2 * (tx + 1) * tw > pd.s[L - 1].w || 2 * (ty + 1) * th > pd.s[L - 1].h) return false;
-    tw /= 2;
-    th /= 2;
-  }
-  return true;
-}
-
-// Tile (tx, ty) when it is interior and scale 0 takes 16-byte row loads: each thread owns a 2x2 block of scale 1 (its
-// 4x4 scale-0 source as 16-byte loads) and so one scale-2 sample, computed in registers; the four scale-2 samples of
-// a scale-3 sample sit in one warp (a warp holds two scale-2 rows) and meet by shuffles; scales 4 and 5 (16 and 4
-// samples) go through shared memory. Every sample is quad_mean of its four sources in mean2x2's order, as the general
-// path computes it for full blocks, so the planes are the same bits.
-// Scales 1-5 of interior tile (tx, ty) from the thread's 2x2 block of scale 1 (v1[row][column][channel], at
-// scale-1 origin (tx * 32 + 2 (t % 16), ty * 32 + 2 (t / 16))).
-__device__ __forceinline__ void pyramid_levels_interior(const PyramidDesc& pd, float* __restrict__ pyr, int tx,
-                                                        int ty, const float (&v1)[2][2][3]) {
-  static_assert(kPyrTW == 32 && kPyrTH == 32 && kPyrThreads == 256, "thread layout of the interior path");
-  __shared__ float l3[3][8][8], l4[3][4][4];
-  const ScaleDesc s1 = pd.s[1];
-  const size_t np1 = (size_t)s1.w * s1.h;
-  const int t = threadIdx.x, bx = t % 16, by = t / 16;
-  const int ox = tx * 32 + 2 * bx, oy = ty * 32 + 2 * by;  // scale-1 origin of the thread's 2x2 block
-  float* dst1 = pyr + s1.off;
-#pragma unroll
-  for (int r = 0; r < 2; r++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float* d = dst1 + c * np1 + (size_t)(oy + r) * s1.w + ox;
-      d[0] = v1[r][0][c];
-      d[1] = v1[r][1][c];
-    }
-  if (pd.nscales < 3) return;
-  const ScaleDesc s2 = pd.s[2];
-  const size_t np2 = (size_t)s2.w * s2.h;
-  float v2[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    v2[c] = quad_mean(v1[0][0][c], v1[0][1][c], v1[1][0][c], v1[1][1][c]);
-    pyr[s2.off + c * np2 + (size_t)(ty * 16 + by) * s2.w + tx * 16 + bx] = v2[c];
-  }
-  if (pd.nscales < 4) return;
-  // Scale 3: lane = 16 * (row parity) + column; the sample at (column pair, warp) takes lanes l, l+1, l+16, l+17.
-  const ScaleDesc s3 = pd.s[3];
-  const size_t np3 = (size_t)s3.w * s3.h;
-  const int lane = t & 31, warp = t >> 5;
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const float q1 = __shfl_down_sync(0xffffffffu, v2[c], 1);
-    const float q2 = __shfl_down_sync(0xffffffffu, v2[c], 16);
-    const float q3 = __shfl_down_sync(0xffffffffu, v2[c], 17);
-    if (lane < 16 && (lane & 1) == 0) {
-      const float v3 = quad_mean(v2[c], q1, q2, q3);
-      const int X = lane / 2, Y = warp;
-      pyr[s3.off + c * np3 + (size_t)(ty * 8 + Y) * s3.w + tx * 8 + X] = v3;
-      l3[c][Y][X] = v3;
-    }
-  }
-  if (pd.nscales < 5) return;
-  __syncthreads();
-  const ScaleDesc s4 = pd.s[4];
-  const size_t np4 = (size_t)s4.w * s4.h;
-  if (t < 16) {
-    const int X = t % 4, Y = t / 4;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float v4 = quad_mean(l3[c][2 * Y][2 * X], l3[c][2 * Y][2 * X + 1], l3[c][2 * Y + 1][2 * X],
-                                 l3[c][2 * Y + 1][2 * X + 1]);
-      pyr[s4.off + c * np4 + (size_t)(ty * 4 + Y) * s4.w + tx * 4 + X] = v4;
-      l4[c][Y][X] = v4;
-    }
-  }
-  if (pd.nscales < 6 || t >= 32) return;
-  __syncwarp();
-  const ScaleDesc s5 = pd.s[5];
-  const size_t np5 = (size_t)s5.w * s5.h;
-  if (t < 4) {
-    const int X = t % 2, Y = t / 2;
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      pyr[s5.off + c * np5 + (size_t)(ty * 2 + Y) * s5.w + tx * 2 + X] =
-          quad_mean(l4[c][2 * Y][2 * X], l4[c][2 * Y][2 * X + 1], l4[c][2 * Y + 1][2 * X], l4[c][2 * Y + 1][2 * X + 1]);
-  }
-}
-
-// Interior tile (tx, ty) from scale 0 in memory: each thread's 4x4 source block as 16-byte row loads.
-__device__ __forceinline__ void pyramid_tile_interior(const PyramidDesc& pd, float* __restrict__ pyr, int tx, int ty) {
-  const ScaleDesc s0 = pd.s[0];
-  const size_t np0 = (size_t)s0.w * s0.h;
-  const float* src0 = pyr + s0.off;
-  const int t = threadIdx.x, bx = t % 16, by = t / 16;
-  const int ox = tx * 32 + 2 * bx, oy = ty * 32 + 2 * by;
-  float v1[2][2][3];  // [row][column][channel]
-#pragma unroll
-  for (int r = 0; r < 2; r++) {
-    float4 a0[3], a1[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float4* p = reinterpret_cast<const float4*>(src0 + c * np0 + (size_t)(2 * (oy + r)) * s0.w + 2 * ox);
-      a0[c] = p[0];
-      a1[c] = p[s0.w / 4];
+      r[c][0] = rq[c].x;
+      r[c][1] = rq[c].y;
+      r[c][2] = rq[c].z;
+      r[c][3] = rq[c].w;
     }
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      v1[r][0][c] = quad_mean(a0[c].x, a0[c].y, a1[c].x, a1[c].y);
-      v1[r][1][c] = quad_mean(a0[c].z, a0[c].w, a1[c].z, a1[c].w);
-    }
-  }
-  pyramid_levels_interior(pd, pyr, tx, ty, v1);
-}
-
-__device__ __forceinline__ bool pyramid_fast_tile(const PyramidDesc& pd, const float* pyr, int tx, int ty) {
-  return (pd.s[0].w & 3) == 0 && ((uintptr_t)(pyr + pd.s[0].off) & 15) == 0 && pyramid_interior(pd, tx, ty);
-}
-
-// Tile (tx, ty) by the general path: scale 1 from scale 0 in memory, then each coarser level from the one above in
-// shared memory.
-template <bool kFresh>
-__device__ __forceinline__ void pyramid_tile_general(const PyramidDesc& pd, float* __restrict__ pyr, int tx, int ty) {
-  __shared__ float buf[2][3][kPyrTH][kPyrTW + 1];
-  const ScaleDesc s0 = pd.s[0], s1 = pd.s[1];
-  scale1_tile<kFresh>(pyr + s0.off, pyr + s1.off, s0, s1, tx, ty, buf[0]);
-  int cur = 0, tw = kPyrTW, th = kPyrTH;
-  for (int L = 2; L < pd.nscales; L++) {
-    __syncthreads();
-    const ScaleDesc a = pd.s[L - 1], b = pd.s[L];
-    const size_t npb = (size_t)b.w * b.h;
-    const int hw = tw / 2, hh = th / 2;
-    const int ax0 = tx * tw, ay0 = ty * th;  // tile origin at level L-1
-    for (int i = threadIdx.x; i < hw * hh; i += blockDim.x) {
-      int lx = i % hw, ly = i / hw;
-      int ox = tx * hw + lx, oy = ty * hh + ly;
-      if (ox < b.w && oy < b.h) {
-        // the 2x2 source block lies in this CTA's level L-1 tile; clip to level L-1's size like mean2x2
-        int x1 = min(ox * 2 + 2, a.w) - ax0, y1 = min(oy * 2 + 2, a.h) - ay0;
+    for (int k = 0; k < 2; k++) pix_diff2(at(r, 0, k), at(r, 1, k), at(r, 2, k), at(l, 0, k), at(l, 1, k), at(l, 2, k), o[k]);
+    put4(g.out + i, np, o);
+  } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          float sum = 0.0f, err = 0.0f;
-          for (int y = 2 * ly; y < y1; y++)
-            for (int x = 2 * lx; x < x1; x++) {
-              float e;
-              sum = two_sum(sum, buf[cur][c][y][x], e);
-              err += e;
-            }
-          float v = __fadd_rn(sum, err) * (1.0f / (float)((y1 - 2 * ly) * (x1 - 2 * lx)));
-          buf[cur ^ 1][c][ly][lx] = v;
-          pyr[b.off + c * npb + (size_t)oy * b.w + ox] = v;
-        }
-      }
-    }
-    cur ^= 1;
-    tw = hw;
-    th = hh;
-  }
-}
-
-// Scale-1 tile `blk` of a pyramid and every coarser tile below it.
-__device__ __forceinline__ void pyramid_tile(const PyramidDesc& pd, float* __restrict__ pyr, const int blk) {
-  const int tiles_x = (pd.s[1].w + kPyrTW - 1) / kPyrTW;
-  const int tx = blk % tiles_x, ty = blk / tiles_x;
-  if (pyramid_fast_tile(pd, pyr, tx, ty)) pyramid_tile_interior(pd, pyr, tx, ty);
-  else pyramid_tile_general<false>(pd, pyr, tx, ty);
-}
-
-__global__ void __launch_bounds__(256, 5) k_pyramid(const __grid_constant__ PyramidDesc pd, float* __restrict__ pyr,
-                                                 const StepDesc* __restrict__ st) {
-  if (st && !st->active) return;
-  pyramid_tile(pd, pyr, blockIdx.x);
-}
-
-// A search candidate's linear planes and pyramid in one pass, for the 4:2:0 layouts of upsample420.cuh. CTA = pyramid
-// tile (tx, ty): its threads upsample the tile's 64 x 64 block of scale 0 (thread t the 4 x 4 block at columns
-// tx * 64 + 4 (t % 16), rows ty * 64 + 4 (t / 16)), write it as scale 0 for the scorer, and, on an interior tile,
-// build scale 1 from the same registers: that 4 x 4 block is exactly the source of the thread's 2 x 2 block of scale
-// 1 in the pyramid's interior path, so scale 0 is never read back (the separate kernels wrote 144 MB at 12 MP and read
-// it back from DRAM). Edge tiles read their block back through L2 after a barrier and take the general path. The
-// planes are the same bits as the decoder's upsampling kernel followed by k_pyramid. Measured per 12 MP candidate:
-// 63.6 us converting the block as two 2-row halves, 61.0 us with all of its loads issued first (upsample_420_quad),
-// against 40.7 + 41.9 us for the two kernels; 72 us at 3 or 5 CTAs per SM.
-__global__ void __launch_bounds__(kPyrThreads, 4) k_upsample_pyramid(const StepDesc* __restrict__ st,
-                                                                    const uint8_t* __restrict__ planes, int w, int h,
-                                                                    const __grid_constant__ PyramidDesc pd,
-                                                                    float* __restrict__ pyr) {
-  if (!st->active) return;
-  __shared__ float lut[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = c_lut8s[i];
-  __syncthreads();
-  const int tiles_x = (pd.s[1].w + kPyrTW - 1) / kPyrTW;
-  const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
-  const int t = threadIdx.x, bx = t % 16, by = t / 16;
-  const int x0 = tx * 2 * kPyrTW + 4 * bx, j0 = ty * kPyrTH + 2 * by;  // columns x0.., chroma rows j0, j0 + 1
-  const size_t np0 = (size_t)w * h;
-  float* lin = pyr + pd.s[0].off;
-  const bool fast = pyramid_fast_tile(pd, pyr, tx, ty);
-  float v1[2][2][3];  // the interior path's scale-1 block: [row][column][channel]
-  if (x0 < w && 2 * j0 < h) {
-    float l[4][3][4];  // [row][channel][column]
-    upsample_420_quad(st, planes, w, h, lut, x0, j0, l);
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int y = 2 * j0 + r;
-      if (y >= h) break;
+    for (int k = 0; k < 2; k++) pix_xyb2(at(l, 0, k), at(l, 1, k), at(l, 2, k), o[k]);
+    put4(g.xyb + i, np, o);
+    if constexpr (kOut == kOutRef) {
 #pragma unroll
       for (int c = 0; c < 3; c++)
-        *reinterpret_cast<float4*>(lin + c * np0 + (size_t)y * w + x0) =
-            make_float4(l[r][c][0], l[r][c][1], l[r][c][2], l[r][c][3]);
-    }
-    if (fast) {
+        *reinterpret_cast<float4*>(g.out + c * np + i) = make_float4(l[c][0], l[c][1], l[c][2], l[c][3]);
+    } else {
 #pragma unroll
-      for (int r = 0; r < 2; r++)
+      for (int k = 0; k < 2; k++)
+        pix_diff2(at(l, 0, k), at(l, 1, k), at(l, 2, k), at(l2, 0, k), at(l2, 1, k), at(l2, 2, k), o[k]);
+      put4(g.out + i, np, o);
+    }
+  }
+}
+
+// The two samples of a row of the coarsest level's 2x2 block.
+template <int kOut>
+__device__ __forceinline__ void emit_pair(const BuildArgs& g, const ScaleDesc& sd, int x, int y, const float (&l)[3][4],
+                                          const float (&l2)[3][4]) {
+  const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
+  auto at = [](const float (&v)[3][4], int c) { return make_float2(v[c][0], v[c][1]); };
+  auto put2 = [&](float* p, const float2 (&v)[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) *reinterpret_cast<float2*>(p + c * np + i) = v[c];
+  };
+  float2 o[3];
+  if constexpr (kOut == kOutDiff) {
+    float2 r[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[c] = __ldg(reinterpret_cast<const float2*>(g.ref + c * np + i));
+    pix_diff2(r[0], r[1], r[2], at(l, 0), at(l, 1), at(l, 2), o);
+    put2(g.out, o);
+  } else {
+    pix_xyb2(at(l, 0), at(l, 1), at(l, 2), o);
+    put2(g.xyb, o);
+    if constexpr (kOut == kOutRef) {
+      const float2 v[3] = {at(l, 0), at(l, 1), at(l, 2)};
+      put2(g.out, v);
+    } else {
+      pix_diff2(at(l, 0), at(l, 1), at(l, 2), at(l2, 0), at(l2, 1), at(l2, 2), o);
+      put2(g.out, o);
+    }
+  }
+}
+
+// Block `blk` of a pyramid. Every thread of the CTA calls it.
+template <int kSrc, int kOut>
+__device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildArgs& g, const int blk) {
+  constexpr int kImgs = kOut == kOutPair ? 2 : 1;
+  __shared__ float lut[256];
+  __shared__ __align__(16) float lev[kImgs][3][kLevFloats];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if constexpr (kSrc != kFromLinear) {
+    lut[t] = c_lut8s[t];
+    __syncthreads();
+  }
+  const ScaleDesc s0 = pd.s[0];
+  const int w = s0.w, h = s0.h;
+  const int bx = (w + kPyrT - 1) / kPyrT, tx = blk % bx, ty = blk / bx;
+  const int quad = t & 15, x0 = tx * kPyrT + 4 * quad;
+  const bool lower = lane >= 16;  // the odd row of the warp's row pair
+#pragma unroll 1
+  for (int slab = 0; slab < kPyrT / 16; slab++) {
+    const int y = ty * kPyrT + slab * 16 + (t >> 4);
+    if (ty * kPyrT + slab * 16 >= h) break;
+    float l[kImgs][3][4];
+    if (x0 < w && y < h) {
+      float4 rq[3];
+      ref_quad<kOut>(g, s0, x0, y, rq);
+      if constexpr (kSrc == kFromPlanes) {
+        planes_quad(g.st, g.planes, w, h, lut, x0, y, l[0]);
+      } else if constexpr (kSrc == kFromLinear) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          v1[r][0][c] = quad_mean(l[2 * r][c][0], l[2 * r][c][1], l[2 * r + 1][c][0], l[2 * r + 1][c][1]);
-          v1[r][1][c] = quad_mean(l[2 * r][c][2], l[2 * r][c][3], l[2 * r + 1][c][2], l[2 * r + 1][c][3]);
+          const float4 q = *reinterpret_cast<const float4*>(g.out + s0.off + c * (size_t)s0.pitch * h +
+                                                            (size_t)y * s0.pitch + x0);
+          l[0][c][0] = q.x;
+          l[0][c][1] = q.y;
+          l[0][c][2] = q.z;
+          l[0][c][3] = q.w;
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < kImgs; m++) image_quad(g.im[m], x0, y, lut, l[m]);
+      }
+      emit_quad<kOut>(g, s0, x0, y, rq, l[0], l[kImgs - 1]);
+    }
+    // Scale 1: the upper half of the warp makes the quad's left sample, the lower half its right one.
+    if (pd.nscales > 1) {
+      const int col = x0 + (lower ? 2 : 0), top = y - (lower ? 1 : 0);
+#pragma unroll
+      for (int m = 0; m < kImgs; m++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float p0 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][0] : l[m][c][2], 16);
+          const float p1 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][1] : l[m][c][3], 16);
+          const float v = lower ? block_mean(p0, p1, l[m][c][2], l[m][c][3], col + 1 < w, top + 1 < h)
+                                : block_mean(l[m][c][0], l[m][c][1], p0, p1, col + 1 < w, top + 1 < h);
+          lev[m][c][(slab * 8 + warp) * lev_pitch(1) + 2 * quad + (lower ? 1 : 0)] = v;
         }
     }
   }
-  if (fast) {
-    pyramid_levels_interior(pd, pyr, tx, ty, v1);
-    return;
+  // Coarser levels, each from the one above in shared memory (level 1 is in place).
+#pragma unroll
+  for (int L = 2; L < kMaxScales; L++) {
+    __syncthreads();
+    if (L >= pd.nscales) break;
+    const int n = kPyrT >> L;
+    if (t < n * n) {
+      const int lx = t % n, ly = t / n;
+      const int ax = 2 * (tx * n + lx), ay = 2 * (ty * n + ly);  // the block's origin in the level above
+      const int aw = pd.s[L - 1].w, ah = pd.s[L - 1].h;
+      if (ax < aw && ay < ah) {
+#pragma unroll
+        for (int m = 0; m < kImgs; m++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            const float* q = &lev[m][c][lev_off(L - 1) + 2 * ly * lev_pitch(L - 1) + 2 * lx];
+            lev[m][c][lev_off(L) + ly * lev_pitch(L) + lx] =
+                block_mean(q[0], q[1], q[lev_pitch(L - 1)], q[lev_pitch(L - 1) + 1], ax + 1 < aw, ay + 1 < ah);
+          }
+      }
+    }
   }
-  __syncthreads();  // the tile's scale 0 is written; a block's global writes are visible to it after the barrier
-  pyramid_tile_general<true>(pd, pyr, tx, ty);
+  __syncthreads();
+  // Then written: the 256 quads of level 1, and in a second trip the 84 of levels 2-4 and the two pairs of level 5.
+#pragma unroll 1
+  for (int trip = 0; trip < 2; trip++) {
+    int L = 1, e = t;
+    if (trip) {
+      if (t >= 86) break;
+      L = t < 64 ? 2 : t < 80 ? 3 : t < 84 ? 4 : 5;
+      e = t - (L == 2 ? 0 : L == 3 ? 64 : L == 4 ? 80 : 84);
+    }
+    if (L >= pd.nscales) continue;
+    const ScaleDesc sd = pd.s[L];
+    const int n = kPyrT >> L, nq = L == 5 ? 1 : n / 4;  // quads of a row (level 5: half a quad)
+    const int lx = 4 * (e % nq), ly = e / nq;
+    const int x = tx * n + lx, y = ty * n + ly;
+    if (x >= sd.w || y >= sd.h) continue;
+    const int at = (L == 1 ? lev_off(1) : L == 2 ? lev_off(2) : L == 3 ? lev_off(3) : L == 4 ? lev_off(4) : lev_off(5)) +
+                   ly * (n + 4) + lx;
+    float l[kImgs][3][4];
+#pragma unroll
+    for (int m = 0; m < kImgs; m++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        // a row is padded by four samples, so the quad of a level-5 pair stays in its row
+        const float2 a = *reinterpret_cast<const float2*>(&lev[m][c][at]);
+        const float2 b = *reinterpret_cast<const float2*>(&lev[m][c][at + 2]);
+        l[m][c][0] = a.x;
+        l[m][c][1] = a.y;
+        l[m][c][2] = b.x;
+        l[m][c][3] = b.y;
+      }
+    if (L < 5) {
+      float4 rq[3];
+      ref_quad<kOut>(g, sd, x, y, rq);
+      emit_quad<kOut>(g, sd, x, y, rq, l[0], l[kImgs - 1]);
+    } else {
+      emit_pair<kOut>(g, sd, x, y, l[0], l[kImgs - 1]);
+    }
+  }
+}
+
+// CTAs per SM: a pair's conversion keeps two images' samples in registers.
+constexpr int build_ctas(int out) { return out == kOutPair ? 3 : 4; }
+
+template <int kSrc, int kOut>
+__global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const __grid_constant__ PyramidDesc pd,
+                                                                        const __grid_constant__ BuildArgs g,
+                                                                        const StepDesc* __restrict__ gate) {
+  if (gate && !gate->active) return;
+  build_block<kSrc, kOut>(pd, g, blockIdx.x);
 }
 
 // ------------------------------------------------------------------------------------------------ work-list scorer
 
 // Many (reference, distorted) pairs of any sizes scored together: one launch per stage over a work-list of every
-// pair's CTAs (linear planes, pyramid tiles, scorer tiles, reductions). Each stage's CTA finds its pair by a binary
-// search over the pairs' first-CTA indices; a pair with no CTAs in a stage has the same first index as the next
-// pair, and the search returns the last pair whose first index is <= the CTA's, so it is never chosen. Pairs that
-// name the same reference (same device pointer, size and format) share the first such pair's reference planes,
-// which are converted once.
+// pair's CTAs (pyramids, scorer tiles, reductions). Each stage's CTA finds its job by a binary search over the jobs'
+// first-CTA indices. Pairs that name the same reference (same device pointer, size and format) share one conversion of
+// it: such a reference is built first (linear and XYB), then its pairs' differences; a reference of one pair is built
+// with it, without linear planes.
 struct ScoreItem {
   PyramidDesc pd;
-  const uint8_t* img[2];  // reference, distorted (interleaved samples)
-  float* pyr[2];          // their pyramids (pyr[0] may be an earlier pair's)
-  int channels, depth;
-  int own_ref;            // 1: this pair converts its reference; 0: it reuses an earlier pair's planes
-  int lin_ctas;           // to_linear CTAs per image
-  int pyr_ctas;           // pyramid CTAs per image
-  long long lin0, pyr0, tile0;  // first CTA / tile of this pair in each stage (own reference first, then distorted)
-  long long part;         // first double of this pair's [18][total_tiles] partial sums
+  long long tile0;  // first tile of this pair
+  long long part;   // first double of this pair's [18][total_tiles] partial sums
+};
+
+// One pyramid (or pair of them) in a builder work-list.
+struct BuildJob {
+  PyramidDesc pd;
+  BuildArgs args;
 };
 
 // One scale of one pair in the tile work-list, with everything a tile needs resolved on the host.
 struct TileSeg {
-  const float* ref;   // channel 0 of this scale's planes
-  const float* dist;
+  const float* ref;   // channel 0 of this scale's XYB planes
+  const float* dist;  // and of its differences
   double* out;        // partial sums of the segment's first band; band k, sum i at out[i * stride + k]
-  int w, h, tiles_x;
+  int w, h, pitch, tiles_x;
   int nch;            // chunks per band
   int stride;         // bands of the pair (the sum-major stride of its partials)
 };
@@ -1172,40 +1062,18 @@ __device__ __forceinline__ int find_first(const long long* __restrict__ first, i
   return lo;
 }
 
-// Which image of the pair (0 reference, 1 distorted) and which CTA of it a stage's pair-local CTA index names.
-__device__ __forceinline__ int split_image(const ScoreItem& it, long long& local, int per_image) {
-  if (it.own_ref && local < per_image) return 0;
-  if (it.own_ref) local -= per_image;
-  return 1;
-}
-
-__global__ void __launch_bounds__(256) k_to_linear_batch(const ScoreItem* __restrict__ items,
-                                                         const long long* __restrict__ lin0, int n,
-                                                         const float* __restrict__ lut16) {
-  __shared__ float lut8[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) lut8[i] = c_lut8s[i];
-  __syncthreads();
-  const int i = find_first(lin0, n, blockIdx.x);
-  const ScoreItem& it = items[i];
-  long long local = (long long)blockIdx.x - it.lin0;
-  const int which = split_image(it, local, it.lin_ctas);
-  to_linear_groups(it.img[which], it.pd.s[0].w, it.pd.s[0].h, it.channels, it.depth, lut16, it.pyr[which],
-                   (size_t)local, lut8);
-}
-
-__global__ void __launch_bounds__(256, 5) k_pyramid_batch(const ScoreItem* __restrict__ items,
-                                                          const long long* __restrict__ pyr0, int n) {
-  const int i = find_first(pyr0, n, blockIdx.x);
-  const ScoreItem& it = items[i];
-  long long local = (long long)blockIdx.x - it.pyr0;
-  const int which = split_image(it, local, it.pyr_ctas);
-  pyramid_tile(it.pd, it.pyr[which], (int)local);
+template <int kOut>
+__global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build_batch(const BuildJob* __restrict__ jobs,
+                                                                              const long long* __restrict__ cta0, int n) {
+  const int i = find_first(cta0, n, blockIdx.x);
+  const BuildJob& j = jobs[i];
+  build_block<kFromImage, kOut>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
 }
 
 // One CTA per tile of the work-list. A persistent form (a fixed grid of k CTAs per SM striding over the list, each
 // CTA reusing its shared memory tile after tile) measured slower on 64 pairs of mixed sizes: 22.7 / 25.4 / 38.9 ms
 // at k = 3 / 2 / 1 against 21.1 ms here, because the block scheduler hands tiles to whichever CTA slot frees first.
-__global__ void __launch_bounds__(kTileThreads, 3)
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(kRefNone))
     k_ssim2_tiles_batch(const TileSeg* __restrict__ segs, const long long* __restrict__ seg0, int nseg) {
   const long long t = blockIdx.x;
   const int g = find_first(seg0, nseg, t);
@@ -1213,6 +1081,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
   ScaleDesc sd;
   sd.w = sg.w;
   sd.h = sg.h;
+  sd.pitch = sg.pitch;
   sd.tiles_x = sg.tiles_x;
   sd.tiles_y = 0;
   sd.tile0 = 0;
@@ -1240,15 +1109,22 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_batch(const ScoreItem* __r
 // The scoring half of one bisection step of every image of a lockstep batch (capi.cu): the candidate pyramids, the
 // tiles and the reductions, each one launch over a work-list of every image's CTAs; an image whose search has
 // finished skips through its StepDesc's `active`.
-__global__ void __launch_bounds__(256, 4) k_pyramid_lock(const LockItem* __restrict__ items, int n) {
+__global__ void __launch_bounds__(kPyrThreads, build_ctas(kOutDiff)) k_build_lock(const LockItem* __restrict__ items,
+                                                                                  int n) {
   const int i = lock_find<&LockItem::p0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   if (!it.st->active) return;
-  pyramid_tile(it.pd, it.dist_pyr, (int)((long long)blockIdx.x - it.p0));
+  BuildArgs g;
+  g.out = it.dist_pyr;
+  g.xyb = nullptr;
+  g.ref = it.ref_pyr;
+  g.planes = it.planes;
+  g.st = it.st;
+  build_block<kFromPlanes, kOutDiff>(it.pd, g, (int)((long long)blockIdx.x - it.p0));
 }
 
 template <int kRef>
-__global__ void __launch_bounds__(kTileThreads, 3) k_ssim2_tiles_lock(const LockItem* __restrict__ items, int n) {
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_lock(const LockItem* __restrict__ items, int n) {
   const int i = lock_find<&LockItem::t0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   if (!it.st->active) return;
@@ -1256,7 +1132,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_ssim2_tiles_lock(const Lock
   int s = 0;
   while (s + 1 < it.pd.nscales && blk >= it.pd.s[s + 1].tile0) s++;
   const ScaleDesc sd = it.pd.s[s];
-  ssim2_band<kRef>(sd, blk - sd.tile0, it.ref_pyr, it.dist_pyr, it.partials + blk, (size_t)it.pd.total_tiles,
+  ssim2_band<kRef>(sd, blk - sd.tile0, it.ref_xyb, it.dist_pyr, it.partials + blk, (size_t)it.pd.total_tiles,
                    it.refm);
 }
 
@@ -1268,47 +1144,78 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_lock(const LockItem* __res
 
 void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_total, long long t_total,
                      int max_scales, int ref_mode) {
-  if (p_total > 0) RCG_LAUNCH(ctx, "pyramid_lock", k_pyramid_lock, (unsigned)p_total, 256, 0, d_items, n);
+  RCG_LAUNCH(ctx, "build_lock", k_build_lock, (unsigned)p_total, kPyrThreads, 0, d_items, n);
   // Every image of the batch is at the same step: the first stores its reference moments, the later ones read them.
   if (ref_mode == kRefWrite)
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefWrite>, (unsigned)t_total, kTileThreads, kTileSmem,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefWrite>, (unsigned)t_total, kTileThreads,
+               tile_smem(kRefWrite),
                d_items, n);
   else if (ref_mode == kRefRead)
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefRead>, (unsigned)t_total, kTileThreads, kTileSmem,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefRead>, (unsigned)t_total, kTileThreads,
+               tile_smem(kRefRead),
                d_items, n);
   else
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefNone>, (unsigned)t_total, kTileThreads, kTileSmem,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefNone>, (unsigned)t_total, kTileThreads,
+               tile_smem(kRefNone),
                d_items, n);
   RCG_LAUNCH(ctx, "ssim2_reduce_lock", k_ssim2_reduce_lock, dim3(max_scales, kScoreSums, n), 256, 0, d_items);
 }
 
-int to_linear(rcg_ctx* ctx, const uint8_t* d_img, int w, int h, int channels, int depth, float* d_pyr) {
-  const float* lut16 = nullptr;
-  if (depth == 16 && channels != 2 && channels != 4) {
-    lut16 = srgb_lut16_device(ctx);
-    if (!lut16) return RCG_NO_MEMORY;
-  }
-  const long long groups = ((long long)w * h + 3) / 4;
-  RCG_LAUNCH(ctx, "to_linear", k_to_linear, (unsigned)((groups + 255) / 256), 256, 0, d_img, w, h, channels, depth,
-             lut16, d_pyr);
+// The source description of an image on the device; false: no memory for the 16-bit table.
+static bool image_src(rcg_ctx* ctx, const uint8_t* d_img, int w, int h, int channels, int depth, ImageSrc* im) {
+  *im = ImageSrc{d_img, w, h, channels, depth, nullptr};
+  if (depth != 16 || channels == 2 || channels == 4) return true;
+  im->lut16 = srgb_lut16_device(ctx);
+  return im->lut16 != nullptr;
+}
+
+int to_linear(rcg_ctx* ctx, const uint8_t* d_img, int w, int h, int pitch, int channels, int depth, float* d_lin) {
+  ImageSrc im;
+  if (!image_src(ctx, d_img, w, h, channels, depth, &im)) return RCG_NO_MEMORY;
+  const long long quads = (long long)((w + 3) / 4) * h;
+  RCG_LAUNCH(ctx, "to_linear", k_to_linear, (unsigned)((quads + 255) / 256), 256, 0, im, pitch, d_lin);
   return RCG_OK;
 }
 
-int build_pyramid_gated(rcg_ctx* ctx, const PyramidDesc& pd, float* d_pyr, const StepDesc* st) {
-  if (pd.nscales < 2) return RCG_OK;
-  RCG_LAUNCH(ctx, "pyramid", k_pyramid, pyramid_ctas(pd), kPyrThreads, 0, pd, d_pyr, st);
+int build_pair(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_ref, const uint8_t* d_dist, int channels, int depth,
+               float* d_xyb, float* d_diff) {
+  BuildArgs g = {};
+  if (!image_src(ctx, d_ref, pd.s[0].w, pd.s[0].h, channels, depth, &g.im[0]) ||
+      !image_src(ctx, d_dist, pd.s[0].w, pd.s[0].h, channels, depth, &g.im[1]))
+    return RCG_NO_MEMORY;
+  g.out = d_diff;
+  g.xyb = d_xyb;
+  RCG_LAUNCH(ctx, "build_pair", (k_build<kFromImage, kOutPair>), pyramid_ctas(pd), kPyrThreads, 0, pd, g, nullptr);
   return RCG_OK;
 }
 
-int build_pyramid(rcg_ctx* ctx, const PyramidDesc& pd, float* d_pyr) {
-  return build_pyramid_gated(ctx, pd, d_pyr, nullptr);
+int build_reference(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_img, int channels, float* d_lin, float* d_xyb) {
+  BuildArgs g = {};
+  if (!image_src(ctx, d_img, pd.s[0].w, pd.s[0].h, channels, 8, &g.im[0])) return RCG_NO_MEMORY;
+  g.out = d_lin;
+  g.xyb = d_xyb;
+  RCG_LAUNCH(ctx, "build_reference", (k_build<kFromImage, kOutRef>), pyramid_ctas(pd), kPyrThreads, 0, pd, g, nullptr);
+  return RCG_OK;
 }
 
-int upsample_pyramid(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, const PyramidDesc& pd,
-                     float* d_pyr) {
-  if (pd.nscales < 2) return upsample_color(ctx, d_step, d_planes, w, h, nullptr, d_pyr + pd.s[0].off);
-  RCG_LAUNCH(ctx, "upsample_pyramid", k_upsample_pyramid, pyramid_ctas(pd), kPyrThreads, 0, d_step, d_planes, w, h,
-             pd, d_pyr);
+int build_decoded(rcg_ctx* ctx, const PyramidDesc& pd, StepDesc* d_step, const uint8_t* d_planes, bool direct,
+                  float* d_out, float* d_xyb, const float* d_ref) {
+  BuildArgs g = {};
+  g.out = d_out;
+  g.xyb = d_xyb;
+  g.ref = d_ref;
+  g.planes = d_planes;
+  g.st = d_step;
+  const int ctas = pyramid_ctas(pd);
+  if (!direct) upsample_color(ctx, d_step, d_planes, pd.s[0].w, pd.s[0].h, nullptr, d_out, pd.s[0].pitch);
+  if (d_ref && direct)
+    RCG_LAUNCH(ctx, "build_diff", (k_build<kFromPlanes, kOutDiff>), ctas, kPyrThreads, 0, pd, g, d_step);
+  else if (d_ref)
+    RCG_LAUNCH(ctx, "build_diff", (k_build<kFromLinear, kOutDiff>), ctas, kPyrThreads, 0, pd, g, d_step);
+  else if (direct)
+    RCG_LAUNCH(ctx, "build_reference", (k_build<kFromPlanes, kOutRef>), ctas, kPyrThreads, 0, pd, g, d_step);
+  else
+    RCG_LAUNCH(ctx, "build_reference", (k_build<kFromLinear, kOutRef>), ctas, kPyrThreads, 0, pd, g, d_step);
   return RCG_OK;
 }
 
@@ -1322,6 +1229,7 @@ PyramidDesc make_pyramid(int w, int h) {
     ScaleDesc& sd = pd.s[s];
     sd.w = w;
     sd.h = h;
+    sd.pitch = (w + 3) / 4 * 4;
     sd.tiles_x = (w + kTileW - 1) / kTileW;
     sd.tiles_y = (h + kTileH - 1) / kTileH;
     sd.tile0 = tiles;
@@ -1329,7 +1237,7 @@ PyramidDesc make_pyramid(int w, int h) {
     sd.chunk0 = tiles;
     sd.off = off;
     tiles += sd.tiles_x * sd.tiles_y;
-    off += 3LL * w * h;
+    off += 3LL * sd.pitch * h;
     pd.nscales = s + 1;
     w = (w + 1) / 2;
     h = (h + 1) / 2;
@@ -1389,21 +1297,21 @@ static cudaError_t scorer_constants(int device) {
   if ((e = cudaMemcpyToSymbol(c_weights, W, sizeof c_weights)) != cudaSuccess) return e;
   if (int ce = codec_upload_lut(lut)) return (cudaError_t)ce;
   if ((e = cudaFuncSetAttribute(k_ssim2_tiles<kRefNone>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess ||
+                                (int)tile_smem(kRefNone))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_ssim2_tiles<kRefWrite>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess ||
+                                (int)tile_smem(kRefWrite))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_ssim2_tiles<kRefRead>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess)
+                                (int)tile_smem(kRefRead))) != cudaSuccess)
     return e;
   if ((e = cudaFuncSetAttribute(k_ssim2_tiles_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess)
+                                (int)tile_smem(kRefNone))) != cudaSuccess)
     return e;
   if ((e = cudaFuncSetAttribute(k_ssim2_tiles_lock<kRefNone>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess ||
+                                (int)tile_smem(kRefNone))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_ssim2_tiles_lock<kRefWrite>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess ||
+                                (int)tile_smem(kRefWrite))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_ssim2_tiles_lock<kRefRead>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kTileSmem)) != cudaSuccess)
+                                (int)tile_smem(kRefRead))) != cudaSuccess)
     return e;
   if (device >= 0 && device < 64) g_scorer_ready[device] = true;
   return cudaSuccess;
@@ -1485,7 +1393,7 @@ static int tune_bands(rcg_ctx* ctx, const PyramidDesc& pd) {
     float t = 1e30f;
     for (int rep = 0; rep < 4; rep++) {
       cudaEventRecord(a, ctx->stream);
-      k_ssim2_tiles<kRefNone><<<pb.total_tiles, kTileThreads, kTileSmem, ctx->stream>>>(pb, pyr, pyr + pd.floats,
+      k_ssim2_tiles<kRefNone><<<pb.total_tiles, kTileThreads, tile_smem(kRefNone), ctx->stream>>>(pb, pyr, pyr + pd.floats,
                                                                                         part, nullptr, nullptr);
       cudaEventRecord(b, ctx->stream);
       cudaEventSynchronize(b);
@@ -1538,13 +1446,13 @@ int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, cons
   unsigned* counter = (unsigned*)ctx->bufs["score_counter"].ptr;
   const PyramidDesc pb = plan_bands(ctx, pd);
   if (!refm || ref_mode == kRefNone)
-    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, pb.total_tiles, kTileThreads, kTileSmem, pb, d_ref, d_dist,
+    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, pb.total_tiles, kTileThreads, tile_smem(kRefNone), pb, d_ref, d_dist,
                partials, step, nullptr);
   else if (ref_mode == kRefWrite)
-    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, pb.total_tiles, kTileThreads, kTileSmem, pb, d_ref,
+    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, pb.total_tiles, kTileThreads, tile_smem(kRefWrite), pb, d_ref,
                d_dist, partials, step, refm);
   else
-    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, pb.total_tiles, kTileThreads, kTileSmem, pb, d_ref,
+    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, pb.total_tiles, kTileThreads, tile_smem(kRefRead), pb, d_ref,
                d_dist, partials, step, refm);
   dim3 rg(pb.nscales, kScoreSums);
   RCG_LAUNCH(ctx, "ssim2_reduce", k_ssim2_reduce, rg, 256, 0, pb, partials, scale_sums, counter, d_score, search,
@@ -1556,107 +1464,156 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
                 const uint32_t* widths, const uint32_t* heights, const int* channels, const int* depths,
                 double** d_scores) {
   std::vector<ScoreItem> items((size_t)n);
-  std::vector<long long> off_ref((size_t)n, -1), off_dist((size_t)n);
-  std::vector<int> ref_of((size_t)n);
   std::map<std::tuple<const uint8_t*, uint32_t, uint32_t, int, int>, int> first_ref;
-  long long lin = 0, pyr = 0, tiles = 0, parts = 0, floats = 0;
+  std::vector<int> ref_of((size_t)n), uses((size_t)n, 0);
+  long long tiles = 0, parts = 0, floats = 0;
   int max_scales = 1;
   bool need16 = false;
-  auto align64 = [](long long f) { return (f + 63) / 64 * 64; };  // 256-byte plane starts (vector stores)
   for (int i = 0; i < n; i++) {
     ScoreItem& it = items[(size_t)i];
     std::memset(&it, 0, sizeof it);
-    const int w = (int)widths[i], h = (int)heights[i];
-    it.pd = make_pyramid(w, h);
-    it.pd = plan_bands(ctx, it.pd);
-    it.img[0] = d_refs[i];
-    it.img[1] = d_dists[i];
-    it.channels = channels[i];
-    it.depth = depths ? depths[i] : 8;
-    auto key = std::make_tuple(d_refs[i], widths[i], heights[i], it.channels, it.depth);
-    auto found = first_ref.find(key);
-    it.own_ref = found == first_ref.end();
-    if (it.own_ref) {
-      first_ref.emplace(key, i);
-      ref_of[(size_t)i] = i;
-      off_ref[(size_t)i] = floats;
-      floats = align64(floats + it.pd.floats);
-    } else {
-      ref_of[(size_t)i] = found->second;
-    }
-    off_dist[(size_t)i] = floats;
-    floats = align64(floats + it.pd.floats);
-    const int copies = it.own_ref ? 2 : 1;
-    it.lin_ctas = (int)((((long long)w * h + 3) / 4 + 255) / 256);
-    it.pyr_ctas = pyramid_ctas(it.pd);
-    it.lin0 = lin;
-    lin += (long long)copies * it.lin_ctas;
-    it.pyr0 = pyr;
-    pyr += (long long)copies * it.pyr_ctas;
+    it.pd = plan_bands(ctx, make_pyramid((int)widths[i], (int)heights[i]));
+    const int depth = depths ? depths[i] : 8;
+    const auto found =
+        first_ref.emplace(std::make_tuple(d_refs[i], widths[i], heights[i], channels[i], depth), i).first;
+    ref_of[(size_t)i] = found->second;
+    uses[(size_t)found->second]++;
     it.tile0 = tiles;
     tiles += it.pd.total_tiles;
     it.part = parts;
     parts += (long long)kScoreSums * it.pd.total_tiles;
     max_scales = std::max(max_scales, it.pd.nscales);
-    need16 |= it.depth == 16 && it.channels != 2 && it.channels != 4;
+    need16 |= depth == 16 && channels[i] != 2 && channels[i] != 4;
   }
-  if (lin > INT32_MAX || pyr > INT32_MAX || tiles > INT32_MAX)
-    return fail(ctx, RCG_INVALID, "batch too large for one launch");
-  float* pyr_base = (float*)workspace(ctx, "batch_pyr", (size_t)floats * sizeof(float));
+  auto alloc = [&](const PyramidDesc& pd) {
+    const long long at = floats;
+    floats = (floats + pd.floats + 63) / 64 * 64;  // 256-byte plane starts (vector stores)
+    return at;
+  };
+  // Per pair the offsets of its reference's XYB and of its differences; per shared reference its linear pyramid.
+  std::vector<long long> off_xyb((size_t)n), off_lin((size_t)n, -1), off_diff((size_t)n);
+  for (int i = 0; i < n; i++) {
+    const int r = ref_of[(size_t)i];
+    if (r == i) {
+      off_xyb[(size_t)i] = alloc(items[(size_t)i].pd);
+      if (uses[(size_t)i] > 1) off_lin[(size_t)i] = alloc(items[(size_t)i].pd);
+    }
+    off_diff[(size_t)i] = alloc(items[(size_t)i].pd);
+  }
+  if (tiles > INT32_MAX) return fail(ctx, RCG_INVALID, "batch too large for one launch");
+  float* base = (float*)workspace(ctx, "batch_pyr", (size_t)floats * sizeof(float));
   double* partials = (double*)workspace(ctx, "batch_partials", (size_t)parts * sizeof(double));
   double* sums = (double*)workspace(ctx, "batch_sums", (size_t)n * kMaxScales * kScoreSums * sizeof(double));
   unsigned* counters = (unsigned*)workspace(ctx, "batch_counters", (size_t)n * sizeof(unsigned));
   double* scores = (double*)workspace(ctx, "batch_scores", (size_t)n * sizeof(double));
-  // The work-list in one upload: pairs, their first to_linear / pyramid CTAs, then the tile segments (one per
-  // pair and scale) and their first tiles.
+  const float* lut16 = need16 ? srgb_lut16_device(ctx) : nullptr;
+  if (!base || !partials || !sums || !counters || !scores || (need16 && !lut16)) return RCG_NO_MEMORY;
+  // Builder jobs in three lists: the shared references, their pairs' differences, the pairs of a reference of their own.
+  constexpr int kLists = 3;
+  std::vector<BuildJob> jobs[kLists];
+  std::vector<long long> first[kLists];
+  long long ctas[kLists] = {0, 0, 0};
+  auto add = [&](int list, int i, const BuildArgs& g) {
+    const PyramidDesc& pd = items[(size_t)i].pd;
+    jobs[list].push_back(BuildJob{pd, g});
+    first[list].push_back(ctas[list]);
+    ctas[list] += pyramid_ctas(pd);
+  };
+  for (int i = 0; i < n; i++) {
+    const int r = ref_of[(size_t)i], depth = depths ? depths[i] : 8, w = (int)widths[i], h = (int)heights[i];
+    const ImageSrc a = {d_refs[i], w, h, channels[i], depth, lut16}, b = {d_dists[i], w, h, channels[i], depth, lut16};
+    BuildArgs g = {};
+    if (uses[(size_t)r] == 1) {
+      g.im[0] = a;
+      g.im[1] = b;
+      g.xyb = base + off_xyb[(size_t)i];
+      g.out = base + off_diff[(size_t)i];
+      add(2, i, g);
+      continue;
+    }
+    if (r == i) {
+      g.im[0] = a;
+      g.xyb = base + off_xyb[(size_t)i];
+      g.out = base + off_lin[(size_t)i];
+      add(0, i, g);
+    }
+    g = {};
+    g.im[0] = b;
+    g.ref = base + off_lin[(size_t)r];
+    g.out = base + off_diff[(size_t)i];
+    add(1, i, g);
+  }
+  // The work-list in one upload: pairs, then the tile segments (one per pair and scale) and their first tiles, then the
+  // builder lists and their first CTAs.
   int nseg = 0;
   for (const ScoreItem& it : items) nseg += it.pd.nscales;
-  const size_t o_lin = (size_t)n * sizeof(ScoreItem), o_pyr = o_lin + (size_t)n * 8,
-               o_seg = o_pyr + (size_t)n * 8, o_seg0 = o_seg + (size_t)nseg * sizeof(TileSeg),
-               list_bytes = o_seg0 + (size_t)nseg * 8;
+  size_t list_bytes = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = list_bytes;
+    list_bytes = (list_bytes + bytes + 15) / 16 * 16;
+    return at;
+  };
+  const size_t o_items = place((size_t)n * sizeof(ScoreItem)), o_seg = place((size_t)nseg * sizeof(TileSeg)),
+               o_seg0 = place((size_t)nseg * 8);
+  size_t o_jobs[kLists], o_first[kLists];
+  for (int k = 0; k < kLists; k++) {
+    if (ctas[k] > INT32_MAX) return fail(ctx, RCG_INVALID, "batch too large for one launch");
+    o_jobs[k] = place(jobs[k].size() * sizeof(BuildJob));
+    o_first[k] = place(first[k].size() * 8);
+  }
   unsigned char* d_list = (unsigned char*)workspace(ctx, "batch_items", list_bytes);
-  const float* lut16 = need16 ? srgb_lut16_device(ctx) : nullptr;
-  if (!pyr_base || !partials || !sums || !counters || !scores || !d_list || (need16 && !lut16)) return RCG_NO_MEMORY;
+  if (!d_list) return RCG_NO_MEMORY;
   std::vector<unsigned char> list(list_bytes);
-  long long* lin0 = (long long*)(list.data() + o_lin);
-  long long* pyr0 = (long long*)(list.data() + o_pyr);
+  std::memcpy(list.data() + o_items, items.data(), (size_t)n * sizeof(ScoreItem));
+  for (int k = 0; k < kLists; k++) {
+    if (jobs[k].empty()) continue;
+    std::memcpy(list.data() + o_jobs[k], jobs[k].data(), jobs[k].size() * sizeof(BuildJob));
+    std::memcpy(list.data() + o_first[k], first[k].data(), first[k].size() * 8);
+  }
   TileSeg* segs = (TileSeg*)(list.data() + o_seg);
   long long* seg0 = (long long*)(list.data() + o_seg0);
-  int g = 0;
+  int gseg = 0;
   for (int i = 0; i < n; i++) {
-    ScoreItem& it = items[(size_t)i];
-    it.pyr[0] = pyr_base + off_ref[(size_t)ref_of[(size_t)i]];
-    it.pyr[1] = pyr_base + off_dist[(size_t)i];
-    lin0[i] = it.lin0;
-    pyr0[i] = it.pyr0;
-    for (int sc = 0; sc < it.pd.nscales; sc++, g++) {
+    const ScoreItem& it = items[(size_t)i];
+    for (int sc = 0; sc < it.pd.nscales; sc++, gseg++) {
       const ScaleDesc& sd = it.pd.s[sc];
-      segs[g].ref = it.pyr[0] + sd.off;
-      segs[g].dist = it.pyr[1] + sd.off;
-      segs[g].out = partials + it.part + sd.tile0;
-      segs[g].w = sd.w;
-      segs[g].h = sd.h;
-      segs[g].tiles_x = sd.tiles_x;
-      segs[g].nch = sd.nch;
-      segs[g].stride = it.pd.total_tiles;
-      seg0[g] = it.tile0 + sd.tile0;
+      TileSeg& sg = segs[gseg];
+      sg.ref = base + off_xyb[(size_t)ref_of[(size_t)i]] + sd.off;
+      sg.dist = base + off_diff[(size_t)i] + sd.off;
+      sg.out = partials + it.part + sd.tile0;
+      sg.w = sd.w;
+      sg.h = sd.h;
+      sg.pitch = sd.pitch;
+      sg.tiles_x = sd.tiles_x;
+      sg.nch = sd.nch;
+      sg.stride = it.pd.total_tiles;
+      seg0[gseg] = it.tile0 + sd.tile0;
     }
   }
-  std::memcpy(list.data(), items.data(), o_lin);
   cudaError_t e = cudaMemcpyAsync(d_list, list.data(), list_bytes, cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch work-list upload");
-  const ScoreItem* d_items = (const ScoreItem*)d_list;
-  const long long* d_lin0 = (const long long*)(d_list + o_lin);
-  const long long* d_pyr0 = (const long long*)(d_list + o_pyr);
+  const ScoreItem* d_items = (const ScoreItem*)(d_list + o_items);
   const TileSeg* d_segs = (const TileSeg*)(d_list + o_seg);
   const long long* d_seg0 = (const long long*)(d_list + o_seg0);
+  auto d_jobs = [&](int k) { return (const BuildJob*)(d_list + o_jobs[k]); };
+  auto d_first = [&](int k) { return (const long long*)(d_list + o_first[k]); };
+  int nj[kLists];
+  for (int k = 0; k < kLists; k++) nj[k] = (int)jobs[k].size();
   // The launches take only the work-list's totals and this context's buffers: a later batch with the same totals
   // replays them (its own pairs come in through the work-list uploaded above).
-  const std::vector<long long> key = {3, n, nseg, lin, pyr, tiles, max_scales, (long long)(uintptr_t)lut16};
+  const std::vector<long long> key = {3,     n,     nseg,    tiles,   max_scales, nj[0],
+                                      nj[1], nj[2], ctas[0], ctas[1], ctas[2]};
   int rc = run_step_loop(ctx, key, [&]() {
-    RCG_LAUNCH(ctx, "to_linear_batch", k_to_linear_batch, (unsigned)lin, 256, 0, d_items, d_lin0, n, lut16);
-    if (pyr > 0) RCG_LAUNCH(ctx, "pyramid_batch", k_pyramid_batch, (unsigned)pyr, 256, 0, d_items, d_pyr0, n);
-    RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, (unsigned)tiles, kTileThreads, kTileSmem, d_segs,
+    if (nj[0])
+      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutRef>, (unsigned)ctas[0], kPyrThreads, 0, d_jobs(0), d_first(0),
+                 nj[0]);
+    if (nj[1])
+      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutDiff>, (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1), d_first(1),
+                 nj[1]);
+    if (nj[2])
+      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutPair>, (unsigned)ctas[2], kPyrThreads, 0, d_jobs(2), d_first(2),
+                 nj[2]);
+    RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, (unsigned)tiles, kTileThreads, tile_smem(kRefNone), d_segs,
                d_seg0, nseg);
     RCG_LAUNCH(ctx, "ssim2_reduce_batch", k_ssim2_reduce_batch, dim3(max_scales, kScoreSums, n), 256, 0, d_items,
                partials, sums, counters, scores);
@@ -1672,13 +1629,13 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
 
 namespace rcg {
 
-// Fixed scratch of rcg_ssimulacra2_device_noalloc: both images' linear pyramids, the per-tile partial sums, the
+// Fixed scratch of rcg_ssimulacra2_device_noalloc: the reference's XYB pyramid and the differences, the per-tile partial sums, the
 // per-scale sums and the reduction's completion counter. Sized for images of at most kNoAllocMaxPixels pixels. CUDA
 // places a module's device arrays on a device when the module is first used there, so every device where any scorer
 // call has run holds it (about 10 MB) until the process exits. The per-device set-up below is cached for the life of
 // the process; a cudaDeviceReset invalidates it and is not supported.
 constexpr long long kNoAllocMaxPixels = 512LL * 512LL;
-constexpr long long kNoAllocPyrFloats = 1200000;  // one image: 3 channels x every scale, with margin
+constexpr long long kNoAllocPyrFloats = 1250000;  // one image: 3 channels x every scale in padded rows (at most 1,202,760)
 constexpr int kNoAllocMaxTiles = 4096;
 constexpr size_t kNoAllocPyrBytes = (size_t)kNoAllocPyrFloats * sizeof(float);
 constexpr size_t kNoAllocPartialOff = 2 * kNoAllocPyrBytes;
@@ -1744,15 +1701,13 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
     cudaGetLastError();
     return RCG_CUDA_ERROR;
   }
-  const unsigned lg = (unsigned)((((long long)w * h + 3) / 4 + 255) / 256);
-  k_to_linear<<<lg, 256, 0, s>>>(d_reference, w, h, channels, 8, nullptr, pyr_ref);
-  k_to_linear<<<lg, 256, 0, s>>>(d_distorted, w, h, channels, 8, nullptr, pyr_dist);
-  if (pd.nscales > 1) {
-    const int pg = pyramid_ctas(pd);
-    k_pyramid<<<pg, kPyrThreads, 0, s>>>(pd, pyr_ref, nullptr);
-    k_pyramid<<<pg, kPyrThreads, 0, s>>>(pd, pyr_dist, nullptr);
-  }
-  k_ssim2_tiles<kRefNone><<<pd.total_tiles, kTileThreads, kTileSmem, s>>>(pd, pyr_ref, pyr_dist, partials, nullptr,
+  BuildArgs g = {};
+  g.im[0] = ImageSrc{d_reference, w, h, channels, 8, nullptr};
+  g.im[1] = ImageSrc{d_distorted, w, h, channels, 8, nullptr};
+  g.xyb = pyr_ref;
+  g.out = pyr_dist;
+  k_build<kFromImage, kOutPair><<<pyramid_ctas(pd), kPyrThreads, 0, s>>>(pd, g, nullptr);
+  k_ssim2_tiles<kRefNone><<<pd.total_tiles, kTileThreads, tile_smem(kRefNone), s>>>(pd, pyr_ref, pyr_dist, partials, nullptr,
                                                                         nullptr);
   k_ssim2_reduce<<<dim3(pd.nscales, kScoreSums), 256, 0, s>>>(pd, partials, sums, counter, d_score, nullptr,
                                                               nullptr);
