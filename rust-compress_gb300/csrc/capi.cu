@@ -642,14 +642,14 @@ int rcg_ctx_set_ref_cache(rcg_ctx* ctx, int on) {
 int rcg_ctx_band_chunks(rcg_ctx* ctx, uint32_t width, uint32_t height) {
   if (!ctx || width < (uint32_t)kMinSide || height < (uint32_t)kMinSide) return 0;
   cudaSetDevice(ctx->device);
-  return band_chunks(ctx, make_pyramid((int)width, (int)height));
+  return band_chunks(ctx, make_pyramid((int)width, (int)height, 3));
 }
 
 // ---- scorer
 
 static int score_device_images(rcg_ctx* ctx, const uint8_t* d_ref, const uint8_t* d_dist, int w, int h, int channels,
                                int depth, double* score) {
-  PyramidDesc pd = make_pyramid(w, h);
+  PyramidDesc pd = make_pyramid(w, h, channels);
   float* ref_pyr = (float*)workspace(ctx, "ref_xyb", (size_t)pd.floats * sizeof(float));
   float* dist_pyr = (float*)workspace(ctx, "dist_pyr", (size_t)pd.floats * sizeof(float));
   double* d_score = (double*)workspace(ctx, "score", sizeof(double));
@@ -1211,7 +1211,7 @@ static int scorer_setup(rcg_ctx* ctx, int metric, int w, int h, int channels, Se
       return RCG_NO_MEMORY;
     return RCG_OK;
   }
-  sc->pd = make_pyramid(w, h);
+  sc->pd = make_pyramid(w, h, channels);
   sc->ref_pyr = (float*)workspace(ctx, "ref_pyr", (size_t)sc->pd.floats * sizeof(float));
   sc->ref_xyb = (float*)workspace(ctx, "ref_xyb", (size_t)sc->pd.floats * sizeof(float));
   sc->dist_pyr = (float*)workspace(ctx, "dist_pyr", (size_t)sc->pd.floats * sizeof(float));
@@ -1247,8 +1247,12 @@ static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st,
   float* lin = (float*)workspace(ctx, "x_lin", 6 * np * sizeof(float), false);
   if (!lin) return RCG_NO_MEMORY;
   const ScaleDesc& s0 = sc.pd.s[0];
-  cudaError_t e = cudaMemcpy2DAsync(lin, (size_t)w * sizeof(float), sc.ref_pyr + s0.off, (size_t)s0.pitch * sizeof(float),
-                                    (size_t)w * sizeof(float), (size_t)3 * h, cudaMemcpyDeviceToDevice, ctx->stream);
+  cudaError_t e = cudaSuccess;
+  for (int c = 0; c < 3 && e == cudaSuccess; c++)  // a gray reference's one plane three times
+    e = cudaMemcpy2DAsync(lin + c * np, (size_t)w * sizeof(float),
+                          sc.ref_pyr + s0.off + (s0.planes == 3 ? c : 0) * (size_t)s0.pitch * h,
+                          (size_t)s0.pitch * sizeof(float), (size_t)w * sizeof(float), (size_t)h, cudaMemcpyDeviceToDevice,
+                          ctx->stream);
   static const int kActive = 1;  // the later steps' tables cleared it; the next step's set it again
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&d_st->active, &kActive, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);

@@ -29,12 +29,13 @@ constexpr int kTileCtas = 4, kTileCtasRead = 6;  // per SM: the scorer's form wi
 
 // ------------------------------------------------------------------------------------------------ descriptors
 
-// One scale of the scorer's pyramid: planes are channel-planar f32, [3][h][pitch], at `off` (floats) in a pyramid
+// One scale of the scorer's pyramid: planes are channel-planar f32, [planes][h][pitch], at `off` (floats) in a pyramid
 // buffer. Rows are padded to whole 16-byte quads (pitch = w rounded up to 4), so every row of every width takes vector
 // loads and stores; the padding's values are never used.
 struct ScaleDesc {
   int w, h;
   int pitch;
+  int planes;  // 3, or 1 for gray images: linear light, or Y (X and B hold no difference between two gray images)
   int tiles_x, tiles_y;  // CTAs across and down (32-column bands of nch chunks of 32 rows; nch = 1: 32x32 tiles)
   int tile0;        // first CTA of this scale in the multi-scale launch
   int nch;          // 32-row chunks per CTA (ssim2.cu, ssim2_band)
@@ -302,7 +303,8 @@ void srgb_lut8(float out[256]);
 const float* srgb_lut16_device(rcg_ctx* ctx);
 
 // Pyramid geometry of the scorer for a w x h image (core/src/ssimulacra2.rs:480-490).
-PyramidDesc make_pyramid(int w, int h);
+// channels: of the image (1 and 2, gray and gray with alpha, give pyramids of one plane).
+PyramidDesc make_pyramid(int w, int h, int channels);
 
 // ---- scorer (ssim2.cu)
 // Upload the 8-bit LUT to constant memory once per device.

@@ -104,12 +104,18 @@ __device__ __forceinline__ float2 row2(float m0, float m1, float m2, float2 r, f
   return __ffma2_rn(two(m0), r, __ffma2_rn(two(m1), g, __fmul2_rn(two(m2), b)));
 }
 
-// The three opsin rows and the exact differences of rows, rounded once.
+// The three opsin rows and the exact differences of rows, rounded once. Every row sums to one, so a difference of rows
+// sums to zero: applied to (r, g, b) it is applied to (r - b, g - b) with its first two entries, which is exactly zero
+// for a gray pixel, as the difference of its cube roots is.
 constexpr float M00 = (float)kM00, M01 = (float)kM01, M02 = (float)kM02;
 constexpr float M10 = (float)kM10, M11 = (float)kM11, M12 = (float)kM12;
 constexpr float M20 = (float)kM20, M21 = (float)kM21, M22 = (float)kM22;
-constexpr float L20r = (float)(kM20 - kM00), L20g = (float)(kM21 - kM01), L20b = (float)(kM22 - kM02);
-constexpr float L21r = (float)(kM20 - kM10), L21g = (float)(kM21 - kM11), L21b = (float)(kM22 - kM12);
+constexpr float L20r = (float)(kM20 - kM00), L20g = (float)(kM21 - kM01);
+constexpr float L21r = (float)(kM20 - kM10), L21g = (float)(kM21 - kM11);
+
+__device__ __forceinline__ float2 diff_row2(float m0, float m1, float2 rb, float2 gb) {
+  return __ffma2_rn(two(m0), rb, __fmul2_rn(two(m1), gb));
+}
 
 // `a` of two pixels.
 __device__ __forceinline__ void pix_xyb2(float2 r, float2 g, float2 b, float2 (&a)[3]) {
@@ -118,8 +124,9 @@ __device__ __forceinline__ void pix_xyb2(float2 r, float2 g, float2 b, float2 (&
                c2 = cbrt2(row2(M20, M21, M22, r, g, b, bias));
   a[0] = __fmul2_rn(two(7.0f), div2(__fmul2_rn(two(0.07f), sub2(r, g)), dsq2(c0, c1)));
   a[1] = sub2(__fmul2_rn(two(0.5f), __fadd2_rn(c0, c1)), two(cbrt_fast(bias)));
-  a[2] = __fmul2_rn(two(0.5f), __fadd2_rn(div2(row2(L20r, L20g, L20b, r, g, b), dsq2(c2, c0)),
-                                          div2(row2(L21r, L21g, L21b, r, g, b), dsq2(c2, c1))));
+  const float2 rb = sub2(r, b), gb = sub2(g, b);
+  a[2] = __fmul2_rn(two(0.5f), __fadd2_rn(div2(diff_row2(L20r, L20g, rb, gb), dsq2(c2, c0)),
+                                          div2(diff_row2(L21r, L21g, rb, gb), dsq2(c2, c1))));
 }
 
 // `d` of two pixels. The quotient difference q_a/D_a - q_b/D_b of a row pair is formed without cancellation as
@@ -146,11 +153,28 @@ __device__ __forceinline__ void pix_diff2(float2 ra, float2 ga, float2 ba, float
   const float2 q01 = qd(__fmul2_rn(two(0.07f), sub2(gb, rb)), __fmul2_rn(two(0.07f), sub2(dr, dg)), ca0, cb0, dc0, s0, ca1,
                         cb1, dc1, s1);
   d[0] = __fmul2_rn(two(7.0f), q01);
-  const float2 q20 = qd(row2(-L20r, -L20g, -L20b, rb, gb, bb), row2(L20r, L20g, L20b, dr, dg, db), ca2, cb2, dc2, s2, ca0,
-                        cb0, dc0, s0);
-  const float2 q21 = qd(row2(-L21r, -L21g, -L21b, rb, gb, bb), row2(L21r, L21g, L21b, dr, dg, db), ca2, cb2, dc2, s2, ca1,
-                        cb1, dc1, s1);
+  const float2 rbb = sub2(rb, bb), gbb = sub2(gb, bb), drb = sub2(dr, db), dgb = sub2(dg, db);
+  const float2 q20 = qd(diff_row2(-L20r, -L20g, rbb, gbb), diff_row2(L20r, L20g, drb, dgb), ca2, cb2, dc2, s2, ca0, cb0, dc0,
+                        s0);
+  const float2 q21 = qd(diff_row2(-L21r, -L21g, rbb, gbb), diff_row2(L21r, L21g, drb, dgb), ca2, cb2, dc2, s2, ca1, cb1, dc1,
+                        s1);
   d[2] = __fmul2_rn(two(0.5f), __fadd2_rn(q20, q21));
+}
+
+// Gray pixels (r = g = b = l): X and B are constants without a difference between two gray images, which the conversions
+// above give as exact zeros, so a gray image has only its Y; the steps are theirs, so it scores as its RGB copy does.
+__device__ __forceinline__ float2 gray_root2(int row, float2 l) {
+  const float bias = (float)kBias;
+  return cbrt2(row ? row2(M10, M11, M12, l, l, l, bias) : row2(M00, M01, M02, l, l, l, bias));
+}
+__device__ __forceinline__ float2 gray_xyb2(float2 l) {
+  return sub2(__fmul2_rn(two(0.5f), __fadd2_rn(gray_root2(0, l), gray_root2(1, l))), two(cbrt_fast((float)kBias)));
+}
+__device__ __forceinline__ float2 gray_diff2(float2 la, float2 lb) {
+  const float2 d = sub2(la, lb);
+  const float2 dc0 = div2(row2(M00, M01, M02, d, d, d), dsq2(gray_root2(0, la), gray_root2(0, lb)));
+  const float2 dc1 = div2(row2(M10, M11, M12, d, d, d), dsq2(gray_root2(1, la), gray_root2(1, lb)));
+  return __fmul2_rn(two(0.5f), __fadd2_rn(dc0, dc1));
 }
 
 // Row index under the top/bottom mirror rule (core/src/ssimulacra2.rs:385-397); -1 for rows no valid output reads.
@@ -236,6 +260,8 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
   const int x0 = tx * kTileW, ybeg = ty * kTileH * nch;
   const int w = sd.w, h = sd.h, pitch = sd.pitch;
   const size_t np = (size_t)pitch * h;
+  // Channels to score: all, or Y alone (ScaleDesc::planes), which is then the only plane.
+  const int ch0 = sd.planes == 1 ? 1 : 0, ch1 = sd.planes == 1 ? 2 : 3;
   const float* pa = xa + sd.off;
   const float* pd = xd + sd.off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -272,8 +298,8 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
     return (unsigned)min(y0 + kTileH / 2, h - 1) * (unsigned)pitch + (unsigned)min(x0 + kTileW / 2, w - 1);
   };
   auto fetch = [&](int ch, int y0, float oa, float od) {
-    const float* ca = pa + ch * np;
-    const float* cd = pd + ch * np;
+    const float* ca = pa + (ch - ch0) * np;
+    const float* cd = pd + (ch - ch0) * np;
 #pragma unroll
     for (int it = 0; it < (kIH * kQuads + kTileThreads - 1) / kTileThreads; it++) {
       const int e = tid + it * kTileThreads;
@@ -297,7 +323,7 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
   };
 
   float oa = __ldg(pa + centre_of(ybeg)), od = __ldg(pd + centre_of(ybeg));
-  fetch(0, ybeg, oa, od);
+  fetch(ch0, ybeg, oa, od);
 #pragma unroll 1
   for (int chunk = 0; chunk < nrun; chunk++) {
     const int y0 = ybeg + chunk * kTileH;
@@ -308,21 +334,21 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
     if constexpr (kRef != kRefNone) rchunk = refm + (size_t)(sd.chunk0 + local * nch + chunk) * kRefChunk;
     if constexpr (kRef == kRefRead) {
       // 8 KB per channel (16-byte aligned, as the bulk prefetch requires: blocks are 24 KB apart from an aligned base).
-      if (tid < 3) {
+      if (tid >= ch0 && tid < ch1) {
         const float2* p = rchunk + tid * kTileH * kTileW;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(kTileH * kTileW * 8) : "memory");
       }
     }
 #pragma unroll 1
-    for (int ch = 0; ch < 3; ch++) {
+    for (int ch = ch0; ch < ch1; ch++) {
       // The next halo: the next channel's, or the next chunk's first.
-      const bool more = ch < 2 || chunk + 1 < nrun;
-      const int nch_ = ch < 2 ? ch + 1 : 0, ny0 = ch < 2 ? y0 : y0 + kTileH;
+      const bool same = ch + 1 < ch1, more = same || chunk + 1 < nrun;
+      const int nch_ = same ? ch + 1 : ch0, ny0 = same ? y0 : y0 + kTileH;
       float noa = 0.f, nod = 0.f;
       if (more) {
         const unsigned nc = centre_of(ny0);
-        noa = __ldg(pa + nch_ * np + nc);
-        nod = __ldg(pd + nch_ * np + nc);
+        noa = __ldg(pa + (nch_ - ch0) * np + nc);
+        nod = __ldg(pd + (nch_ - ch0) * np + nc);
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();  // this halo is in place; the previous vertical pass is done with hb
@@ -813,22 +839,38 @@ __device__ __forceinline__ void put4(float* __restrict__ p, size_t np, const flo
 }
 
 // The reference's linear samples of quad (x, y) of a scale (kOutDiff), asked for before the image's own are converted.
-template <int kOut>
+template <int kOut, bool kGray>
 __device__ __forceinline__ void ref_quad(const BuildArgs& g, const ScaleDesc& sd, int x, int y, float4 (&r)[3]) {
   if constexpr (kOut == kOutDiff) {
     const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
 #pragma unroll
-    for (int c = 0; c < 3; c++) r[c] = __ldg(reinterpret_cast<const float4*>(g.ref + c * np + i));
+    for (int c = 0; c < (kGray ? 1 : 3); c++) r[c] = __ldg(reinterpret_cast<const float4*>(g.ref + c * np + i));
   }
 }
 
 // Write quad (x, y) of a scale: l the linear samples of the image (kOutPair: of the first, l2 of the second), rq its
 // ref_quad.
-template <int kOut>
+template <int kOut, bool kGray>
 __device__ __forceinline__ void emit_quad(const BuildArgs& g, const ScaleDesc& sd, int x, int y, const float4 (&rq)[3],
                                           const float (&l)[3][4], const float (&l2)[3][4]) {
   const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
   auto at = [](const float (&v)[3][4], int c, int k) { return make_float2(v[c][2 * k], v[c][2 * k + 1]); };
+  if constexpr (kGray) {
+    auto put = [&](float* p, auto f) {
+      const float2 a = f(0), b = f(1);
+      *reinterpret_cast<float4*>(p + i) = make_float4(a.x, a.y, b.x, b.y);
+    };
+    if constexpr (kOut == kOutDiff) {
+      put(g.out, [&](int k) {
+        return gray_diff2(k ? make_float2(rq[0].z, rq[0].w) : make_float2(rq[0].x, rq[0].y), at(l, 0, k));
+      });
+    } else {
+      put(g.xyb, [&](int k) { return gray_xyb2(at(l, 0, k)); });
+      if constexpr (kOut == kOutRef) put(g.out, [&](int k) { return at(l, 0, k); });
+      else put(g.out, [&](int k) { return gray_diff2(at(l, 0, k), at(l2, 0, k)); });
+    }
+    return;
+  }
   float2 o[2][3];
   if constexpr (kOut == kOutDiff) {
     float r[3][4];
@@ -860,41 +902,43 @@ __device__ __forceinline__ void emit_quad(const BuildArgs& g, const ScaleDesc& s
 }
 
 // The two samples of a row of the coarsest level's 2x2 block.
-template <int kOut>
+template <int kOut, bool kGray>
 __device__ __forceinline__ void emit_pair(const BuildArgs& g, const ScaleDesc& sd, int x, int y, const float (&l)[3][4],
                                           const float (&l2)[3][4]) {
   const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
   auto at = [](const float (&v)[3][4], int c) { return make_float2(v[c][0], v[c][1]); };
   auto put2 = [&](float* p, const float2 (&v)[3]) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) *reinterpret_cast<float2*>(p + c * np + i) = v[c];
+    for (int c = 0; c < (kGray ? 1 : 3); c++) *reinterpret_cast<float2*>(p + c * np + i) = v[c];
   };
   float2 o[3];
   if constexpr (kOut == kOutDiff) {
     float2 r[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) r[c] = __ldg(reinterpret_cast<const float2*>(g.ref + c * np + i));
-    pix_diff2(r[0], r[1], r[2], at(l, 0), at(l, 1), at(l, 2), o);
+    for (int c = 0; c < (kGray ? 1 : 3); c++) r[c] = __ldg(reinterpret_cast<const float2*>(g.ref + c * np + i));
+    if constexpr (kGray) o[0] = gray_diff2(r[0], at(l, 0));
+    else pix_diff2(r[0], r[1], r[2], at(l, 0), at(l, 1), at(l, 2), o);
     put2(g.out, o);
   } else {
-    pix_xyb2(at(l, 0), at(l, 1), at(l, 2), o);
+    if constexpr (kGray) o[0] = gray_xyb2(at(l, 0));
+    else pix_xyb2(at(l, 0), at(l, 1), at(l, 2), o);
     put2(g.xyb, o);
     if constexpr (kOut == kOutRef) {
       const float2 v[3] = {at(l, 0), at(l, 1), at(l, 2)};
       put2(g.out, v);
     } else {
-      pix_diff2(at(l, 0), at(l, 1), at(l, 2), at(l2, 0), at(l2, 1), at(l2, 2), o);
+      if constexpr (kGray) o[0] = gray_diff2(at(l, 0), at(l2, 0));
+      else pix_diff2(at(l, 0), at(l, 1), at(l, 2), at(l2, 0), at(l2, 1), at(l2, 2), o);
       put2(g.out, o);
     }
   }
 }
 
 // Block `blk` of a pyramid. Every thread of the CTA calls it.
-template <int kSrc, int kOut>
-__device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildArgs& g, const int blk) {
-  constexpr int kImgs = kOut == kOutPair ? 2 : 1;
-  __shared__ float lut[256];
-  __shared__ __align__(16) float lev[kImgs][3][kLevFloats];
+template <int kSrc, int kOut, bool kGray>
+__device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildArgs& g, const int blk, float* lut,
+                                             float (*lev)[3][kLevFloats]) {
+  constexpr int kImgs = kOut == kOutPair ? 2 : 1, kCh = kGray ? 1 : 3;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if constexpr (kSrc != kFromLinear) {
     lut[t] = c_lut8s[t];
@@ -912,12 +956,12 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
     float l[kImgs][3][4];
     if (x0 < w && y < h) {
       float4 rq[3];
-      ref_quad<kOut>(g, s0, x0, y, rq);
+      ref_quad<kOut, kGray>(g, s0, x0, y, rq);
       if constexpr (kSrc == kFromPlanes) {
         planes_quad(g.st, g.planes, w, h, lut, x0, y, l[0]);
       } else if constexpr (kSrc == kFromLinear) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
+        for (int c = 0; c < kCh; c++) {
           const float4 q = *reinterpret_cast<const float4*>(g.out + s0.off + c * (size_t)s0.pitch * h +
                                                             (size_t)y * s0.pitch + x0);
           l[0][c][0] = q.x;
@@ -929,7 +973,7 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
 #pragma unroll
         for (int m = 0; m < kImgs; m++) image_quad(g.im[m], x0, y, lut, l[m]);
       }
-      emit_quad<kOut>(g, s0, x0, y, rq, l[0], l[kImgs - 1]);
+      emit_quad<kOut, kGray>(g, s0, x0, y, rq, l[0], l[kImgs - 1]);
     }
     // Scale 1: the upper half of the warp makes the quad's left sample, the lower half its right one.
     if (pd.nscales > 1) {
@@ -937,7 +981,7 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
 #pragma unroll
       for (int m = 0; m < kImgs; m++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
+        for (int c = 0; c < kCh; c++) {
           const float p0 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][0] : l[m][c][2], 16);
           const float p1 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][1] : l[m][c][3], 16);
           const float v = lower ? block_mean(p0, p1, l[m][c][2], l[m][c][3], col + 1 < w, top + 1 < h)
@@ -960,7 +1004,7 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
 #pragma unroll
         for (int m = 0; m < kImgs; m++)
 #pragma unroll
-          for (int c = 0; c < 3; c++) {
+          for (int c = 0; c < kCh; c++) {
             const float* q = &lev[m][c][lev_off(L - 1) + 2 * ly * lev_pitch(L - 1) + 2 * lx];
             lev[m][c][lev_off(L) + ly * lev_pitch(L) + lx] =
                 block_mean(q[0], q[1], q[lev_pitch(L - 1)], q[lev_pitch(L - 1) + 1], ax + 1 < aw, ay + 1 < ah);
@@ -990,7 +1034,7 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
 #pragma unroll
     for (int m = 0; m < kImgs; m++)
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < kCh; c++) {
         // a row is padded by four samples, so the quad of a level-5 pair stays in its row
         const float2 a = *reinterpret_cast<const float2*>(&lev[m][c][at]);
         const float2 b = *reinterpret_cast<const float2*>(&lev[m][c][at + 2]);
@@ -1001,23 +1045,44 @@ __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildAr
       }
     if (L < 5) {
       float4 rq[3];
-      ref_quad<kOut>(g, sd, x, y, rq);
-      emit_quad<kOut>(g, sd, x, y, rq, l[0], l[kImgs - 1]);
+      ref_quad<kOut, kGray>(g, sd, x, y, rq);
+      emit_quad<kOut, kGray>(g, sd, x, y, rq, l[0], l[kImgs - 1]);
     } else {
-      emit_pair<kOut>(g, sd, x, y, l[0], l[kImgs - 1]);
+      emit_pair<kOut, kGray>(g, sd, x, y, l[0], l[kImgs - 1]);
     }
   }
+}
+
+// Of either kind (the work-lists, whose images may be mixed).
+template <int kSrc, int kOut>
+__device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildArgs& g, const int blk) {
+  __shared__ float lut[256];
+  __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
+  if (pd.s[0].planes == 1) build_planes<kSrc, kOut, true>(pd, g, blk, lut, lev);
+  else build_planes<kSrc, kOut, false>(pd, g, blk, lut, lev);
 }
 
 // CTAs per SM: a pair's conversion keeps two images' samples in registers.
 constexpr int build_ctas(int out) { return out == kOutPair ? 3 : 4; }
 
-template <int kSrc, int kOut>
+template <int kSrc, int kOut, bool kGray>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const __grid_constant__ PyramidDesc pd,
                                                                         const __grid_constant__ BuildArgs g,
                                                                         const StepDesc* __restrict__ gate) {
   if (gate && !gate->active) return;
-  build_block<kSrc, kOut>(pd, g, blockIdx.x);
+  __shared__ float lut[256];
+  __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
+  build_planes<kSrc, kOut, kGray>(pd, g, blockIdx.x, lut, lev);
+}
+
+// Queue one builder launch (st: the step that gates it, nullable). Samples that come as linear planes are never gray
+// ones: a gray layout is always read directly.
+template <int kSrc, int kOut>
+void launch_build(const PyramidDesc& pd, const BuildArgs& g, const StepDesc* st, cudaStream_t stream) {
+  if (kSrc != kFromLinear && pd.s[0].planes == 1)
+    k_build<kSrc, kOut, kSrc != kFromLinear><<<pyramid_ctas(pd), kPyrThreads, 0, stream>>>(pd, g, st);
+  else
+    k_build<kSrc, kOut, false><<<pyramid_ctas(pd), kPyrThreads, 0, stream>>>(pd, g, st);
 }
 
 // ------------------------------------------------------------------------------------------------ work-list scorer
@@ -1044,7 +1109,7 @@ struct TileSeg {
   const float* ref;   // channel 0 of this scale's XYB planes
   const float* dist;  // and of its differences
   double* out;        // partial sums of the segment's first band; band k, sum i at out[i * stride + k]
-  int w, h, pitch, tiles_x;
+  int w, h, pitch, planes, tiles_x;
   int nch;            // chunks per band
   int stride;         // bands of the pair (the sum-major stride of its partials)
 };
@@ -1082,6 +1147,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRefNone))
   sd.w = sg.w;
   sd.h = sg.h;
   sd.pitch = sg.pitch;
+  sd.planes = sg.planes;
   sd.tiles_x = sg.tiles_x;
   sd.tiles_y = 0;
   sd.tile0 = 0;
@@ -1185,7 +1251,10 @@ int build_pair(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_ref, const 
     return RCG_NO_MEMORY;
   g.out = d_diff;
   g.xyb = d_xyb;
-  RCG_LAUNCH(ctx, "build_pair", (k_build<kFromImage, kOutPair>), pyramid_ctas(pd), kPyrThreads, 0, pd, g, nullptr);
+  cudaEvent_t ea, eb;
+  launch_begin(ctx, "build_pair", &ea, &eb);
+  launch_build<kFromImage, kOutPair>(pd, g, nullptr, ctx->stream);
+  launch_end(ctx, "build_pair", ea, eb);
   return RCG_OK;
 }
 
@@ -1194,7 +1263,10 @@ int build_reference(rcg_ctx* ctx, const PyramidDesc& pd, const uint8_t* d_img, i
   if (!image_src(ctx, d_img, pd.s[0].w, pd.s[0].h, channels, 8, &g.im[0])) return RCG_NO_MEMORY;
   g.out = d_lin;
   g.xyb = d_xyb;
-  RCG_LAUNCH(ctx, "build_reference", (k_build<kFromImage, kOutRef>), pyramid_ctas(pd), kPyrThreads, 0, pd, g, nullptr);
+  cudaEvent_t ea, eb;
+  launch_begin(ctx, "build_reference", &ea, &eb);
+  launch_build<kFromImage, kOutRef>(pd, g, nullptr, ctx->stream);
+  launch_end(ctx, "build_reference", ea, eb);
   return RCG_OK;
 }
 
@@ -1206,20 +1278,23 @@ int build_decoded(rcg_ctx* ctx, const PyramidDesc& pd, StepDesc* d_step, const u
   g.ref = d_ref;
   g.planes = d_planes;
   g.st = d_step;
-  const int ctas = pyramid_ctas(pd);
   if (!direct) upsample_color(ctx, d_step, d_planes, pd.s[0].w, pd.s[0].h, nullptr, d_out, pd.s[0].pitch);
+  const char* name = d_ref ? "build_diff" : "build_reference";
+  cudaEvent_t ea, eb;
+  launch_begin(ctx, name, &ea, &eb);
   if (d_ref && direct)
-    RCG_LAUNCH(ctx, "build_diff", (k_build<kFromPlanes, kOutDiff>), ctas, kPyrThreads, 0, pd, g, d_step);
+    launch_build<kFromPlanes, kOutDiff>(pd, g, d_step, ctx->stream);
   else if (d_ref)
-    RCG_LAUNCH(ctx, "build_diff", (k_build<kFromLinear, kOutDiff>), ctas, kPyrThreads, 0, pd, g, d_step);
+    launch_build<kFromLinear, kOutDiff>(pd, g, d_step, ctx->stream);
   else if (direct)
-    RCG_LAUNCH(ctx, "build_reference", (k_build<kFromPlanes, kOutRef>), ctas, kPyrThreads, 0, pd, g, d_step);
+    launch_build<kFromPlanes, kOutRef>(pd, g, d_step, ctx->stream);
   else
-    RCG_LAUNCH(ctx, "build_reference", (k_build<kFromLinear, kOutRef>), ctas, kPyrThreads, 0, pd, g, d_step);
+    launch_build<kFromLinear, kOutRef>(pd, g, d_step, ctx->stream);
+  launch_end(ctx, name, ea, eb);
   return RCG_OK;
 }
 
-PyramidDesc make_pyramid(int w, int h) {
+PyramidDesc make_pyramid(int w, int h, int channels) {
   PyramidDesc pd;
   std::memset(&pd, 0, sizeof pd);
   long long off = 0;
@@ -1230,6 +1305,7 @@ PyramidDesc make_pyramid(int w, int h) {
     sd.w = w;
     sd.h = h;
     sd.pitch = (w + 3) / 4 * 4;
+    sd.planes = channels <= 2 ? 1 : 3;
     sd.tiles_x = (w + kTileW - 1) / kTileW;
     sd.tiles_y = (h + kTileH - 1) / kTileH;
     sd.tile0 = tiles;
@@ -1237,7 +1313,7 @@ PyramidDesc make_pyramid(int w, int h) {
     sd.chunk0 = tiles;
     sd.off = off;
     tiles += sd.tiles_x * sd.tiles_y;
-    off += 3LL * sd.pitch * h;
+    off += (long long)sd.planes * sd.pitch * h;
     pd.nscales = s + 1;
     w = (w + 1) / 2;
     h = (h + 1) / 2;
@@ -1364,10 +1440,10 @@ __global__ void k_tune_fill(float* __restrict__ p, long long n) {
 static std::mutex g_band_mu;
 static std::map<std::pair<int, int>, int> g_band_choice;  // (device, size class) -> chunks per band
 
-// Size class: scale-0 tiles in half-octave steps.
+// Size class: scale-0 tiles in half-octave steps, gray images (one channel's work per tile) apart.
 static int band_class(const PyramidDesc& pd) {
   const double t = (double)pd.s[0].tiles_x * pd.s[0].tiles_y;
-  return (int)std::floor(2.0 * std::log2(std::max(1.0, t)));
+  return (int)std::floor(2.0 * std::log2(std::max(1.0, t))) + (pd.s[0].planes == 1 ? 1000 : 0);
 }
 
 // Time k_ssim2_tiles for each candidate on a stand-in pair of this geometry (own allocation, freed after); the
@@ -1472,7 +1548,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   for (int i = 0; i < n; i++) {
     ScoreItem& it = items[(size_t)i];
     std::memset(&it, 0, sizeof it);
-    it.pd = plan_bands(ctx, make_pyramid((int)widths[i], (int)heights[i]));
+    it.pd = plan_bands(ctx, make_pyramid((int)widths[i], (int)heights[i], channels[i]));
     const int depth = depths ? depths[i] : 8;
     const auto found =
         first_ref.emplace(std::make_tuple(d_refs[i], widths[i], heights[i], channels[i], depth), i).first;
@@ -1584,6 +1660,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
       sg.w = sd.w;
       sg.h = sd.h;
       sg.pitch = sd.pitch;
+      sg.planes = sd.planes;
       sg.tiles_x = sd.tiles_x;
       sg.nch = sd.nch;
       sg.stride = it.pd.total_tiles;
@@ -1685,7 +1762,7 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   if (width < (uint32_t)kMinSide || height < (uint32_t)kMinSide) return RCG_INVALID;
   if ((long long)width * (long long)height > kNoAllocMaxPixels) return RCG_INVALID;
   const int w = (int)width, h = (int)height;
-  PyramidDesc pd = make_pyramid(w, h);
+  PyramidDesc pd = make_pyramid(w, h, channels);
   if (pd.floats > kNoAllocPyrFloats || pd.total_tiles > kNoAllocMaxTiles) return RCG_INVALID;
   unsigned char* base = nullptr;
   int rc = noalloc_setup(&base);
@@ -1706,7 +1783,7 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   g.im[1] = ImageSrc{d_distorted, w, h, channels, 8, nullptr};
   g.xyb = pyr_ref;
   g.out = pyr_dist;
-  k_build<kFromImage, kOutPair><<<pyramid_ctas(pd), kPyrThreads, 0, s>>>(pd, g, nullptr);
+  launch_build<kFromImage, kOutPair>(pd, g, nullptr, s);
   k_ssim2_tiles<kRefNone><<<pd.total_tiles, kTileThreads, tile_smem(kRefNone), s>>>(pd, pyr_ref, pyr_dist, partials, nullptr,
                                                                         nullptr);
   k_ssim2_reduce<<<dim3(pd.nscales, kScoreSums), 256, 0, s>>>(pd, partials, sums, counter, d_score, nullptr,
