@@ -7,8 +7,14 @@
 // through the SSIM and edge maps to the moments and the XYB samples (one-sided derivatives at the max(., 0) and |.|
 // kinks); through the blurs (the zero-padded row blur is its own transpose, the mirrored column blur scatters
 // back); through XYB to linear light; plus the coarser scales' gradients spread back over their 2x2 blocks; and
-// finally through the sRGB curve. The blur intermediates are recomputed per scale in the backward pass, not kept
-// from the forward one. Plane kernels, one thread per sample, templated on the real type: FP64 (the checked
+// finally through the sRGB curve. Every scale and channel (up to 18 planes) goes through one launch per step, each CTA
+// finding its plane in a job table: the planes are independent in all steps but the pyramid and its adjoint, and most of
+// them are far too small to fill the GPU alone. Where their moments fit a budget they are kept from the forward pass for
+// the backward one, else the planes go in groups that are blurred again. Measured against one launch per plane (222 in
+// all, the moments blurred twice): FP64 768x512 4.9 -> 2.3 ms a call, 290x250 2.2 -> 0.6 (bound by the narrow FP64 pipe
+// then), FP32 inside a 1620x1080 perceptual search 2.1 -> 0.7 ms (memory). Row runs inside the row without their border
+// checks measured slower (their warps diverge at every row's ends). Plane kernels, templated on the real type: FP64 (the
+// checked
 // gradient: it matches the FP64 CPU gradient to rounding) and FP32 (the perceptual weights, where a few significant
 // digits suffice: the variances' cancellation error, ~1e-8, is small against the SSIM constant 9e-4 that bounds
 // every denominator, and GB300's FP32 rate is many times its FP64 rate). Sums of the maps are f64 across threads in
@@ -49,12 +55,46 @@ template <> __device__ __forceinline__ float tap<float>(int t) { return c_k32[t]
 __device__ __forceinline__ double cbrt_t(double x) { return cbrt(x); }
 __device__ __forceinline__ float cbrt_t(float x) { return cbrtf(x); }
 
+// x^0.4 = y + lo for x > 0, the fifth root of x^2 = a + ea: r = a^(-1/5) from an f32 seed by two steps of Newton's
+// iteration for the inverse root (r <- r (6 - a r^5) / 5; an error e becomes 3 e^2, 1e-6 -> 3e-12 -> 3e-23), then y = a
+// r^4 and one Newton step on y^5 = a + ea whose residual carries the rounding errors of a, y^2 and y^4, kept apart as lo.
+// About 30 FP64 operations where pow takes some two hundred; products formed with y and lo round once more, so the curve
+// below is within an ulp, as pow is. False for values outside the f32 range (those go to pow).
+__device__ __forceinline__ bool pow04(double x, double& a, double& ea, double& y, double& lo) {
+  a = x * x;
+  ea = fma(x, x, -a);
+  if (!(a > 1e-30 && a < 1e30)) return false;
+  const float l2 = log2f((float)a);
+  double r = (double)exp2f(-0.2f * l2);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const double r2 = r * r, r5 = r2 * r2 * r;
+    r = r * fma(-0.2 * a, r5, 1.2);
+  }
+  const double r2 = r * r, r4 = r2 * r2;
+  y = a * r4;
+  const double y2 = y * y, e2 = fma(y, y, -y2);
+  const double y4 = y2 * y2, e4 = fma(2.0 * y2, e2, fma(y2, y2, -y4));
+  lo = (fma(-y4, y, a) + fma(-e4, y, ea)) * 0.2 * r4;  // y = 1 / r, so 1 / (5 y^4) = r^4 / 5
+  // The curve's exponents 2.4 and 1.4 are f64 values, both 8.88e-17 below the decimals: x^-8.88e-17 = 1 - 8.88e-17 ln x.
+  lo = fma(y, -8.881784197001252e-17 * 0.34657359027997264 * (double)l2, lo);
+  return true;
+}
+
 __device__ __forceinline__ double srgb64(double v) {
-  return v <= 0.04045 ? v / 12.92 : pow((v + 0.055) / 1.055, 2.4);
+  if (v <= 0.04045) return v / 12.92;
+  const double x = (v + 0.055) / 1.055;
+  double a, ea, y, lo;
+  if (!pow04(x, a, ea, y, lo)) return pow(x, 2.4);
+  return fma(a, y, fma(a, lo, ea * y));
 }
 __device__ __forceinline__ double srgb64_deriv(double v255) {
   const double v = v255 / 255.0;
-  return v <= 0.04045 ? 1.0 / (12.92 * 255.0) : 2.4 * pow((v + 0.055) / 1.055, 1.4) / (1.055 * 255.0);
+  if (v <= 0.04045) return 1.0 / (12.92 * 255.0);
+  const double x = (v + 0.055) / 1.055;
+  double a, ea, y, lo;
+  const double p = pow04(x, a, ea, y, lo) ? fma(x, y, x * lo) : pow(x, 1.4);
+  return 2.4 * p / (1.055 * 255.0);
 }
 
 __device__ __forceinline__ long long tid1() { return (long long)blockIdx.x * blockDim.x + threadIdx.x; }
@@ -82,15 +122,37 @@ __global__ void k_lin(const uint8_t* __restrict__ ref, const float* __restrict__
     }
 }
 
-// 2x2 means (:225-247), fewer samples at odd edges; 3 channels.
-// Grid (output columns, rows, channels): see grid_rows.
+// One plane (a channel of a scale): its samples start at `x` in the buffers that hold a plane per channel (XYB, the
+// gradient), its five moments at `m`.
+struct AdjJob {
+  int w, h;
+  long long n, x, m;
+};
+constexpr int kMaxJobs = 3 * kMaxScales;
+// The planes of a launch and the first CTA of each (cta0[count] is the grid's size).
+struct AdjJobs {
+  int count;
+  unsigned cta0[kMaxJobs + 1];
+  AdjJob j[kMaxJobs];
+};
+
+__device__ __forceinline__ int job_of(const AdjJobs& jobs, unsigned cta) {
+  int k = 0;
+  while (k + 1 < jobs.count && cta >= jobs.cta0[k + 1]) k++;
+  return k;
+}
+
+// 2x2 means (:225-247), fewer samples at odd edges; 3 channels of both images (grid z).
+// Grid (output columns, rows, planes): see grid_rows.
 template <typename T>
-__global__ void k_down(const T* __restrict__ src, int w, int h, T* __restrict__ dst, int ow, int oh) {
+__global__ void k_down(const T* __restrict__ src_a, const T* __restrict__ src_b, int w, int h, T* __restrict__ dst_a,
+                       T* __restrict__ dst_b, int ow, int oh) {
   const int ox = blockIdx.x * blockDim.x + threadIdx.x;
   if (ox >= ow) return;
   const long long n = (long long)ow * oh;
-  const int c = blockIdx.z;
-  const T* p = src + (long long)c * w * h;
+  const int c = blockIdx.z % 3;
+  const T* p = (blockIdx.z < 3 ? src_a : src_b) + (long long)c * w * h;
+  T* dst = blockIdx.z < 3 ? dst_a : dst_b;
   const int x1 = min(2 * ox + 2, w);
   for (int oy = blockIdx.y; oy < oh; oy += gridDim.y) {
     const int y1 = min(2 * oy + 2, h);
@@ -101,13 +163,19 @@ __global__ void k_down(const T* __restrict__ src, int w, int h, T* __restrict__ 
   }
 }
 
-// XYB (:249-258) of 3 linear planes.
+// XYB (:249-258) of 3 linear planes: one job per scale (its first channel's), both images (grid y).
 template <typename T>
-__global__ void k_xyb(const T* __restrict__ lin, long long n, T* __restrict__ xyb) {
+__global__ void k_xyb(const __grid_constant__ AdjJobs jobs, const T* __restrict__ lin_a, const T* __restrict__ lin_b,
+                      T* __restrict__ xyb_a, T* __restrict__ xyb_b) {
+  const int job = job_of(jobs, blockIdx.x);
+  const long long n = jobs.j[job].n, i = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const T* lin = (blockIdx.y ? lin_b : lin_a) + jobs.j[job].x;
+  T* xyb = (blockIdx.y ? xyb_b : xyb_a) + jobs.j[job].x;
   const T M00 = (T)kM00, M01 = (T)kM01, M02 = (T)kM02, M10 = (T)kM10, M11 = (T)kM11, M12 = (T)kM12;
   const T M20 = (T)kM20, M21 = (T)kM21, M22 = (T)kM22, bias = (T)kBiasD;
   const T cb = cbrt_t(bias);
-  for (long long i = tid1(); i < n; i += (long long)gridDim.x * blockDim.x) {
+  {
     const T r = lin[i], g = lin[n + i], b = lin[2 * n + i];
     const T m0 = cbrt_t(fmax(M00 * r + M01 * g + M02 * b + bias, (T)0)) - cb;
     const T m1 = cbrt_t(fmax(M10 * r + M11 * g + M12 * b + bias, (T)0)) - cb;
@@ -119,51 +187,38 @@ __global__ void k_xyb(const T* __restrict__ lin, long long n, T* __restrict__ xy
   }
 }
 
-// The plane kernels below run on a (columns / 256, rows, planes) grid: a thread owns one column of one plane and
-// strides over the rows, so no sample index is divided back into (plane, row, column).
+// k_down's grid: a thread owns one column of one plane and strides over the rows.
 dim3 grid_rows(int w, int h, int planes) {
   return dim3((unsigned)((w + 255) / 256), (unsigned)std::min(h, 65535), (unsigned)planes);
 }
 
 // Outputs per thread of the row blurs: a run of kHRun consecutive outputs reads its kHRun + 10 source samples once
-// (in registers) instead of 11 per output; every output still sums its in-range taps in the same order.
+// (in registers) instead of 11 per output; every output still sums its in-range taps in the same order. A plane's runs
+// are numbered along its rows, so narrow planes fill their CTAs too.
 constexpr int kHRun = 4;
+__host__ __device__ inline long long row_runs(int w, int h) { return (long long)((w + kHRun - 1) / kHRun) * h; }
 
-// The row blurs' grid: (column runs / 256, rows, planes).
-dim3 grid_row_runs(int w, int h, int planes) {
-  return dim3((unsigned)(((w + kHRun - 1) / kHRun + 255) / 256), (unsigned)std::min(h, 65535), (unsigned)planes);
-}
-
-// Row blur (zero outside) of one plane: the backward pass's rows (the zero-padded row blur is its own transpose).
-// One plane per grid z.
+// Row blur (zero outside) of one run of a plane: the backward pass's rows (the zero-padded row blur is its own
+// transpose).
 template <typename T>
-__global__ void k_hblur(const T* __restrict__ src, int w, int h, T* __restrict__ dst) {
-  const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) * kHRun;
-  if (x0 >= w) return;
-  const long long n = (long long)w * h;
-  const T* sp = src + blockIdx.z * n;
-  T* dp = dst + blockIdx.z * n;
-  for (int y = blockIdx.y; y < h; y += gridDim.y) {
-    const T* row = sp + (long long)y * w;
-    T v[kHRun + 2 * kR];
+__device__ __forceinline__ void hblur_run(const T* __restrict__ row, int w, int x0, T (&out)[kHRun]) {
+  T v[kHRun + 2 * kR];
 #pragma unroll
-    for (int k = 0; k < kHRun + 2 * kR; k++) {
-      const int xx = x0 + k - kR;
-      v[k] = xx >= 0 && xx < w ? row[xx] : (T)0;
+  for (int k = 0; k < kHRun + 2 * kR; k++) {
+    const int xx = x0 + k - kR;
+    v[k] = xx >= 0 && xx < w ? row[xx] : (T)0;
+  }
+#pragma unroll
+  for (int o = 0; o < kHRun; o++) {
+    const int x = x0 + o;
+    T s = 0;
+#pragma unroll
+    for (int t = 0; t <= 2 * kR; t++) {
+      const int xx = x + t - kR;
+      if (xx < 0 || xx >= w) continue;
+      s += tap<T>(t) * v[o + t];
     }
-#pragma unroll
-    for (int o = 0; o < kHRun; o++) {
-      const int x = x0 + o;
-      if (x >= w) break;
-      T s = 0;
-#pragma unroll
-      for (int t = 0; t <= 2 * kR; t++) {
-        const int xx = x + t - kR;
-        if (xx < 0 || xx >= w) continue;
-        s += tap<T>(t) * v[o + t];
-      }
-      dp[(long long)y * w + x] = s;
-    }
+    out[o] = s;
   }
 }
 
@@ -196,12 +251,20 @@ __device__ __forceinline__ void store_run5(T* __restrict__ dst, long long n, lon
 // The five products of the forward pass blurred along rows in one sweep: dst + q * n for q = 0 xa, 1 xb, 2 xa^2,
 // 3 xb^2, 4 xa xb (each output summed over the taps in the same order as k_hblur).
 template <typename T>
-__global__ void k_hblur5(const T* __restrict__ xa, const T* __restrict__ xb, int w, int h, T* __restrict__ dst) {
-  const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) * kHRun;
-  if (x0 >= w) return;
-  const long long n = (long long)w * h;
-  for (int y = blockIdx.y; y < h; y += gridDim.y) {
-    const long long rowi = (long long)y * w;
+__global__ void __launch_bounds__(256) k_hblur5(const __grid_constant__ AdjJobs jobs, const T* __restrict__ xa_all,
+                                                const T* __restrict__ xb_all, T* __restrict__ dst_all) {
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const int w = J.w, h = J.h, runs = (w + kHRun - 1) / kHRun;
+  const long long n = J.n, e = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x;
+  const long long y = e / runs;
+  if (y >= h) return;
+  const int x0 = (int)(e - y * runs) * kHRun;
+  const T* xa = xa_all + J.x;
+  const T* xb = xb_all + J.x;
+  T* dst = dst_all + J.m;
+  {
+    const long long rowi = y * w;
     T va[kHRun + 2 * kR], vb[kHRun + 2 * kR];
 #pragma unroll
     for (int k = 0; k < kHRun + 2 * kR; k++) {
@@ -243,47 +306,53 @@ __device__ __forceinline__ int mirror64(int yy, int h) { return yy < 0 ? -yy - 1
 // 16 (0.94 against 1.18 ms per perceptual search at 12 MP with 8), its transpose runs of 8 (0.39 against 0.47 with 16).
 constexpr int kRunN = 16, kRun = 8;
 
-// Column blur with mirrored rows (:385-397), one plane per grid z, grid y over runs of kRunN rows.
+// Column blur with mirrored rows (:385-397) of a job's five planes (grid y); a CTA's threads take consecutive columns of
+// runs of kRunN rows, the runs one after another.
 template <typename T>
-__global__ void k_vblur_n(const T* __restrict__ src, int w, int h, T* __restrict__ dst) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= w) return;
-  const long long n = (long long)w * h;
-  const T* sp = src + blockIdx.z * n + x;
-  T* dp = dst + blockIdx.z * n + x;
-  const int runs = (h + kRunN - 1) / kRunN;
-  for (int r = blockIdx.y; r < runs; r += gridDim.y) {
-    const int y0 = r * kRunN;
-    T v[kRunN + 2 * kR];
+__global__ void __launch_bounds__(256) k_vblur_n(const __grid_constant__ AdjJobs jobs, const T* __restrict__ src,
+                                                 T* __restrict__ dst) {
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const int w = J.w, h = J.h;
+  const long long e = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x, r = e / w;
+  if (r >= (h + kRunN - 1) / kRunN) return;
+  const int x = (int)(e - r * w);
+  const T* sp = src + J.m + blockIdx.y * J.n + x;
+  T* dp = dst + J.m + blockIdx.y * J.n + x;
+  const int y0 = (int)r * kRunN;
+  T v[kRunN + 2 * kR];
 #pragma unroll
-    for (int k = 0; k < kRunN + 2 * kR; k++) {
-      const int yy = y0 + k - kR;
-      v[k] = yy <= h - 1 + kR ? sp[(long long)mirror64(yy, h) * w] : (T)0;  // rows past a short last run: unused
-    }
+  for (int k = 0; k < kRunN + 2 * kR; k++) {
+    const int yy = y0 + k - kR;
+    v[k] = yy <= h - 1 + kR ? sp[(long long)mirror64(yy, h) * w] : (T)0;  // rows past a short last run: unused
+  }
 #pragma unroll
-    for (int o = 0; o < kRunN; o++) {
-      if (y0 + o >= h) break;
-      T s = 0;
+  for (int o = 0; o < kRunN; o++) {
+    if (y0 + o >= h) break;
+    T s = 0;
 #pragma unroll
-      for (int t = 0; t <= 2 * kR; t++) s += tap<T>(t) * v[o + t];
-      dp[(long long)(y0 + o) * w] = s;
-    }
+    for (int t = 0; t <= 2 * kR; t++) s += tap<T>(t) * v[o + t];
+    dp[(long long)(y0 + o) * w] = s;
   }
 }
 
 // Transpose of the column blur as a gather: row y' receives tap t from the rows y whose mirrored source row is y', i.e.
 // from source index y' (y = y' - t + R), -y' - 1 (mirrored at the top) and 2h - 1 - y' (at the bottom).
-// One plane per grid z, grid y over runs of kRun rows; a run inside the interior reads its rows once.
+// A job's three gradient planes (grid y), threads as in k_vblur_n with runs of kRun rows; a run inside the interior reads
+// its rows once.
 template <typename T>
-__global__ void k_vblur_t(const T* __restrict__ gsrc, int w, int h, T* __restrict__ dst) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= w) return;
-  const long long n = (long long)w * h;
-  const T* g = gsrc + blockIdx.z * n;
-  T* dp = dst + blockIdx.z * n;
-  const int runs = (h + kRun - 1) / kRun;
-  for (int r = blockIdx.y; r < runs; r += gridDim.y) {
-    const int y0 = r * kRun;
+__global__ void __launch_bounds__(256) k_vblur_t(const __grid_constant__ AdjJobs jobs, const T* __restrict__ gsrc,
+                                                 T* __restrict__ dst) {
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const int w = J.w, h = J.h;
+  const long long e = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x, r = e / w;
+  if (r >= (h + kRun - 1) / kRun) return;
+  const int x = (int)(e - r * w);
+  const T* g = gsrc + J.m + blockIdx.y * J.n;
+  T* dp = dst + J.m + blockIdx.y * J.n;
+  {
+    const int y0 = (int)r * kRun;
     if (y0 >= kR && y0 + kRun - 1 < h - kR) {
       // every output row of the run is interior: row yp takes tap t from source row yp - t + kR
       T v[kRun + 2 * kR];
@@ -296,7 +365,7 @@ __global__ void k_vblur_t(const T* __restrict__ gsrc, int w, int h, T* __restric
         for (int t = 0; t <= 2 * kR; t++) s += tap<T>(t) * v[o + 2 * kR - t];
         dp[(long long)(y0 + o) * w + x] = s;
       }
-      continue;
+      return;
     }
     for (int yp = y0; yp < min(y0 + kRun, h); yp++) {
       T s = 0;
@@ -320,13 +389,22 @@ __global__ void k_vblur_t(const T* __restrict__ gsrc, int w, int h, T* __restric
 
 // The six map sums of one channel (:421-440): per-thread sums in T, then f64 per-CTA partials (parts[block][6]);
 // k_sum_parts adds them in a fixed order, so the score and the gradient are the same bits on every run.
+// One job's CTAs take its samples in turn.
 template <typename T>
-__global__ void __launch_bounds__(256) k_maps(const T* __restrict__ mom, const T* __restrict__ xa,
-                                              const T* __restrict__ xb, long long n, double* __restrict__ parts) {
+__global__ void __launch_bounds__(256) k_maps(const __grid_constant__ AdjJobs jobs, const T* __restrict__ mom_all,
+                                              const T* __restrict__ xa_all, const T* __restrict__ xb_all,
+                                              double* __restrict__ parts) {
   __shared__ double red[6][8];
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const long long n = J.n, first = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x,
+                  step = (long long)(jobs.cta0[job + 1] - jobs.cta0[job]) * blockDim.x;
+  const T* mom = mom_all + J.m;
+  const T* xa = xa_all + J.x;
+  const T* xb = xb_all + J.x;
   const T one = 1, c2 = (T)kC2;
   T acc[6] = {0, 0, 0, 0, 0, 0};
-  for (long long i = tid1(); i < n; i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = first; i < n; i += step) {
     const T m1 = mom[i], m2 = mom[n + i], s11 = mom[2 * n + i], s22 = mom[3 * n + i], s12 = mom[4 * n + i];
     const T num_m = one - (m1 - m2) * (m1 - m2);
     const T num_s = (T)2 * (s12 - m1 * m2) + c2;
@@ -358,10 +436,17 @@ __global__ void __launch_bounds__(256) k_maps(const T* __restrict__ mom, const T
   }
 }
 
-// sums[k] = the nparts partials of column k, one warp per column, lanes strided then a shuffle tree.
-__global__ void __launch_bounds__(192) k_sum_parts(const double* __restrict__ parts, int nparts,
-                                                   double* __restrict__ sums) {
+// sums[job][k] = the job's partials of column k, one CTA per job, one warp per column, lanes strided then a shuffle
+// tree. `at`: where each job's six sums go.
+struct AdjSums {
+  int at[kMaxJobs];
+};
+__global__ void __launch_bounds__(192) k_sum_parts(const __grid_constant__ AdjJobs jobs, const __grid_constant__ AdjSums to,
+                                                   const double* __restrict__ parts_all, double* __restrict__ sums_all) {
   const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* parts = parts_all + (size_t)jobs.cta0[blockIdx.x] * 6;
+  const int nparts = (int)(jobs.cta0[blockIdx.x + 1] - jobs.cta0[blockIdx.x]);
+  double* sums = sums_all + to.at[blockIdx.x];
   double v = 0.0;
   for (int i = lane; i < nparts; i += 32) v += parts[(size_t)i * 6 + k];
 #pragma unroll
@@ -375,11 +460,28 @@ __global__ void __launch_bounds__(192) k_sum_parts(const double* __restrict__ pa
 struct NormCoef {
   double g1[3], g4[3];
 };
+struct NormCoefs {
+  NormCoef job[kMaxJobs];
+};
 
+// The three moments' gradients go to the job's first three planes of gq.
 template <typename T>
-__global__ void k_mapgrad(const T* __restrict__ mom, const T* __restrict__ xa, const T* __restrict__ xb, long long n,
-                          NormCoef ncd, T* __restrict__ g_m2, T* __restrict__ g_s22, T* __restrict__ g_s12,
-                          T* __restrict__ g_xb) {
+__global__ void __launch_bounds__(256) k_mapgrad(const __grid_constant__ AdjJobs jobs,
+                                                 const __grid_constant__ NormCoefs coefs, const T* __restrict__ mom_all,
+                                                 const T* __restrict__ xa_all, const T* __restrict__ xb_all,
+                                                 T* __restrict__ gq, T* __restrict__ gx) {
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const NormCoef& ncd = coefs.job[job];
+  const long long n = J.n, i = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const T* mom = mom_all + J.m;
+  const T* xa = xa_all + J.x;
+  const T* xb = xb_all + J.x;
+  T* g_m2 = gq + J.m;
+  T* g_s22 = g_m2 + n;
+  T* g_s12 = g_s22 + n;
+  T* g_xb = gx + J.x;
   const T one = 1, two = 2, zero = 0, c2 = (T)kC2;
   T g1[3], g4[3];
 #pragma unroll
@@ -387,7 +489,7 @@ __global__ void k_mapgrad(const T* __restrict__ mom, const T* __restrict__ xa, c
     g1[m] = (T)ncd.g1[m];
     g4[m] = (T)ncd.g4[m];
   }
-  for (long long i = tid1(); i < n; i += (long long)gridDim.x * blockDim.x) {
+  {
     const T m1 = mom[i], m2 = mom[n + i], s11 = mom[2 * n + i], s22 = mom[3 * n + i], s12 = mom[4 * n + i];
     const T num_m = one - (m1 - m2) * (m1 - m2);
     const T num_s = two * (s12 - m1 * m2) + c2;
@@ -415,12 +517,27 @@ __global__ void k_mapgrad(const T* __restrict__ mom, const T* __restrict__ xa, c
   }
 }
 
-// d score / d xb = direct + G^T(g_m2) + 2 xb G^T(g_s22) + xa G^T(g_s12) for one channel.
+// d score / d xb = direct + G^T(g_m2) + 2 xb G^T(g_s22) + xa G^T(g_s12): the row blurs of a job's three planes (already
+// through the transposed column blur), combined where they are made. A thread takes one run of outputs.
 template <typename T>
-__global__ void k_combine(const T* __restrict__ t_m2, const T* __restrict__ t_s22, const T* __restrict__ t_s12,
-                          const T* __restrict__ xa, const T* __restrict__ xb, long long n, T* __restrict__ g_xb) {
-  for (long long i = tid1(); i < n; i += (long long)gridDim.x * blockDim.x)
-    g_xb[i] += t_m2[i] + (T)2 * xb[i] * t_s22[i] + xa[i] * t_s12[i];
+__global__ void __launch_bounds__(256) k_hblur_combine(const __grid_constant__ AdjJobs jobs, const T* __restrict__ src,
+                                                       const T* __restrict__ xa_all, const T* __restrict__ xb_all,
+                                                       T* __restrict__ gx) {
+  const int job = job_of(jobs, blockIdx.x);
+  const AdjJob& J = jobs.j[job];
+  const int w = J.w, runs = (w + kHRun - 1) / kHRun;
+  const long long n = J.n, e = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x, y = e / runs;
+  if (y >= J.h) return;
+  const int x0 = (int)(e - y * runs) * kHRun;
+  const T* row = src + J.m + y * w;
+  T t_m2[kHRun], t_s22[kHRun], t_s12[kHRun];
+  hblur_run(row, w, x0, t_m2);
+  hblur_run(row + n, w, x0, t_s22);
+  hblur_run(row + 2 * n, w, x0, t_s12);
+  const long long i0 = J.x + y * w + x0;
+#pragma unroll
+  for (int o = 0; o < kHRun; o++)
+    if (x0 + o < w) gx[i0 + o] += t_m2[o] + (T)2 * xb_all[i0 + o] * t_s22[o] + xa_all[i0 + o] * t_s12[o];
 }
 
 // XYB adjoint to the linear planes of this scale, plus the coarser scale's gradient spread over its 2x2 blocks.
@@ -476,6 +593,10 @@ unsigned grid_of(long long n) {
   return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152 * 32));
 }
 
+// Moments of planes blurred together: their two buffers of five planes each stay within this (320 bytes a pixel in FP64:
+// images of up to 80 MP go as one group, in FP32 of up to 160 MP).
+constexpr long long kAdjBudgetBytes = 24ll << 30;
+
 // The whole pass in real type T; workspace buffers are named per type.
 template <typename T>
 int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, int h, double* score, double* d_grad) {
@@ -520,44 +641,83 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
   const int ns = (int)sc.size();
   if (ns == 0) return fail(ctx, RCG_INVALID, "SSIMULACRA 2 needs at least 8x8 pixels");
   const long long n0 = sc[0].n;
+  // Every channel of every scale, and the groups of them that go through the blurs together: all, when their moments
+  // (ten planes each, of which five are kept for the backward pass) fit the budget.
+  struct Plane {
+    int s, c;
+  };
+  std::vector<std::vector<Plane>> groups;
+  const long long budget = std::max<long long>(5 * n0, kAdjBudgetBytes / (2 * (long long)sizeof(T)));
+  long long used = 0, most = 0;
+  for (int s = 0; s < ns; s++)
+    for (int c = 0; c < 3; c++) {
+      if (groups.empty() || used + 5 * sc[s].n > budget) {
+        groups.emplace_back();
+        used = 0;
+      }
+      groups.back().push_back({s, c});
+      used += 5 * sc[s].n;
+      most = std::max(most, used);
+    }
+  const bool keep = groups.size() == 1;
   T* pa = ws("pa", total);
   T* pb = ws("pb", total);
-  T* xa = ws("xa", 3 * n0);
-  T* xb = ws("xb", 3 * n0);
-  T* hb5 = ws("hb5", 5 * n0);  // row-blurred products (forward), column-blurred gradients (backward)
-  T* mom = ws("mom", 5 * n0);
-  T* gq = ws("gq", 3 * n0);  // g_m2, g_s22, g_s12
-  T* tq = ws("tq", 3 * n0);  // their blur adjoints
-  T* gx = ws("gx", 3 * n0);  // d score / d xb
-  T* gl = ws("gl", total);   // d score / d linear, per scale
-  double* sums = (double*)workspace(ctx, (pfx + "sums").c_str(), sizeof(double) * kMaxScales * 18);
-  double* parts = (double*)workspace(ctx, (pfx + "parts").c_str(), sizeof(double) * 6 * grid_of(n0));
-  if (!pa || !pb || !xa || !xb || !hb5 || !mom || !gq || !tq || !gx || !gl || !sums || !parts)
-    return RCG_NO_MEMORY;
-  RCG_LAUNCH(ctx, "adj_lin", k_lin<T>, grid_of(n0), 256, 0, d_ref, d_dist, n0, pa, pb);
-  for (int s = 1; s < ns; s++) {
-    RCG_LAUNCH(ctx, "adj_down", k_down<T>, grid_rows(sc[s].w, sc[s].h, 3), 256, 0, pa + sc[s - 1].off, sc[s - 1].w,
-               sc[s - 1].h, pa + sc[s].off, sc[s].w, sc[s].h);
-    RCG_LAUNCH(ctx, "adj_down", k_down<T>, grid_rows(sc[s].w, sc[s].h, 3), 256, 0, pb + sc[s - 1].off, sc[s - 1].w,
-               sc[s - 1].h, pb + sc[s].off, sc[s].w, sc[s].h);
-  }
-  // forward: the moments and map sums of every scale
-  auto moments = [&](int s, int c) {
-    const long long n = sc[s].n;
-    RCG_LAUNCH(ctx, "adj_hblur5", k_hblur5<T>, grid_row_runs(sc[s].w, sc[s].h, 1), 256, 0, xa + c * n, xb + c * n,
-               sc[s].w, sc[s].h, hb5);
-    RCG_LAUNCH(ctx, "adj_vblur", k_vblur_n<T>, grid_rows(sc[s].w, (sc[s].h + kRunN - 1) / kRunN, 5), 256, 0, hb5,
-               sc[s].w, sc[s].h, mom);
-  };
-  for (int s = 0; s < ns; s++) {
-    const long long n = sc[s].n;
-    RCG_LAUNCH(ctx, "adj_xyb", k_xyb<T>, grid_of(n), 256, 0, pa + sc[s].off, n, xa);
-    RCG_LAUNCH(ctx, "adj_xyb", k_xyb<T>, grid_of(n), 256, 0, pb + sc[s].off, n, xb);
-    for (int c = 0; c < 3; c++) {
-      moments(s, c);
-      RCG_LAUNCH(ctx, "adj_maps", k_maps<T>, grid_of(n), 256, 0, mom, xa + c * n, xb + c * n, n, parts);
-      RCG_LAUNCH(ctx, "adj_sum_parts", k_sum_parts, 1, 192, 0, parts, (int)grid_of(n), sums + s * 18 + c * 6);
+  T* xa = ws("xa", total);
+  T* xb = ws("xb", total);
+  T* hb5 = ws("hb5", most);  // row-blurred products; the gradients of the moments
+  T* mom = ws("mom", most);  // moments; the gradients through the transposed column blur
+  T* gx = ws("gx", total);   // d score / d xb
+  T* gl = ws("gl", total);   // d score / d linear
+  // The jobs of a group with `ctas` CTAs each (by plane size).
+  auto jobs_of = [&](const std::vector<Plane>& g, auto ctas) {
+    AdjJobs jobs;
+    std::memset(&jobs, 0, sizeof jobs);
+    long long m = 0, at = 0;
+    for (const Plane& p : g) {
+      AdjJob& j = jobs.j[jobs.count];
+      j = AdjJob{sc[p.s].w, sc[p.s].h, sc[p.s].n, sc[p.s].off + p.c * sc[p.s].n, m};
+      m += 5 * j.n;
+      jobs.cta0[jobs.count++] = (unsigned)at;
+      at += (long long)ctas(j);
     }
+    jobs.cta0[jobs.count] = (unsigned)at;
+    return jobs;
+  };
+  auto grid = [](const AdjJobs& j) { return j.cta0[j.count]; };
+  auto by_samples = [](const AdjJob& j) { return (j.n + 255) / 256; };
+  auto by_row_runs = [](const AdjJob& j) { return (row_runs(j.w, j.h) + 255) / 256; };
+  auto by_runs = [](int rows) {
+    return [rows](const AdjJob& j) { return ((long long)((j.h + rows - 1) / rows) * j.w + 255) / 256; };
+  };
+  auto by_grid = [](const AdjJob& j) { return (long long)grid_of(j.n); };
+  size_t max_parts = 0;
+  for (const auto& g : groups) max_parts = std::max<size_t>(max_parts, grid(jobs_of(g, by_grid)));
+  double* sums = (double*)workspace(ctx, (pfx + "sums").c_str(), sizeof(double) * kMaxScales * 18);
+  double* parts = (double*)workspace(ctx, (pfx + "parts").c_str(), sizeof(double) * 6 * max_parts);
+  if (!pa || !pb || !xa || !xb || !hb5 || !mom || !gx || !gl || !sums || !parts) return RCG_NO_MEMORY;
+  RCG_LAUNCH(ctx, "adj_lin", k_lin<T>, grid_of(n0), 256, 0, d_ref, d_dist, n0, pa, pb);
+  for (int s = 1; s < ns; s++)
+    RCG_LAUNCH(ctx, "adj_down", k_down<T>, grid_rows(sc[s].w, sc[s].h, 6), 256, 0, pa + sc[s - 1].off,
+               pb + sc[s - 1].off, sc[s - 1].w, sc[s - 1].h, pa + sc[s].off, pb + sc[s].off, sc[s].w, sc[s].h);
+  {
+    std::vector<Plane> first;  // a scale's three channels go by its first
+    for (int s = 0; s < ns; s++) first.push_back({s, 0});
+    const AdjJobs jobs = jobs_of(first, by_samples);
+    RCG_LAUNCH(ctx, "adj_xyb", k_xyb<T>, dim3(grid(jobs), 2), 256, 0, jobs, pa, pb, xa, xb);
+  }
+  // forward: the moments and map sums of every plane
+  auto moments = [&](const std::vector<Plane>& g) {
+    const AdjJobs rows = jobs_of(g, by_row_runs), cols = jobs_of(g, by_runs(kRunN));
+    RCG_LAUNCH(ctx, "adj_hblur5", k_hblur5<T>, grid(rows), 256, 0, rows, xa, xb, hb5);
+    RCG_LAUNCH(ctx, "adj_vblur", k_vblur_n<T>, dim3(grid(cols), 5), 256, 0, cols, hb5, mom);
+  };
+  for (const auto& g : groups) {
+    moments(g);
+    const AdjJobs jobs = jobs_of(g, by_grid);
+    AdjSums to;
+    for (size_t k = 0; k < g.size(); k++) to.at[k] = g[k].s * 18 + g[k].c * 6;
+    RCG_LAUNCH(ctx, "adj_maps", k_maps<T>, grid(jobs), 256, 0, jobs, mom, xa, xb, parts);
+    RCG_LAUNCH(ctx, "adj_sum_parts", k_sum_parts, (unsigned)g.size(), 192, 0, jobs, to, parts, sums);
   }
   double hs[kMaxScales * 18];
   cudaMemcpyAsync(hs, sums, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
@@ -597,32 +757,29 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
   const double dsum = -10.0 * ex * std::pow(P, ex - 1.0) *
                       (2.326765642916932 - 2.0 * 0.020884521182843837 * q + 3.0 * 6.248496625763138e-05 * q * q) *
                       kq;
-  // backward, coarsest scale first
-  for (int s = ns - 1; s >= 0; s--) {
-    const long long n = sc[s].n;
-    const double count = (double)n;
-    RCG_LAUNCH(ctx, "adj_xyb", k_xyb<T>, grid_of(n), 256, 0, pa + sc[s].off, n, xa);
-    RCG_LAUNCH(ctx, "adj_xyb", k_xyb<T>, grid_of(n), 256, 0, pb + sc[s].off, n, xb);
-    for (int c = 0; c < 3; c++) {
-      NormCoef nc;
+  // backward: d score / d xb of every plane, then to linear light from the coarsest scale to the finest
+  for (const auto& g : groups) {
+    if (!keep) moments(g);
+    NormCoefs coefs;
+    std::memset(&coefs, 0, sizeof coefs);
+    for (size_t k = 0; k < g.size(); k++) {
+      const int s = g[k].s, c = g[k].c;
+      const double count = (double)sc[s].n;
       for (int m = 0; m < 3; m++) {
-        nc.g1[m] = dsum * wst[s][c][2 * m] / count;
+        coefs.job[k].g1[m] = dsum * wst[s][c][2 * m] / count;
         const double mean4 = hs[s * 18 + c * 6 + 2 * m + 1] / count;
-        nc.g4[m] = mean4 > 0.0 ? dsum * wst[s][c][2 * m + 1] * std::pow(mean4, -0.75) / count : 0.0;
+        coefs.job[k].g4[m] = mean4 > 0.0 ? dsum * wst[s][c][2 * m + 1] * std::pow(mean4, -0.75) / count : 0.0;
       }
-      moments(s, c);  // recomputed, not stored
-      RCG_LAUNCH(ctx, "adj_mapgrad", k_mapgrad<T>, grid_of(n), 256, 0, mom, xa + c * n, xb + c * n, n, nc, gq,
-                 gq + n, gq + 2 * n, gx + c * n);
-      // the three gradient planes through the transposed column blur, then the row blur (its own transpose)
-      RCG_LAUNCH(ctx, "adj_vblur_t", k_vblur_t<T>, grid_rows(sc[s].w, (sc[s].h + kRun - 1) / kRun, 3), 256, 0, gq,
-                 sc[s].w, sc[s].h, hb5);
-      RCG_LAUNCH(ctx, "adj_hblur", k_hblur<T>, grid_row_runs(sc[s].w, sc[s].h, 3), 256, 0, hb5, sc[s].w, sc[s].h, tq);
-      RCG_LAUNCH(ctx, "adj_combine", k_combine<T>, grid_of(n), 256, 0, tq, tq + n, tq + 2 * n, xa + c * n,
-                 xb + c * n, n, gx + c * n);
     }
-    RCG_LAUNCH(ctx, "adj_xyb_adj", k_xyb_adj<T>, grid_of(n), 256, 0, pb + sc[s].off, gx, sc[s].w, sc[s].h,
-               s + 1 < ns ? gl + sc[s + 1].off : nullptr, s + 1 < ns ? sc[s + 1].w : 0, gl + sc[s].off);
+    const AdjJobs all = jobs_of(g, by_samples), cols = jobs_of(g, by_runs(kRun)), rows = jobs_of(g, by_row_runs);
+    RCG_LAUNCH(ctx, "adj_mapgrad", k_mapgrad<T>, grid(all), 256, 0, all, coefs, mom, xa, xb, hb5, gx);
+    // the three gradient planes through the transposed column blur, then the row blur (its own transpose)
+    RCG_LAUNCH(ctx, "adj_vblur_t", k_vblur_t<T>, dim3(grid(cols), 3), 256, 0, cols, hb5, mom);
+    RCG_LAUNCH(ctx, "adj_hblur", k_hblur_combine<T>, grid(rows), 256, 0, rows, mom, xa, xb, gx);
   }
+  for (int s = ns - 1; s >= 0; s--)
+    RCG_LAUNCH(ctx, "adj_xyb_adj", k_xyb_adj<T>, grid_of(sc[s].n), 256, 0, pb + sc[s].off, gx + sc[s].off, sc[s].w,
+               sc[s].h, s + 1 < ns ? gl + sc[s + 1].off : nullptr, s + 1 < ns ? sc[s + 1].w : 0, gl + sc[s].off);
   RCG_LAUNCH(ctx, "adj_out", k_grad_out<T>, grid_of(npx), 256, 0, gl + sc[0].off, d_dist, npx, d_grad);
   return RCG_OK;
 }
