@@ -9,13 +9,14 @@
 // found there is not an RSTn, that segment and all later ones read zero bits).
 //
 // The device decodes each segment in parallel by self-synchronization. A decoding state at a codeword boundary is
-// (bit position, block of the MCU, next coefficient index). The segment's bits are cut into spans of 2048 bits, one
-// thread each, and each span into pieces of 256 bits. Round after round every thread decodes its span from its
-// current start state, records the state and the block count and DC-difference sums at every piece boundary, and
-// hands the state where it crosses into the next span to its successor. The first span of a segment starts from
-// the exact state, so the states become exact from front to back; Huffman codes resynchronize within a few
-// codewords, but the block-of-the-MCU part of the state only when a desynchronization happens to realign it, which
-// takes a few MCUs, hence spans long enough to settle in a few rounds. When a round changes nothing, every piece
+// (bit position, block of the MCU, next coefficient index). The segment's bits are cut into spans of 1024 bits, one
+// thread each, and each span into pieces of 256 bits. Turn after turn the threads whose start state has changed decode
+// their spans from it, record the state and the block count and DC-difference sums at every piece boundary, and
+// hand the state where they cross into the next span to its successor: inside a CTA until nothing changes, from CTA to
+// CTA between launches (rounds). The first span of a segment starts from the exact state, so the states become exact
+// from front to back; Huffman codes resynchronize within a few codewords, but the block-of-the-MCU part of the state
+// only when a desynchronization happens to realign it, which can take tens of MCUs (the worst of a 5.5 MB file's
+// spans: 16 kbit), and no better first guess shortens that. When a round changes nothing, every piece
 // start is exact; prefix sums of the counts give each piece its first block and DC predictions, and a last pass,
 // one thread per piece, decodes again and writes the coefficients. If the rounds do not settle within a bound, one
 // thread per segment follows the chain of states instead.
@@ -25,6 +26,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -35,9 +37,11 @@ namespace rcg {
 namespace {
 
 constexpr int kSubBits = 256;   // a piece: the unit of the writing pass
-constexpr int kSpanSubs = 8;    // a span (8 pieces, 2048 bits): the unit of the synchronization rounds
-constexpr int kDecThreads = 64;
-constexpr int kFirstBatch = 3;  // rounds launched before the first convergence check
+constexpr int kSpanSubs = 4;    // a span (4 pieces, 1024 bits): the unit of synchronization
+constexpr int kSyncThreads = 192;  // spans per CTA of a synchronization round
+constexpr int kDecThreads = 128;   // pieces per CTA of the writing pass
+constexpr int kPrefixSpans = 4;    // spans per thread of the prefix sums
+constexpr int kRoundBatch = 4;     // rounds launched between looks at which have settled; those past that return at once
 constexpr int kMaxRounds = 48;
 constexpr int kMaxMcuBlocks = 48;
 constexpr unsigned long long kMaxPixels = 150000000ull;  // core/src/image.rs:33 (MAX_PIXELS)
@@ -87,6 +91,56 @@ bool build_huff(const uint8_t bits[16], const uint8_t* vals, size_t nvals, DevHu
   return true;
 }
 
+// The same table for the span decoder: a 10-bit lookup of what a code does to the decoder's state (0: longer code, or a
+// DC size past 15). Otherwise the canonical search: codes of growing length take growing left-justified ranges, so the
+// length is the first one whose range ends past the next 16 bits, the symbol vals[off + code].
+constexpr int kFastBits = 10;
+struct SeqHuff {
+  uint16_t fast[1 << kFastBits];  // seq_entry
+  uint32_t lim[17];               // [len]: left-justified end of the codes of up to len bits
+  int32_t off[17];
+  uint8_t vals[256];
+  int32_t dc;
+  uint32_t pad;
+};
+static_assert(sizeof(SeqHuff) % 16 == 0, "tables are copied in 16-byte words");
+// The distinct tables of a scan (three components of one DC and one AC table each at most).
+struct SeqTables {
+  int n, pad[3];
+  SeqHuff t[6];
+};
+
+// A symbol as the span decoder sees it: bits 0..5 the bits it takes (code and value), bits 6..11 how far the coefficient
+// index moves, from bit 12 the value's size. A DC symbol (its byte is the size) moves by one; an AC symbol (run, size)
+// by run + 1, ZRL by 16; an end of block or of a band run moves by kEob, past any band, and holds its run in place of
+// the size (the run's extra bits are not counted: only AC first scans have any).
+constexpr uint32_t kEob = 63;
+__host__ __device__ __forceinline__ uint32_t seq_entry(int len, uint32_t sym, bool dc) {
+  const uint32_t run = sym >> 4, sz = sym & 15;
+  if (dc) return (uint32_t)(len + sym) | (1u << 6) | (sym << 12);
+  if (sz == 0 && run < 15) return (uint32_t)len | (kEob << 6) | (run << 12);
+  return (uint32_t)(len + sz) | ((run + 1) << 6) | (sz << 12);
+}
+
+void seq_huff(const DevHuff& h, bool dc, SeqHuff* q) {
+  std::memset(q, 0, sizeof *q);
+  std::memcpy(q->vals, h.vals, sizeof q->vals);
+  q->dc = dc;
+  uint32_t end = 0;  // left-justified end of the codes so far
+  for (int len = 1; len <= 16; len++) {
+    const int n = h.maxcode[len] < 0 ? 0 : h.maxcode[len] - h.mincode[len] + 1;
+    for (int i = 0; i < n && len <= kFastBits; i++) {
+      const int c = h.mincode[len] + i, shift = kFastBits - len;
+      const int sym = h.vals[h.valptr[len] + i];
+      if (dc && sym > 15) continue;
+      for (int f = 0; f < (1 << shift); f++) q->fast[(c << shift) | f] = (uint16_t)seq_entry(len, sym, dc);
+    }
+    if (n > 0) end = (uint32_t)(h.maxcode[len] + 1) << (16 - len);
+    q->lim[len] = end;
+    q->off[len] = h.valptr[len] - h.mincode[len];
+  }
+}
+
 struct Segment {
   long long byte0;    // first destuffed byte of the segment in the scan's buffer
   long long nbytes;   // destuffed bytes of the segment (reads beyond give zeros)
@@ -115,6 +169,7 @@ struct ScanDesc {
   int mcu_dy[kMaxMcuBlocks], mcu_dx[kMaxMcuBlocks];
   int comp[4];                // frame component of each scan component
   int dc[4], ac[4];           // table slot of each scan component
+  int tdc[4], tac[4];         // and its entry in the scan's SeqTables
   CompDesc fc[3];             // frame components (block grids, offsets)
   int nseg;
   long long nsub;   // pieces of the scan
@@ -131,6 +186,12 @@ struct SubCount {
   long long blocks;  // blocks completed
   uint32_t dc[4];    // sums of DC differences per scan component (wrapping, as the reference's i32 predictor)
 };
+
+__device__ __forceinline__ void add_count(SubCount& a, const SubCount& b) {
+  a.blocks += b.blocks;
+#pragma unroll
+  for (int q = 0; q < 4; q++) a.dc[q] += b.dc[q];
+}
 
 // Bit reader over a segment's unstuffed bytes: reads past the segment's end give zeros (decode.rs:30-60). Bytes
 // inside a shared-memory window (the CTA's slice of the buffer, loaded once, coalesced) come from there; the rest
@@ -217,90 +278,182 @@ __device__ __forceinline__ int huff_decode(const DevHuff& h, Reader& r) {
   return -1;
 }
 
-__device__ __forceinline__ int extend_bits(uint32_t v, int t) {
-  if (t == 0) return 0;
-  return v < (1u << (t - 1)) ? (int)v - (1 << t) + 1 : (int)v;
-}
-
 struct Tables {
   DevHuff dc[4], ac[4];
 };
 
-// Decodes from `st` until the bit position reaches `stop_bit` or `max_blocks` blocks are complete. WRITE: also
-// stores the coefficients of block `block_base + blocks` onward (zigzag order), with DC predictors `pred`.
-// Returns 0, or 1 on a bad code (decode.rs:1482-1506).
-template <bool WRITE>
-__device__ __forceinline__ int decode_run(const Tables& tb, const ScanDesc& sd, Reader& r, SubState& st, long long stop_bit,
-                          long long max_blocks, SubCount& cnt, long long block_base, uint32_t* pred,
-                          int16_t* __restrict__ out) {
-  int u = st.u, k = st.k;
-  uint32_t d0 = cnt.dc[0], d1 = cnt.dc[1], d2 = cnt.dc[2], d3 = cnt.dc[3];
-  const uint32_t p0 = WRITE ? pred[0] - d0 : 0u, p1 = WRITE ? pred[1] - d1 : 0u, p2 = WRITE ? pred[2] - d2 : 0u,
-                 p3 = WRITE ? pred[3] - d3 : 0u;
+// What the span decoder's CTAs keep in shared memory: the scan's tables, per block of the MCU its tables and component
+// and where its blocks lie in the coefficients, and the CTA's slice of the entropy-coded data as big-endian words.
+struct BlockAt {
+  long long base, row, col;  // block index = base + MCU row * row + MCU column * col
+};
+template <int kWinWords>
+struct SeqShared {
+  SeqTables tab;
+  ScanDesc sd;
+  BlockAt at[kMaxMcuBlocks];
+  uint32_t pat[kMaxMcuBlocks];  // DC table | AC table << 8 | scan component << 16
+  uint32_t win[kWinWords];
+  long long w0;  // the slice: words [w0, w0 + nwin) of the scan buffer
+  int nwin;
+};
+
+// A place in a segment: the 64 bits (hi, lo) around bit p and the word after them, p and the words counted from the word
+// of the last seek. Words past the segment's end read as zero (decode.rs:30-60). kWin: from the CTA's slice, which holds
+// all that its spans or pieces read (and nothing outside it is read); else from the buffer.
+template <bool kWin>
+struct Bits {
+  const uint32_t* win;
+  const uint32_t* src;
+  uint32_t end, next;  // words that hold data; next word to load
+  uint32_t hi, lo, nx, p;
+  long long base;      // the segment's bit at p == 0
+  __device__ __forceinline__ uint32_t word(uint32_t i) const {
+    return i < end ? (kWin ? win[i] : __byte_perm(__ldg(src + i), 0, 0x0123)) : 0u;
+  }
+  template <int kWinWords>
+  __device__ __forceinline__ void seek(const SeqShared<kWinWords>& sh, const uint8_t* data, const Segment& sg,
+                                       long long bit) {
+    const long long first = sg.byte0 / 4, at = first + (bit >> 5);  // segments start at a word
+    long long left = first + (sg.nbytes + 3) / 4 - at;
+    if (kWin) {
+      const bool held = at >= sh.w0 && at < sh.w0 + sh.nwin;
+      win = sh.win + (held ? at - sh.w0 : 0);
+      left = held ? min(left, sh.w0 + sh.nwin - at) : 0;
+    } else {
+      src = reinterpret_cast<const uint32_t*>(data) + at;
+    }
+    end = (uint32_t)min(max(left, 0ll), 0x7fffffffll);
+    hi = word(0);
+    lo = word(1);
+    nx = word(2);
+    next = 3;
+    p = (uint32_t)bit & 31u;
+    base = bit - p;
+  }
+  __device__ __forceinline__ long long bit() const { return base + p; }
+  __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(lo, hi, p); }
+  __device__ __forceinline__ void skip(uint32_t n) {  // n <= 32: at most one word boundary
+    const uint32_t q = p + n;
+    if ((q ^ p) & 32u) {
+      hi = lo;
+      lo = nx;
+      nx = word(next);
+      next += next < end;
+    }
+    p = q;
+  }
+};
+
+__device__ __forceinline__ int value_of(uint32_t w, uint32_t len, uint32_t sz) {  // decode.rs:190-200 (receive, extend)
+  const uint32_t raw = sz ? (w << len) >> (32 - sz) : 0u;  // len <= 16
+  return sz && !(raw >> (sz - 1)) ? (int)raw - (1 << sz) + 1 : (int)raw;
+}
+
+// Decodes from block u of the MCU, coefficient k, until the position reaches `stop` (p of `r`; kEndless: never) or, when
+// writing, `max_blocks` blocks are complete. kWrite: also stores the coefficients of block `block0` onward (zigzag
+// order), with DC predictors `pred`. Returns 0, or 1 on a bad code (decode.rs:1482-1506).
+//
+// decode_sequential (decode.rs:1482-1506) with every effect of a symbol in its table entry: a DC symbol is a size and as
+// many bits; an AC symbol (run, size) is EOB (size 0, run < 15), ZRL (size 0, run 15: k += 16) or a coefficient at
+// k + run (error past 63); the block ends when k reaches 64 or at EOB. The progressive first scans are the same loop:
+// decode_dc_first (:1509-1517) is a DC symbol per block, its value shifted left by al; decode_ac_first (:1519-1547)
+// runs k from ss (>= 1), ends the block past se, shifts values by al, and an EOB symbol there is an end-of-band run:
+// 2^run - 1 + (run extra bits) further blocks read no bits at all.
+//
+// What bounds it: the latency of a symbol. A thread's symbols are a serial chain (shift, lookup, add, shift), and a round
+// waits for the span of the most symbols. So the chain carries only the position, the index and the table (about 160
+// cycles a symbol, from 1500 with separate code and value reads, 64-bit positions and bytes gathered four at a time);
+// the next word is loaded a word ahead, values are formed for DC sums and when writing only.
+constexpr uint32_t kEndless = 0xffffffffu;
+template <bool kWrite, bool kWin, int kWinWords>
+__device__ __forceinline__ int decode_run(const SeqShared<kWinWords>& sh, Bits<kWin>& r, int& u, int& k, uint32_t stop,
+                                          uint32_t max_blocks, SubCount& cnt, long long block0,
+                                          const uint32_t* pred, int16_t* __restrict__ out) {
+  const ScanDesc& sd = sh.sd;
+  const bool ac_first = sd.kind == kAcFirst;
+  const int kend = sd.kind == kDcFirst ? 0 : ac_first ? sd.se : 63, shift = sd.al, k0 = sd.k0, bmcu = sd.bmcu;
+  uint32_t pat = sh.pat[u];
+  const SeqHuff* h = &sh.tab.t[k == 0 ? pat & 255 : (pat >> 8) & 255];
+  uint32_t blocks = 0, d0 = 0, d1 = 0, d2 = 0;
   int16_t* blk = nullptr;
-  auto block_ptr = [&](long long b) -> int16_t* {
-    const long long mcu = b / sd.bmcu;
-    const int uu = (int)(b - mcu * sd.bmcu);
-    const int si = sd.mcu_si[uu];
-    const CompDesc& c = sd.fc[sd.comp[si]];
-    const long long my = mcu / sd.mcus_x, mx = mcu - my * sd.mcus_x;
-    const long long row = my * (sd.bmcu == 1 ? 1 : c.v) + sd.mcu_dy[uu];
-    const long long col = mx * (sd.bmcu == 1 ? 1 : c.h) + sd.mcu_dx[uu];
-    return out + (c.blk0 + row * c.bw + col) * 64;
-  };
-  if (WRITE && cnt.blocks < max_blocks) blk = block_ptr(block_base + cnt.blocks);
+  long long my = 0, mx = 0;
+  if (kWrite) {
+    const long long mcu = block0 / bmcu;
+    my = mcu / sd.mcus_x;
+    mx = mcu - my * sd.mcus_x;
+    blk = out + (sh.at[u].base + my * sh.at[u].row + mx * sh.at[u].col) * 64;
+    d0 = pred[0];
+    d1 = pred[1];
+    d2 = pred[2];
+  }
   int err = 0;
-  // One symbol per iteration with a single code path for DC and AC symbols (the lanes of a warp decode different
-  // streams; branches would serialize them). decode_sequential (decode.rs:1482-1506) in select form: a DC symbol is
-  // a size t <= 16 and t extra bits; an AC symbol (run, size) is EOB (size 0, run < 15), ZRL (size 0, run 15: k += 16)
-  // or a coefficient at k + run (error past 63); the block ends when k reaches 64 or at EOB. The progressive first
-  // scans are the same loop: decode_dc_first (:1509-1517) is a DC symbol per block, its value shifted left by al;
-  // decode_ac_first (:1519-1547) runs k from ss, ends the block past se, shifts values by al, and an EOB symbol
-  // there is an end-of-band run: 2^run - 1 + (run extra bits) further blocks read no bits at all.
-  const bool dc_only = sd.kind == kDcFirst, ac_first = sd.kind == kAcFirst;
-  const int kend = ac_first ? sd.se : 63, shift = sd.al;
-  long long blocks = cnt.blocks;
-  while (blocks < max_blocks && r.bit < stop_bit) {
-    const int si = sd.mcu_si[u];
-    const bool dc = dc_only || (!ac_first && k == 0);
-    const int sym = huff_decode(dc ? tb.dc[sd.dc[si]] : tb.ac[sd.ac[si]], r);
-    const int run = dc ? 0 : (sym >> 4);
-    const int sz = dc ? sym : (sym & 15);
-    if (sym < 0 || sz > 16 || (!dc && sz > 0 && k + run > 63)) {
-      err = 1;
-      break;
+  while (r.p < stop || (kWrite && stop == kEndless)) {
+    const uint32_t w = r.peek();
+    uint32_t e = h->fast[w >> (32 - kFastBits)];
+    if (e == 0) {
+      const uint32_t c = w >> 16;
+      int len = 1;
+      while (len < 17 && c >= h->lim[len]) len++;
+      const uint32_t sym = len < 17 ? h->vals[h->off[len] + (int)(c >> (16 - len))] : 255u;
+      if (len == 17 || (h->dc && sym > 16)) {
+        err = 1;
+        break;
+      }
+      e = seq_entry(len, sym, h->dc);
     }
-    const int v = extend_bits(r.bits(sz), sz);
-    // end-of-band run of an AC first scan (sz == 0 here, so no value bits were read)
-    const long long skip = (ac_first && sz == 0 && run < 15) ? (long long)((1u << run) - 1u + r.bits(run)) : 0;
-    const uint32_t ud = dc ? (uint32_t)v : 0u;  // selects instead of indexing by si: the sums stay in registers
-    d0 += si == 0 ? ud : 0u;
-    d1 += si == 1 ? ud : 0u;
-    d2 += si == 2 ? ud : 0u;
-    d3 += si == 3 ? ud : 0u;
-    if (WRITE) {
-      if (dc)
-        blk[0] = (int16_t)((si == 0 ? p0 + d0 : si == 1 ? p1 + d1 : si == 2 ? p2 + d2 : p3 + d3) << shift);
-      else if (sz > 0)
-        blk[k + run] = (int16_t)((uint32_t)v << shift);
+    const uint32_t adv = e & 63u, step = (e >> 6) & 63u, sz = e >> 12;
+    if (k == 0) {
+      const uint32_t v = (uint32_t)value_of(w, adv - sz, sz);
+      const uint32_t si = pat >> 16;
+      d0 += si == 0 ? v : 0u;  // selects instead of indexing by si: the sums stay in registers
+      d1 += si == 1 ? v : 0u;
+      d2 += si == 2 ? v : 0u;
+      if (kWrite) blk[0] = (int16_t)((si == 0 ? d0 : si == 1 ? d1 : d2) << shift);
+      h = &sh.tab.t[(pat >> 8) & 255];
+    } else if (kWrite && sz > 0 && step != kEob) {
+      if (k + (int)step > 64) {
+        err = 1;
+        break;
+      }
+      blk[k + step - 1] = (int16_t)((uint32_t)value_of(w, adv - sz, sz) << shift);
     }
-    const int nk = dc ? (dc_only ? 64 : 1) : (sz == 0 ? (run == 15 ? k + 16 : 64) : k + run + 1);
-    const bool end = nk > kend;
-    k = end ? sd.k0 : nk;
-    if (end) {
-      u = u + 1 == sd.bmcu ? 0 : u + 1;
-      blocks += 1 + skip;
-      if (WRITE && blocks < max_blocks) blk = block_ptr(block_base + blocks);
+    r.skip(adv);
+    k += (int)step;
+    if (k > kend) {
+      if (!kWrite && k > 64 && sz > 0 && step != kEob) {
+        err = 1;
+        break;
+      }
+      uint32_t more = 0;
+      if (ac_first && step == kEob) {
+        more = (1u << sz) - 1u + (sz ? r.peek() >> (32 - sz) : 0u);
+        r.skip(sz);
+      }
+      k = k0;
+      blocks += 1 + more;
+      u = u + 1 == bmcu ? 0 : u + 1;
+      pat = sh.pat[u];
+      h = &sh.tab.t[ac_first ? (pat >> 8) & 255 : pat & 255];
+      if (kWrite) {
+        if (blocks >= max_blocks) break;
+        if (more) {  // a scan of one component, a block per MCU
+          const long long mcu = block0 + blocks;
+          my = mcu / sd.mcus_x;
+          mx = mcu - my * sd.mcus_x;
+        } else if (u == 0 && ++mx == sd.mcus_x) {
+          mx = 0;
+          my++;
+        }
+        blk = out + (sh.at[u].base + my * sh.at[u].row + mx * sh.at[u].col) * 64;
+      }
     }
   }
   cnt.blocks = blocks;
-  st.bit = r.bit;
-  st.u = u;
-  st.k = k;
   cnt.dc[0] = d0;
   cnt.dc[1] = d1;
   cnt.dc[2] = d2;
-  cnt.dc[3] = d3;
+  cnt.dc[3] = 0;
   return err;
 }
 
@@ -338,13 +491,6 @@ __device__ __forceinline__ void unit_window(const Segment* segs, int nseg, long 
   *hi = min(h, l + cap);
 }
 
-// Copies scan-buffer bytes [lo, hi) (16-byte aligned; the buffer is padded past its end) into shared memory.
-__device__ __forceinline__ void load_window(const uint8_t* data, long long lo, long long hi, uint8_t* win) {
-  const int4* src = reinterpret_cast<const int4*>(data + lo);
-  int4* dst = reinterpret_cast<int4*>(win);
-  for (long long i = threadIdx.x; i < (hi - lo) / 16; i += blockDim.x) dst[i] = __ldg(src + i);
-}
-
 __device__ __forceinline__ void load_tables(Tables& sh, const Tables* g) {
   const int4* src = reinterpret_cast<const int4*>(g);
   int4* dst = reinterpret_cast<int4*>(&sh);
@@ -352,191 +498,285 @@ __device__ __forceinline__ void load_tables(Tables& sh, const Tables* g) {
   __syncthreads();
 }
 
-// One round, one thread per span: decode the span's pieces from the span's current start, record the state and
-// the counts at every piece boundary, and propose the state at the span's end as the next span's start.
-__global__ void __launch_bounds__(kDecThreads) k_seq_sync(const ScanDesc* __restrict__ sdp, const Tables* __restrict__ tg,
-                                                          const Segment* __restrict__ segs,
-                                                          const uint8_t* __restrict__ data,
-                                                          const SubState* __restrict__ cur, SubState* __restrict__ nxt,
-                                                          SubState* __restrict__ piece_state,
-                                                          SubCount* __restrict__ counts, int* __restrict__ changed) {
-  __shared__ __align__(16) Tables tb;
-  __shared__ ScanDesc sd;
-  if (threadIdx.x == 0) sd = *sdp;
-  load_tables(tb, tg);
-  constexpr long long kWin = (long long)kDecThreads * (kSpanSubs * kSubBits / 8 + 4) + kTail + 32;
-  __shared__ __align__(16) uint8_t win[kWin];
-  __shared__ long long w_lo, w_hi;
-  const long long t0 = (long long)blockIdx.x * blockDim.x;
-  if (threadIdx.x == 0) unit_window(segs, sd.nseg, t0, blockDim.x, sd.nspan, true, kWin & ~15ll, &w_lo, &w_hi);
+// Fills the CTA's shared state: tables, scan, MCU pattern and, for units [t0, t0 + count) (none: count 0), their bytes as
+// big-endian words (the buffer is padded past its end).
+template <int kWinWords>
+__device__ __forceinline__ void load_shared(SeqShared<kWinWords>& sh, const ScanDesc* sdp, const SeqTables* tg,
+                                            const Segment* segs, const uint8_t* data, long long t0, long long count,
+                                            bool spans) {
+  const int n = tg->n;
+  for (int i = threadIdx.x; i < 1 + n * (int)(sizeof(SeqHuff) / 16); i += blockDim.x)
+    reinterpret_cast<int4*>(&sh.tab)[i] = __ldg(reinterpret_cast<const int4*>(tg) + i);
+  for (int i = threadIdx.x; i < (int)(sizeof(ScanDesc) / 4); i += blockDim.x)
+    reinterpret_cast<int*>(&sh.sd)[i] = reinterpret_cast<const int*>(sdp)[i];
+  if (threadIdx.x == 0) {
+    long long lo = 0, hi = 0;
+    if (count > 0)
+      unit_window(segs, sdp->nseg, t0, count, spans ? sdp->nspan : sdp->nsub, spans, ((long long)kWinWords * 4) & ~15ll,
+                  &lo, &hi);
+    sh.w0 = lo / 4;
+    sh.nwin = (int)((hi - lo) / 4);
+  }
   __syncthreads();
-  load_window(data, w_lo, w_hi, win);
+  const ScanDesc& sd = sh.sd;
+  for (int u = threadIdx.x; u < sd.bmcu; u += blockDim.x) {
+    const int si = sd.mcu_si[u];
+    const CompDesc& c = sd.fc[sd.comp[si]];
+    const long long v = sd.bmcu == 1 ? 1 : c.v, h = sd.bmcu == 1 ? 1 : c.h;
+    sh.at[u] = BlockAt{c.blk0 + (long long)sd.mcu_dy[u] * c.bw + sd.mcu_dx[u], v * c.bw, h};
+    sh.pat[u] = (uint32_t)sd.tdc[si] | ((uint32_t)sd.tac[si] << 8) | ((uint32_t)si << 16);
+  }
+  const int4* src = reinterpret_cast<const int4*>(data + sh.w0 * 4);
+  for (int i = threadIdx.x; i < sh.nwin / 4; i += blockDim.x) {
+    const int4 v = __ldg(src + i);
+    sh.win[4 * i] = __byte_perm((uint32_t)v.x, 0, 0x0123);
+    sh.win[4 * i + 1] = __byte_perm((uint32_t)v.y, 0, 0x0123);
+    sh.win[4 * i + 2] = __byte_perm((uint32_t)v.z, 0, 0x0123);
+    sh.win[4 * i + 3] = __byte_perm((uint32_t)v.w, 0, 0x0123);
+  }
   __syncthreads();
-  const long long t = t0 + threadIdx.x;
-  if (t >= sd.nspan) return;
-  const SubRef ref = find_sub(segs, sd.nseg, t, true);
-  const Segment& sg = segs[ref.seg];
-  if (ref.local == 0) nxt[t] = SubState{0, 0, sd.k0};
-  const int f0 = ref.local * kSpanSubs, f1 = min(f0 + kSpanSubs, sg.nsub);
-  SubState st = cur[t];
-  piece_state[sg.sub0 + f0] = st;
-  Reader r;
-  r.init(data, sg.byte0, sg.nbytes, st.bit, win, w_lo, w_hi);
-  for (int f = f0; f < f1 && f + 1 < sg.nsub; f++) {
-    SubCount cnt{};
+}
+
+// Units of one CTA: their bytes, each segment's padding to a word, the bytes read past the last, both ends' rounding.
+constexpr int window_words(int threads, int unit_bytes) { return (threads * (unit_bytes + 4) + kTail + 32) / 4; }
+
+__device__ __forceinline__ bool same(const SubState& a, const SubState& b) {
+  return a.bit == b.bit && a.u == b.u && a.k == b.k;
+}
+
+// A state at a piece's boundary, packed: the bits past the boundary (a codeword at most), block of the MCU, coefficient.
+__device__ __forceinline__ uint32_t pack_state(const SubState& st, long long boundary) {
+  return (uint32_t)(st.bit - boundary) | ((uint32_t)st.u << 8) | ((uint32_t)st.k << 16);
+}
+
+// Decodes span `local` of a segment from `st` (to the state at its end): the state at every piece's start and the counts
+// of every piece. A bad code leaves the decoder desynchronized; any state will do to go on from. seen[f]: the states
+// past piece f of an earlier turn (kNotSeen: none). Where one is met again, the rest of the span is as it was then:
+// returns false (the state at the span's end is unchanged too).
+constexpr uint32_t kNotSeen = 0xffffffffu;
+template <bool kWin, int kWinWords>
+__device__ __forceinline__ bool decode_span(const SeqShared<kWinWords>& sh, const uint8_t* data, const Segment& sg,
+                                            int local, SubState& st, uint32_t (&seen)[kSpanSubs],
+                                            SubState* __restrict__ piece_state, SubCount* __restrict__ counts) {
+  const int f0 = local * kSpanSubs;
+  Bits<kWin> r;
+  r.seek(sh, data, sg, st.bit);
+#pragma unroll
+  for (int i = 0; i < kSpanSubs; i++) {
+    const int f = f0 + i;
+    if (f < sg.nsub) piece_state[sg.sub0 + f] = st;
+    if (f + 1 >= sg.nsub) return true;  // the segment's last piece is decoded when it is written
     const long long stop = (long long)(f + 1) * kSubBits;
-    if (decode_run<false>(tb, sd, r, st, stop, LLONG_MAX, cnt, 0, nullptr, nullptr)) {
-      st = SubState{stop, 0, sd.k0};  // desynchronized: any guess will do
-      r.init(data, sg.byte0, sg.nbytes, stop, win, w_lo, w_hi);
+    SubCount cnt;
+    if (decode_run<false>(sh, r, st.u, st.k, (uint32_t)max(stop - r.base, 0ll), 0, cnt, 0, nullptr, nullptr)) {
+      st.u = 0;
+      st.k = sh.sd.k0;
+      r.seek(sh, data, sg, stop);
     }
+    st.bit = r.bit();
     counts[sg.sub0 + f] = cnt;
-    piece_state[sg.sub0 + f + 1] = st;
+    const uint32_t now = pack_state(st, stop);
+    if (now == seen[i]) return false;
+    seen[i] = now;
   }
-  if (ref.local + 1 >= sg.nspan) return;  // the segment's last span proposes nothing
-  nxt[t + 1] = st;
-  const SubState& old = cur[t + 1];
-  if (old.bit != st.bit || old.u != st.u || old.k != st.k) atomicOr(changed, 1);
+  return true;
 }
 
-// Fallback when the rounds do not settle: one thread per segment follows the chain of exact piece states.
-__global__ void k_seq_chain(const ScanDesc* __restrict__ sdp, const Tables* __restrict__ tg,
-                            const Segment* __restrict__ segs, const uint8_t* __restrict__ data,
-                            SubState* __restrict__ piece_state, SubCount* __restrict__ counts) {
-  __shared__ __align__(16) Tables tb;
-  __shared__ ScanDesc sd;
-  if (threadIdx.x == 0) sd = *sdp;
-  load_tables(tb, tg);
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < sd.nseg; s += gridDim.x * blockDim.x) {
-    const Segment& sg = segs[s];
-    SubState st{0, 0, sd.k0};
-    Reader r;
-    r.init(data, sg.byte0, sg.nbytes, 0);
-    for (int i = 0; i + 1 < sg.nsub; i++) {
-      piece_state[sg.sub0 + i] = st;
-      SubCount cnt{};
-      const long long stop = (long long)(i + 1) * kSubBits;
-      if (decode_run<false>(tb, sd, r, st, stop, LLONG_MAX, cnt, 0, nullptr, nullptr)) {
-        st = SubState{stop, 0, sd.k0};
-        r.init(data, sg.byte0, sg.nbytes, stop);
-      }
-      counts[sg.sub0 + i] = cnt;
+// One round, one thread per span and kSyncThreads spans per CTA. A thread decodes its span from the span's current
+// start and proposes the state at its end as the next span's start; inside a CTA this is repeated, by the threads whose
+// start has changed, until no start changes (a CTA's n-th span is settled after n turns at most). The state at the end
+// of a CTA's last span goes to the next CTA in the next round: edge_nxt[c] is the start of CTA c's first span. Round 0
+// starts every span at its first bit, the MCU's first block, a block's first coefficient. A round after one that moved
+// no edge (changed[round - 1] == 0) returns at once.
+// What bounds it: the longest chain of spans that start wrong, a few lanes decoding one after the other while the chip
+// waits. Measured for 5.5 MB (6 MP 4:2:0, quality 92): 880 us (690 for round 0, 180 for round 1) against 2170 for eight
+// rounds of 2048-bit spans that each decoded every span; spans of 512 / 2048 bits 917 / 958, 96 spans a CTA 864.
+__global__ void __launch_bounds__(kSyncThreads) k_seq_sync(const ScanDesc* __restrict__ sdp,
+                                                           const SeqTables* __restrict__ tg,
+                                                           const Segment* __restrict__ segs,
+                                                           const uint8_t* __restrict__ data,
+                                                           SubState* __restrict__ start,
+                                                           const SubState* __restrict__ edge_cur,
+                                                           SubState* __restrict__ edge_nxt,
+                                                           SubState* __restrict__ piece_state,
+                                                           SubCount* __restrict__ counts,
+                                                           SubCount* __restrict__ span_counts,
+                                                           int* __restrict__ changed, int round) {
+  if (round > 0 && changed[round - 1] == 0) return;
+  constexpr int kWords = window_words(kSyncThreads, kSpanSubs * kSubBits / 8);
+  __shared__ __align__(16) SeqShared<kWords> sh;
+  __shared__ SubState proposed[kSyncThreads + 1];
+  const int tid = threadIdx.x;
+  const long long t0 = (long long)blockIdx.x * kSyncThreads, t = t0 + tid;
+  load_shared(sh, sdp, tg, segs, data, t0, kSyncThreads, true);
+  const ScanDesc& sd = sh.sd;
+  const bool live = t < sd.nspan, more = t0 + kSyncThreads < sd.nspan;  // more: the next CTA has spans
+  const SubRef ref = live ? find_sub(segs, sd.nseg, t, true) : SubRef{0, 0};
+  const Segment& sg = segs[ref.seg];
+  SubState st{(long long)ref.local * kSpanSubs * kSubBits, 0, sd.k0};
+  bool need = live;
+  if (round > 0 && live) {
+    st = start[t];
+    need = false;
+    if (tid == 0 && ref.local > 0) {
+      const SubState in = edge_cur[blockIdx.x];
+      need = !same(in, st);
+      st = in;
     }
-    piece_state[sg.sub0 + sg.nsub - 1] = st;
+  }
+  uint32_t seen[kSpanSubs];
+#pragma unroll
+  for (int i = 0; i < kSpanSubs; i++) seen[i] = kNotSeen;
+  if (round > 0 && live) {  // the state past the last piece is not kept: it is decoded again
+#pragma unroll
+    for (int i = 0; i + 1 < kSpanSubs; i++) {
+      const int f = ref.local * kSpanSubs + i + 1;
+      if (f < sg.nsub) seen[i] = pack_state(piece_state[sg.sub0 + f], (long long)f * kSubBits);
+    }
+  }
+  proposed[tid] = st;
+  if (tid == 0) proposed[kSyncThreads] = round > 0 && more ? edge_cur[blockIdx.x + 1] : SubState{0, 0, sd.k0};
+  __syncthreads();
+  bool decoded = false;
+  do {
+    if (need) {
+      SubState end = st;
+      const bool moved = decode_span<true>(sh, data, sg, ref.local, end, seen, piece_state, counts);
+      if (moved && ref.local + 1 < sg.nspan) proposed[tid + 1] = end;  // the next segment starts from its own first bit
+      decoded = true;
+    }
+    __syncthreads();
+    need = false;
+    if (live && tid > 0 && ref.local > 0) {
+      const SubState in = proposed[tid];
+      need = !same(in, st);
+      st = in;
+    }
+  } while (__syncthreads_or(need));
+  if (decoded) {
+    start[t] = st;
+    SubCount sum{};
+    if (ref.local + 1 < sg.nspan)  // no span follows a segment's last one
+      for (int i = 0; i < kSpanSubs; i++) add_count(sum, counts[sg.sub0 + ref.local * kSpanSubs + i]);
+    span_counts[t] = sum;
+  }
+  if (tid == 0 && more) {
+    const SubState out = proposed[kSyncThreads];
+    edge_nxt[blockIdx.x + 1] = out;
+    if (round == 0 || !same(out, edge_cur[blockIdx.x + 1])) changed[round] = 1;
   }
 }
 
-// Per segment, exclusive prefix sums of the pieces' block counts and DC sums (one CTA per segment, 1024 pieces at a
-// time: warp shuffles, then the 32 warp totals).
-__global__ void __launch_bounds__(1024) k_seq_prefix(const ScanDesc* __restrict__ sdp, const Segment* __restrict__ segs,
-                                                     const SubCount* __restrict__ counts, SubCount* __restrict__ base) {
-  __shared__ long long wb[32];
-  __shared__ uint32_t wd[4][32];
-  const ScanDesc& sd = *sdp;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int s = blockIdx.x; s < sd.nseg; s += gridDim.x) {
+// Fallback when the rounds do not settle: one thread per segment follows the chain of exact states.
+__global__ void __launch_bounds__(128) k_seq_chain(const ScanDesc* __restrict__ sdp, const SeqTables* __restrict__ tg,
+                                                   const Segment* __restrict__ segs, const uint8_t* __restrict__ data,
+                                                   SubState* __restrict__ piece_state, SubCount* __restrict__ counts,
+                                                   SubCount* __restrict__ span_counts) {
+  __shared__ __align__(16) SeqShared<4> sh;
+  load_shared(sh, sdp, tg, segs, data, 0, 0, true);
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < sh.sd.nseg; s += gridDim.x * blockDim.x) {
     const Segment& sg = segs[s];
-    long long carry_b = 0;
-    uint32_t carry_d[4] = {0, 0, 0, 0};
-    for (int off = 0; off < sg.nsub; off += 1024) {
-      const int i = off + threadIdx.x;
-      // piece i starts after pieces 0..i-1 (the last piece's counts are never needed)
-      SubCount c{};
-      if (i >= 1 && i < sg.nsub) c = counts[sg.sub0 + i - 1];
-      long long b = c.blocks;
-      uint32_t d[4] = {c.dc[0], c.dc[1], c.dc[2], c.dc[3]};
+    SubState st{0, 0, sh.sd.k0};
+    for (int i = 0; i < sg.nspan; i++) {
+      uint32_t seen[kSpanSubs];
+      for (int f = 0; f < kSpanSubs; f++) seen[f] = kNotSeen;
+      decode_span<false>(sh, data, sg, i, st, seen, piece_state, counts);
+      SubCount sum{};
+      for (int f = 0; f < kSpanSubs && i + 1 < sg.nspan; f++) add_count(sum, counts[sg.sub0 + i * kSpanSubs + f]);
+      span_counts[sg.span0 + i] = sum;
+    }
+  }
+}
+
+// Per segment, exclusive prefix sums of the spans' block counts and DC sums (one CTA per segment, kPrefixSpans x 1024
+// spans at a time: a thread's own spans, warp shuffles, then the 32 warp totals). The pieces inside a span are summed by
+// the threads that write them: one pass over every piece here took 96 us for 5.5 MB, this 31.
+__global__ void __launch_bounds__(1024) k_seq_prefix(const ScanDesc* __restrict__ sdp, const Segment* __restrict__ segs,
+                                                     const SubCount* __restrict__ span_counts,
+                                                     SubCount* __restrict__ base) {
+  __shared__ SubCount total[32];
+  const int nseg = sdp->nseg;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto scan_warp = [&](SubCount& c) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const long long bo = __shfl_up_sync(0xffffffffu, b, o);
-        uint32_t dq[4];
+    for (int o = 1; o < 32; o <<= 1) {
+      SubCount x;
+      x.blocks = __shfl_up_sync(0xffffffffu, c.blocks, o);
 #pragma unroll
-        for (int q = 0; q < 4; q++) dq[q] = __shfl_up_sync(0xffffffffu, d[q], o);
-        if (lane >= o) {
-          b += bo;
+      for (int q = 0; q < 4; q++) x.dc[q] = __shfl_up_sync(0xffffffffu, c.dc[q], o);
+      if (lane >= o) add_count(c, x);
+    }
+  };
+  for (int s = blockIdx.x; s < nseg; s += gridDim.x) {
+    const long long span0 = segs[s].span0;
+    const int nspan = segs[s].nspan;
+    SubCount carry{};
+    for (int off = 0; off < nspan; off += 1024 * kPrefixSpans) {
+      const int i0 = off + threadIdx.x * kPrefixSpans;
+      SubCount own[kPrefixSpans], c{};
 #pragma unroll
-          for (int q = 0; q < 4; q++) d[q] += dq[q];
-        }
-      }
-      if (lane == 31) {
-        wb[warp] = b;
+      for (int q = 0; q < kPrefixSpans; q++) own[q] = i0 + q < nspan ? span_counts[span0 + i0 + q] : SubCount{};
 #pragma unroll
-        for (int q = 0; q < 4; q++) wd[q][warp] = d[q];
-      }
+      for (int q = 0; q < kPrefixSpans; q++) add_count(c, own[q]);
+      scan_warp(c);
+      if (lane == 31) total[warp] = c;
+      SubCount before;  // the spans of the lanes before this one
+      before.blocks = __shfl_up_sync(0xffffffffu, c.blocks, 1);
+#pragma unroll
+      for (int q = 0; q < 4; q++) before.dc[q] = __shfl_up_sync(0xffffffffu, c.dc[q], 1);
+      if (lane == 0) before = SubCount{};
       __syncthreads();
       if (warp == 0) {
-        long long x = wb[lane];
-        uint32_t y[4] = {wd[0][lane], wd[1][lane], wd[2][lane], wd[3][lane]};
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const long long xo = __shfl_up_sync(0xffffffffu, x, o);
-          uint32_t yo[4];
-#pragma unroll
-          for (int q = 0; q < 4; q++) yo[q] = __shfl_up_sync(0xffffffffu, y[q], o);
-          if (lane >= o) {
-            x += xo;
-#pragma unroll
-            for (int q = 0; q < 4; q++) y[q] += yo[q];
-          }
-        }
-        wb[lane] = x;
-#pragma unroll
-        for (int q = 0; q < 4; q++) wd[q][lane] = y[q];
+        SubCount x = total[lane];
+        scan_warp(x);
+        total[lane] = x;
       }
       __syncthreads();
-      if (warp > 0) {
-        b += wb[warp - 1];
+      if (warp > 0) add_count(before, total[warp - 1]);
+      add_count(before, carry);
 #pragma unroll
-        for (int q = 0; q < 4; q++) d[q] += wd[q][warp - 1];
+      for (int q = 0; q < kPrefixSpans; q++) {
+        if (i0 + q < nspan) base[span0 + i0 + q] = before;
+        add_count(before, own[q]);
       }
-      if (i < sg.nsub) {
-        SubCount o;
-        o.blocks = carry_b + b;
-#pragma unroll
-        for (int q = 0; q < 4; q++) o.dc[q] = carry_d[q] + d[q];
-        base[sg.sub0 + i] = o;
-      }
-      carry_b += wb[31];
-#pragma unroll
-      for (int q = 0; q < 4; q++) carry_d[q] += wd[q][31];
+      add_count(carry, total[31]);
       __syncthreads();
     }
   }
 }
 
-// Final pass: decode each subsequence from its exact start and write the coefficients.
-__global__ void __launch_bounds__(kDecThreads) k_seq_write(const ScanDesc* __restrict__ sdp, const Tables* __restrict__ tg,
-                                                   const Segment* __restrict__ segs, const uint8_t* __restrict__ data,
-                                                   const SubState* __restrict__ states,
-                                                   const SubCount* __restrict__ base, int16_t* __restrict__ out,
-                                                   int* __restrict__ error) {
-  __shared__ __align__(16) Tables tb;
-  __shared__ ScanDesc sd;
-  if (threadIdx.x == 0) sd = *sdp;
-  load_tables(tb, tg);
-  constexpr long long kWin = (long long)kDecThreads * (kSubBits / 8 + 4) + kTail + 32;
-  __shared__ __align__(16) uint8_t win[kWin];
-  __shared__ long long w_lo, w_hi;
+// Final pass: decode each piece from its exact start and write the coefficients (5.5 MB: 49 us, from 69).
+__global__ void __launch_bounds__(kDecThreads) k_seq_write(const ScanDesc* __restrict__ sdp,
+                                                           const SeqTables* __restrict__ tg,
+                                                           const Segment* __restrict__ segs,
+                                                           const uint8_t* __restrict__ data,
+                                                           const SubState* __restrict__ states,
+                                                           const SubCount* __restrict__ counts,
+                                                           const SubCount* __restrict__ base, int16_t* __restrict__ out,
+                                                           int* __restrict__ error) {
+  constexpr int kWords = window_words(kDecThreads, kSubBits / 8);
+  __shared__ __align__(16) SeqShared<kWords> sh;
   const long long t0 = (long long)blockIdx.x * blockDim.x;
-  if (threadIdx.x == 0) unit_window(segs, sd.nseg, t0, blockDim.x, sd.nsub, false, kWin & ~15ll, &w_lo, &w_hi);
-  __syncthreads();
-  load_window(data, w_lo, w_hi, win);
-  __syncthreads();
+  load_shared(sh, sdp, tg, segs, data, t0, blockDim.x, false);
+  const ScanDesc& sd = sh.sd;
   const long long t = t0 + threadIdx.x;
   if (t >= sd.nsub) return;
   const SubRef ref = find_sub(segs, sd.nseg, t, false);
   const Segment& sg = segs[ref.seg];
-  const SubCount b = base[t];
+  SubCount b = base[sg.span0 + ref.local / kSpanSubs];
+  for (int f = ref.local / kSpanSubs * kSpanSubs; f < ref.local; f++) add_count(b, counts[sg.sub0 + f]);
   if (b.blocks >= sg.nblocks) return;  // past the segment's last block: padding
   SubState st = states[t];
   if (st.u != (int)((sg.block0 + b.blocks) % sd.bmcu)) {
     atomicCAS(error, 0, 2);  // inconsistent start (cannot happen for exact states)
     return;
   }
-  SubCount cnt{};
-  uint32_t pred[4] = {b.dc[0], b.dc[1], b.dc[2], b.dc[3]};
-  Reader r;
-  r.init(data, sg.byte0, sg.nbytes, st.bit, win, w_lo, w_hi);
-  const long long stop = ref.local + 1 < sg.nsub ? (long long)(ref.local + 1) * kSubBits : LLONG_MAX;
-  if (decode_run<true>(tb, sd, r, st, stop, sg.nblocks - b.blocks, cnt, sg.block0 + b.blocks, pred, out))
+  Bits<true> r;
+  r.seek(sh, data, sg, st.bit);
+  const uint32_t stop =
+      ref.local + 1 < sg.nsub ? (uint32_t)max((long long)(ref.local + 1) * kSubBits - r.base, 0ll) : kEndless;
+  SubCount cnt;
+  if (decode_run<true>(sh, r, st.u, st.k, stop, (uint32_t)(sg.nblocks - b.blocks), cnt, sg.block0 + b.blocks, b.dc, out))
     atomicCAS(error, 0, 1);
 }
 
@@ -713,6 +953,7 @@ struct HostComp {
 struct HostScan {
   ScanDesc sd;
   Tables tables;
+  SeqTables seq;  // the distinct ones, for the span decoder
   std::vector<Segment> segs;
   std::vector<uint8_t> bytes;  // destuffed segments
 };
@@ -853,6 +1094,7 @@ int parse_jpeg(rcg_ctx* ctx, const uint8_t* d, size_t len, Parsed& P) {
       HostScan sc;
       std::memset(&sc.sd, 0, sizeof sc.sd);
       std::memset(&sc.tables, 0, sizeof sc.tables);
+      sc.seq.n = 0;
       sc.sd.ns = ns;
       for (int i = 0; i < ns; i++) {
         const uint8_t cid = b[1 + 2 * i], t = b[2 + 2 * i];
@@ -899,6 +1141,15 @@ int parse_jpeg(rcg_ctx* ctx, const uint8_t* d, size_t len, Parsed& P) {
           return fail_parse(ctx, RCG_INVALID, "scan uses undefined huffman table");
         if (has_dc[sc.sd.dc[i]]) sc.tables.dc[sc.sd.dc[i]] = dct[sc.sd.dc[i]];
         if (has_ac[sc.sd.ac[i]]) sc.tables.ac[sc.sd.ac[i]] = act[sc.sd.ac[i]];
+        // An entry shared with an earlier component of the same slot; a scan without DC (or AC) symbols uses any.
+        auto entry = [&](const DevHuff& h, bool dc, const int* slot, const int* at) {
+          for (int j = 0; j < i; j++)
+            if (slot[j] == slot[i]) return at[j];
+          seq_huff(h, dc, &sc.seq.t[sc.seq.n]);
+          return sc.seq.n++;
+        };
+        sc.sd.tdc[i] = need_dc ? entry(sc.tables.dc[sc.sd.dc[i]], true, sc.sd.dc, sc.sd.tdc) : 0;
+        sc.sd.tac[i] = need_ac ? entry(sc.tables.ac[sc.sd.ac[i]], false, sc.sd.ac, sc.sd.tac) : 0;
       }
       // MCU pattern and geometry (decode.rs:1251-1258, :1270-1275)
       const bool inter = ns > 1;
@@ -1032,23 +1283,26 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
   if (!d_out || !d_err || !d_sd || !d_tab) return RCG_NO_MEMORY;
   cudaMemsetAsync(d_out, 0, (size_t)nblocks * 128, ctx->stream);
   cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream);
-  int h_changed = 0;
   int rounds_max = 0;
   bool fell_back = false;
   for (HostScan& sc : P.scans) {
     std::memcpy(sc.sd.fc, fc, sizeof fc);
     const long long nsub = sc.sd.nsub, nspan = sc.sd.nspan;
     // Padded: a CTA's shared-memory window covers whole units plus kTail bytes, rounded up to 16, so it may run up
-    // to one span (256 B) + kTail + 15 bytes past the last segment's data.
+    // to one span (128 B) + kTail + 15 bytes past the last segment's data.
     uint8_t* d_bytes = (uint8_t*)workspace(ctx, "dec_bytes", sc.bytes.size() + 1024);
     Segment* d_segs = (Segment*)workspace(ctx, "dec_segs", sizeof(Segment) * sc.segs.size());
-    SubState* d_s0 = (SubState*)workspace(ctx, "dec_state0", sizeof(SubState) * (size_t)nspan);
-    SubState* d_s1 = (SubState*)workspace(ctx, "dec_state1", sizeof(SubState) * (size_t)nspan);
+    const unsigned grid_span = (unsigned)((nspan + kSyncThreads - 1) / kSyncThreads);
+    SubState* d_start = (SubState*)workspace(ctx, "dec_starts", sizeof(SubState) * (size_t)nspan);
+    SubState* d_edges = (SubState*)workspace(ctx, "dec_edges", sizeof(SubState) * 2 * (size_t)grid_span);
     SubState* d_piece = (SubState*)workspace(ctx, "dec_pieces", sizeof(SubState) * (size_t)nsub);
     SubCount* d_cnt = (SubCount*)workspace(ctx, "dec_counts", sizeof(SubCount) * (size_t)nsub);
-    SubCount* d_base = (SubCount*)workspace(ctx, "dec_base", sizeof(SubCount) * (size_t)nsub);
-    int* d_changed = (int*)workspace(ctx, "dec_changed", sizeof(int));
-    if (!d_bytes || !d_segs || !d_s0 || !d_s1 || !d_piece || !d_cnt || !d_base || !d_changed) return RCG_NO_MEMORY;
+    SubCount* d_spans = (SubCount*)workspace(ctx, "dec_spans", sizeof(SubCount) * (size_t)nspan);
+    SubCount* d_base = (SubCount*)workspace(ctx, "dec_base", sizeof(SubCount) * (size_t)nspan);
+    int* d_changed = (int*)workspace(ctx, "dec_changed", sizeof(int) * kMaxRounds);
+    SeqTables* d_seq = (SeqTables*)workspace(ctx, "dec_seq_tables", sizeof(SeqTables));
+    if (!d_seq || !d_bytes || !d_segs || !d_start || !d_edges || !d_piece || !d_cnt || !d_spans || !d_base || !d_changed)
+      return RCG_NO_MEMORY;
     if (!sc.bytes.empty() && (rc = copy_to_device(ctx, d_bytes, sc.bytes.data(), sc.bytes.size())) != RCG_OK)
       return rc;
     cudaMemcpyAsync(d_segs, sc.segs.data(), sizeof(Segment) * sc.segs.size(), cudaMemcpyHostToDevice, ctx->stream);
@@ -1067,36 +1321,33 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
                  kRefineThreads, 0, d_sd, d_tab, d_segs, d_bytes, d_out, d_err);
       continue;
     }
-    // Initial guesses: every span starts at its first bit, first block of the MCU, at a block's first coefficient.
-    std::vector<SubState> init((size_t)nspan);
-    for (const Segment& g : sc.segs)
-      for (int i = 0; i < g.nspan; i++)
-        init[g.span0 + i] = SubState{(long long)i * kSpanSubs * kSubBits, 0, sc.sd.k0};
-    cudaMemcpyAsync(d_s0, init.data(), sizeof(SubState) * (size_t)nspan, cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemsetAsync(d_cnt, 0, sizeof(SubCount) * (size_t)nsub, ctx->stream);
-    const unsigned grid_span = (unsigned)((nspan + kDecThreads - 1) / kDecThreads);
+    cudaMemcpyAsync(d_seq, &sc.seq, offsetof(SeqTables, t) + sizeof(SeqHuff) * (size_t)sc.seq.n, cudaMemcpyHostToDevice,
+                    ctx->stream);
+    cudaMemsetAsync(d_changed, 0, sizeof(int) * kMaxRounds, ctx->stream);
     const unsigned grid = (unsigned)((nsub + kDecThreads - 1) / kDecThreads);
-    SubState* cur = d_s0;
-    SubState* nxt = d_s1;
+    SubState* edge_cur = d_edges;
+    SubState* edge_nxt = d_edges + grid_span;
     bool settled = false;
-    int round = 0;
-    while (round < kMaxRounds) {
-      // A few rounds back to back (most streams settle within them), then one round per check: the check of a
-      // batch looks at its last round only, which changes nothing exactly when the states have settled.
-      const int batch = round == 0 ? kFirstBatch : 1;
-      for (int b = 0; b < batch; b++, round++) {
-        if (b == batch - 1) cudaMemsetAsync(d_changed, 0, sizeof(int), ctx->stream);
-        RCG_LAUNCH(ctx, "seq_sync", k_seq_sync, grid_span, kDecThreads, 0, d_sd, d_tab, d_segs, d_bytes, cur, nxt,
-                   d_piece, d_cnt, d_changed);
-        std::swap(cur, nxt);
+    int round = 0, launched = 0;
+    while (launched < kMaxRounds && !settled) {
+      // A batch of rounds back to back, then one look at which of them changed anything. Every start is exact after as
+      // many rounds as there are CTAs.
+      const int until = (int)std::min<unsigned>(launched + std::min<unsigned>(kRoundBatch, grid_span), kMaxRounds);
+      for (; launched < until; launched++) {
+        RCG_LAUNCH(ctx, "seq_sync", k_seq_sync, grid_span, kSyncThreads, 0, d_sd, d_seq, d_segs, d_bytes, d_start,
+                   edge_cur, edge_nxt, d_piece, d_cnt, d_spans, d_changed, launched);
+        std::swap(edge_cur, edge_nxt);
       }
-      cudaMemcpyAsync(&h_changed, d_changed, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-      cudaError_t e = cudaStreamSynchronize(ctx->stream);
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "JPEG decode");
-      if (!h_changed) {
+      if (grid_span == 1) {
         settled = true;
+        round = 1;
         break;
       }
+      int h_changed[kMaxRounds];
+      cudaMemcpyAsync(h_changed, d_changed, sizeof(int) * (size_t)launched, cudaMemcpyDeviceToHost, ctx->stream);
+      cudaError_t e = cudaStreamSynchronize(ctx->stream);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "JPEG decode");
+      for (; round < launched && !settled; round++) settled = h_changed[round] == 0;
     }
     if (settled)
       rounds_max = std::max(rounds_max, round);
@@ -1104,12 +1355,12 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
       fell_back = true;
     if (!settled) {
       RCG_LAUNCH(ctx, "seq_chain", k_seq_chain, (unsigned)std::min<long long>((sc.sd.nseg + 127) / 128, 1024), 128, 0,
-                 d_sd, d_tab, d_segs, d_bytes, d_piece, d_cnt);
+                 d_sd, d_seq, d_segs, d_bytes, d_piece, d_cnt, d_spans);
     }
-    RCG_LAUNCH(ctx, "seq_prefix", k_seq_prefix, (unsigned)std::min(sc.sd.nseg, 1024), 1024, 0, d_sd, d_segs, d_cnt,
+    RCG_LAUNCH(ctx, "seq_prefix", k_seq_prefix, (unsigned)std::min(sc.sd.nseg, 1024), 1024, 0, d_sd, d_segs, d_spans,
                d_base);
-    RCG_LAUNCH(ctx, "seq_write", k_seq_write, grid, kDecThreads, 0, d_sd, d_tab, d_segs, d_bytes, d_piece, d_base,
-               d_out, d_err);
+    RCG_LAUNCH(ctx, "seq_write", k_seq_write, grid, kDecThreads, 0, d_sd, d_seq, d_segs, d_bytes, d_piece, d_cnt,
+               d_base, d_out, d_err);
   }
   int h_err = 0;
   cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
