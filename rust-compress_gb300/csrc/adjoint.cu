@@ -108,6 +108,7 @@ __device__ __forceinline__ int sample8(float v) {
 template <typename T>
 __global__ void k_lin(const uint8_t* __restrict__ ref, const float* __restrict__ dist, long long n,
                       T* __restrict__ la, T* __restrict__ lb) {
+  grid_chain();
   __shared__ T lut[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (T)c_lin8[i];
   __syncthreads();
@@ -147,6 +148,7 @@ __device__ __forceinline__ int job_of(const AdjJobs& jobs, unsigned cta) {
 template <typename T>
 __global__ void k_down(const T* __restrict__ src_a, const T* __restrict__ src_b, int w, int h, T* __restrict__ dst_a,
                        T* __restrict__ dst_b, int ow, int oh) {
+  grid_chain();
   const int ox = blockIdx.x * blockDim.x + threadIdx.x;
   if (ox >= ow) return;
   const long long n = (long long)ow * oh;
@@ -167,6 +169,7 @@ __global__ void k_down(const T* __restrict__ src_a, const T* __restrict__ src_b,
 template <typename T>
 __global__ void k_xyb(const __grid_constant__ AdjJobs jobs, const T* __restrict__ lin_a, const T* __restrict__ lin_b,
                       T* __restrict__ xyb_a, T* __restrict__ xyb_b) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const long long n = jobs.j[job].n, i = (long long)(blockIdx.x - jobs.cta0[job]) * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -253,6 +256,7 @@ __device__ __forceinline__ void store_run5(T* __restrict__ dst, long long n, lon
 template <typename T>
 __global__ void __launch_bounds__(256) k_hblur5(const __grid_constant__ AdjJobs jobs, const T* __restrict__ xa_all,
                                                 const T* __restrict__ xb_all, T* __restrict__ dst_all) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
   const int w = J.w, h = J.h, runs = (w + kHRun - 1) / kHRun;
@@ -311,6 +315,7 @@ constexpr int kRunN = 16, kRun = 8;
 template <typename T>
 __global__ void __launch_bounds__(256) k_vblur_n(const __grid_constant__ AdjJobs jobs, const T* __restrict__ src,
                                                  T* __restrict__ dst) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
   const int w = J.w, h = J.h;
@@ -343,6 +348,7 @@ __global__ void __launch_bounds__(256) k_vblur_n(const __grid_constant__ AdjJobs
 template <typename T>
 __global__ void __launch_bounds__(256) k_vblur_t(const __grid_constant__ AdjJobs jobs, const T* __restrict__ gsrc,
                                                  T* __restrict__ dst) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
   const int w = J.w, h = J.h;
@@ -394,6 +400,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_maps(const __grid_constant__ AdjJobs jobs, const T* __restrict__ mom_all,
                                               const T* __restrict__ xa_all, const T* __restrict__ xb_all,
                                               double* __restrict__ parts) {
+  grid_chain();
   __shared__ double red[6][8];
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
@@ -443,6 +450,7 @@ struct AdjSums {
 };
 __global__ void __launch_bounds__(192) k_sum_parts(const __grid_constant__ AdjJobs jobs, const __grid_constant__ AdjSums to,
                                                    const double* __restrict__ parts_all, double* __restrict__ sums_all) {
+  grid_chain();
   const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double* parts = parts_all + (size_t)jobs.cta0[blockIdx.x] * 6;
   const int nparts = (int)(jobs.cta0[blockIdx.x + 1] - jobs.cta0[blockIdx.x]);
@@ -470,6 +478,7 @@ __global__ void __launch_bounds__(256) k_mapgrad(const __grid_constant__ AdjJobs
                                                  const __grid_constant__ NormCoefs coefs, const T* __restrict__ mom_all,
                                                  const T* __restrict__ xa_all, const T* __restrict__ xb_all,
                                                  T* __restrict__ gq, T* __restrict__ gx) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
   const NormCoef& ncd = coefs.job[job];
@@ -523,6 +532,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_hblur_combine(const __grid_constant__ AdjJobs jobs, const T* __restrict__ src,
                                                        const T* __restrict__ xa_all, const T* __restrict__ xb_all,
                                                        T* __restrict__ gx) {
+  grid_chain();
   const int job = job_of(jobs, blockIdx.x);
   const AdjJob& J = jobs.j[job];
   const int w = J.w, runs = (w + kHRun - 1) / kHRun;
@@ -544,6 +554,7 @@ __global__ void __launch_bounds__(256) k_hblur_combine(const __grid_constant__ A
 template <typename T>
 __global__ void k_xyb_adj(const T* __restrict__ lin, const T* __restrict__ g_xyb, int w, int h,
                           const T* __restrict__ g_coarse, int cw, T* __restrict__ g_lin) {
+  grid_chain();
   const T M00 = (T)kM00, M01 = (T)kM01, M02 = (T)kM02, M10 = (T)kM10, M11 = (T)kM11, M12 = (T)kM12;
   const T M20 = (T)kM20, M21 = (T)kM21, M22 = (T)kM22, bias = (T)kBiasD;
   const T zero = 0, one = 1, three = 3, half = (T)0.5, seven = 7;
@@ -577,6 +588,7 @@ __global__ void k_xyb_adj(const T* __restrict__ lin, const T* __restrict__ g_xyb
 template <typename T>
 __global__ void k_grad_out(const T* __restrict__ g_lin, const float* __restrict__ dist, long long n,
                            double* __restrict__ grad) {
+  grid_chain();
   __shared__ double dlut[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) dlut[i] = c_dlin8[i];
   __syncthreads();

@@ -223,6 +223,7 @@ __device__ __forceinline__ int comp_of(const StepDesc* st, long long gb) {
 // jpeg/src/encode.rs:451-477: edge-replicated Y/Cb/Cr planes over the padded grid (Gray: Y only).
 __global__ void k_color_pad(const uint8_t* __restrict__ src, int w, int h, int channels, int pw, int ph,
                             uint8_t* __restrict__ yp, uint8_t* __restrict__ cbp, uint8_t* __restrict__ crp) {
+  grid_chain();
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= pw) return;
   for (int r = blockIdx.y; r < ph; r += gridDim.y) {
@@ -250,6 +251,7 @@ int color_pad(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, in
 // jpeg/src/encode.rs:478-499 (down): (sum + n/2) / n over fx*fy samples. Source stride pw, output (pw/fx)x(ph/fy).
 __global__ void k_chroma_down(const uint8_t* __restrict__ p, int stride, int pw, int ph, int fx, int fy,
                               uint8_t* __restrict__ o) {
+  grid_chain();
   int cw = pw / fx, ch = ph / fy;
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= cw) return;
@@ -311,6 +313,7 @@ __device__ __forceinline__ void transpose8(float (&b)[64]) {
 // One thread per block: level shift (x - 128), FDCT (jpeg/src/dct.rs:59-65), store in zigzag order
 // (flat[ZZ_T[k]], jpeg/src/encode.rs:201-211) as cache[k*nb + b].
 __global__ void k_fdct_cache(const uint8_t* __restrict__ plane, int stride, int bw, int bh, float* __restrict__ cache) {
+  grid_chain();
   long long nb = (long long)bw * bh;
   long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
@@ -415,6 +418,7 @@ __device__ __forceinline__ void quantize_body(StepDesc* __restrict__ st, const C
 }
 
 __global__ void __launch_bounds__(128, 4) k_quantize(StepDesc* __restrict__ st, CacheSet cs) {
+  grid_chain();
   quantize_body(st, cs, blockIdx.x);
 }
 
@@ -474,7 +478,7 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
   if (t == 0) st->eob[comp] = fmul(lambda, len[0]);
 }
 
-__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) { rate_tables_body(st, blockIdx.x); }
+__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) { grid_chain(); rate_tables_body(st, blockIdx.x); }
 
 int rate_tables(rcg_ctx* ctx, StepDesc* d_step) {
   RCG_LAUNCH(ctx, "rate_tables", k_rate_tables, 3, 288, 0, d_step);
@@ -723,6 +727,7 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
 
 template <bool kWeighted>
 __global__ void __launch_bounds__(128, 7) k_trellis(StepDesc* __restrict__ st, CacheSet cs) {
+  grid_chain();
   trellis_body<kWeighted>(st, cs, blockIdx.x);
 }
 
@@ -819,6 +824,7 @@ __device__ __forceinline__ void dequant_idct_body(const StepDesc* __restrict__ s
 
 __global__ void __launch_bounds__(128) k_dequant_idct(const StepDesc* __restrict__ st,
                                                      const int16_t* __restrict__ coefs, uint8_t* __restrict__ planes) {
+  grid_chain();
   dequant_idct_body(st, coefs, planes, blockIdx.x);
 }
 
@@ -971,6 +977,7 @@ __global__ void __launch_bounds__(128, 10) k_upsample_color(const StepDesc* __re
                                                              const uint8_t* __restrict__ planes, int w, int h,
                                                              uint8_t* __restrict__ rgb, float* __restrict__ lin,
                                                              int pitch) {
+  grid_chain();
   upsample_color_body(st, planes, w, h, rgb, lin, pitch, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
@@ -1032,6 +1039,7 @@ __device__ __forceinline__ void step_tables_body(const SearchState* __restrict__
 __global__ void __launch_bounds__(192) k_step_tables(const SearchState* __restrict__ ss, StepDesc* __restrict__ st,
                                                      int w, int h, int16_t* slots, long long slot_stride,
                                                      const float* pweights) {
+  grid_chain();
   step_tables_body(ss, st, w, h, slots, slot_stride, pweights);
 }
 
@@ -1047,6 +1055,7 @@ int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int w, in
 // One bisection step of every image of a lockstep batch: the same kernel bodies as one search, each launch over a
 // work-list of every image's CTAs (an image whose search has finished skips through its StepDesc's `active`).
 __global__ void __launch_bounds__(192) k_step_tables_lock(const LockItem* __restrict__ items) {
+  grid_chain();
   const LockItem& it = items[blockIdx.x];
   step_tables_body(it.ss, it.st, it.w, it.h, it.slots, it.slot_stride, nullptr);
 }
@@ -1059,22 +1068,26 @@ __device__ __forceinline__ CacheSet lock_caches(const LockItem& it) {
 }
 
 __global__ void __launch_bounds__(128, 4) k_quantize_lock(const LockItem* __restrict__ items, int n) {
+  grid_chain();
   const int i = lock_find<&LockItem::q0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   quantize_body(it.st, lock_caches(it), (long long)blockIdx.x - it.q0);
 }
 
 __global__ void __launch_bounds__(288) k_rate_tables_lock(const LockItem* __restrict__ items) {
+  grid_chain();
   rate_tables_body(items[blockIdx.y].st, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(128, 7) k_trellis_lock(const LockItem* __restrict__ items, int n) {
+  grid_chain();
   const int i = lock_find<&LockItem::q0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   trellis_body<false>(it.st, lock_caches(it), (long long)blockIdx.x - it.q0);
 }
 
 __global__ void __launch_bounds__(128) k_dequant_idct_lock(const LockItem* __restrict__ items, int n) {
+  grid_chain();
   const int i = lock_find<&LockItem::q0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   dequant_idct_body(it.st, nullptr, it.planes, (long long)blockIdx.x - it.q0);
@@ -1160,6 +1173,7 @@ void host_requant_tables(StepDesc* st, int quality, int trellis, int tq_out[3], 
 // coefficient); each component's Rdo median is the element of rank 31 among its q[1..63].
 __global__ void __launch_bounds__(192) k_step_tables_rq(const SearchState* __restrict__ ss, StepDesc* __restrict__ st,
                                                         int16_t* slots, long long slot_stride) {
+  grid_chain();
   __shared__ float rq[3][64];
   __shared__ float median[3];
   const int t = threadIdx.x;
@@ -1218,6 +1232,7 @@ int step_tables_requant(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, i
 // When the trellis pass follows, also the AC symbol histogram of the result over the blocks of the MCU grid
 // (ac_code_lengths, :155 -> :223-227, :376-398).
 __global__ void __launch_bounds__(128) k_requant_plain(StepDesc* __restrict__ st) {
+  grid_chain();
   __shared__ unsigned int sh[2][256];
   if (!st->active) return;
   const bool hist = st->use_trellis != 0;

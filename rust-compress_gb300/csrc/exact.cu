@@ -47,6 +47,7 @@ constexpr double kXC2 = 0.0009;
 // downsample (:223-247): one output sample of channel blockIdx.y.
 __global__ void __launch_bounds__(256) k_x_down(const float* __restrict__ src, int w, int h,
                                                 float* __restrict__ dst, int ow, int oh) {
+  grid_chain();
   const long long n = (long long)ow * oh;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -76,6 +77,7 @@ __device__ __forceinline__ void xyb_ref(double r, double g, double b, double out
 // XYB of rows [lo, lo + rows) of both images (:353-367): planes [3][rows][w] each.
 __global__ void __launch_bounds__(256) k_x_xyb(const float* __restrict__ a, const float* __restrict__ b, int w, int h,
                                                int lo, int rows, double* __restrict__ xa, double* __restrict__ xb) {
+  grid_chain();
   const long long n = (long long)rows * w;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -105,6 +107,7 @@ __device__ __forceinline__ double quantity(int q, const double* ra, const double
 // blur_row (:273-319) of the five quantities of one channel at one sample: h5 [5][rows][w].
 __global__ void __launch_bounds__(256) k_x_hblur(const double* __restrict__ xa, const double* __restrict__ xb, int w,
                                                  int rows, double* __restrict__ h5) {
+  grid_chain();
   const long long n = (long long)rows * w;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(256) k_x_hblur(const double* __restrict__ xa, 
 __global__ void __launch_bounds__(256) k_x_vmaps(const double* __restrict__ h5, const double* __restrict__ xa,
                                                  const double* __restrict__ xb, int w, int h, int lo, int rows,
                                                  int y0, int y1, double* __restrict__ maps) {
+  grid_chain();
   const long long no = (long long)(y1 - y0) * w;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= no) return;
@@ -178,6 +182,7 @@ __global__ void __launch_bounds__(256) k_x_vmaps(const double* __restrict__ h5, 
 // order from zero, one serial chain. maps: [3][6][orows][w] of the group; parts: [stripe][18] (c * 6 + k).
 __global__ void __launch_bounds__(32) k_x_sums(const double* __restrict__ maps, int w, int orows, int nstripes,
                                                int stripe0, double* __restrict__ parts) {
+  grid_chain();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nstripes * kScoreSums) return;
   const int j = t / kScoreSums, ck = t - j * kScoreSums;
@@ -210,6 +215,7 @@ __global__ void __launch_bounds__(32) k_x_sums(const double* __restrict__ maps, 
 
 // scale_stats (:446-466): the stripes added in order, then means and 4th roots; stats [3][6] of this scale.
 __global__ void k_x_stats(const double* __restrict__ parts, int nstripes, int w, int h, double* __restrict__ stats) {
+  grid_chain();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double count = (double)((long long)w * h);
   for (int c = 0; c < 3; c++)
@@ -223,6 +229,7 @@ __global__ void k_x_stats(const double* __restrict__ parts, int nstripes, int w,
 // ssimulacra2 (:491-511): 108 weighted terms in the reference's order, then the mapping. NaN for the reference's
 // non-finite Err.
 __global__ void k_x_final(const double* __restrict__ stats, int nscales, double* __restrict__ score) {
+  grid_chain();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double ssim = 0.0;
   int i = 0;
@@ -246,6 +253,7 @@ __global__ void k_x_final(const double* __restrict__ stats, int nscales, double*
 
 // A paused search (search_record, near tie) takes its candidate's exact score and goes on.
 __global__ void k_search_resume(SearchState* ss, const double* __restrict__ score) {
+  grid_chain();
   if (threadIdx.x != 0 || blockIdx.x != 0 || ss->done != 2) return;
   const double s = *score;
   ss->done = 0;

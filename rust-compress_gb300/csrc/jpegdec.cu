@@ -602,6 +602,7 @@ __global__ void __launch_bounds__(kSyncThreads) k_seq_sync(const ScanDesc* __res
                                                            SubCount* __restrict__ counts,
                                                            SubCount* __restrict__ span_counts,
                                                            int* __restrict__ changed, int round) {
+  grid_chain();
   if (round > 0 && changed[round - 1] == 0) return;
   constexpr int kWords = window_words(kSyncThreads, kSpanSubs * kSubBits / 8);
   __shared__ __align__(16) SeqShared<kWords> sh;
@@ -672,6 +673,7 @@ __global__ void __launch_bounds__(128) k_seq_chain(const ScanDesc* __restrict__ 
                                                    const Segment* __restrict__ segs, const uint8_t* __restrict__ data,
                                                    SubState* __restrict__ piece_state, SubCount* __restrict__ counts,
                                                    SubCount* __restrict__ span_counts) {
+  grid_chain();
   __shared__ __align__(16) SeqShared<4> sh;
   load_shared(sh, sdp, tg, segs, data, 0, 0, true);
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < sh.sd.nseg; s += gridDim.x * blockDim.x) {
@@ -694,6 +696,7 @@ __global__ void __launch_bounds__(128) k_seq_chain(const ScanDesc* __restrict__ 
 __global__ void __launch_bounds__(1024) k_seq_prefix(const ScanDesc* __restrict__ sdp, const Segment* __restrict__ segs,
                                                      const SubCount* __restrict__ span_counts,
                                                      SubCount* __restrict__ base) {
+  grid_chain();
   __shared__ SubCount total[32];
   const int nseg = sdp->nseg;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -754,6 +757,7 @@ __global__ void __launch_bounds__(kDecThreads) k_seq_write(const ScanDesc* __res
                                                            const SubCount* __restrict__ counts,
                                                            const SubCount* __restrict__ base, int16_t* __restrict__ out,
                                                            int* __restrict__ error) {
+  grid_chain();
   constexpr int kWords = window_words(kDecThreads, kSubBits / 8);
   __shared__ __align__(16) SeqShared<kWords> sh;
   const long long t0 = (long long)blockIdx.x * blockDim.x;
@@ -797,6 +801,7 @@ __device__ __forceinline__ int16_t* scan_block(const ScanDesc& sd, int16_t* out,
 __global__ void __launch_bounds__(256) k_dc_refine(const ScanDesc* __restrict__ sdp, const Segment* __restrict__ segs,
                                                    const uint8_t* __restrict__ data, long long nblocks,
                                                    int16_t* __restrict__ out) {
+  grid_chain();
   const ScanDesc& sd = *sdp;
   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
@@ -857,6 +862,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_ac_refine(const ScanDesc* __
                                                               const Segment* __restrict__ segs,
                                                               const uint8_t* __restrict__ data,
                                                               int16_t* __restrict__ out, int* __restrict__ error) {
+  grid_chain();
   __shared__ __align__(16) Tables tb;
   __shared__ ScanDesc sd;
   __shared__ __align__(16) int16_t rows[kRefineThreads][64];

@@ -41,6 +41,7 @@ template <int CH>
 __global__ void __launch_bounds__(256) k_ssim_rows(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b,
                                                    int w, int nx, int ny, double* __restrict__ rowsums,
                                                    const StepDesc* __restrict__ st) {
+  grid_chain();
   if (st && !st->active) return;
   __shared__ int gs[kWinTile + 1][CH][5];
   __shared__ double vals[kWinTile];
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(256) k_ssim_rows(const uint8_t* __restrict__ a
 
 __global__ void k_ssim_final(const double* __restrict__ rowsums, int nx, int ny, double* __restrict__ score,
                              SearchState* __restrict__ ss, const StepDesc* __restrict__ st) {
+  grid_chain();
   if (st && !st->active) return;
   if (threadIdx.x != 0) return;
   double sum = 0.0;
@@ -111,6 +113,7 @@ template <int CH>
 __global__ void __launch_bounds__(256) k_ssim_global(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b,
                                                      int w, int h, double* __restrict__ score,
                                                      SearchState* __restrict__ ss, const StepDesc* __restrict__ st) {
+  grid_chain();
   if (st && !st->active) return;
   __shared__ unsigned long long sums[CH][5];
   if (threadIdx.x < CH * 5) (&sums[0][0])[threadIdx.x] = 0;
@@ -151,6 +154,7 @@ __global__ void __launch_bounds__(256) k_ssim_global(const uint8_t* __restrict__
 // Sum of squared sample differences (psnr, core/src/metrics.rs:70): exact in 64-bit integers.
 __global__ void __launch_bounds__(256) k_sq_err(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b,
                                                 size_t n, unsigned long long* __restrict__ out) {
+  grid_chain();
   unsigned long long acc = 0;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int d = (int)a[i] - (int)b[i];
@@ -163,6 +167,7 @@ __global__ void __launch_bounds__(256) k_sq_err(const uint8_t* __restrict__ a, c
 
 // luma (core/src/metrics.rs:75-87): Gray as is, GrayAlpha's gray, else (299R + 587G + 114B + 500) / 1000.
 __global__ void k_luma(const uint8_t* __restrict__ a, size_t npx, int ch, uint8_t* __restrict__ out) {
+  grid_chain();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += (size_t)gridDim.x * blockDim.x) {
     const uint8_t* p = a + i * ch;
     out[i] = ch <= 2 ? p[0] : (uint8_t)((299u * p[0] + 587u * p[1] + 114u * p[2] + 500u) / 1000u);
@@ -171,6 +176,7 @@ __global__ void k_luma(const uint8_t* __restrict__ a, size_t npx, int ch, uint8_
 
 // downsample2 (core/src/metrics.rs:89-106): floor of the 2x2 mean, odd edges dropped.
 __global__ void k_down2(const uint8_t* __restrict__ in, int w, int nw, int nh, uint8_t* __restrict__ out) {
+  grid_chain();
   const size_t n = (size_t)nw * nh;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(i / nw), x = (int)(i % nw);

@@ -78,6 +78,7 @@ __device__ __forceinline__ int up_taps(int i, int f, int n_full, int n_c, int* x
 template <typename T>
 __global__ void __launch_bounds__(256) k_coef_grad(const double* __restrict__ g, PullDesc d,
                                                    double* __restrict__ coef_grad, double* __restrict__ energy) {
+  grid_chain();
   __shared__ double gs[4][64];
   __shared__ double tmp[4][64];
   __shared__ double wsum[8];
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(256) k_coef_grad(const double* __restrict__ g,
 // Neighbourhood RMS of the block energies (edge-replicated window, rows then columns in order).
 __global__ void k_block_sensitivity(PullDesc d, const double* __restrict__ energy, int radius,
                                     double* __restrict__ sens) {
+  grid_chain();
   const long long gb = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gb >= d.nblocks) return;
   const PullComp& pc = d.c[comp_of_block(d, gb)];
@@ -169,6 +171,7 @@ __global__ void k_block_sensitivity(PullDesc d, const double* __restrict__ energ
 // Mean sensitivity of each component: one CTA per component, fixed summation order (deterministic).
 __global__ void __launch_bounds__(1024) k_component_mean(PullDesc d, const double* __restrict__ sens,
                                                          double* __restrict__ mean) {
+  grid_chain();
   __shared__ double part[1024];
   const PullComp& pc = d.c[blockIdx.x];
   const long long nb = (long long)pc.bw * pc.bh;
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(1024) k_component_mean(PullDesc d, const doubl
 // warp writes the 32 blocks' 2048 floats as coalesced float4 rows (each value taken from its block's lane).
 __global__ void k_weights(PullDesc d, const double* __restrict__ sens, const double* __restrict__ mean,
                           PerceptualParams p, float* __restrict__ weights) {
+  grid_chain();
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 5;  // first block of the warp
   const int lane = threadIdx.x & 31;
   if (warp0 >= d.nblocks) return;
@@ -210,6 +214,7 @@ __global__ void k_weights(PullDesc d, const double* __restrict__ sens, const dou
 // 8-bit Gray or RGB -> 8-bit RGB and/or f32 RGB (Gray replicated, as the scorer does: core/src/ssimulacra2.rs:192-203).
 __global__ void k_expand_rgb(const uint8_t* __restrict__ src, int channels, size_t npx, uint8_t* __restrict__ rgb8,
                              float* __restrict__ rgbf) {
+  grid_chain();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += (size_t)gridDim.x * blockDim.x) {
     uint8_t v[3];
     if (channels == 1) {

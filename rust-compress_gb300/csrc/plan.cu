@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(kThreads) k_plan_blocks(const PlanDesc* __rest
                                                           const int16_t* __restrict__ coefs, ScanStats* stats,
                                                           uint16_t* __restrict__ flags, int* __restrict__ chunk_last,
                                                           unsigned long long* __restrict__ chunk_pend) {
+  grid_chain();
   __shared__ unsigned hist[2][2][256];
   __shared__ int s_scan, last_sym;
   __shared__ unsigned long long pend_sum;
@@ -324,6 +325,7 @@ __device__ __forceinline__ void block_scan(int m, unsigned long long p, int* m_e
 __global__ void __launch_bounds__(1024) k_plan_chunks(const PlanDesc* __restrict__ pd, const int* chunk_last,
                                                       const unsigned long long* chunk_pend, int* chunk_prev,
                                                       unsigned long long* chunk_pbase) {
+  grid_chain();
   const ScanDesc sc = pd->scan[blockIdx.x];
   if (sc.kind != kAcFirst && sc.kind != kAcRefine) return;
   const long long nch = (sc.npos + kChunk - 1) / kChunk;
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(kThreads) k_plan_prefix(const PlanDesc* __rest
                                                           const unsigned long long* __restrict__ chunk_pbase,
                                                           int* __restrict__ prev, unsigned long long* __restrict__ P,
                                                           int* __restrict__ prev_end) {
+  grid_chain();
   __shared__ int s_scan;
   const long long chunk = blockIdx.x;
   if (threadIdx.x == 0) s_scan = find_scan(pd, chunk);
@@ -397,6 +400,7 @@ __global__ void __launch_bounds__(kThreads) k_plan_eobruns(const PlanDesc* __res
                                                            const int* __restrict__ prev,
                                                            const unsigned long long* __restrict__ P,
                                                            const int* __restrict__ prev_end, ScanStats* stats) {
+  grid_chain();
   __shared__ int s_scan;
   __shared__ unsigned cnt[16];
   __shared__ unsigned long long raw_sh;
@@ -475,6 +479,7 @@ __global__ void __launch_bounds__(kThreads) k_plan_eobruns(const PlanDesc* __res
 // (encode.rs:552-560), empty or not.
 __global__ void __launch_bounds__(288) k_plan_tables(const PlanDesc* __restrict__ pd, const ScanStats* stats,
                                                      unsigned long long* table_bits, int* dht_bytes) {
+  grid_chain();
   __shared__ unsigned freq[kHuffSyms];
   __shared__ unsigned char lens[kHuffSyms];
   __shared__ HuffScratch scratch;
@@ -519,6 +524,7 @@ __global__ void __launch_bounds__(288) k_plan_tables(const PlanDesc* __restrict_
 __global__ void __launch_bounds__(256) k_plan_choose(const PlanDesc* __restrict__ pd, const ScanStats* stats,
                                                      const unsigned long long* table_bits, const int* dht_bytes,
                                                      PlanOut* out) {
+  grid_chain();
   __shared__ unsigned long long cost[kMaxScans];
   __shared__ unsigned long long best_v[256];
   __shared__ int best_i[256];

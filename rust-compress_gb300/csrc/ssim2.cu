@@ -581,6 +581,7 @@ template <int kRef>
 __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
     k_ssim2_tiles(PyramidDesc pd, const float* __restrict__ ref, const float* __restrict__ dist,
                   double* __restrict__ partials, const StepDesc* __restrict__ st, float2* __restrict__ refm) {
+  grid_chain();
   if (st && !st->active) return;
   const int blk = blockIdx.x;
   int s = 0;
@@ -653,6 +654,7 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce(PyramidDesc pd, const doub
                                                       double* __restrict__ scale_sums, unsigned* __restrict__ counter,
                                                       double* __restrict__ score_out, SearchState* __restrict__ ss,
                                                       const StepDesc* __restrict__ st) {
+  grid_chain();
   if (st && !st->active) return;
   reduce_scale_sum(pd, partials, scale_sums, counter, score_out, ss);
 }
@@ -746,6 +748,7 @@ __device__ __forceinline__ void image_quad(const ImageSrc& im, int x0, int y, co
 
 // Linear planes [3][h][pitch] of an image (the reference-order scorer's input).
 __global__ void __launch_bounds__(256) k_to_linear(const ImageSrc im, int pitch, float* __restrict__ out) {
+  grid_chain();
   // The table lives in shared memory: per-thread indices differ, which would serialize constant-memory reads.
   __shared__ float lut8[256];
   lut8[threadIdx.x] = c_lut8s[threadIdx.x];
@@ -1069,6 +1072,7 @@ template <int kSrc, int kOut, bool kGray>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const __grid_constant__ PyramidDesc pd,
                                                                         const __grid_constant__ BuildArgs g,
                                                                         const StepDesc* __restrict__ gate) {
+  grid_chain();
   if (gate && !gate->active) return;
   __shared__ float lut[256];
   __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
@@ -1080,9 +1084,9 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const _
 template <int kSrc, int kOut>
 void launch_build(const PyramidDesc& pd, const BuildArgs& g, const StepDesc* st, cudaStream_t stream) {
   if (kSrc != kFromLinear && pd.s[0].planes == 1)
-    k_build<kSrc, kOut, kSrc != kFromLinear><<<pyramid_ctas(pd), kPyrThreads, 0, stream>>>(pd, g, st);
+    launch_chained(pyramid_ctas(pd), kPyrThreads, 0, stream, k_build<kSrc, kOut, kSrc != kFromLinear>, pd, g, st);
   else
-    k_build<kSrc, kOut, false><<<pyramid_ctas(pd), kPyrThreads, 0, stream>>>(pd, g, st);
+    launch_chained(pyramid_ctas(pd), kPyrThreads, 0, stream, k_build<kSrc, kOut, false>, pd, g, st);
 }
 
 // ------------------------------------------------------------------------------------------------ work-list scorer
@@ -1130,6 +1134,7 @@ __device__ __forceinline__ int find_first(const long long* __restrict__ first, i
 template <int kOut>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build_batch(const BuildJob* __restrict__ jobs,
                                                                               const long long* __restrict__ cta0, int n) {
+  grid_chain();
   const int i = find_first(cta0, n, blockIdx.x);
   const BuildJob& j = jobs[i];
   build_block<kFromImage, kOut>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
@@ -1140,6 +1145,7 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build_batch(c
 // at k = 3 / 2 / 1 against 21.1 ms here, because the block scheduler hands tiles to whichever CTA slot frees first.
 __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRefNone))
     k_ssim2_tiles_batch(const TileSeg* __restrict__ segs, const long long* __restrict__ seg0, int nseg) {
+  grid_chain();
   const long long t = blockIdx.x;
   const int g = find_first(seg0, nseg, t);
   const TileSeg sg = segs[g];
@@ -1163,6 +1169,7 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_batch(const ScoreItem* __r
                                                             double* __restrict__ scale_sums,
                                                             unsigned* __restrict__ counters,
                                                             double* __restrict__ scores) {
+  grid_chain();
   const int p = blockIdx.z;
   const ScoreItem& it = items[p];
   if ((int)blockIdx.x >= it.pd.nscales) return;
@@ -1177,6 +1184,7 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_batch(const ScoreItem* __r
 // finished skips through its StepDesc's `active`.
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOutDiff)) k_build_lock(const LockItem* __restrict__ items,
                                                                                   int n) {
+  grid_chain();
   const int i = lock_find<&LockItem::p0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   if (!it.st->active) return;
@@ -1191,6 +1199,7 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOutDiff)) k_build_loc
 
 template <int kRef>
 __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_lock(const LockItem* __restrict__ items, int n) {
+  grid_chain();
   const int i = lock_find<&LockItem::t0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
   if (!it.st->active) return;
@@ -1203,6 +1212,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_l
 }
 
 __global__ void __launch_bounds__(256) k_ssim2_reduce_lock(const LockItem* __restrict__ items) {
+  grid_chain();
   const LockItem& it = items[blockIdx.z];
   if (!it.st->active || (int)blockIdx.x >= it.pd.nscales) return;
   reduce_scale_sum(it.pd, it.partials, it.scale_sums, it.counter, it.score, it.ss);
@@ -1429,6 +1439,7 @@ PyramidDesc banded(const PyramidDesc& pd, int nch0, int min_tiles) {
 // Deterministic stand-in content for the tuning runs (linear values in [0, 1), the second image a perturbed copy);
 // the kernel's time does not depend on the values.
 __global__ void k_tune_fill(float* __restrict__ p, long long n) {
+  grid_chain();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     uint32_t x = (uint32_t)(i % (n / 2)) * 2654435761u;
     x ^= x >> 15;
@@ -1784,9 +1795,9 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   g.xyb = pyr_ref;
   g.out = pyr_dist;
   launch_build<kFromImage, kOutPair>(pd, g, nullptr, s);
-  k_ssim2_tiles<kRefNone><<<pd.total_tiles, kTileThreads, tile_smem(kRefNone), s>>>(pd, pyr_ref, pyr_dist, partials, nullptr,
-                                                                        nullptr);
-  k_ssim2_reduce<<<dim3(pd.nscales, kScoreSums), 256, 0, s>>>(pd, partials, sums, counter, d_score, nullptr,
+  launch_chained(pd.total_tiles, kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref, pyr_dist,
+                 partials, nullptr, nullptr);
+  launch_chained(dim3(pd.nscales, kScoreSums), 256, 0, s, k_ssim2_reduce, pd, partials, sums, counter, d_score, nullptr,
                                                               nullptr);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? RCG_OK : RCG_CUDA_ERROR;
