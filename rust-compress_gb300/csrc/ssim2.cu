@@ -227,7 +227,7 @@ __device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) 
 // moment pairs that share a tap weight as packed two-lane f32 FMAs, each lane exactly fmaf.
 // Offsets: every chunk takes the XYB and XYB difference at its own centre.
 // Band `local` of scale `sd` (sd.tiles_x bands across; sd.nch chunks each); the band's 18 sums go to out[i * stride],
-// i < 18.
+// i < 18. one: the channel to score (its six sums are written), -1: all; every thread of the CTA passes the same.
 // Reference moments (kRef). The offsets a chunk subtracts from `a` come from the reference alone, so the blurred a' and
 // a'^2 of every output pixel depend on the reference and the band layout only. A search scores every candidate against
 // one reference: its first candidate runs kRef = kRefWrite, which also stores (blur a', blur a'^2) per output pixel and
@@ -245,8 +245,8 @@ __device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) 
 // measured 282, 4 287), 4 for the other forms (5 faster at 4K by 1%, slower in a batch by 4%). Quad offsets kept over a
 // chunk's channels measured 278, the maps of two rows as packed operations 273 but 242 plain: neither was kept.
 template <int kRef>
-__device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, const float* __restrict__ xa,
-                                           const float* __restrict__ xd, double* __restrict__ out,
+__device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, const int one,
+                                           const float* __restrict__ xa, const float* __restrict__ xd, double* __restrict__ out,
                                            const size_t stride, float2* __restrict__ refm) {
   extern __shared__ float4 smem4[];
   float* const xs = reinterpret_cast<float*>(smem4);  // the channel's a, then its d
@@ -260,10 +260,12 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
   const int x0 = tx * kTileW, ybeg = ty * kTileH * nch;
   const int w = sd.w, h = sd.h, pitch = sd.pitch;
   const size_t np = (size_t)pitch * h;
-  // Channels to score: all, or Y alone (ScaleDesc::planes), which is then the only plane.
-  const int ch0 = sd.planes == 1 ? 1 : 0, ch1 = sd.planes == 1 ? 2 : 3;
-  const float* pa = xa + sd.off;
-  const float* pd = xd + sd.off;
+  // Channels to score: all, or Y alone (ScaleDesc::planes), which is then the only plane, or channel `one` of three.
+  const bool split = one >= 0 && sd.planes != 1;
+  if (one > 0 && !split) return;
+  const int ch0 = sd.planes == 1 ? 1 : split ? one : 0, ch1 = sd.planes == 1 ? 2 : split ? one + 1 : 3;
+  const float* pa = xa + sd.off + (split ? one * np : 0);  // the planes of channel ch0
+  const float* pd = xd + sd.off + (split ? one * np : 0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   float sums[kScoreSums];
@@ -570,12 +572,20 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
     if (lane == 0) s_red[warp][i] = v;
   }
   __syncthreads();
-  if (tid < kScoreSums) {
+  if (tid < kScoreSums && (!split || tid / 6 == one)) {
     double acc = 0.0;
     for (int wi = 0; wi < kTileThreads / 32; wi++) acc += (double)s_red[wi][tid];
     out[(size_t)tid * stride] = acc;  // sum-major: the reduction reads each sum contiguously
   }
 }
+
+// Launches of few bands are latency-bound (a CTA's three channels one after the other): there each band is three CTAs, one
+// per channel. The sums are per channel, so they are the same bits. Measured, whole bands / split: 66 bands (240x180)
+// 17.9 / 10.6 us, 340 (512x512, without reference moments) 20.0 / 18.0, 977 (0.8 MP) 43.3 / 41.4, 2300 (1.7 MP) 56.5 /
+// 57.5, 12 MP 278 / 304: a CTA's start and end weigh more once the bands fill the chip.
+constexpr int kSplitTiles = 1024;
+__device__ __forceinline__ int channel_of_cta() { return gridDim.y == 1 ? -1 : (int)blockIdx.y; }
+dim3 tile_grid(long long ctas) { return dim3((unsigned)ctas, ctas <= kSplitTiles ? 3 : 1); }
 
 template <int kRef>
 __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
@@ -587,7 +597,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
   int s = 0;
   while (s + 1 < pd.nscales && blk >= pd.s[s + 1].tile0) s++;
   const ScaleDesc sd = pd.s[s];
-  ssim2_band<kRef>(sd, blk - sd.tile0, ref, dist, partials + blk, (size_t)pd.total_tiles, refm);
+  ssim2_band<kRef>(sd, blk - sd.tile0, channel_of_cta(), ref, dist, partials + blk, (size_t)pd.total_tiles, refm);
 }
 
 // Deterministic reduction of the per-tile sums: CTA (scale, sum index); the last CTA to finish computes the score
@@ -1160,7 +1170,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRefNone))
   sd.nch = sg.nch;
   sd.off = 0;
   const int local = (int)(t - __ldg(seg0 + g));
-  ssim2_band<kRefNone>(sd, local, sg.ref, sg.dist, sg.out + local, (size_t)sg.stride, nullptr);
+  ssim2_band<kRefNone>(sd, local, channel_of_cta(), sg.ref, sg.dist, sg.out + local, (size_t)sg.stride, nullptr);
 }
 
 // CTA (scale, sum, pair); scale_sums [n][kMaxScales][18], counters and scores [n].
@@ -1207,7 +1217,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_l
   int s = 0;
   while (s + 1 < it.pd.nscales && blk >= it.pd.s[s + 1].tile0) s++;
   const ScaleDesc sd = it.pd.s[s];
-  ssim2_band<kRef>(sd, blk - sd.tile0, it.ref_xyb, it.dist_pyr, it.partials + blk, (size_t)it.pd.total_tiles,
+  ssim2_band<kRef>(sd, blk - sd.tile0, channel_of_cta(), it.ref_xyb, it.dist_pyr, it.partials + blk, (size_t)it.pd.total_tiles,
                    it.refm);
 }
 
@@ -1223,15 +1233,15 @@ void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_t
   RCG_LAUNCH(ctx, "build_lock", k_build_lock, (unsigned)p_total, kPyrThreads, 0, d_items, n);
   // Every image of the batch is at the same step: the first stores its reference moments, the later ones read them.
   if (ref_mode == kRefWrite)
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefWrite>, (unsigned)t_total, kTileThreads,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefWrite>, tile_grid(t_total), kTileThreads,
                tile_smem(kRefWrite),
                d_items, n);
   else if (ref_mode == kRefRead)
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefRead>, (unsigned)t_total, kTileThreads,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefRead>, tile_grid(t_total), kTileThreads,
                tile_smem(kRefRead),
                d_items, n);
   else
-    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefNone>, (unsigned)t_total, kTileThreads,
+    RCG_LAUNCH(ctx, "ssim2_tiles_lock", k_ssim2_tiles_lock<kRefNone>, tile_grid(t_total), kTileThreads,
                tile_smem(kRefNone),
                d_items, n);
   RCG_LAUNCH(ctx, "ssim2_reduce_lock", k_ssim2_reduce_lock, dim3(max_scales, kScoreSums, n), 256, 0, d_items);
@@ -1533,13 +1543,13 @@ int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, cons
   unsigned* counter = (unsigned*)ctx->bufs["score_counter"].ptr;
   const PyramidDesc pb = plan_bands(ctx, pd);
   if (!refm || ref_mode == kRefNone)
-    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, pb.total_tiles, kTileThreads, tile_smem(kRefNone), pb, d_ref, d_dist,
+    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefNone), pb, d_ref, d_dist,
                partials, step, nullptr);
   else if (ref_mode == kRefWrite)
-    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, pb.total_tiles, kTileThreads, tile_smem(kRefWrite), pb, d_ref,
+    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefWrite), pb, d_ref,
                d_dist, partials, step, refm);
   else
-    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, pb.total_tiles, kTileThreads, tile_smem(kRefRead), pb, d_ref,
+    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefRead), pb, d_ref,
                d_dist, partials, step, refm);
   dim3 rg(pb.nscales, kScoreSums);
   RCG_LAUNCH(ctx, "ssim2_reduce", k_ssim2_reduce, rg, 256, 0, pb, partials, scale_sums, counter, d_score, search,
@@ -1701,7 +1711,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
     if (nj[2])
       RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutPair>, (unsigned)ctas[2], kPyrThreads, 0, d_jobs(2), d_first(2),
                  nj[2]);
-    RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, (unsigned)tiles, kTileThreads, tile_smem(kRefNone), d_segs,
+    RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, tile_grid(tiles), kTileThreads, tile_smem(kRefNone), d_segs,
                d_seg0, nseg);
     RCG_LAUNCH(ctx, "ssim2_reduce_batch", k_ssim2_reduce_batch, dim3(max_scales, kScoreSums, n), 256, 0, d_items,
                partials, sums, counters, scores);
@@ -1795,7 +1805,7 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   g.xyb = pyr_ref;
   g.out = pyr_dist;
   launch_build<kFromImage, kOutPair>(pd, g, nullptr, s);
-  launch_chained(pd.total_tiles, kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref, pyr_dist,
+  launch_chained(tile_grid(pd.total_tiles), kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref, pyr_dist,
                  partials, nullptr, nullptr);
   launch_chained(dim3(pd.nscales, kScoreSums), 256, 0, s, k_ssim2_reduce, pd, partials, sums, counter, d_score, nullptr,
                                                               nullptr);
