@@ -830,16 +830,17 @@ struct BuildArgs {
   ImageSrc im[2];         // kFromImage
 };
 
-constexpr int kPyrT = 64;         // scale-0 block of a CTA
+constexpr int kPyrT = 64;       // scale-0 block of a CTA
+constexpr int kPyrTSmall = 32;  // of a small image (kSmallBuild)
 constexpr int kPyrThreads = 256;
 // Rows of a level's block in shared memory, padded so that quads stay 16-byte aligned; where each level starts.
-__device__ __forceinline__ constexpr int lev_pitch(int L) { return (kPyrT >> L) + 4; }
-__device__ __forceinline__ constexpr int lev_off(int L) {
+__device__ __forceinline__ constexpr int lev_pitch(int T, int L) { return (T >> L) + 4; }
+__device__ __forceinline__ constexpr int lev_off(int T, int L) {
   int o = 0;
-  for (int k = 1; k < L; k++) o += lev_pitch(k) * (kPyrT >> k);
+  for (int k = 1; k < L; k++) o += lev_pitch(T, k) * (T >> k);
   return o;
 }
-constexpr int kLevFloats = 36 * 32 + 20 * 16 + 12 * 8 + 8 * 4 + 6 * 2;  // one channel's levels 1-5
+constexpr int kLevFloats = 36 * 32 + 20 * 16 + 12 * 8 + 8 * 4 + 6 * 2;  // one channel's levels 1-5 (of the larger block)
 
 int pyramid_ctas(const PyramidDesc& pd) {
   return ((pd.s[0].w + kPyrT - 1) / kPyrT) * ((pd.s[0].h + kPyrT - 1) / kPyrT);
@@ -914,21 +915,27 @@ __device__ __forceinline__ void emit_quad(const BuildArgs& g, const ScaleDesc& s
   }
 }
 
-// The two samples of a row of the coarsest level's 2x2 block.
+// The two samples of a row of a level's 2x2 block, or its only one (`single`).
 template <int kOut, bool kGray>
-__device__ __forceinline__ void emit_pair(const BuildArgs& g, const ScaleDesc& sd, int x, int y, const float (&l)[3][4],
-                                          const float (&l2)[3][4]) {
+__device__ __forceinline__ void emit_pair(const BuildArgs& g, const ScaleDesc& sd, int x, int y, bool single,
+                                          const float (&l)[3][4], const float (&l2)[3][4]) {
   const size_t np = (size_t)sd.pitch * sd.h, i = (size_t)sd.off + (size_t)y * sd.pitch + x;
   auto at = [](const float (&v)[3][4], int c) { return make_float2(v[c][0], v[c][1]); };
   auto put2 = [&](float* p, const float2 (&v)[3]) {
 #pragma unroll
-    for (int c = 0; c < (kGray ? 1 : 3); c++) *reinterpret_cast<float2*>(p + c * np + i) = v[c];
+    for (int c = 0; c < (kGray ? 1 : 3); c++) {
+      if (single) p[c * np + i] = v[c].x;
+      else *reinterpret_cast<float2*>(p + c * np + i) = v[c];
+    }
   };
   float2 o[3];
   if constexpr (kOut == kOutDiff) {
     float2 r[3];
 #pragma unroll
-    for (int c = 0; c < (kGray ? 1 : 3); c++) r[c] = __ldg(reinterpret_cast<const float2*>(g.ref + c * np + i));
+    for (int c = 0; c < (kGray ? 1 : 3); c++) {
+      const float* q = g.ref + c * np + i;
+      r[c] = single ? make_float2(__ldg(q), 0.f) : __ldg(reinterpret_cast<const float2*>(q));
+    }
     if constexpr (kGray) o[0] = gray_diff2(r[0], at(l, 0));
     else pix_diff2(r[0], r[1], r[2], at(l, 0), at(l, 1), at(l, 2), o);
     put2(g.out, o);
@@ -948,24 +955,25 @@ __device__ __forceinline__ void emit_pair(const BuildArgs& g, const ScaleDesc& s
 }
 
 // Block `blk` of a pyramid. Every thread of the CTA calls it.
-template <int kSrc, int kOut, bool kGray>
+template <int kSrc, int kOut, bool kGray, int T>
 __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildArgs& g, const int blk, float* lut,
                                              float (*lev)[3][kLevFloats]) {
   constexpr int kImgs = kOut == kOutPair ? 2 : 1, kCh = kGray ? 1 : 3;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  constexpr int kRowQuads = T / 4, kRows = kPyrThreads / kRowQuads;  // of a slab
+  const int t = threadIdx.x, lane = t & 31;
   if constexpr (kSrc != kFromLinear) {
     lut[t] = c_lut8s[t];
     __syncthreads();
   }
   const ScaleDesc s0 = pd.s[0];
   const int w = s0.w, h = s0.h;
-  const int bx = (w + kPyrT - 1) / kPyrT, tx = blk % bx, ty = blk / bx;
-  const int quad = t & 15, x0 = tx * kPyrT + 4 * quad;
-  const bool lower = lane >= 16;  // the odd row of the warp's row pair
+  const int bx = (w + T - 1) / T, tx = blk % bx, ty = blk / bx;
+  const int quad = t % kRowQuads, x0 = tx * T + 4 * quad;
+  const bool lower = (lane & kRowQuads) != 0;  // the odd row of a row pair
 #pragma unroll 1
-  for (int slab = 0; slab < kPyrT / 16; slab++) {
-    const int y = ty * kPyrT + slab * 16 + (t >> 4);
-    if (ty * kPyrT + slab * 16 >= h) break;
+  for (int slab = 0; slab < T / kRows; slab++) {
+    const int y = ty * T + slab * kRows + t / kRowQuads;
+    if (ty * T + slab * kRows >= h) break;
     float l[kImgs][3][4];
     if (x0 < w && y < h) {
       float4 rq[3];
@@ -988,18 +996,18 @@ __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildA
       }
       emit_quad<kOut, kGray>(g, s0, x0, y, rq, l[0], l[kImgs - 1]);
     }
-    // Scale 1: the upper half of the warp makes the quad's left sample, the lower half its right one.
+    // Scale 1: the row pair's upper lane makes the quad's left sample, the lower one its right one.
     if (pd.nscales > 1) {
       const int col = x0 + (lower ? 2 : 0), top = y - (lower ? 1 : 0);
 #pragma unroll
       for (int m = 0; m < kImgs; m++)
 #pragma unroll
         for (int c = 0; c < kCh; c++) {
-          const float p0 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][0] : l[m][c][2], 16);
-          const float p1 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][1] : l[m][c][3], 16);
+          const float p0 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][0] : l[m][c][2], kRowQuads);
+          const float p1 = __shfl_xor_sync(0xffffffffu, lower ? l[m][c][1] : l[m][c][3], kRowQuads);
           const float v = lower ? block_mean(p0, p1, l[m][c][2], l[m][c][3], col + 1 < w, top + 1 < h)
                                 : block_mean(l[m][c][0], l[m][c][1], p0, p1, col + 1 < w, top + 1 < h);
-          lev[m][c][(slab * 8 + warp) * lev_pitch(1) + 2 * quad + (lower ? 1 : 0)] = v;
+          lev[m][c][(slab * kRows + t / kRowQuads) / 2 * lev_pitch(T, 1) + 2 * quad + (lower ? 1 : 0)] = v;
         }
     }
   }
@@ -1008,7 +1016,7 @@ __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildA
   for (int L = 2; L < kMaxScales; L++) {
     __syncthreads();
     if (L >= pd.nscales) break;
-    const int n = kPyrT >> L;
+    const int n = T >> L;
     if (t < n * n) {
       const int lx = t % n, ly = t / n;
       const int ax = 2 * (tx * n + lx), ay = 2 * (ty * n + ly);  // the block's origin in the level above
@@ -1018,37 +1026,40 @@ __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildA
         for (int m = 0; m < kImgs; m++)
 #pragma unroll
           for (int c = 0; c < kCh; c++) {
-            const float* q = &lev[m][c][lev_off(L - 1) + 2 * ly * lev_pitch(L - 1) + 2 * lx];
-            lev[m][c][lev_off(L) + ly * lev_pitch(L) + lx] =
-                block_mean(q[0], q[1], q[lev_pitch(L - 1)], q[lev_pitch(L - 1) + 1], ax + 1 < aw, ay + 1 < ah);
+            const float* q = &lev[m][c][lev_off(T, L - 1) + 2 * ly * lev_pitch(T, L - 1) + 2 * lx];
+            lev[m][c][lev_off(T, L) + ly * lev_pitch(T, L) + lx] =
+                block_mean(q[0], q[1], q[lev_pitch(T, L - 1)], q[lev_pitch(T, L - 1) + 1], ax + 1 < aw, ay + 1 < ah);
           }
       }
     }
   }
   __syncthreads();
-  // Then written: the 256 quads of level 1, and in a second trip the 84 of levels 2-4 and the two pairs of level 5.
+  // Then written. Of a 64 block: the 256 quads of level 1, and in a second trip the 84 of levels 2-4 and the two pairs of
+  // level 5. Of a 32 block, in one: the 84 quads of levels 1-3, the two pairs of level 4 and the sample of level 5.
 #pragma unroll 1
-  for (int trip = 0; trip < 2; trip++) {
+  for (int trip = 0; trip < (T == 64 ? 2 : 1); trip++) {
     int L = 1, e = t;
-    if (trip) {
-      if (t >= 86) break;
-      L = t < 64 ? 2 : t < 80 ? 3 : t < 84 ? 4 : 5;
-      e = t - (L == 2 ? 0 : L == 3 ? 64 : L == 4 ? 80 : 84);
+    if (T == 32 || trip) {
+      if (t >= (T == 64 ? 86 : 87)) break;
+      const int k = t < 64 ? 0 : t < 80 ? 1 : t < 84 ? 2 : t < 86 ? 3 : 4;
+      L = k + (T == 64 ? 2 : 1);
+      e = t - (k == 0 ? 0 : k == 1 ? 64 : k == 2 ? 80 : k == 3 ? 84 : 86);
     }
     if (L >= pd.nscales) continue;
     const ScaleDesc sd = pd.s[L];
-    const int n = kPyrT >> L, nq = L == 5 ? 1 : n / 4;  // quads of a row (level 5: half a quad)
+    const int n = T >> L, nq = n < 4 ? 1 : n / 4;  // quads of a row (a pair or a sample counts as one)
     const int lx = 4 * (e % nq), ly = e / nq;
     const int x = tx * n + lx, y = ty * n + ly;
     if (x >= sd.w || y >= sd.h) continue;
-    const int at = (L == 1 ? lev_off(1) : L == 2 ? lev_off(2) : L == 3 ? lev_off(3) : L == 4 ? lev_off(4) : lev_off(5)) +
+    const int at = (L == 1 ? lev_off(T, 1) : L == 2 ? lev_off(T, 2) : L == 3 ? lev_off(T, 3) : L == 4 ? lev_off(T, 4)
+                                                                                                 : lev_off(T, 5)) +
                    ly * (n + 4) + lx;
     float l[kImgs][3][4];
 #pragma unroll
     for (int m = 0; m < kImgs; m++)
 #pragma unroll
       for (int c = 0; c < kCh; c++) {
-        // a row is padded by four samples, so the quad of a level-5 pair stays in its row
+        // a row is padded by four samples, so the quad of a pair or a single sample stays in its row
         const float2 a = *reinterpret_cast<const float2*>(&lev[m][c][at]);
         const float2 b = *reinterpret_cast<const float2*>(&lev[m][c][at + 2]);
         l[m][c][0] = a.x;
@@ -1056,12 +1067,12 @@ __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildA
         l[m][c][2] = b.x;
         l[m][c][3] = b.y;
       }
-    if (L < 5) {
+    if (n >= 4) {
       float4 rq[3];
       ref_quad<kOut, kGray>(g, sd, x, y, rq);
       emit_quad<kOut, kGray>(g, sd, x, y, rq, l[0], l[kImgs - 1]);
     } else {
-      emit_pair<kOut, kGray>(g, sd, x, y, l[0], l[kImgs - 1]);
+      emit_pair<kOut, kGray>(g, sd, x, y, n == 1, l[0], l[kImgs - 1]);
     }
   }
 }
@@ -1071,14 +1082,14 @@ template <int kSrc, int kOut>
 __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildArgs& g, const int blk) {
   __shared__ float lut[256];
   __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
-  if (pd.s[0].planes == 1) build_planes<kSrc, kOut, true>(pd, g, blk, lut, lev);
-  else build_planes<kSrc, kOut, false>(pd, g, blk, lut, lev);
+  if (pd.s[0].planes == 1) build_planes<kSrc, kOut, true, kPyrT>(pd, g, blk, lut, lev);
+  else build_planes<kSrc, kOut, false, kPyrT>(pd, g, blk, lut, lev);
 }
 
 // CTAs per SM: a pair's conversion keeps two images' samples in registers.
 constexpr int build_ctas(int out) { return out == kOutPair ? 3 : 4; }
 
-template <int kSrc, int kOut, bool kGray>
+template <int kSrc, int kOut, bool kGray, int T>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const __grid_constant__ PyramidDesc pd,
                                                                         const __grid_constant__ BuildArgs g,
                                                                         const StepDesc* __restrict__ gate) {
@@ -1086,17 +1097,32 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const _
   if (gate && !gate->active) return;
   __shared__ float lut[256];
   __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
-  build_planes<kSrc, kOut, kGray>(pd, g, blockIdx.x, lut, lev);
+  build_planes<kSrc, kOut, kGray, T>(pd, g, blockIdx.x, lut, lev);
 }
+
+// Images of at most this many 64x64 blocks are built by 32x32 blocks: one slab of level 0 and one trip for the others per
+// CTA, where a 64 block takes four and two, one after the other. The same samples either way. Measured, 64 / 32: 12 blocks
+// (240x180) 16.6 / 10.7 us, 64 (512x512, a pair) 22.8 / 14.9, 294 (0.8 MP) 24.4 / 26.4, 442 (1.7 MP) 30.8 / 35.0: most
+// threads of a 32 block idle while the levels above 0 are converted.
+constexpr int kSmallBuild = 152;
 
 // Queue one builder launch (st: the step that gates it, nullable). Samples that come as linear planes are never gray
 // ones: a gray layout is always read directly.
 template <int kSrc, int kOut>
 void launch_build(const PyramidDesc& pd, const BuildArgs& g, const StepDesc* st, cudaStream_t stream) {
-  if (kSrc != kFromLinear && pd.s[0].planes == 1)
-    launch_chained(pyramid_ctas(pd), kPyrThreads, 0, stream, k_build<kSrc, kOut, kSrc != kFromLinear>, pd, g, st);
-  else
-    launch_chained(pyramid_ctas(pd), kPyrThreads, 0, stream, k_build<kSrc, kOut, false>, pd, g, st);
+  constexpr bool kGray = kSrc != kFromLinear;
+  const int ctas = pyramid_ctas(pd);
+  if (ctas <= kSmallBuild) {
+    const int n = ((pd.s[0].w + kPyrTSmall - 1) / kPyrTSmall) * ((pd.s[0].h + kPyrTSmall - 1) / kPyrTSmall);
+    if (kGray && pd.s[0].planes == 1)
+      launch_chained(n, kPyrThreads, 0, stream, k_build<kSrc, kOut, kGray, kPyrTSmall>, pd, g, st);
+    else
+      launch_chained(n, kPyrThreads, 0, stream, k_build<kSrc, kOut, false, kPyrTSmall>, pd, g, st);
+  } else if (kGray && pd.s[0].planes == 1) {
+    launch_chained(ctas, kPyrThreads, 0, stream, k_build<kSrc, kOut, kGray, kPyrT>, pd, g, st);
+  } else {
+    launch_chained(ctas, kPyrThreads, 0, stream, k_build<kSrc, kOut, false, kPyrT>, pd, g, st);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ work-list scorer

@@ -1,5 +1,6 @@
-"""A scorer launch of few bands scores one channel per CTA. That changes no sum, so a score has the same bits as in a work-list
-of many bands."""
+"""Small images take forms of their own in the scorer: a launch of few bands scores one channel per CTA, and an image of few
+64x64 blocks is built by 32x32 blocks. Neither changes a sample or a sum, so a score has the same bits as in a work-list
+large enough to take the forms of large images."""
 
 import numpy as np
 import pytest
@@ -17,7 +18,8 @@ def _pair(w, h, gray, seed):
     return ref, np.clip(ref.astype(int) + noise, 0, 255).astype(np.uint8)
 
 
-# Up to 1024 bands (768 + 192 + 48 + 12 + 3 + 1) and a few more.
+# Single samples and pairs at the last scales; one 32 block and its neighbours; 152 blocks of 64 and one more; 1024 bands
+# (768 + 192 + 48 + 12 + 3 + 1) and a few more.
 @pytest.mark.parametrize("w,h", [(8, 8), (9, 31), (32, 32), (33, 65), (64, 64), (65, 31), (97, 161), (240, 180), (512, 512),
                                  (1216, 512), (1217, 512), (1024, 768), (1030, 769)])
 @pytest.mark.parametrize("gray", [False, True])
