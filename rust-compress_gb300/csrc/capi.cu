@@ -1224,10 +1224,11 @@ static int scorer_setup(rcg_ctx* ctx, int metric, int w, int h, int channels, Se
   return score_workspace(ctx, sc->pd);
 }
 
-// Decoded planes of one candidate -> score -> one bisection step (all gated by the step's `active`). Step `s` of the
+// Decoded planes of one candidate -> score -> one bisection step and the next one's tables (SSIMULACRA2), all gated by the
+// step's `active`. Step `s` of the
 // loop: the first candidate of a search (s = 0, always active) stores the reference moments, later ones read them.
 static void score_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st, const uint8_t* planes, int w,
-                            int h, int channels, SearchState* d_ss, int s) {
+                            int h, int channels, SearchState* d_ss, int s, const NextStep& next) {
   if (sc.metric == RCG_METRIC_SSIM) {
     upsample_color(ctx, d_st, planes, w, h, sc.cand_px, nullptr);
     ssim_score(ctx, sc.ref_px, sc.cand_px, w, h, channels, sc.d_score, d_ss, d_st);
@@ -1235,7 +1236,7 @@ static void score_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st
   }
   build_decoded(ctx, sc.pd, d_st, planes, sc.direct, sc.dist_pyr, nullptr, sc.ref_pyr);
   score_pyramids(ctx, sc.pd, sc.ref_xyb, sc.dist_pyr, sc.d_score, d_ss, d_st, sc.ref_moments,
-                 s == 0 ? kRefWrite : kRefRead);
+                 s == 0 ? kRefWrite : kRefRead, next);
 }
 
 // The reference-order FP64 score of a paused search's candidate to d_exact. Its planes are still the paused candidate's
@@ -1266,9 +1267,10 @@ static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st,
 // done = 2) with its decoded planes still in place (every later step was
 // inactive). Here it is rescored in the reference's f64 arithmetic and order on the GPU (exact_candidate), the bisection
 // records that score and goes on, and the remaining steps run as plain launches; repeated while a later candidate
-// pauses again. `issue_step(s)` issues step s's kernels.
+// pauses again. `issue_step(s, first)` issues step s's kernels; `first`: its tables too, which no step before it fills.
 static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, SearchState* hs, StepDesc* d_st,
-                       const uint8_t* planes, int max_steps, int w, int h, const std::function<void(int)>& issue_step) {
+                       const uint8_t* planes, int max_steps, int w, int h,
+                       const std::function<void(int, bool)>& issue_step) {
   while (hs->done == 2) {
     if (sc.metric != RCG_METRIC_SSIMULACRA2) return fail(ctx, RCG_INVALID, "paused search without a rescorer");
     double* d_exact = (double*)workspace(ctx, "x_score", sizeof(double), false);
@@ -1277,7 +1279,7 @@ static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, 
     if (rc != RCG_OK) return rc;
     search_resume(ctx, d_ss, d_exact);
     ctx->tie_rescores++;
-    for (int s = hs->step + 1; s < max_steps; s++) issue_step(s);
+    for (int s = hs->step + 1; s < max_steps; s++) issue_step(s, s == hs->step + 1);
     cudaMemcpyAsync(hs, d_ss, sizeof *hs, cudaMemcpyDeviceToHost, ctx->stream);
     if ((rc = finish(ctx, "search after a near tie")) != RCG_OK) return rc;
   }
@@ -1392,16 +1394,17 @@ static int search_impl(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int cha
   const int nsteps = step_limit > 0 ? std::min(step_limit, run.max_steps) : run.max_steps;
   const std::vector<long long> key = {1, (long long)(uintptr_t)d_src, w, h, channels, metric, subsampling, trellis_on,
                                       nsteps, (long long)(uintptr_t)d_weights};
-  auto issue_step = [&](int s) {
-    step_tables(ctx, d_ss, d_st, w, h, run.slots, es.max_coefs, d_weights);
+  const NextStep next = {kNextEncode, w, h, run.slots, es.max_coefs, d_weights};
+  auto issue_step = [&](int s, bool first) {
+    if (first || metric == RCG_METRIC_SSIM) step_tables(ctx, d_ss, d_st, next);
     quantize(ctx, d_st, es.caches, es.max_blocks);
     rate_tables(ctx, d_st);
     trellis(ctx, d_st, es.caches, es.max_blocks, d_weights != nullptr);
     dequant_idct(ctx, d_st, nullptr, run.planes, es.max_blocks);
-    score_candidate(ctx, sc, d_st, run.planes, w, h, channels, d_ss, s);
+    score_candidate(ctx, sc, d_st, run.planes, w, h, channels, d_ss, s, next);
   };
   rc = run_step_loop(ctx, key, [&]() {
-    for (int s = 0; s < nsteps; s++) issue_step(s);
+    for (int s = 0; s < nsteps; s++) issue_step(s, s == 0);
   });
   if (rc != RCG_OK) return rc;
   SearchState hs;
@@ -1641,15 +1644,15 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
   double* d_exact = (double*)workspace(ctx, "x_score", sizeof(double), false);
   if (!d_items || !d_exact) return RCG_NO_MEMORY;
   cudaMemcpyAsync(d_items, items.data(), sizeof(LockItem) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
-  auto issue_step = [&](int s) {
-    lock_step_codec(ctx, d_items, n, q_total);
+  auto issue_step = [&](int s, bool first) {
+    lock_step_codec(ctx, d_items, n, q_total, first);
     lock_step_score(ctx, d_items, n, p_total, t_total, max_scales,
                     ctx->ref_cache ? (s == 0 ? kRefWrite : kRefRead) : kRefNone);
   };
   // The grids follow from the totals; the images' buffers come in through the work-list uploaded above.
   const std::vector<long long> key = {5, n, max_steps, q_total, p_total, t_total, max_scales};
   rc = run_step_loop(ctx, key, [&]() {
-    for (int s = 0; s < max_steps; s++) issue_step(s);
+    for (int s = 0; s < max_steps; s++) issue_step(s, s == 0);
   });
   if (rc != RCG_OK) return rc;
   std::vector<SearchState> hs((size_t)n);
@@ -1672,7 +1675,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
       from = std::min(from, hs[(size_t)i].step + 1);
     }
     if (from == max_steps) break;
-    for (int s = from; s < max_steps; s++) issue_step(s);
+    for (int s = from; s < max_steps; s++) issue_step(s, s == from);
     if ((rc = read_states()) != RCG_OK) return rc;
   }
   // Results, each through its image's context (the step loop is complete: the states were read after it), in
@@ -1816,16 +1819,17 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
     const CompDesc& cd = st->comp[c];
     key.insert(key.end(), {cd.bw, cd.bh, cd.h, cd.v, cd.blk0, cd.plane_off});
   }
-  auto issue_step = [&](int s) {
-    step_tables_requant(ctx, d_ss, d_st, slots, nblocks * 64);
+  const NextStep next = {kNextRequant, w, h, slots, nblocks * 64, nullptr};
+  auto issue_step = [&](int s, bool first) {
+    if (first || metric == RCG_METRIC_SSIM) step_tables(ctx, d_ss, d_st, next);
     requantize_plain(ctx, d_st, nblocks);
     rate_tables(ctx, d_st);
     rcg::trellis(ctx, d_st, no_caches, nblocks);
     dequant_idct(ctx, d_st, nullptr, planes, nblocks);
-    score_candidate(ctx, sc, d_st, planes, w, h, channels, d_ss, s);
+    score_candidate(ctx, sc, d_st, planes, w, h, channels, d_ss, s, next);
   };
   rc = run_step_loop(ctx, key, [&]() {
-    for (int s = 0; s < max_steps; s++) issue_step(s);
+    for (int s = 0; s < max_steps; s++) issue_step(s, s == 0);
   });
   if (rc != RCG_OK) {
     delete st;

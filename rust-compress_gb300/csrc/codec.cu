@@ -20,67 +20,11 @@
 
 #include "rcg_internal.cuh"
 #include "huffman.cuh"
+#include "step_tables.cuh"
 
 namespace rcg {
 
 // ------------------------------------------------------------------------------------------------ tables
-
-// jpeg/src/lib.rs:14-19
-__host__ __device__ inline int zigzag(int k) {
-  constexpr int Z[64] = {0,  1,  8,  16, 9,  2,  3,  10, 17, 24, 32, 25, 18, 11, 4,  5,  12, 19, 26, 33, 40, 48,
-                         41, 34, 27, 20, 13, 6,  7,  14, 21, 28, 35, 42, 49, 56, 57, 50, 43, 36, 29, 22, 15, 23,
-                         30, 37, 44, 51, 58, 59, 52, 45, 38, 31, 39, 46, 53, 60, 61, 54, 47, 55, 62, 63};
-  return Z[k];
-}
-
-// jpeg/src/dct.rs:8 (AAN scale factors)
-__host__ __device__ inline float aan(int i) {
-  constexpr float A[8] = {1.0f, 1.3870398f, 1.306563f, 1.1758756f, 1.0f, 0.78569495f, 0.5411961f, 0.27589938f};
-  return A[i];
-}
-
-// jpeg/src/quality.rs:26-35
-__host__ __device__ inline uint8_t perceptual_q(int i) {
-  constexpr uint8_t P[64] = {16, 16, 16,  18,  25,  37,  56,  85,  16, 17, 20,  27,  34,  40,  53,  75,
-                             16, 20, 24,  31,  43,  62,  91,  135, 18, 27, 31,  40,  53,  74,  106, 156,
-                             25, 34, 43,  53,  69,  94,  131, 189, 37, 40, 62,  74,  94,  124, 169, 238,
-                             56, 53, 91,  106, 131, 169, 226, 255, 85, 75, 135, 156, 189, 238, 255, 255};
-  return P[i];
-}
-
-// Exact f32 arithmetic on host and device: round-to-nearest, never contracted.
-__host__ __device__ inline float fadd(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fadd_rn(a, b);
-#else
-  volatile float r = a + b;
-  return r;
-#endif
-}
-__host__ __device__ inline float fsub(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fsub_rn(a, b);
-#else
-  volatile float r = a - b;
-  return r;
-#endif
-}
-__host__ __device__ inline float fmul(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fmul_rn(a, b);
-#else
-  volatile float r = a * b;
-  return r;
-#endif
-}
-__host__ __device__ inline float fdiv(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fdiv_rn(a, b);
-#else
-  volatile float r = a / b;
-  return r;
-#endif
-}
 
 // jpeg/src/dct.rs:125-129: round half to even for |x| < 2^22; wrapping integer arithmetic beyond, as the reference.
 __device__ __forceinline__ int round_f32(float x) {
@@ -89,80 +33,10 @@ __device__ __forceinline__ int round_f32(float x) {
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 
-// Sampling factors build_coefs chooses (jpeg/src/encode.rs:428-439).
-__host__ __device__ inline void sampling(int channels, int subsampling, int quality, int* hmax, int* vmax) {
-  if (channels == 1) {
-    *hmax = 1;
-    *vmax = 1;
-    return;
-  }
-  switch (subsampling) {
-    case RCG_SUB_420: *hmax = 2; *vmax = 2; break;
-    case RCG_SUB_422: *hmax = 2; *vmax = 1; break;
-    case RCG_SUB_444: *hmax = 1; *vmax = 1; break;
-    default:
-      if (quality < 90) { *hmax = 2; *vmax = 2; } else { *hmax = 1; *vmax = 1; }
-  }
-}
-
-// FDCT cache slot of a component for a sampling layout: 3 caches (Y, Cb, Cr) per layout kind.
-__host__ __device__ inline int layout_kind(int hmax, int vmax) { return hmax == 2 ? (vmax == 2 ? 0 : 1) : 2; }
-
-// One entry of the per-quality tables, shared by the host (fill_step) and the device (k_step_tables) so both give
-// identical bits. `q` is the quantization table (natural order).
-//   quant value at natural index n (jpeg/src/quality.rs:6-15)
-__host__ __device__ inline uint8_t qtable_entry(int quality, int n) {
-  unsigned q = (unsigned)(quality < 1 ? 1 : (quality > 100 ? 100 : quality));
-  unsigned scale = q < 50 ? 5000 / q : 200 - 2 * q;
-  unsigned v = ((unsigned)perceptual_q(n) * scale + 50) / 100;
-  return (uint8_t)(v < 1 ? 1 : (v > 255 ? 255 : v));
-}
-//   fdct divisor for zigzag position k: fdct_divisors stores 1 / (q[v*8+u] * AAN[u] * AAN[v] * 8) at [u*8+v]
-//   (jpeg/src/encode.rs:174-183) and quantize_plane reads it at ZZ_T[k] = (n%8)*8 + n/8 (:202), i.e. u = n%8,
-//   v = n/8, q[v*8+u] = q[n]
-__host__ __device__ inline float divz_entry(const uint8_t* q, int k) {
-  int n = zigzag(k);
-  return fdiv(1.0f, fmul(fmul(fmul((float)q[n], aan(n % 8)), aan(n / 8)), 8.0f));
-}
-//   dequantization multiplier at natural index n = v*8+u: q[v*8+u] * AAN[u] * AAN[v] (jpeg/src/decode.rs:1316-1321)
-__host__ __device__ inline float mult_entry(const uint8_t* q, int n) {
-  return fmul(fmul((float)q[n], aan(n % 8)), aan(n / 8));
-}
-
-// Block layout of a candidate (jpeg/src/encode.rs:428-443, :511-517).
-__host__ __device__ inline void fill_layout(StepDesc* st, int quality, int subsampling, int channels, int trellis,
-                                            int w, int h) {
-  st->quality = quality;
-  st->use_trellis = (trellis && quality < 100) ? 1 : 0;
-  int hmax, vmax;
-  sampling(channels, subsampling, quality, &hmax, &vmax);
-  st->hmax = hmax;
-  st->vmax = vmax;
-  int pw = (w + 8 * hmax - 1) / (8 * hmax) * 8 * hmax;
-  int ph = (h + 8 * vmax - 1) / (8 * vmax) * 8 * vmax;
-  st->ncomp = channels == 1 ? 1 : 3;
-  long long blk = 0, poff = 0;
-  int kind = layout_kind(hmax, vmax);
-  for (int c = 0; c < st->ncomp; c++) {
-    CompDesc& cd = st->comp[c];
-    cd.h = c == 0 ? hmax : 1;
-    cd.v = c == 0 ? vmax : 1;
-    cd.bw = c == 0 ? pw / 8 : pw / hmax / 8;
-    cd.bh = c == 0 ? ph / 8 : ph / vmax / 8;
-    cd.cls = c == 0 ? 0 : 1;
-    cd.cache = kind * 3 + c;
-    cd.blk0 = blk;
-    cd.plane_off = poff;
-    blk += (long long)cd.bw * cd.bh;
-    poff += (long long)cd.bw * 8 * cd.bh * 8;
-  }
-  st->nblocks = blk;
-}
-
 // The per-quality tables of one candidate: quantization tables (jpeg/src/quality.rs), fdct divisors
 // (jpeg/src/encode.rs:174-183), dequantization multipliers (jpeg/src/decode.rs:1316-1321), the Rdo parameters that
 // do not depend on the rate model (jpeg/src/rdo.rs:28-45), and the block layout (jpeg/src/encode.rs:440-517).
-// Host version (single calls); k_step_tables computes the same entries in parallel on the device.
+// Host version (single calls); step_tables_body computes the same entries in parallel on the device.
 inline void fill_step(StepDesc* st, int quality, int subsampling, int channels, int trellis, int w, int h) {
   const float kappa = 0.02f;  // TRELLIS_KAPPA, jpeg/src/encode.rs:42
   fill_layout(st, quality, subsampling, channels, trellis, w, h);
@@ -797,7 +671,7 @@ __device__ __forceinline__ void dequant_idct_body(const StepDesc* __restrict__ s
     for (int j = 0; j < 8; j++) {
       int k = g * 8 + j;
       int v = (int)(short)((w4[j >> 1] >> (16 * (j & 1))) & 0xFFFF);
-      int n = zigzag(k);
+      int n = zigzag_known(k);
       blk[n] = fmul((float)v, mult[n]);
     }
   }
@@ -991,62 +865,16 @@ int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int 
 
 // ------------------------------------------------------------------------------------------------ step tables
 
-// First kernel of every search step: the bisection state names the quality; fill the candidate's tables. 192
-// threads: one per (component, coefficient) entry; the Rdo median is the element of rank 31 among q[1..63] (ties
-// broken by index, which leaves the value unchanged), the same value the reference's sort yields.
-__device__ __forceinline__ void step_tables_body(const SearchState* __restrict__ ss, StepDesc* __restrict__ st,
-                                                 int w, int h, int16_t* slots, long long slot_stride,
-                                                 const float* pweights) {
-  __shared__ uint8_t qt[64];
-  __shared__ float rq[64];
-  __shared__ float median;
-  const int t = threadIdx.x;
-  if (ss->done) {
-    if (t == 0) st->active = 0;
-    return;
-  }
-  const int step = ss->step;
-  const int q = ss->qs[step];
-  if (t == 0) {
-    st->active = 1;
-    st->requant = 0;
-    fill_layout(st, q, ss->subsampling, ss->channels, ss->trellis, w, h);
-    st->coefs = slots + (long long)step * slot_stride;
-    st->pweights = pweights;
-  }
-  if (t < 64) qt[t] = qtable_entry(q, t);
-  __syncthreads();
-  // luma_table == chroma_table (jpeg/src/quality.rs:37-43): every component gets the same entries
-  const int c = t / 64, k = t % 64;
-  st->qt[c][k] = qt[k];
-  st->divz[c][k] = divz_entry(qt, k);
-  st->mult[c][k] = mult_entry(qt, k);
-  float rk = (float)qt[zigzag(k)];
-  st->rq[c][k] = rk;
-  if (c == 0) rq[k] = rk;
-  for (int i = t; i < 512; i += blockDim.x) (&st->hist[0][0])[i] = 0;
-  __syncthreads();
-  if (c == 0 && k >= 1) {
-    int rank = 0;
-    for (int j = 1; j < 64; j++) rank += (rq[j] < rk || (rq[j] == rk && j < k)) ? 1 : 0;
-    if (rank == 31) median = rk;
-  }
-  __syncthreads();
-  st->rw[c][k] = k == 0 ? 1.0f : fdiv(median, rk);
-  if (k == 0) st->lambda[c] = fmul(fmul(0.02f, median), median);  // TRELLIS_KAPPA (jpeg/src/encode.rs:42)
-}
-
-__global__ void __launch_bounds__(192) k_step_tables(const SearchState* __restrict__ ss, StepDesc* __restrict__ st,
-                                                     int w, int h, int16_t* slots, long long slot_stride,
-                                                     const float* pweights) {
+// A search's first step (and the first one after a near tie): the later ones' tables are filled where the step before is
+// scored (ssim2_reduce), unless the search's metric is another.
+__global__ void __launch_bounds__(kStepThreads) k_step_tables(const SearchState* __restrict__ ss,
+                                                              StepDesc* __restrict__ st, const NextStep next) {
   grid_chain();
-  step_tables_body(ss, st, w, h, slots, slot_stride, pweights);
+  step_tables_body(*ss, st, next);
 }
 
-int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int w, int h, int16_t* d_coef_slots,
-                long long slot_stride, const float* d_pweights) {
-  RCG_LAUNCH(ctx, "step_tables", k_step_tables, 1, 192, 0, d_search, d_step, w, h, d_coef_slots, slot_stride,
-             d_pweights);
+int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, const NextStep& next) {
+  RCG_LAUNCH(ctx, "step_tables", k_step_tables, 1, kStepThreads, 0, d_search, d_step, next);
   return RCG_OK;
 }
 
@@ -1054,10 +882,10 @@ int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int w, in
 
 // One bisection step of every image of a lockstep batch: the same kernel bodies as one search, each launch over a
 // work-list of every image's CTAs (an image whose search has finished skips through its StepDesc's `active`).
-__global__ void __launch_bounds__(192) k_step_tables_lock(const LockItem* __restrict__ items) {
+__global__ void __launch_bounds__(kStepThreads) k_step_tables_lock(const LockItem* __restrict__ items) {
   grid_chain();
   const LockItem& it = items[blockIdx.x];
-  step_tables_body(it.ss, it.st, it.w, it.h, it.slots, it.slot_stride, nullptr);
+  step_tables_body(*it.ss, it.st, NextStep{kNextEncode, it.w, it.h, it.slots, it.slot_stride, nullptr});
 }
 
 __device__ __forceinline__ CacheSet lock_caches(const LockItem& it) {
@@ -1093,8 +921,8 @@ __global__ void __launch_bounds__(128) k_dequant_idct_lock(const LockItem* __res
   dequant_idct_body(it.st, nullptr, it.planes, (long long)blockIdx.x - it.q0);
 }
 
-void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total) {
-  RCG_LAUNCH(ctx, "step_tables_lock", k_step_tables_lock, n, 192, 0, d_items);
+void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total, bool first) {
+  if (first) RCG_LAUNCH(ctx, "step_tables_lock", k_step_tables_lock, n, kStepThreads, 0, d_items);
   RCG_LAUNCH(ctx, "quantize_lock", k_quantize_lock, (unsigned)q_total, 128, 0, d_items, n);
   RCG_LAUNCH(ctx, "rate_tables_lock", k_rate_tables_lock, dim3(3, n), 288, 0, d_items);
   RCG_LAUNCH(ctx, "trellis_lock", k_trellis_lock, (unsigned)q_total, 128, 0, d_items, n);
@@ -1108,16 +936,9 @@ int codec_upload_lut(const float* lut8) {
 
 // ------------------------------------------------------------------------------------------------ requantization
 
-// Table of one component for a requantization to `quality` (jpeg/src/encode.rs:121-126): the quality's table,
-// never finer than the source's.
-__host__ __device__ inline uint8_t requant_entry(const uint8_t* old, int quality, int n) {
-  uint8_t t = qtable_entry(quality, n);
-  return t > old[n] ? t : old[n];
-}
-
 // Slot assignment of jpeg/src/encode.rs:139-148: components with equal tables share a slot, a new table takes the
 // first free one. Also reports whether any table changed (:127) and the slot tables.
-__host__ __device__ inline int requant_slots(const StepDesc* st, int* tq, uint8_t (*slot_qt)[64], int* present) {
+inline int requant_slots(const StepDesc* st, int* tq, uint8_t (*slot_qt)[64], int* present) {
   int changed = 0;
   for (int sl = 0; sl < 4; sl++) present[sl] = 0;
   for (int c = 0; c < st->ncomp; c++) {
@@ -1167,65 +988,6 @@ void host_requant_tables(StepDesc* st, int quality, int trellis, int tq_out[3], 
   st->changed = requant_slots(st, tq_out, slot_qt_out, present_out);
   st->use_trellis = (trellis && st->changed) ? 1 : 0;
   std::memset(st->hist, 0, sizeof st->hist);
-}
-
-// Search step of the JPEG->JPEG search: the same tables as host_requant_tables, 192 threads (component,
-// coefficient); each component's Rdo median is the element of rank 31 among its q[1..63].
-__global__ void __launch_bounds__(192) k_step_tables_rq(const SearchState* __restrict__ ss, StepDesc* __restrict__ st,
-                                                        int16_t* slots, long long slot_stride) {
-  grid_chain();
-  __shared__ float rq[3][64];
-  __shared__ float median[3];
-  const int t = threadIdx.x;
-  if (ss->done) {
-    if (t == 0) st->active = 0;
-    return;
-  }
-  const int step = ss->step;
-  const int q = ss->qs[step];
-  const int c = t / 64, k = t % 64;
-  const bool live = c < st->ncomp;
-  if (live) {
-    int n = zigzag(k);
-    uint8_t nn = requant_entry(st->src_qt[c], q, n);
-    st->qt[c][n] = nn;
-    st->ratio[c][k] = fdiv((float)st->src_qt[c][n], (float)nn);
-    st->rq[c][k] = (float)nn;
-    rq[c][k] = (float)nn;
-  }
-  for (int i = t; i < 512; i += blockDim.x) (&st->hist[0][0])[i] = 0;
-  __syncthreads();
-  if (live) {
-    st->mult[c][k] = mult_entry(st->qt[c], k);
-    if (k >= 1) {
-      float rk = rq[c][k];
-      int rank = 0;
-      for (int j = 1; j < 64; j++) rank += (rq[c][j] < rk || (rq[c][j] == rk && j < k)) ? 1 : 0;
-      if (rank == 31) median[c] = rk;
-    }
-  }
-  __syncthreads();
-  if (live) {
-    st->rw[c][k] = k == 0 ? 1.0f : fdiv(median[c], rq[c][k]);
-    if (k == 0) st->lambda[c] = fmul(fmul(0.02f, median[c]), median[c]);
-  }
-  if (t == 0) {
-    int tq[3];
-    uint8_t slot_qt[4][64];
-    int present[4];
-    st->active = 1;
-    st->requant = 1;
-    st->quality = q;
-    st->changed = requant_slots(st, tq, slot_qt, present);
-    st->use_trellis = (ss->trellis && st->changed) ? 1 : 0;
-    st->coefs = slots + (long long)step * slot_stride;
-  }
-}
-
-int step_tables_requant(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int16_t* d_coef_slots,
-                        long long slot_stride) {
-  RCG_LAUNCH(ctx, "step_tables", k_step_tables_rq, 1, 192, 0, d_search, d_step, d_coef_slots, slot_stride);
-  return RCG_OK;
 }
 
 // Plain requantization (jpeg/src/encode.rs:132-138): round_f32(coef * old/new) clamped to +-2047, every position.

@@ -156,6 +156,16 @@ __device__ __forceinline__ void search_record(SearchState* ss, double sv, bool m
   }
 }
 
+// What fills the tables of a search's next candidate (step_tables.cuh), where its step is scored.
+enum { kNextNone = 0, kNextEncode = 1, kNextRequant = 2 };
+struct NextStep {
+  int kind = kNextNone;
+  int w = 0, h = 0;                // of the image (kNextEncode)
+  int16_t* slots = nullptr;        // coefficient slots, one per step
+  long long slot_stride = 0;
+  const float* pweights = nullptr; // weights of the perceptual trellis (nullable)
+};
+
 // One image of a lockstep batch of searches (capi.cu, rcg_search_batch_lockstep): every bisection step of every
 // image runs as one work-list launch per stage, each CTA finding its image by the first-CTA offsets below.
 struct LockItem {
@@ -356,10 +366,11 @@ constexpr int kRefChunk = 3 * kTileH * kTileW;
 constexpr int kRefNone = 0, kRefWrite = 1, kRefRead = 2;
 // Score of a reference's XYB pyramid and a candidate's XYB differences: per-tile sums of every scale, then the final
 // mapping. `d_score` receives the score (f64); when
-// `search` is non-null the final kernel also advances the device-side bisection. `refm`/`ref_mode`: the reference
-// moments (nullptr / kRefNone: none).
+// `search` is non-null the final kernel also advances the device-side bisection and fills the tables of the step that
+// comes `next` in *step. `refm`/`ref_mode`: the reference moments (nullptr / kRefNone: none).
 int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_xyb, const float* d_diff, double* d_score,
-                   SearchState* search, StepDesc* step, float2* refm = nullptr, int ref_mode = kRefNone);
+                   SearchState* search, StepDesc* step, float2* refm = nullptr, int ref_mode = kRefNone,
+                   const NextStep& next = NextStep());
 // The reference-order FP64 score (exact.cu) of two images given as scale-0 linear planes ([3][h][w] f32, as
 // to_linear writes them): to d_score (NaN for the reference's non-finite Err), queued on the context stream.
 int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, int h, double* d_score);
@@ -386,7 +397,8 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
                 double** d_scores);
 
 // ---- lockstep batch (work-list launches over the LockItems of a batch; totals are the grids' CTA counts)
-void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total);
+// first: the step's tables too (else the step before has filled them).
+void lock_step_codec(rcg_ctx* ctx, const LockItem* d_items, int n, long long q_total, bool first);
 void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_total, long long t_total,
                      int max_scales, int ref_mode = kRefNone);
 
@@ -450,11 +462,8 @@ int codec_upload_lut(const float* lut8);
 // tables in st->src_qt, on the host (single calls) and on the device (search steps): identical bits.
 void host_requant_tables(StepDesc* st, int quality, int trellis, int tq_out[3], uint8_t slot_qt_out[4][64],
                          int present_out[4]);
-int step_tables_requant(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int16_t* d_coef_slots,
-                        long long slot_stride);
-// Device-side: fill the step tables from the quality the search state holds.
-int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, int w, int h, int16_t* d_coef_slots,
-                long long slot_stride, const float* d_pweights = nullptr);
+// A search's (next) step: the tables of the quality that its state holds, by a launch of their own.
+int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, const NextStep& next);
 
 // ---- perceptual trellis weights (perceptual.cu)
 struct PerceptualParams {

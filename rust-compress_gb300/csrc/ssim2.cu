@@ -36,6 +36,7 @@
 
 #include "rcg_internal.cuh"
 #include "planes_quad.cuh"
+#include "step_tables.cuh"
 
 namespace rcg {
 
@@ -600,27 +601,52 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
   ssim2_band<kRef>(sd, blk - sd.tile0, channel_of_cta(), ref, dist, partials + blk, (size_t)pd.total_tiles, refm);
 }
 
-// Deterministic reduction of the per-tile sums: CTA (scale, sum index); the last CTA to finish computes the score
-// (core/src/ssimulacra2.rs:457-511) and, in a search, advances the bisection (jpeg/src/target.rs:29-56).
-// CTA (scale blockIdx.x, sum blockIdx.y) of one score; the last of its nscales x 18 CTAs maps the sums.
+// Deterministic reduction of the per-tile sums: CTA (scale, sum index) of one score; the last of its nscales x 18 CTAs to
+// finish computes the score (core/src/ssimulacra2.rs:457-511) and, in a search, advances the bisection
+// (jpeg/src/target.rs:29-56) and fills the next step's tables.
+// What bounds it: latency (partial sums, a counter, the last CTA's serial end) and FP64 operations, of which an SM starts
+// a warp's only every 16 cycles or so: warps without sums or terms leave them out. What the end needs and no CTA writes
+// (weights, sample counts, the search's state) is loaded at the start by every CTA, and the bisection works on a copy in
+// shared memory. Measured at 240x180: 12.7 us with the next step's tables, from 12.5 and a launch of 5.0 for the tables
+// (10 requantizing), whose lookups went through stack copies of the constant tables; a search 622 -> 567 us.
 __device__ __forceinline__ void reduce_scale_sum(const PyramidDesc& pd, const double* __restrict__ partials,
                                                  double* __restrict__ scale_sums, unsigned* __restrict__ counter,
-                                                 double* __restrict__ score_out, SearchState* __restrict__ ss) {
+                                                 double* __restrict__ score_out, SearchState* __restrict__ ss,
+                                                 StepDesc* __restrict__ st, const NextStep& next) {
+  constexpr int kStateWords = sizeof(SearchState) / 4;
+  static_assert(kStateWords <= 256 && sizeof(SearchState) % 4 == 0, "copied a word per thread");
   __shared__ double red[8];
   __shared__ bool last;
-  const int s = blockIdx.x, i = blockIdx.y;
+  __shared__ __align__(8) int state[kStateWords];
+  const int s = blockIdx.x, i = blockIdx.y, t = threadIdx.x;
   const ScaleDesc sd = pd.s[s];
   const int n = sd.tiles_x * sd.tiles_y;
+  if (ss && t < kStateWords) state[t] = reinterpret_cast<const int*>(ss)[t];
+  // Term t follows the reference's weight order: channel, scale, norm (mean, 4-norm), then (ssim, artifact, detail)
+  // (core/src/ssimulacra2.rs:491-506).
+  const int ns = pd.nscales, nterms = 3 * ns * 6;
+  int from = 0, nrm = 0;
+  double weight = 0.0, count = 1.0;
+  if (t < nterms) {
+    const int c = t / (ns * 6), rem = t % (ns * 6), sc = rem / 6, r2 = rem % 6, k = r2 % 3;
+    nrm = r2 / 3;
+    from = sc * kScoreSums + c * 6 + 2 * k + nrm;
+    weight = c_weights[t];
+    count = (double)pd.s[sc].w * (double)pd.s[sc].h;
+  }
   double acc = 0.0;
   const double* col = partials + (size_t)i * pd.total_tiles + sd.tile0;
-  for (int t = threadIdx.x; t < n; t += 256) acc += col[t];
+  for (int u = t; u < n; u += 256) acc += col[u];
+  const int warps = min(8, (n + 31) / 32);  // those that hold sums
+  if ((t >> 5) < warps) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if ((t & 31) == 0) red[t >> 5] = acc;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (t == 0) {
     double tot = 0.0;
-    for (int wi = 0; wi < 8; wi++) tot += red[wi];
+    for (int wi = 0; wi < warps; wi++) tot += red[wi];
     scale_sums[s * kScoreSums + i] = tot;
     __threadfence();
     unsigned prev = atomicAdd(counter, 1u);
@@ -629,44 +655,46 @@ __device__ __forceinline__ void reduce_scale_sum(const PyramidDesc& pd, const do
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // The last CTA maps the per-scale sums to the score. Term t follows the reference's weight order: channel, scale,
-  // norm (mean, 4-norm), then (ssim, artifact, detail) (core/src/ssimulacra2.rs:491-506); one thread per term, then
-  // the terms summed by a fixed pairwise tree (18.4 against 20.5 us per launch for the serial sum).
-  __shared__ double terms[3 * kMaxScales * 6];
-  const volatile double* vs = scale_sums;
-  const int ns = pd.nscales, nterms = 3 * ns * 6, t = threadIdx.x;
+  // The last CTA maps the per-scale sums to the score: one thread per term, then the terms summed by a fixed pairwise
+  // tree (neighbours first; deterministic).
+  double term = 0.0;
   if (t < nterms) {
-    int c = t / (ns * 6), rem = t % (ns * 6), sc = rem / 6, r2 = rem % 6, nrm = r2 / 3, k = r2 % 3;
-    double count = (double)pd.s[sc].w * (double)pd.s[sc].h;
-    double v = vs[sc * kScoreSums + c * 6 + 2 * k + nrm] / count;
+    double v = reinterpret_cast<const volatile double*>(scale_sums)[from] / count;
     if (nrm == 1) v = sqrt(sqrt(v));  // (sum of 4th powers / count)^0.25 (:462)
-    terms[t] = c_weights[t] * fabs(v);
+    term = weight * fabs(v);
+  }
+  if (t < 128) {  // 108 terms at most
+#pragma unroll
+    for (int span = 1; span < 32; span *= 2) term += __shfl_down_sync(0xffffffffu, term, span);
+    if ((t & 31) == 0) red[t >> 5] = term;
   }
   __syncthreads();
-  // Fixed-order pairwise sum of the terms (deterministic; the same tree on every call).
-  for (int span = 1; span < nterms; span *= 2) {
-    if (t % (2 * span) == 0 && t + span < nterms) terms[t] += terms[t + span];
-    __syncthreads();
+  SearchState* const copy = reinterpret_cast<SearchState*>(state);
+  if (t == 0) {
+    *counter = 0;
+    double ssim = (red[0] + red[1]) + (red[2] + red[3]);
+    ssim *= 0.9562382616834844;
+    ssim = 2.326765642916932 * ssim - 0.020884521182843837 * ssim * ssim + 6.248496625763138e-05 * ssim * ssim * ssim;
+    double score = ssim > 0.0 ? 100.0 - 10.0 * pow(ssim, 0.6276336467831387) : 100.0;
+    // A non-finite score is the reference's Err, which the search maps to f64::MIN (cli/src/pipeline.rs:218).
+    bool finite = isfinite(score);
+    *score_out = finite ? score : NAN;
+    if (ss) search_record(copy, finite ? score : -1.7976931348623157e308);
   }
-  if (t != 0) return;
-  *counter = 0;
-  double ssim = terms[0];
-  ssim *= 0.9562382616834844;
-  ssim = 2.326765642916932 * ssim - 0.020884521182843837 * ssim * ssim + 6.248496625763138e-05 * ssim * ssim * ssim;
-  double score = ssim > 0.0 ? 100.0 - 10.0 * pow(ssim, 0.6276336467831387) : 100.0;
-  // A non-finite score is the reference's Err, which the search maps to f64::MIN (cli/src/pipeline.rs:218).
-  bool finite = isfinite(score);
-  *score_out = finite ? score : NAN;
-  if (ss) search_record(ss, finite ? score : -1.7976931348623157e308);
+  if (!ss) return;
+  __syncthreads();
+  if (t < kStateWords) reinterpret_cast<int*>(ss)[t] = state[t];
+  if (next.kind != kNextNone) step_tables_body(*copy, st, next);
 }
 
-__global__ void __launch_bounds__(256) k_ssim2_reduce(PyramidDesc pd, const double* __restrict__ partials,
+__global__ void __launch_bounds__(256) k_ssim2_reduce(const __grid_constant__ PyramidDesc pd,
+                                                      const double* __restrict__ partials,
                                                       double* __restrict__ scale_sums, unsigned* __restrict__ counter,
                                                       double* __restrict__ score_out, SearchState* __restrict__ ss,
-                                                      const StepDesc* __restrict__ st) {
+                                                      StepDesc* __restrict__ st, const NextStep next) {
   grid_chain();
   if (st && !st->active) return;
-  reduce_scale_sum(pd, partials, scale_sums, counter, score_out, ss);
+  reduce_scale_sum(pd, partials, scale_sums, counter, score_out, ss, st, next);
 }
 
 // ------------------------------------------------------------------------------------------------ planes, pyramid
@@ -1210,7 +1238,7 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_batch(const ScoreItem* __r
   const ScoreItem& it = items[p];
   if ((int)blockIdx.x >= it.pd.nscales) return;
   reduce_scale_sum(it.pd, partials + it.part, scale_sums + (size_t)p * kMaxScales * kScoreSums, counters + p,
-                   scores + p, nullptr);
+                   scores + p, nullptr, nullptr, NextStep());
 }
 
 // ------------------------------------------------------------------------------------------------ lockstep batch
@@ -1251,7 +1279,8 @@ __global__ void __launch_bounds__(256) k_ssim2_reduce_lock(const LockItem* __res
   grid_chain();
   const LockItem& it = items[blockIdx.z];
   if (!it.st->active || (int)blockIdx.x >= it.pd.nscales) return;
-  reduce_scale_sum(it.pd, it.partials, it.scale_sums, it.counter, it.score, it.ss);
+  reduce_scale_sum(it.pd, it.partials, it.scale_sums, it.counter, it.score, it.ss, it.st,
+                   NextStep{kNextEncode, it.w, it.h, it.slots, it.slot_stride, nullptr});
 }
 
 void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_total, long long t_total,
@@ -1562,7 +1591,7 @@ int score_workspace(rcg_ctx* ctx, const PyramidDesc& pd) {
 }
 
 int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, const float* d_dist, double* d_score,
-                   SearchState* search, StepDesc* step, float2* refm, int ref_mode) {
+                   SearchState* search, StepDesc* step, float2* refm, int ref_mode, const NextStep& next) {
   if (score_workspace(ctx, pd) != RCG_OK) return RCG_NO_MEMORY;
   double* partials = (double*)ctx->bufs["score_partials"].ptr;
   double* scale_sums = (double*)ctx->bufs["score_scale_sums"].ptr;
@@ -1579,7 +1608,7 @@ int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, cons
                d_dist, partials, step, refm);
   dim3 rg(pb.nscales, kScoreSums);
   RCG_LAUNCH(ctx, "ssim2_reduce", k_ssim2_reduce, rg, 256, 0, pb, partials, scale_sums, counter, d_score, search,
-             step);
+             step, next);
   return RCG_OK;
 }
 
@@ -1834,7 +1863,7 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   launch_chained(tile_grid(pd.total_tiles), kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref, pyr_dist,
                  partials, nullptr, nullptr);
   launch_chained(dim3(pd.nscales, kScoreSums), 256, 0, s, k_ssim2_reduce, pd, partials, sums, counter, d_score, nullptr,
-                                                              nullptr);
+                                                              nullptr, NextStep());
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? RCG_OK : RCG_CUDA_ERROR;
 }
