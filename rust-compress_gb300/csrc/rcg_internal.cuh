@@ -237,13 +237,6 @@ struct rcg_ctx {
   float* lut16 = nullptr;  // 65536-entry sRGB->linear table for 16-bit samples (allocated on first use)
   std::vector<rcg_ctx*> workers;  // sub-contexts of rcg_search_batch (own streams and workspaces)
   std::vector<rcg_ctx*> lock_subs;  // per-image sub-contexts of rcg_search_batch_lockstep (buffers, set-up streams)
-  // Pinned host staging for host-buffer calls (grow-only): pageable copies go through the driver's own staging and
-  // serialize across threads; these let a worker thread do its memcpy in parallel with other workers' GPU work.
-  bool stage_copies = false;  // set on batch worker contexts
-  void* pinned_in = nullptr;
-  size_t pinned_in_bytes = 0;
-  void* pinned_out = nullptr;
-  size_t pinned_out_bytes = 0;
   // Step loops of the device searches captured as CUDA graphs (capi.cu, run_step_loop). A loop's launches and their
   // arguments follow from the image shape, the options and the workspace pointers, so the key holds the first two
   // and ws_gen stands for the third: every workspace (re)allocation bumps it and makes older graphs stale.
@@ -281,9 +274,8 @@ int cuda_fail(rcg_ctx* ctx, cudaError_t e, const char* what);
 // scorer's) move without making the graphs stale.
 void* workspace(rcg_ctx* ctx, const char* name, size_t bytes, bool in_graphs = true);
 
-// Host<->device copies of caller buffers: the driver's path for single calls; on batch worker contexts direct DMA when
-// the caller's memory is pinned, else through the context's pinned staging buffer. copy_to_device is asynchronous on the context stream (the source may be reused as soon as it
-// returns); copy_to_host synchronizes the stream.
+// Host<->device copies of caller buffers. copy_to_device is asynchronous on the context stream (the source may be reused
+// as soon as it returns); copy_to_host synchronizes the stream.
 int copy_to_device(rcg_ctx* ctx, void* dst, const void* src, size_t bytes);
 int copy_to_host(rcg_ctx* ctx, void* dst, const void* src, size_t bytes);
 

@@ -197,6 +197,22 @@ class CoefImage:
     def flat(self):
         return np.concatenate([c.coefs for c in self.comps]).astype(np.int16, copy=False)
 
+    def _joined(self):
+        """(array, address, count) of the components' coefficients back to back, for a call that reads them: in place
+        where they lie so (as every call of this library returns them), else put together. Keep `array` meanwhile."""
+        arrs = [c.coefs for c in self.comps]
+        end = None
+        for a in arrs:
+            if not (isinstance(a, np.ndarray) and a.dtype == np.int16 and a.ndim == 1 and a.flags.c_contiguous
+                    and (end is None or a.ctypes.data == end)):
+                break
+            end = a.ctypes.data + a.nbytes
+        else:
+            if arrs:
+                return arrs, arrs[0].ctypes.data, sum(a.size for a in arrs)
+        flat = np.ascontiguousarray(self.flat())
+        return flat, flat.ctypes.data, flat.size
+
     def layout(self):
         lay = _Layout()
         lay.ncomp = len(self.comps)
@@ -753,17 +769,17 @@ class Context:
     def reconstruct(self, ci):
         """jpeg/src/decode.rs:334: the pixels a viewer would show (Gray (h, w) or Rgb (h, w, 3) uint8)."""
         lay = ci.layout()
-        flat = np.ascontiguousarray(ci.flat())
+        keep, at, _ = ci._joined()
         nc = len(ci.comps)
         out = np.zeros((ci.height, ci.width, nc), dtype=np.uint8)
         if ci.present is None:
             qt = np.ascontiguousarray(ci.qtables, dtype=np.uint8)
             self._check(_lib.rcg_reconstruct(self._ptr, ci.width, ci.height, ctypes.byref(lay), qt.ctypes.data,
-                                             flat.ctypes.data, out.ctypes.data, out.size))
+                                             at, out.ctypes.data, out.size))
         else:
             t = ci.table_slots()
             self._check(_lib.rcg_reconstruct_tables(self._ptr, ci.width, ci.height, ctypes.byref(lay),
-                                                    ctypes.byref(t), flat.ctypes.data, out.ctypes.data, out.size))
+                                                    ctypes.byref(t), at, out.ctypes.data, out.size))
         return out[:, :, 0] if nc == 1 else out
 
     def decode_coefs(self, data):
@@ -812,9 +828,9 @@ class Context:
     def plan(self, ci):
         """write_best's plan of a CoefImage (jpeg/src/encode.rs:543-565): statistics, costs and choice on the GPU."""
         lay = ci.layout()
-        flat = np.ascontiguousarray(ci.flat())
+        keep, at, count = ci._joined()
         r = _PlanResult()
-        self._check(_lib.rcg_plan(self._ptr, ci.width, ci.height, ctypes.byref(lay), flat.ctypes.data, flat.size,
+        self._check(_lib.rcg_plan(self._ptr, ci.width, ci.height, ctypes.byref(lay), at, count,
                                   ctypes.byref(r)))
         return _plan(r)
 
@@ -828,23 +844,23 @@ class Context:
     def requantize(self, ci, quality, trellis=True):
         """CoefImage::requantize (jpeg/src/encode.rs:111) of a copy of `ci`; returns the new CoefImage."""
         lay = ci.layout()
-        flat = np.ascontiguousarray(ci.flat())
-        out = np.empty_like(flat)
+        keep, at, count = ci._joined()
+        out = np.empty(count, dtype=np.int16)
         t_in, t_out = ci.table_slots(), _QTables()
         self._check(_lib.rcg_requantize(self._ptr, ci.width, ci.height, ctypes.byref(lay), ctypes.byref(t_in),
-                                        flat.ctypes.data, int(quality), 1 if trellis else 0, out.ctypes.data,
+                                        at, int(quality), 1 if trellis else 0, out.ctypes.data,
                                         out.size, ctypes.byref(t_out)))
         return _general_image(ci, out, t_out)
 
     def find_quality_requantize(self, ci, target, max_quality=100, trellis=True, metric=METRIC_SSIMULACRA2):
         """The JPEG -> JPEG --target-ssimulacra2 search (cli/src/pipeline.rs:369-386) over requantizations of `ci`."""
         lay = ci.layout()
-        flat = np.ascontiguousarray(ci.flat())
-        out = np.empty_like(flat)
+        keep, at, count = ci._joined()
+        out = np.empty(count, dtype=np.int16)
         t_in, t_out = ci.table_slots(), _QTables()
         f = _Found()
         self._check(_lib.rcg_search_requantize(self._ptr, ci.width, ci.height, ctypes.byref(lay),
-                                               ctypes.byref(t_in), flat.ctypes.data, int(metric), float(target),
+                                               ctypes.byref(t_in), at, int(metric), float(target),
                                                int(max_quality), 1 if trellis else 0, ctypes.byref(f),
                                                out.ctypes.data, out.size, ctypes.byref(t_out)))
         trace = [(int(f.trace_q[i]), float(f.trace_score[i])) for i in range(f.nsteps)]
