@@ -768,8 +768,8 @@ int rcg_ssimulacra2_batch(rcg_ctx* ctx, int n, const uint8_t* const* references,
 
 // ---- rate-quality sweep
 
-// Device bytes one image of a sweep holds until its group is scored: the image and its candidates (8-bit), and both
-// sides' linear pyramids in the scorer (3 channels, 4/3 for the coarser scales, 4-byte floats: 16 B per pixel).
+// Device bytes one image of a sweep holds until its group is scored: the image and its candidates' planes (8-bit), and both
+// sides' pyramids in the scorer (3 channels, 4/3 for the coarser scales, 4-byte floats: 16 B per pixel).
 static size_t sweep_bytes(uint32_t w, uint32_t h, int channels, int nq) {
   const size_t px = (size_t)w * h;
   return (px * channels + 16 * px) * (size_t)(nq + 1);
@@ -778,47 +778,58 @@ constexpr size_t kSweepGroupBytes = 8ull << 30;  // images per group: as many as
 
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-// A group of images of rcg_sweep_qualities: every image's candidates at every quality encoded and decoded to 8-bit
-// pixels on the device, then all of the group's pairs scored by one work-list scorer call (each image converted once
-// as the reference of its candidates).
+// A group of images of rcg_sweep_qualities: every image's candidates at every quality encoded and decoded to component
+// planes on the device, then all of the group's pairs scored from them by one work-list scorer call (each image converted
+// once as the reference of its candidates). An image's candidates are encoded together, a launch per stage, as many at a
+// time as kSweepCoefBytes holds the coefficients of: eight of 2 MP one by one left most of the chip idle (40 launches,
+// 740 us with a colour image made of each; together four launches, 180 us).
+constexpr size_t kSweepCoefBytes = 512ull << 20;
 static int sweep_group(rcg_ctx* ctx, int n, const uint8_t* const* images, const uint32_t* widths,
                        const uint32_t* heights, const int* channels, int nq, const int* qualities,
                        const rcg_encode_options* opts, double* scores) {
   int rc;
-  std::vector<size_t> img_off((size_t)n), cand_off((size_t)n), img_bytes((size_t)n);
+  std::vector<size_t> img_off((size_t)n), cand_off((size_t)n), cand_bytes((size_t)n), img_bytes((size_t)n);
   size_t tot_img = 0, tot_cand = 0;
-  for (int i = 0; i < n; i++) {
-    img_bytes[(size_t)i] = (size_t)widths[i] * heights[i] * channels[i];
-    img_off[(size_t)i] = tot_img;
-    tot_img += align256(img_bytes[(size_t)i]);
-    cand_off[(size_t)i] = tot_cand;
-    tot_cand += align256(img_bytes[(size_t)i]) * (size_t)nq;
-  }
   // build_coefs' tables per (image, quality) (jpeg/src/encode.rs:426-539), one descriptor per candidate.
   std::vector<StepDesc> st((size_t)n * nq);
-  long long max_coefs = 0, max_planes = 0;
-  for (int i = 0; i < n; i++)
+  size_t coef_bytes = 0;
+  std::vector<int> chunk((size_t)n);  // candidates encoded at a time
+  std::vector<long long> max_coefs((size_t)n, 0);
+  for (int i = 0; i < n; i++) {
+    long long planes = 0;
     for (int k = 0; k < nq; k++) {
       StepDesc& d = st[(size_t)i * nq + k];
       host_step_tables(&d, qualities[k], opts->subsampling, channels[i], opts->trellis, (int)widths[i],
                        (int)heights[i]);
-      max_coefs = std::max(max_coefs, d.nblocks * 64);
-      max_planes = std::max(max_planes, plane_bytes(&d));
+      max_coefs[(size_t)i] = std::max(max_coefs[(size_t)i], d.nblocks * 64);
+      planes = std::max(planes, plane_bytes(&d));
     }
+    img_bytes[(size_t)i] = (size_t)widths[i] * heights[i] * channels[i];
+    img_off[(size_t)i] = tot_img;
+    tot_img += align256(img_bytes[(size_t)i]);
+    cand_bytes[(size_t)i] = align256((size_t)planes);
+    cand_off[(size_t)i] = tot_cand;
+    tot_cand += cand_bytes[(size_t)i] * (size_t)nq;
+    const size_t each = (size_t)max_coefs[(size_t)i] * 2;
+    chunk[(size_t)i] = (int)std::max<size_t>(1, std::min<size_t>((size_t)nq, kSweepCoefBytes / each));
+    coef_bytes = std::max(coef_bytes, each * (size_t)chunk[(size_t)i]);
+  }
   uint8_t* d_imgs = (uint8_t*)workspace(ctx, "sweep_imgs", tot_img);
   uint8_t* d_cand = (uint8_t*)workspace(ctx, "sweep_cands", tot_cand);
-  int16_t* d_coefs = (int16_t*)workspace(ctx, "sweep_coefs", (size_t)max_coefs * 2);
-  uint8_t* d_planes = (uint8_t*)workspace(ctx, "sweep_planes", (size_t)max_planes);
+  int16_t* d_coefs = (int16_t*)workspace(ctx, "sweep_coefs", coef_bytes);
   StepDesc* d_sts = (StepDesc*)workspace(ctx, "sweep_steps", sizeof(StepDesc) * st.size());
-  if (!d_imgs || !d_cand || !d_coefs || !d_planes || !d_sts) return RCG_NO_MEMORY;
-  for (StepDesc& d : st) d.coefs = d_coefs;  // one candidate at a time, in stream order
+  if (!d_imgs || !d_cand || !d_coefs || !d_sts) return RCG_NO_MEMORY;
+  for (int i = 0; i < n; i++)
+    for (int k = 0; k < nq; k++)  // a chunk's candidates side by side, the next chunk after it in stream order
+      st[(size_t)i * nq + k].coefs = d_coefs + (k % chunk[(size_t)i]) * max_coefs[(size_t)i];
   // Host copies first: a pageable copy waits for the stream, so they go before any kernel of the group.
   for (int i = 0; i < n; i++)
     if ((rc = copy_to_device(ctx, d_imgs + img_off[(size_t)i], images[i], img_bytes[(size_t)i])) != RCG_OK) return rc;
   cudaError_t e = cudaMemcpyAsync(d_sts, st.data(), sizeof(StepDesc) * st.size(), cudaMemcpyHostToDevice,
                                   ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep tables upload");
-  std::vector<const uint8_t*> refs(st.size()), dists(st.size());
+  std::vector<const uint8_t*> refs(st.size());
+  std::vector<Decoded> decoded(st.size());
   std::vector<uint32_t> ws(st.size()), hs(st.size());
   std::vector<int> cs(st.size());
   for (int i = 0; i < n; i++) {
@@ -827,25 +838,28 @@ static int sweep_group(rcg_ctx* ctx, int n, const uint8_t* const* images, const 
     if ((rc = setup_encoder(ctx, d_src, (int)widths[i], (int)heights[i], channels[i], opts->subsampling, &es)) !=
         RCG_OK)
       return rc;
+    uint8_t* planes = d_cand + cand_off[(size_t)i];
+    const long long stride = (long long)cand_bytes[(size_t)i];
+    for (int k = 0; k < nq; k += chunk[(size_t)i]) {
+      StepDesc* d_st = d_sts + (size_t)i * nq + k;
+      const int count = std::min(chunk[(size_t)i], nq - k);
+      quantize(ctx, d_st, es.caches, es.max_blocks, count);
+      rate_tables(ctx, d_st, count);
+      trellis(ctx, d_st, es.caches, es.max_blocks, false, count);
+      dequant_idct(ctx, d_st, nullptr, planes + k * stride, es.max_blocks, count, stride);
+    }
     for (int k = 0; k < nq; k++) {
       const size_t j = (size_t)i * nq + k;
-      StepDesc* d_st = d_sts + j;
-      quantize(ctx, d_st, es.caches, es.max_blocks);
-      rate_tables(ctx, d_st);
-      trellis(ctx, d_st, es.caches, es.max_blocks);
-      dequant_idct(ctx, d_st, nullptr, d_planes, es.max_blocks);  // reconstruct (jpeg/src/decode.rs:334-389)
-      uint8_t* out = d_cand + cand_off[(size_t)i] + align256(img_bytes[(size_t)i]) * (size_t)k;
-      upsample_color(ctx, d_st, d_planes, (int)widths[i], (int)heights[i], out, nullptr);
       refs[j] = d_src;
-      dists[j] = out;
+      decoded[j] = Decoded{planes + k * stride, d_sts + j};
       ws[j] = widths[i];
       hs[j] = heights[i];
       cs[j] = channels[i];
     }
   }
   double* d_scores = nullptr;
-  if ((rc = score_batch(ctx, (int)st.size(), refs.data(), dists.data(), ws.data(), hs.data(), cs.data(), nullptr,
-                        &d_scores)) != RCG_OK)
+  if ((rc = score_batch(ctx, (int)st.size(), refs.data(), nullptr, ws.data(), hs.data(), cs.data(), nullptr, &d_scores,
+                        decoded.data())) != RCG_OK)
     return rc;
   if ((rc = copy_to_host(ctx, scores, d_scores, sizeof(double) * st.size())) != RCG_OK) return rc;
   return finish(ctx, "sweep");

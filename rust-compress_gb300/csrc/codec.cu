@@ -293,13 +293,13 @@ __device__ __forceinline__ void quantize_body(StepDesc* __restrict__ st, const C
 
 __global__ void __launch_bounds__(128, 4) k_quantize(StepDesc* __restrict__ st, CacheSet cs) {
   grid_chain();
-  quantize_body(st, cs, blockIdx.x);
+  quantize_body(st + blockIdx.y, cs, blockIdx.x);  // blockIdx.y: the candidate of several encoded at once
 }
 
-int quantize(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks) {
+int quantize(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, int count) {
   CacheSet cs;
   for (int i = 0; i < 9; i++) cs.p[i] = d_caches[i];
-  int grid = (int)((max_blocks + 127) / 128);
+  const dim3 grid((unsigned)((max_blocks + 127) / 128), (unsigned)count);
   RCG_LAUNCH(ctx, "quantize", k_quantize, grid, 128, 0, d_step, cs);
   return RCG_OK;
 }
@@ -352,10 +352,10 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
   if (t == 0) st->eob[comp] = fmul(lambda, len[0]);
 }
 
-__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) { grid_chain(); rate_tables_body(st, blockIdx.x); }
+__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) { grid_chain(); rate_tables_body(st + blockIdx.y, blockIdx.x); }
 
-int rate_tables(rcg_ctx* ctx, StepDesc* d_step) {
-  RCG_LAUNCH(ctx, "rate_tables", k_rate_tables, 3, 288, 0, d_step);
+int rate_tables(rcg_ctx* ctx, StepDesc* d_step, int count) {
+  RCG_LAUNCH(ctx, "rate_tables", k_rate_tables, dim3(3, (unsigned)count), 288, 0, d_step);
   return RCG_OK;
 }
 
@@ -602,13 +602,14 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
 template <bool kWeighted>
 __global__ void __launch_bounds__(128, 7) k_trellis(StepDesc* __restrict__ st, CacheSet cs) {
   grid_chain();
-  trellis_body<kWeighted>(st, cs, blockIdx.x);
+  trellis_body<kWeighted>(st + blockIdx.y, cs, blockIdx.x);
 }
 
-int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted) {
+int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted,
+            int count) {
   CacheSet cs;
   for (int i = 0; i < 9; i++) cs.p[i] = d_caches ? d_caches[i] : nullptr;
-  int grid = (int)((max_blocks + 127) / 128);
+  const dim3 grid((unsigned)((max_blocks + 127) / 128), (unsigned)count);
   if (weighted)
     RCG_LAUNCH(ctx, "trellis_weighted", k_trellis<true>, grid, 128, 0, d_step, cs);
   else
@@ -697,14 +698,16 @@ __device__ __forceinline__ void dequant_idct_body(const StepDesc* __restrict__ s
 }
 
 __global__ void __launch_bounds__(128) k_dequant_idct(const StepDesc* __restrict__ st,
-                                                     const int16_t* __restrict__ coefs, uint8_t* __restrict__ planes) {
+                                                     const int16_t* __restrict__ coefs, uint8_t* __restrict__ planes,
+                                                     long long planes_stride) {
   grid_chain();
-  dequant_idct_body(st, coefs, planes, blockIdx.x);
+  dequant_idct_body(st + blockIdx.y, coefs, planes + blockIdx.y * planes_stride, blockIdx.x);
 }
 
-int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks) {
-  int grid = (int)((max_blocks + 127) / 128);
-  RCG_LAUNCH(ctx, "dequant_idct", k_dequant_idct, grid, 128, 0, d_step, d_coefs, d_planes);
+int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks,
+                 int count, long long planes_stride) {
+  const dim3 grid((unsigned)((max_blocks + 127) / 128), (unsigned)count);
+  RCG_LAUNCH(ctx, "dequant_idct", k_dequant_idct, grid, 128, 0, d_step, d_coefs, d_planes, planes_stride);
   return RCG_OK;
 }
 

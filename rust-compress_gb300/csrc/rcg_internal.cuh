@@ -384,9 +384,15 @@ inline size_t ref_moment_bytes(const PyramidDesc& banded_pd) {
 int score_workspace(rcg_ctx* ctx, const PyramidDesc& pd);
 // Score n device-resident pairs (checked sizes and formats; depths nullable = 8) with the work-list kernels;
 // *d_scores receives the device array of the n scores (NaN where a score is not finite), ready once the stream is.
+// `decoded` (nullable): the distorted images are an encoder's decoded planes instead (d_dists is not read; 8-bit).
+struct Decoded {
+  const uint8_t* planes;
+  const StepDesc* st;  // on the device: their layout
+};
 int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t* const* d_dists,
                 const uint32_t* widths, const uint32_t* heights, const int* channels, const int* depths,
-                double** d_scores);
+                double** d_scores,
+                const Decoded* decoded = nullptr);
 
 // ---- lockstep batch (work-list launches over the LockItems of a batch; totals are the grids' CTA counts)
 // first: the step's tables too (else the step before has filled them).
@@ -402,15 +408,17 @@ int color_pad(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, in
 int chroma_down(rcg_ctx* ctx, const uint8_t* d_src, int src_stride, int pw, int ph, int fx, int fy, uint8_t* d_dst);
 // FDCT of every block of a plane into the zigzag [k][block] cache (quality-independent; jpeg/src/encode.rs:189-196).
 int fdct_cache(rcg_ctx* ctx, const uint8_t* d_plane, int stride, int bw, int bh, float* d_cache);
-// Per-candidate pipeline pieces, all driven by a device StepDesc.
-int quantize(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks);
+// Per-candidate pipeline pieces, all driven by a device StepDesc (or `count` consecutive ones of one image at once).
+int quantize(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, int count = 1);
 // Plain requantization of st->coef_src into st->coefs, with the AC histogram when the trellis pass follows.
 int requantize_plain(rcg_ctx* ctx, StepDesc* d_step, long long max_blocks);
-int rate_tables(rcg_ctx* ctx, StepDesc* d_step);
+int rate_tables(rcg_ctx* ctx, StepDesc* d_step, int count = 1);
 // weighted: the perceptual mode (d_step->pweights); otherwise the reference's plain trellis.
-int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted = false);
-// d_coefs null: decode the candidate's own coefficients (d_step->coefs).
-int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks);
+int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted = false,
+            int count = 1);
+// d_coefs null: decode the candidate's own coefficients (d_step->coefs). The planes of several are planes_stride apart.
+int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks,
+                 int count = 1, long long planes_stride = 0);
 // Upsample + YCbCr->RGB (jpeg/src/decode.rs:1404-1444). Writes interleaved 8-bit pixels to d_rgb (nullable)
 // and/or linear planes [3][h][pitch] to d_lin (nullable).
 int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, uint8_t* d_rgb,

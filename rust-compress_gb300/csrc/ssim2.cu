@@ -1195,13 +1195,13 @@ __device__ __forceinline__ int find_first(const long long* __restrict__ first, i
   return lo;
 }
 
-template <int kOut>
+template <int kSrc, int kOut>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build_batch(const BuildJob* __restrict__ jobs,
                                                                               const long long* __restrict__ cta0, int n) {
   grid_chain();
   const int i = find_first(cta0, n, blockIdx.x);
   const BuildJob& j = jobs[i];
-  build_block<kFromImage, kOut>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
+  build_block<kSrc, kOut>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
 }
 
 // One CTA per tile of the work-list. A persistent form (a fixed grid of k CTAs per SM striding over the list, each
@@ -1614,7 +1614,7 @@ int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, cons
 
 int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t* const* d_dists,
                 const uint32_t* widths, const uint32_t* heights, const int* channels, const int* depths,
-                double** d_scores) {
+                double** d_scores, const Decoded* decoded) {
   std::vector<ScoreItem> items((size_t)n);
   std::map<std::tuple<const uint8_t*, uint32_t, uint32_t, int, int>, int> first_ref;
   std::vector<int> ref_of((size_t)n), uses((size_t)n, 0);
@@ -1648,7 +1648,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
     const int r = ref_of[(size_t)i];
     if (r == i) {
       off_xyb[(size_t)i] = alloc(items[(size_t)i].pd);
-      if (uses[(size_t)i] > 1) off_lin[(size_t)i] = alloc(items[(size_t)i].pd);
+      if (uses[(size_t)i] > 1 || decoded) off_lin[(size_t)i] = alloc(items[(size_t)i].pd);
     }
     off_diff[(size_t)i] = alloc(items[(size_t)i].pd);
   }
@@ -1673,9 +1673,10 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   };
   for (int i = 0; i < n; i++) {
     const int r = ref_of[(size_t)i], depth = depths ? depths[i] : 8, w = (int)widths[i], h = (int)heights[i];
-    const ImageSrc a = {d_refs[i], w, h, channels[i], depth, lut16}, b = {d_dists[i], w, h, channels[i], depth, lut16};
+    const ImageSrc a = {d_refs[i], w, h, channels[i], depth, lut16},
+                   b = {decoded ? nullptr : d_dists[i], w, h, channels[i], depth, lut16};
     BuildArgs g = {};
-    if (uses[(size_t)r] == 1) {
+    if (uses[(size_t)r] == 1 && !decoded) {
       g.im[0] = a;
       g.im[1] = b;
       g.xyb = base + off_xyb[(size_t)i];
@@ -1690,7 +1691,12 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
       add(0, i, g);
     }
     g = {};
-    g.im[0] = b;
+    if (decoded) {
+      g.planes = decoded[i].planes;
+      g.st = decoded[i].st;
+    } else {
+      g.im[0] = b;
+    }
     g.ref = base + off_lin[(size_t)r];
     g.out = base + off_diff[(size_t)i];
     add(1, i, g);
@@ -1755,16 +1761,19 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   // The launches take only the work-list's totals and this context's buffers: a later batch with the same totals
   // replays them (its own pairs come in through the work-list uploaded above).
   const std::vector<long long> key = {3,     n,     nseg,    tiles,   max_scales, nj[0],
-                                      nj[1], nj[2], ctas[0], ctas[1], ctas[2]};
+                                      nj[1], nj[2], ctas[0], ctas[1], ctas[2], decoded != nullptr};
   int rc = run_step_loop(ctx, key, [&]() {
     if (nj[0])
-      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutRef>, (unsigned)ctas[0], kPyrThreads, 0, d_jobs(0), d_first(0),
+      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutRef>), (unsigned)ctas[0], kPyrThreads, 0, d_jobs(0), d_first(0),
                  nj[0]);
-    if (nj[1])
-      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutDiff>, (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1), d_first(1),
-                 nj[1]);
+    if (nj[1] && decoded)
+      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromPlanes, kOutDiff>), (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1),
+                 d_first(1), nj[1]);
+    else if (nj[1])
+      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutDiff>), (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1),
+                 d_first(1), nj[1]);
     if (nj[2])
-      RCG_LAUNCH(ctx, "build_batch", k_build_batch<kOutPair>, (unsigned)ctas[2], kPyrThreads, 0, d_jobs(2), d_first(2),
+      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutPair>), (unsigned)ctas[2], kPyrThreads, 0, d_jobs(2), d_first(2),
                  nj[2]);
     RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, tile_grid(tiles), kTileThreads, tile_smem(kRefNone), d_segs,
                d_seg0, nseg);
