@@ -796,7 +796,7 @@ def main():
     prof = {}
     for k in ("ssim2_tiles_cached", "ssim2_tiles_store", "ssim2_tiles", "trellis", "quantize", "dequant_idct",
               "build_diff", "build_reference", "ssim2_reduce", "rate_tables", "step_tables",
-              "fdct_cache", "color_pad", "chroma_down"):
+              "fdct_image"):
         n, ms = ctx.kernel_time(k)
         prof[k] = {"launches": n, "ms": ms}
     ctx.set_profiling(False)

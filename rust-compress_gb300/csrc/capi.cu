@@ -294,45 +294,24 @@ static int setup_encoder(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int c
     }
   }
   const int hv[3][2] = {{2, 2}, {2, 1}, {1, 1}};
-  int pw_max = 0, ph_max = 0;
-  for (int k = 0; k < 3; k++) {
-    if (!kinds[k]) continue;
-    int hm = channels == 1 ? 1 : hv[k][0], vm = channels == 1 ? 1 : hv[k][1];
-    pw_max = std::max(pw_max, (w + 8 * hm - 1) / (8 * hm) * 8 * hm);
-    ph_max = std::max(ph_max, (h + 8 * vm - 1) / (8 * vm) * 8 * vm);
-  }
-  size_t plane = (size_t)pw_max * ph_max;
-  uint8_t* yp = (uint8_t*)workspace(ctx, "plane_y", plane);
-  uint8_t* cbp = channels == 1 ? nullptr : (uint8_t*)workspace(ctx, "plane_cb", plane);
-  uint8_t* crp = channels == 1 ? nullptr : (uint8_t*)workspace(ctx, "plane_cr", plane);
-  if (!yp || (channels == 3 && (!cbp || !crp))) return RCG_NO_MEMORY;
-  color_pad(ctx, d_src, w, h, channels, pw_max, ph_max, yp, cbp, crp);
   for (int k = 0; k < 3; k++) {
     if (!kinds[k]) continue;
     int hm = channels == 1 ? 1 : hv[k][0], vm = channels == 1 ? 1 : hv[k][1];
     int pw = (w + 8 * hm - 1) / (8 * hm) * 8 * hm, ph = (h + 8 * vm - 1) / (8 * vm) * 8 * vm;
     long long blocks = 0, pbytes = 0;
+    int bws[3], bhs[3];
+    float* caches[3] = {nullptr, nullptr, nullptr};
     for (int c = 0; c < (channels == 1 ? 1 : 3); c++) {
       int cw = c == 0 ? pw : pw / hm, chh = c == 0 ? ph : ph / vm;
-      int bw = cw / 8, bh = chh / 8;
+      int bw = bws[c] = cw / 8, bh = bhs[c] = chh / 8;
       std::string name = "fdct_cache_" + std::to_string(k * 3 + c);
       float* cache = (float*)workspace(ctx, name.c_str(), (size_t)bw * bh * 64 * sizeof(float));
       if (!cache) return RCG_NO_MEMORY;
-      const uint8_t* src = c == 0 ? yp : (c == 1 ? cbp : crp);
-      int stride = pw_max;
-      if (c > 0 && hm * vm > 1) {
-        std::string dn = "plane_sub_" + std::to_string(k * 3 + c);
-        uint8_t* sub = (uint8_t*)workspace(ctx, dn.c_str(), (size_t)cw * chh);
-        if (!sub) return RCG_NO_MEMORY;
-        chroma_down(ctx, src, pw_max, pw, ph, hm, vm, sub);
-        src = sub;
-        stride = cw;
-      }
-      fdct_cache(ctx, src, stride, bw, bh, cache);
-      es->caches[k * 3 + c] = cache;
+      es->caches[k * 3 + c] = caches[c] = cache;
       blocks += (long long)bw * bh;
       pbytes += (long long)cw * chh;
     }
+    fdct_image(ctx, d_src, w, h, channels, hm, vm, caches, bws, bhs);
     es->max_blocks = std::max(es->max_blocks, blocks);
     es->max_coefs = std::max(es->max_coefs, blocks * 64);
     es->max_plane_bytes = std::max(es->max_plane_bytes, pbytes);

@@ -6,7 +6,6 @@
 // (colour conversion, subsampling, upsampling, histograms) are exact by construction.
 //
 // Layouts in HBM:
-//   padded planes      u8, row-major, stride = padded width (the MCU-padded grid of jpeg/src/encode.rs:440-443)
 //   FDCT cache         f32, [64][nblocks] per component: zigzag coefficient k of block b at k*nblocks + b, so a
 //                      thread-per-block kernel reads one coalesced row per coefficient. Quality-independent: the
 //                      reference recomputes it for every candidate (jpeg/src/encode.rs:189-196).
@@ -92,59 +91,7 @@ __device__ __forceinline__ int comp_of(const StepDesc* st, long long gb) {
   return c;
 }
 
-// ------------------------------------------------------------------------------------------------ K1 colour + pad
-
-// jpeg/src/encode.rs:451-477: edge-replicated Y/Cb/Cr planes over the padded grid (Gray: Y only).
-__global__ void k_color_pad(const uint8_t* __restrict__ src, int w, int h, int channels, int pw, int ph,
-                            uint8_t* __restrict__ yp, uint8_t* __restrict__ cbp, uint8_t* __restrict__ crp) {
-  grid_chain();
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= pw) return;
-  for (int r = blockIdx.y; r < ph; r += gridDim.y) {
-    int sr = min(r, h - 1), sx = min(x, w - 1);
-    size_t o = (size_t)r * pw + x;
-    if (channels == 1) {
-      yp[o] = src[(size_t)sr * w + sx];
-      continue;
-    }
-    size_t i = ((size_t)sr * w + sx) * 3;
-    int rr = src[i], gg = src[i + 1], bb = src[i + 2];
-    yp[o] = (uint8_t)((19595 * rr + 38470 * gg + 7471 * bb + 32768) >> 16);
-    cbp[o] = (uint8_t)((-11059 * rr - 21709 * gg + 32768 * bb + (128 << 16) + 32767) >> 16);
-    crp[o] = (uint8_t)((32768 * rr - 27439 * gg - 5329 * bb + (128 << 16) + 32767) >> 16);
-  }
-}
-
-int color_pad(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int pw, int ph, uint8_t* d_y,
-              uint8_t* d_cb, uint8_t* d_cr) {
-  dim3 grid((pw + 255) / 256, std::min(ph, 65535));
-  RCG_LAUNCH(ctx, "color_pad", k_color_pad, grid, 256, 0, d_src, w, h, channels, pw, ph, d_y, d_cb, d_cr);
-  return RCG_OK;
-}
-
-// jpeg/src/encode.rs:478-499 (down): (sum + n/2) / n over fx*fy samples. Source stride pw, output (pw/fx)x(ph/fy).
-__global__ void k_chroma_down(const uint8_t* __restrict__ p, int stride, int pw, int ph, int fx, int fy,
-                              uint8_t* __restrict__ o) {
-  grid_chain();
-  int cw = pw / fx, ch = ph / fy;
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= cw) return;
-  for (int r = blockIdx.y; r < ch; r += gridDim.y) {
-    unsigned s = 0;
-    for (int dy = 0; dy < fy; dy++)
-      for (int dx = 0; dx < fx; dx++) s += p[(size_t)(fy * r + dy) * stride + fx * x + dx];
-    unsigned n = (unsigned)(fx * fy);
-    o[(size_t)r * cw + x] = (uint8_t)((s + n / 2) / n);
-  }
-}
-
-int chroma_down(rcg_ctx* ctx, const uint8_t* d_src, int src_stride, int pw, int ph, int fx, int fy, uint8_t* d_dst) {
-  dim3 grid((pw / fx + 255) / 256, std::min(ph / fy, 65535));
-  RCG_LAUNCH(ctx, "chroma_down", k_chroma_down, grid, 256, 0, d_src, src_stride, pw, ph, fx, fy, d_dst);
-  return RCG_OK;
-}
-
-// ------------------------------------------------------------------------------------------------ K2 FDCT cache
+// ------------------------------------------------------------------------------------------------ K1, K2 image to FDCT
 
 // jpeg/src/dct.rs:20-57 (fdct_pass) on column j of a row-major 8x8 block held in registers.
 __device__ __forceinline__ void fdct_pass(float (&d)[64]) {
@@ -184,42 +131,146 @@ __device__ __forceinline__ void transpose8(float (&b)[64]) {
     }
 }
 
-// One thread per block: level shift (x - 128), FDCT (jpeg/src/dct.rs:59-65), store in zigzag order
-// (flat[ZZ_T[k]], jpeg/src/encode.rs:201-211) as cache[k*nb + b].
-__global__ void k_fdct_cache(const uint8_t* __restrict__ plane, int stride, int bw, int bh, float* __restrict__ cache) {
+// From the image to the FDCT caches of one sampling layout. A CTA takes 256 x 16 pixels of the padded grid: the colour
+// conversion with edge replication (jpeg/src/encode.rs:451-477) into shared memory, the chroma box filter
+// (sum + n/2) / n (:478-499), then a thread per block: level shift (x - 128), FDCT (jpeg/src/dct.rs:59-65), stored in
+// zigzag order (flat[ZZ_T[k]], jpeg/src/encode.rs:201-211) as cache[k * blocks + b], 32 blocks of a row side by side.
+// What bounds it: the store of the caches (72 MB at 12 MP 4:2:0) at large sizes, its latency and launch at small ones.
+// Measured against a launch each for the planes, either chroma plane and the three caches, whose planes made two trips
+// through memory, converted and filtered a byte at a time: 12 MP 4:2:0 124 -> 48 us, 2 MP 56 -> 16, 240x180 4:4:4 26 -> 11.
+constexpr int kFdW = 256, kFdH = 16, kFdThreads = 128;
+
+struct FdctOut {
+  float* cache[3];
+  int bw[3], bh[3];
+};
+
+template <int kFx, int kFy, bool kGray>
+__global__ void __launch_bounds__(kFdThreads) k_fdct_image(const uint8_t* __restrict__ src, int w, int h,
+                                                           const FdctOut out) {
   grid_chain();
-  long long nb = (long long)bw * bh;
-  long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  int by = (int)(b / bw), bx = (int)(b % bw);
-  float blk[64];
+  constexpr bool kDown = !kGray && kFx * kFy > 1;
+  constexpr int kSubW = kFdW / kFx, kSubH = kFdH / kFy;
+  __shared__ __align__(16) uint8_t px[kGray ? 1 : 3][kFdH][kFdW];
+  __shared__ __align__(16) uint8_t sub[2][kDown ? kSubH : 1][kDown ? kSubW : 8];
+  const int t = threadIdx.x, x0 = blockIdx.x * kFdW, y0 = blockIdx.y * kFdH;
+  constexpr int kBytes = kGray ? 4 : 12;  // of four pixels
+  const size_t total = (size_t)w * h * (kBytes / 4);
+#pragma unroll 2
+  for (int e = t; e < kFdW / 4 * kFdH; e += kFdThreads) {
+    const int q = e % (kFdW / 4), r = e / (kFdW / 4), gx = x0 + 4 * q;
+    if (gx >= out.bw[0] * 8) continue;  // past the padded grid
+    const size_t row = (size_t)min(y0 + r, h - 1) * w, at = (row + gx) * (kBytes / 4);
+    uint32_t b[3] = {0, 0, 0};
+    const int mis = (int)((uintptr_t)(src + at) & 3);
+    // Bytes of any alignment: the aligned words that hold them and a funnel shift, where those lie in the image.
+    if (gx + 4 <= w && at >= (size_t)mis && (mis == 0 || at + kBytes + 4 - mis <= total)) {
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(src + at - mis);
+      uint32_t v[4];
 #pragma unroll
-  for (int y = 0; y < 8; y++) {
-    const uint8_t* src = plane + (size_t)(by * 8 + y) * stride + bx * 8;
-    uint2 v = *reinterpret_cast<const uint2*>(src);
+      for (int k = 0; k < kBytes / 4; k++) v[k] = __ldg(p + k);
+      v[kBytes / 4] = mis ? __ldg(p + kBytes / 4) : 0u;
 #pragma unroll
-    for (int x = 0; x < 8; x++) {
-      unsigned word = x < 4 ? v.x : v.y;
-      unsigned byte = (word >> (8 * (x & 3))) & 0xFF;
-      blk[y * 8 + x] = fsub((float)byte, 128.0f);
+      for (int k = 0; k < kBytes / 4; k++) b[k] = __funnelshift_r(v[k], v[k + 1], 8 * mis);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kBytes; k++) {
+        const int px4 = kGray ? k : k / 3, c = kGray ? 0 : k % 3;
+        const uint32_t v = src[(row + min(gx + px4, w - 1)) * (kBytes / 4) + c];
+        b[k / 4] |= v << (8 * (k % 4));
+      }
+    }
+    if (kGray) {
+      *reinterpret_cast<uint32_t*>(&px[0][r][4 * q]) = b[0];
+    } else {
+      uint32_t yy = 0, cb = 0, cr = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        auto byte = [&](int i) { return (int)((b[i / 4] >> (8 * (i % 4))) & 0xFF); };
+        const int rr = byte(3 * k), gg = byte(3 * k + 1), bb = byte(3 * k + 2);
+        yy |= (uint32_t)(uint8_t)((19595 * rr + 38470 * gg + 7471 * bb + 32768) >> 16) << (8 * k);
+        cb |= (uint32_t)(uint8_t)((-11059 * rr - 21709 * gg + 32768 * bb + (128 << 16) + 32767) >> 16) << (8 * k);
+        cr |= (uint32_t)(uint8_t)((32768 * rr - 27439 * gg - 5329 * bb + (128 << 16) + 32767) >> 16) << (8 * k);
+      }
+      *reinterpret_cast<uint32_t*>(&px[0][r][4 * q]) = yy;
+      *reinterpret_cast<uint32_t*>(&px[kGray ? 0 : 1][r][4 * q]) = cb;
+      *reinterpret_cast<uint32_t*>(&px[kGray ? 0 : 2][r][4 * q]) = cr;
     }
   }
-  fdct_pass(blk);
-  transpose8(blk);
-  fdct_pass(blk);
+  __syncthreads();
+  if constexpr (kDown) {
+    static_assert(kFx == 2, "chroma is halved across");
+    for (int e = t; e < 2 * kSubH * (kSubW / 4); e += kFdThreads) {
+      const int q = e % (kSubW / 4), r = e / (kSubW / 4) % kSubH, c = e / (kSubW / 4 * kSubH);
+      uint32_t v = 0;
 #pragma unroll
-  for (int k = 0; k < 64; k++) {
-    constexpr int ZT[64] = {0,  8,  1,  2,  9,  16, 24, 17, 10, 3,  4,  11, 18, 25, 32, 40, 33, 26, 19, 12, 5,  6,
-                            13, 20, 27, 34, 41, 48, 56, 49, 42, 35, 28, 21, 14, 7,  15, 22, 29, 36, 43, 50, 57, 58,
-                            51, 44, 37, 30, 23, 31, 38, 45, 52, 59, 60, 53, 46, 39, 47, 54, 61, 62, 55, 63};
-    cache[(long long)k * nb + b] = blk[ZT[k]];
+      for (int k = 0; k < 4; k++) {
+        unsigned sum = 0;
+#pragma unroll
+        for (int dy = 0; dy < kFy; dy++) {
+          const uint2 p = *reinterpret_cast<const uint2*>(&px[1 + c][kFy * r + dy][8 * q]);
+          const uint32_t word = k < 2 ? p.x : p.y;
+          sum += ((word >> (16 * (k & 1))) & 0xFF) + ((word >> (16 * (k & 1) + 8)) & 0xFF);
+        }
+        v |= ((sum + kFx * kFy / 2) / (kFx * kFy)) << (8 * k);
+      }
+      *reinterpret_cast<uint32_t*>(&sub[c][r][4 * q]) = v;
+    }
+    __syncthreads();
+  }
+  constexpr int kLuma = kFdW / 8 * (kFdH / 8), kChroma = kGray ? 0 : kSubW / 8 * (kSubH / 8);
+#pragma unroll 1
+  for (int i = t; i < kLuma + 2 * kChroma; i += kFdThreads) {
+    const int c = i < kLuma ? 0 : i < kLuma + kChroma ? 1 : 2;
+    const int e = i - (c == 0 ? 0 : c == 1 ? kLuma : kLuma + kChroma), across = c == 0 ? kFdW / 8 : kSubW / 8;
+    const int lx = e % across, ly = e / across;
+    const int bx = blockIdx.x * across + lx, by = blockIdx.y * (c == 0 ? kFdH / 8 : kSubH / 8) + ly;
+    if (bx >= out.bw[c] || by >= out.bh[c]) continue;
+    const bool down = kDown && c > 0;
+    const uint8_t* from = down ? &sub[c - 1][ly * 8][lx * 8] : &px[kGray ? 0 : c][ly * 8][lx * 8];
+    float blk[64];
+#pragma unroll
+    for (int y = 0; y < 8; y++) {
+      const uint2 v = *reinterpret_cast<const uint2*>(from + y * (down ? kSubW : kFdW));
+#pragma unroll
+      for (int x = 0; x < 8; x++) {
+        const unsigned word = x < 4 ? v.x : v.y;
+        blk[y * 8 + x] = fsub((float)((word >> (8 * (x & 3))) & 0xFF), 128.0f);
+      }
+    }
+    fdct_pass(blk);
+    transpose8(blk);
+    fdct_pass(blk);
+    const long long nb = (long long)out.bw[c] * out.bh[c], b = (long long)by * out.bw[c] + bx;
+    float* cache = out.cache[c] + b;
+#pragma unroll
+    for (int k = 0; k < 64; k++) {
+      constexpr int ZT[64] = {0,  8,  1,  2,  9,  16, 24, 17, 10, 3,  4,  11, 18, 25, 32, 40, 33, 26, 19, 12, 5,  6,
+                              13, 20, 27, 34, 41, 48, 56, 49, 42, 35, 28, 21, 14, 7,  15, 22, 29, 36, 43, 50, 57, 58,
+                              51, 44, 37, 30, 23, 31, 38, 45, 52, 59, 60, 53, 46, 39, 47, 54, 61, 62, 55, 63};
+      cache[(long long)k * nb] = blk[ZT[k]];
+    }
   }
 }
 
-int fdct_cache(rcg_ctx* ctx, const uint8_t* d_plane, int stride, int bw, int bh, float* d_cache) {
-  long long nb = (long long)bw * bh;
-  int grid = (int)((nb + 127) / 128);
-  RCG_LAUNCH(ctx, "fdct_cache", k_fdct_cache, grid, 128, 0, d_plane, stride, bw, bh, d_cache);
+int fdct_image(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int fx, int fy, float* const* d_caches,
+               const int* bw, const int* bh) {
+  FdctOut out;
+  std::memset(&out, 0, sizeof out);
+  for (int c = 0; c < (channels == 1 ? 1 : 3); c++) {
+    out.cache[c] = d_caches[c];
+    out.bw[c] = bw[c];
+    out.bh[c] = bh[c];
+  }
+  const dim3 grid((unsigned)((bw[0] * 8 + kFdW - 1) / kFdW), (unsigned)((bh[0] * 8 + kFdH - 1) / kFdH));
+  if (channels == 1)
+    RCG_LAUNCH(ctx, "fdct_image", (k_fdct_image<1, 1, true>), grid, kFdThreads, 0, d_src, w, h, out);
+  else if (fy == 2)
+    RCG_LAUNCH(ctx, "fdct_image", (k_fdct_image<2, 2, false>), grid, kFdThreads, 0, d_src, w, h, out);
+  else if (fx == 2)
+    RCG_LAUNCH(ctx, "fdct_image", (k_fdct_image<2, 1, false>), grid, kFdThreads, 0, d_src, w, h, out);
+  else
+    RCG_LAUNCH(ctx, "fdct_image", (k_fdct_image<1, 1, false>), grid, kFdThreads, 0, d_src, w, h, out);
   return RCG_OK;
 }
 

@@ -401,13 +401,11 @@ void lock_step_score(rcg_ctx* ctx, const LockItem* d_items, int n, long long p_t
                      int max_scales, int ref_mode = kRefNone);
 
 // ---- codec (codec.cu)
-// Colour conversion + edge padding (jpeg/src/encode.rs:463-477): full-resolution padded Y/Cb/Cr planes.
-int color_pad(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int pw, int ph, uint8_t* d_y,
-              uint8_t* d_cb, uint8_t* d_cr);
-// 2-D box downsample of a padded chroma plane (jpeg/src/encode.rs:478-499).
-int chroma_down(rcg_ctx* ctx, const uint8_t* d_src, int src_stride, int pw, int ph, int fx, int fy, uint8_t* d_dst);
-// FDCT of every block of a plane into the zigzag [k][block] cache (quality-independent; jpeg/src/encode.rs:189-196).
-int fdct_cache(rcg_ctx* ctx, const uint8_t* d_plane, int stride, int bw, int bh, float* d_cache);
+// An image's FDCT caches in one sampling layout (chroma reduced by fx x fy; quality-independent): colour conversion and
+// edge padding (jpeg/src/encode.rs:451-477), chroma downsampling (:478-499) and the FDCT of every block, zigzag
+// [k][block] (:189-196). bw, bh: blocks of each component.
+int fdct_image(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int fx, int fy, float* const* d_caches,
+               const int* bw, const int* bh);
 // Per-candidate pipeline pieces, all driven by a device StepDesc (or `count` consecutive ones of one image at once).
 int quantize(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, int count = 1);
 // Plain requantization of st->coef_src into st->coefs, with the AC histogram when the trellis pass follows.
