@@ -794,7 +794,7 @@ def main():
     for _ in range(3):
         step_device()
     prof = {}
-    for k in ("ssim2_tiles_cached", "ssim2_tiles_store", "ssim2_tiles", "trellis", "quantize", "dequant_idct",
+    for k in ("ssim2_tiles_cached", "ssim2_tiles_store", "ssim2_tiles", "trellis", "trellis_decode", "quantize", "dequant_idct",
               "build_diff", "build_reference", "ssim2_reduce", "rate_tables", "step_tables",
               "fdct_image"):
         n, ms = ctx.kernel_time(k)

@@ -1343,8 +1343,7 @@ static int search_impl(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int cha
     if (first || metric == RCG_METRIC_SSIM) step_tables(ctx, d_ss, d_st, next);
     quantize(ctx, d_st, es.caches, es.max_blocks);
     rate_tables(ctx, d_st);
-    trellis(ctx, d_st, es.caches, es.max_blocks, d_weights != nullptr);
-    dequant_idct(ctx, d_st, nullptr, run.planes, es.max_blocks);
+    trellis_decode(ctx, d_st, es.caches, es.max_blocks, d_weights != nullptr, run.planes);
     score_candidate(ctx, sc, d_st, run.planes, w, h, channels, d_ss, s, next);
   };
   rc = run_step_loop(ctx, key, [&]() {
@@ -1765,8 +1764,7 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
     if (first || metric == RCG_METRIC_SSIM) step_tables(ctx, d_ss, d_st, next);
     requantize_plain(ctx, d_st, nblocks);
     rate_tables(ctx, d_st);
-    rcg::trellis(ctx, d_st, no_caches, nblocks);
-    dequant_idct(ctx, d_st, nullptr, planes, nblocks);
+    trellis_decode(ctx, d_st, no_caches, nblocks, false, planes);
     score_candidate(ctx, sc, d_st, planes, w, h, channels, d_ss, s, next);
   };
   rc = run_step_loop(ctx, key, [&]() {

@@ -762,6 +762,37 @@ int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t
   return RCG_OK;
 }
 
+// The trellis and the decoding of its result by the same thread, for candidates of few blocks (the decoder's launch costs
+// them more than the trellis's occupancy): the registers of the two phases do not add up, but the decoder's leave room for
+// four CTAs per SM instead of seven, so the line lies at one wave of those. Measured per search, apart / together: 17 CTAs
+// (240x180) 551 / 542 us, 408 (0.8 MP) 1082 / 1076, 474 (3.9 MP gray) 1280 / 1265; 1107 (6 MP, requantizing) 4877 / 5015.
+constexpr int kDecodeCtas = 4;
+constexpr long long kTrellisDecodeCtas = kDecodeCtas * 152;
+
+template <bool kWeighted>
+__global__ void __launch_bounds__(128, kDecodeCtas) k_trellis_decode(StepDesc* __restrict__ st, CacheSet cs,
+                                                                     uint8_t* __restrict__ planes) {
+  grid_chain();
+  trellis_body<kWeighted>(st, cs, blockIdx.x);
+  dequant_idct_body(st, nullptr, planes, blockIdx.x);  // a thread's own block: its coefficients are its own stores
+}
+
+int trellis_decode(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted,
+                   uint8_t* d_planes) {
+  const long long ctas = (max_blocks + 127) / 128;
+  if (ctas > kTrellisDecodeCtas) {
+    trellis(ctx, d_step, d_caches, max_blocks, weighted);
+    return dequant_idct(ctx, d_step, nullptr, d_planes, max_blocks);
+  }
+  CacheSet cs;
+  for (int i = 0; i < 9; i++) cs.p[i] = d_caches ? d_caches[i] : nullptr;
+  if (weighted)
+    RCG_LAUNCH(ctx, "trellis_decode", k_trellis_decode<true>, (unsigned)ctas, 128, 0, d_step, cs, d_planes);
+  else
+    RCG_LAUNCH(ctx, "trellis_decode", k_trellis_decode<false>, (unsigned)ctas, 128, 0, d_step, cs, d_planes);
+  return RCG_OK;
+}
+
 // ------------------------------------------------------------------------------------------------ K7 upsample+colour
 
 __constant__ float c_lut8[256];

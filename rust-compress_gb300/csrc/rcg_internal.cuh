@@ -414,6 +414,9 @@ int rate_tables(rcg_ctx* ctx, StepDesc* d_step, int count = 1);
 // weighted: the perceptual mode (d_step->pweights); otherwise the reference's plain trellis.
 int trellis(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted = false,
             int count = 1);
+// trellis, then dequant_idct of its result (in one launch where that is faster).
+int trellis_decode(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches, long long max_blocks, bool weighted,
+                   uint8_t* d_planes);
 // d_coefs null: decode the candidate's own coefficients (d_step->coefs). The planes of several are planes_stride apart.
 int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks,
                  int count = 1, long long planes_stride = 0);
