@@ -955,7 +955,7 @@ int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int 
 __global__ void __launch_bounds__(kStepThreads) k_step_tables(const SearchState* __restrict__ ss,
                                                               StepDesc* __restrict__ st, const NextStep next) {
   grid_chain();
-  step_tables_body(*ss, st, next);
+  step_tables_body(*ss, st, next, step_prepare(st, next));
 }
 
 int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, const NextStep& next) {
@@ -970,7 +970,8 @@ int step_tables(rcg_ctx* ctx, SearchState* d_search, StepDesc* d_step, const Nex
 __global__ void __launch_bounds__(kStepThreads) k_step_tables_lock(const LockItem* __restrict__ items) {
   grid_chain();
   const LockItem& it = items[blockIdx.x];
-  step_tables_body(*it.ss, it.st, NextStep{kNextEncode, it.w, it.h, it.slots, it.slot_stride, nullptr});
+  const NextStep next = {kNextEncode, it.w, it.h, it.slots, it.slot_stride, nullptr};
+  step_tables_body(*it.ss, it.st, next, step_prepare(it.st, next));
 }
 
 __device__ __forceinline__ CacheSet lock_caches(const LockItem& it) {

@@ -634,6 +634,8 @@ __device__ __forceinline__ void reduce_scale_sum(const PyramidDesc& pd, const do
     weight = c_weights[t];
     count = (double)pd.s[sc].w * (double)pd.s[sc].h;
   }
+  StepPre pre = {};
+  if (next.kind != kNextNone) pre = step_prepare(st, next);
   double acc = 0.0;
   const double* col = partials + (size_t)i * pd.total_tiles + sd.tile0;
   for (int u = t; u < n; u += 256) acc += col[u];
@@ -684,7 +686,7 @@ __device__ __forceinline__ void reduce_scale_sum(const PyramidDesc& pd, const do
   if (!ss) return;
   __syncthreads();
   if (t < kStateWords) reinterpret_cast<int*>(ss)[t] = state[t];
-  if (next.kind != kNextNone) step_tables_body(*copy, st, next);
+  if (next.kind != kNextNone) step_tables_body(*copy, st, next, pre);
 }
 
 __global__ void __launch_bounds__(256) k_ssim2_reduce(const __grid_constant__ PyramidDesc pd,

@@ -6,8 +6,8 @@
 
 namespace rcg {
 
-// The constant tables, for the host and in constant memory (an array local to a function that is indexed at run time is
-// written to the stack by every thread).
+// The constant tables, for the host and in device memory (an array local to a function that is indexed at run time is
+// written to the stack by every thread; in constant memory every lane's own index costs a turn).
 #define RCG_ZIGZAG                                                                                                \
   {0,  1,  8,  16, 9,  2,  3,  10, 17, 24, 32, 25, 18, 11, 4,  5,  12, 19, 26, 33, 40, 48, 41, 34, 27, 20, 13, 6, \
    7,  14, 21, 28, 35, 42, 49, 56, 57, 50, 43, 36, 29, 22, 15, 23, 30, 37, 44, 51, 58, 59, 52, 45, 38, 31, 39,    \
@@ -21,11 +21,11 @@ namespace rcg {
 static const uint8_t h_zigzag[64] = RCG_ZIGZAG;
 static const float h_aan[8] = RCG_AAN;
 static const uint8_t h_perceptual_q[64] = RCG_PERCEPTUAL_Q;
-static __constant__ uint8_t c_zigzag[64] = RCG_ZIGZAG;
-static __constant__ float c_aan[8] = RCG_AAN;
-static __constant__ uint8_t c_perceptual_q[64] = RCG_PERCEPTUAL_Q;
+static __device__ const uint8_t d_zigzag[64] = RCG_ZIGZAG;
+static __device__ const float d_aan[8] = RCG_AAN;
+static __device__ const uint8_t d_perceptual_q[64] = RCG_PERCEPTUAL_Q;
 #ifdef __CUDA_ARCH__
-#define RCG_TABLE(name) c_##name
+#define RCG_TABLE(name) d_##name
 #else
 #define RCG_TABLE(name) h_##name
 #endif
@@ -38,9 +38,6 @@ __host__ __device__ constexpr int zigzag_known(int k) {
 __host__ __device__ inline float aan(int i) { return RCG_TABLE(aan)[i]; }      // jpeg/src/dct.rs:8 (AAN scale factors)
 __host__ __device__ inline uint8_t perceptual_q(int i) { return RCG_TABLE(perceptual_q)[i]; }  // jpeg/src/quality.rs:26-35
 #undef RCG_TABLE
-#undef RCG_ZIGZAG
-#undef RCG_AAN
-#undef RCG_PERCEPTUAL_Q
 
 // Exact f32 arithmetic on host and device: round-to-nearest, never contracted.
 __host__ __device__ inline float fadd(float a, float b) {
@@ -97,24 +94,21 @@ __host__ __device__ inline int layout_kind(int hmax, int vmax) { return hmax == 
 
 // One entry of the per-quality tables, shared by the host (fill_step) and the device (step_tables_body) so both give
 // identical bits. `q` is the quantization table (natural order).
-//   quant value at natural index n (jpeg/src/quality.rs:6-15)
-__host__ __device__ inline uint8_t qtable_entry(int quality, int n) {
+//   quant value at a natural index whose perceptual entry is p (jpeg/src/quality.rs:6-15)
+__host__ __device__ inline uint8_t quality_entry(int quality, unsigned p) {
   unsigned q = (unsigned)(quality < 1 ? 1 : (quality > 100 ? 100 : quality));
   unsigned scale = q < 50 ? 5000 / q : 200 - 2 * q;
-  unsigned v = ((unsigned)perceptual_q(n) * scale + 50) / 100;
+  unsigned v = (p * scale + 50) / 100;
   return (uint8_t)(v < 1 ? 1 : (v > 255 ? 255 : v));
 }
+__host__ __device__ inline uint8_t qtable_entry(int quality, int n) { return quality_entry(quality, perceptual_q(n)); }
+//   dequantization multiplier at natural index n = v*8+u: q[v*8+u] * AAN[u] * AAN[v] (jpeg/src/decode.rs:1316-1321)
+__host__ __device__ inline float mult_of(uint8_t q, float aan_u, float aan_v) { return fmul(fmul((float)q, aan_u), aan_v); }
+__host__ __device__ inline float mult_entry(const uint8_t* q, int n) { return mult_of(q[n], aan(n % 8), aan(n / 8)); }
 //   fdct divisor for zigzag position k: fdct_divisors stores 1 / (q[v*8+u] * AAN[u] * AAN[v] * 8) at [u*8+v]
 //   (jpeg/src/encode.rs:174-183) and quantize_plane reads it at ZZ_T[k] = (n%8)*8 + n/8 (:202), i.e. u = n%8,
 //   v = n/8, q[v*8+u] = q[n]
-__host__ __device__ inline float divz_entry(const uint8_t* q, int k) {
-  int n = zigzag(k);
-  return fdiv(1.0f, fmul(fmul(fmul((float)q[n], aan(n % 8)), aan(n / 8)), 8.0f));
-}
-//   dequantization multiplier at natural index n = v*8+u: q[v*8+u] * AAN[u] * AAN[v] (jpeg/src/decode.rs:1316-1321)
-__host__ __device__ inline float mult_entry(const uint8_t* q, int n) {
-  return fmul(fmul((float)q[n], aan(n % 8)), aan(n / 8));
-}
+__host__ __device__ inline float divz_entry(const uint8_t* q, int k) { return fdiv(1.0f, fmul(mult_entry(q, zigzag(k)), 8.0f)); }
 
 // Block layout of a candidate (jpeg/src/encode.rs:428-443, :511-517).
 __host__ __device__ inline void fill_layout(StepDesc* st, int quality, int subsampling, int channels, int trellis,
@@ -154,16 +148,54 @@ __host__ __device__ inline uint8_t requant_entry(const uint8_t* old, int quality
 }
 
 // The candidate that the bisection state names: its quality, layout and tables, or active = 0 once the search has
-// finished (or paused). kStepThreads threads: one per (component, coefficient) entry; the Rdo median is the element of
-// rank 31 among q[1..63] (ties broken by index, which leaves the value unchanged), the same value the reference's sort
-// yields. One CTA: bound by its own latency (a launch of its own took 5 us a step, 10 requantizing), so a search fills
-// them at the end of the launch that scored the step before.
-constexpr int kStepThreads = 192;
+// finished (or paused). kStepThreads threads, one per (component, coefficient) entry and one for the layout; the Rdo
+// median is the value of rank 31 among q[1..63], the one the reference's sort yields. One CTA: bound by its own latency
+// (a launch of its own took 5 us a step, 10 requantizing), so a search fills them at the end of the launch that scored the
+// step before, and what does not depend on the quality is loaded before that end (step_prepare; 2.4 us of the 12.7 that
+// launch took at 240x180 were spent here without it, 1.5 with).
+constexpr int kStepThreads = 256;
 
-// Every thread of the CTA calls it (threads past kStepThreads help with nothing).
-__device__ __forceinline__ void step_tables_body(const SearchState& ss, StepDesc* __restrict__ st, const NextStep& next) {
-  __shared__ uint8_t qt[64];
-  __shared__ float rq[3][64];
+// What a thread's entries are made of, by k: one load of 32 bytes, none of them waiting for another.
+struct __align__(16) StepPre {
+  float au, av, nu, nv;          // AAN factors of the natural index k and of n
+  int n;                         // natural index of zigzag position k
+  uint8_t pk, pn;                // perceptual entries of both
+  uint8_t old_k, old_n;          // requantization: the source's entries
+  int ncomp;
+  int pad;
+};
+struct StepPreTable {
+  StepPre e[64];
+};
+constexpr StepPreTable step_pre_table() {
+  constexpr int Z[64] = RCG_ZIGZAG;
+  constexpr float A[8] = RCG_AAN;
+  constexpr uint8_t P[64] = RCG_PERCEPTUAL_Q;
+  StepPreTable t = {};
+  for (int k = 0; k < 64; k++)
+    t.e[k] = StepPre{A[k % 8], A[k / 8], A[Z[k] % 8], A[Z[k] / 8], Z[k], P[k], P[Z[k]], 0, 0, 3, 0};
+  return t;
+}
+static __device__ const StepPreTable d_step_pre = step_pre_table();
+#undef RCG_ZIGZAG
+#undef RCG_AAN
+#undef RCG_PERCEPTUAL_Q
+
+__device__ __forceinline__ StepPre step_prepare(const StepDesc* st, const NextStep& next) {
+  const int c = threadIdx.x / 64, k = threadIdx.x % 64;
+  StepPre p = d_step_pre.e[k];
+  if (next.kind == kNextRequant && c < 3) {
+    p.old_k = st->src_qt[c][k];
+    p.old_n = st->src_qt[c][p.n];
+    p.ncomp = st->ncomp;
+  }
+  return p;
+}
+
+// Every thread of the CTA (kStepThreads of them) calls it.
+__device__ __forceinline__ void step_tables_body(const SearchState& ss, StepDesc* __restrict__ st, const NextStep& next,
+                                                 const StepPre& p) {
+  __shared__ __align__(16) float rq[3][64];
   __shared__ float median[3];
   const int t = threadIdx.x;
   if (ss.done) {
@@ -174,7 +206,7 @@ __device__ __forceinline__ void step_tables_body(const SearchState& ss, StepDesc
   const int q = ss.qs[step];
   const bool requant = next.kind == kNextRequant;
   const int c = t / 64, k = t % 64;
-  if (t == 0) {
+  if (t == 192) {
     st->active = 1;
     st->requant = requant ? 1 : 0;
     st->coefs = next.slots + (long long)step * next.slot_stride;
@@ -185,40 +217,41 @@ __device__ __forceinline__ void step_tables_body(const SearchState& ss, StepDesc
       st->pweights = next.pweights;
     }
   }
-  for (int i = t; i < 512; i += blockDim.x) (&st->hist[0][0])[i] = 0;
+  for (int i = t; i < 512; i += kStepThreads) (&st->hist[0][0])[i] = 0;
   // luma_table == chroma_table (jpeg/src/quality.rs:37-43): every component gets the same entries. A requantization
   // keeps each component's own (never finer than the source's); its components' count is the source's.
-  const bool live = c < 3 && (!requant || c < st->ncomp);
+  const bool live = c < p.ncomp && c < 3;
   bool differs = false;
-  if (requant) {
-    if (live) {
-      const int n = zigzag(k);
-      const uint8_t old = st->src_qt[c][n], nn = requant_entry(st->src_qt[c], q, n);
-      differs = nn != old;
-      st->qt[c][n] = nn;
-      st->ratio[c][k] = fdiv((float)old, (float)nn);
-      st->mult[c][n] = fmul(fmul((float)nn, aan(n % 8)), aan(n / 8));
-      rq[c][k] = (float)nn;
-      st->rq[c][k] = (float)nn;
+  if (live) {
+    uint8_t qk = quality_entry(q, p.pk), qn = quality_entry(q, p.pn);
+    if (requant) {  // requant_entry
+      qk = max(qk, p.old_k);
+      qn = max(qn, p.old_n);
+      differs = qk != p.old_k;
+      st->ratio[c][k] = fdiv((float)p.old_n, (float)qn);
+    } else {
+      st->divz[c][k] = fdiv(1.0f, fmul(mult_of(qn, p.nu, p.nv), 8.0f));
     }
-  } else {
-    if (t < 64) qt[t] = qtable_entry(q, t);
-    __syncthreads();
-    if (live) {
-      st->qt[c][k] = qt[k];
-      st->divz[c][k] = divz_entry(qt, k);
-      st->mult[c][k] = mult_entry(qt, k);
-      rq[c][k] = (float)qt[zigzag(k)];
-      st->rq[c][k] = rq[c][k];
-    }
+    st->qt[c][k] = qk;
+    st->mult[c][k] = mult_of(qk, p.au, p.av);
+    rq[c][k] = (float)qn;
+    st->rq[c][k] = (float)qn;
   }
   const bool changed = __syncthreads_or(differs);
   if (live && k >= 1) {
     const float rk = rq[c][k];
-    int rank = 0;
-#pragma unroll 9
-    for (int j = 1; j < 64; j++) rank += (rq[c][j] < rk || (rq[c][j] == rk && j < k)) ? 1 : 0;
-    if (rank == 31) median[c] = rk;
+    int below = 0, upto = 0;
+#pragma unroll 4
+    for (int j = 0; j < 16; j++) {
+      const float4 v = *reinterpret_cast<const float4*>(&rq[c][4 * j]);
+      if (j > 0) {
+        below += v.x < rk;
+        upto += v.x <= rk;
+      }
+      below += (v.y < rk) + (v.z < rk) + (v.w < rk);
+      upto += (v.y <= rk) + (v.z <= rk) + (v.w <= rk);
+    }
+    if (below <= 31 && upto > 31) median[c] = rk;  // several threads of one value may write it
   }
   __syncthreads();
   if (live) {
