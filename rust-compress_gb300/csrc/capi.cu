@@ -198,16 +198,43 @@ void collect_times(rcg_ctx* ctx) {
 
 // ------------------------------------------------------------------------------------------------ host copies
 
-// Straight from and to the caller's memory, whatever its kind and thread: the GPU reads a Grace host's pageable pages at
-// the link's rate (18 MB: 121 us pageable, 101 pinned), where one core's copy into a pinned buffer takes 900.
+static bool is_pinned(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+static void* grow_pinned(void** buf, size_t* cap, size_t bytes) {
+  if (*buf && *cap >= bytes) return *buf;
+  if (*buf) cudaFreeHost(*buf);
+  *buf = nullptr;
+  *cap = 0;
+  if (cudaHostAlloc(buf, bytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    *buf = nullptr;
+    return nullptr;
+  }
+  *cap = bytes;
+  return *buf;
+}
+
+// Straight from the caller's memory, whatever its kind and thread: the GPU reads a Grace host's pageable pages at the
+// link's rate (18 MB: 121 us pageable, 101 pinned), where one core's copy into a pinned buffer takes 900.
 int copy_to_device(rcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
   cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
   return e == cudaSuccess ? RCG_OK : cuda_fail(ctx, e, "host to device copy");
 }
 
+// The other way too, but not from several threads at once into memory that was never touched, as results usually are:
+// the GPU's page faults then queue up (64 images of 166 MP: 566 ms, through a pinned buffer per worker 81).
 int copy_to_host(rcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+  void* st = ctx->stage_results && !is_pinned(dst) ? grow_pinned(&ctx->pinned_out, &ctx->pinned_out_bytes, bytes) : nullptr;
+  cudaError_t e = cudaMemcpyAsync(st ? st : dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess && st) std::memcpy(dst, st, bytes);
   return e == cudaSuccess ? RCG_OK : cuda_fail(ctx, e, "device to host copy");
 }
 
@@ -454,6 +481,7 @@ void rcg_ctx_destroy(rcg_ctx* ctx) {
   for (auto& kv : ctx->bufs)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
   if (ctx->lut16) cudaFree(ctx->lut16);
+  if (ctx->pinned_out) cudaFreeHost(ctx->pinned_out);
   for (auto& p : ctx->pending) {
     cudaEventDestroy(p.a);
     cudaEventDestroy(p.b);
@@ -1438,6 +1466,7 @@ int rcg_search_batch(rcg_ctx* ctx, int n, const uint8_t* const* srcs, const uint
     rcg_ctx* wk = nullptr;
     int crc = rcg_ctx_create(ctx->device, &wk);
     if (crc != RCG_OK) return fail(ctx, crc, "cannot create a batch worker context");
+    wk->stage_results = true;
     ctx->workers.push_back(wk);
   }
   // Largest images first, handed out one at a time: the workers finish at about the same time.
@@ -1500,6 +1529,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     rcg_ctx* sub = nullptr;
     int crc = rcg_ctx_create(ctx->device, &sub);
     if (crc != RCG_OK) return fail(ctx, crc, "cannot create a batch image context");
+    sub->stage_results = true;
     ctx->lock_subs.push_back(sub);
   }
   // Per image, on its own context's stream (the images' set-ups overlap one another): upload, colour planes, FDCTs,

@@ -237,6 +237,10 @@ struct rcg_ctx {
   float* lut16 = nullptr;  // 65536-entry sRGB->linear table for 16-bit samples (allocated on first use)
   std::vector<rcg_ctx*> workers;  // sub-contexts of rcg_search_batch (own streams and workspaces)
   std::vector<rcg_ctx*> lock_subs;  // per-image sub-contexts of rcg_search_batch_lockstep (buffers, set-up streams)
+  // Pinned buffer for results on their way to the caller's memory (grow-only), on batch contexts only (copy_to_host).
+  bool stage_results = false;
+  void* pinned_out = nullptr;
+  size_t pinned_out_bytes = 0;
   // Step loops of the device searches captured as CUDA graphs (capi.cu, run_step_loop). A loop's launches and their
   // arguments follow from the image shape, the options and the workspace pointers, so the key holds the first two
   // and ws_gen stands for the third: every workspace (re)allocation bumps it and makes older graphs stale.
