@@ -872,9 +872,9 @@ __device__ __forceinline__ constexpr int lev_off(int T, int L) {
 }
 constexpr int kLevFloats = 36 * 32 + 20 * 16 + 12 * 8 + 8 * 4 + 6 * 2;  // one channel's levels 1-5 (of the larger block)
 
-int pyramid_ctas(const PyramidDesc& pd) {
-  return ((pd.s[0].w + kPyrT - 1) / kPyrT) * ((pd.s[0].h + kPyrT - 1) / kPyrT);
-}
+static int blocks_of(const PyramidDesc& pd, int t) { return ((pd.s[0].w + t - 1) / t) * ((pd.s[0].h + t - 1) / t); }
+
+int pyramid_ctas(const PyramidDesc& pd) { return blocks_of(pd, kPyrT); }
 
 __device__ __forceinline__ void put4(float* __restrict__ p, size_t np, const float2 (&v)[2][3]) {
 #pragma unroll
@@ -1108,12 +1108,12 @@ __device__ __forceinline__ void build_planes(const PyramidDesc& pd, const BuildA
 }
 
 // Of either kind (the work-lists, whose images may be mixed).
-template <int kSrc, int kOut>
+template <int kSrc, int kOut, int T>
 __device__ __forceinline__ void build_block(const PyramidDesc& pd, const BuildArgs& g, const int blk) {
   __shared__ float lut[256];
   __shared__ __align__(16) float lev[kOut == kOutPair ? 2 : 1][3][kLevFloats];
-  if (pd.s[0].planes == 1) build_planes<kSrc, kOut, true, kPyrT>(pd, g, blk, lut, lev);
-  else build_planes<kSrc, kOut, false, kPyrT>(pd, g, blk, lut, lev);
+  if (pd.s[0].planes == 1) build_planes<kSrc, kOut, true, T>(pd, g, blk, lut, lev);
+  else build_planes<kSrc, kOut, false, T>(pd, g, blk, lut, lev);
 }
 
 // CTAs per SM: a pair's conversion keeps two images' samples in registers.
@@ -1143,7 +1143,7 @@ void launch_build(const PyramidDesc& pd, const BuildArgs& g, const StepDesc* st,
   constexpr bool kGray = kSrc != kFromLinear;
   const int ctas = pyramid_ctas(pd);
   if (ctas <= kSmallBuild) {
-    const int n = ((pd.s[0].w + kPyrTSmall - 1) / kPyrTSmall) * ((pd.s[0].h + kPyrTSmall - 1) / kPyrTSmall);
+    const int n = blocks_of(pd, kPyrTSmall);
     if (kGray && pd.s[0].planes == 1)
       launch_chained(n, kPyrThreads, 0, stream, k_build<kSrc, kOut, kGray, kPyrTSmall>, pd, g, st);
     else
@@ -1197,13 +1197,13 @@ __device__ __forceinline__ int find_first(const long long* __restrict__ first, i
   return lo;
 }
 
-template <int kSrc, int kOut>
+template <int kSrc, int kOut, int T>
 __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build_batch(const BuildJob* __restrict__ jobs,
                                                                               const long long* __restrict__ cta0, int n) {
   grid_chain();
   const int i = find_first(cta0, n, blockIdx.x);
   const BuildJob& j = jobs[i];
-  build_block<kSrc, kOut>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
+  build_block<kSrc, kOut, T>(j.pd, j.args, (int)((long long)blockIdx.x - __ldg(cta0 + i)));
 }
 
 // One CTA per tile of the work-list. A persistent form (a fixed grid of k CTAs per SM striding over the list, each
@@ -1260,7 +1260,7 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOutDiff)) k_build_loc
   g.ref = it.ref_pyr;
   g.planes = it.planes;
   g.st = it.st;
-  build_block<kFromPlanes, kOutDiff>(it.pd, g, (int)((long long)blockIdx.x - it.p0));
+  build_block<kFromPlanes, kOutDiff, kPyrT>(it.pd, g, (int)((long long)blockIdx.x - it.p0));
 }
 
 template <int kRef>
@@ -1703,6 +1703,17 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
     g.out = base + off_diff[(size_t)i];
     add(1, i, g);
   }
+  // A list of few blocks is built by 32x32 ones, as one small image is (kSmallBuild).
+  bool small[kLists];
+  for (int k = 0; k < kLists; k++) {
+    small[k] = ctas[k] <= kSmallBuild;
+    if (!small[k]) continue;
+    ctas[k] = 0;
+    for (size_t j = 0; j < jobs[k].size(); j++) {
+      first[k][j] = ctas[k];
+      ctas[k] += blocks_of(jobs[k][j].pd, kPyrTSmall);
+    }
+  }
   // The work-list in one upload: pairs, then the tile segments (one per pair and scale) and their first tiles, then the
   // builder lists and their first CTAs.
   int nseg = 0;
@@ -1763,20 +1774,20 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   // The launches take only the work-list's totals and this context's buffers: a later batch with the same totals
   // replays them (its own pairs come in through the work-list uploaded above).
   const std::vector<long long> key = {3,     n,     nseg,    tiles,   max_scales, nj[0],
-                                      nj[1], nj[2], ctas[0], ctas[1], ctas[2], decoded != nullptr};
+                                      nj[1], nj[2], ctas[0], ctas[1], ctas[2], decoded != nullptr,
+                                      small[0], small[1], small[2]};
   int rc = run_step_loop(ctx, key, [&]() {
-    if (nj[0])
-      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutRef>), (unsigned)ctas[0], kPyrThreads, 0, d_jobs(0), d_first(0),
-                 nj[0]);
-    if (nj[1] && decoded)
-      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromPlanes, kOutDiff>), (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1),
-                 d_first(1), nj[1]);
-    else if (nj[1])
-      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutDiff>), (unsigned)ctas[1], kPyrThreads, 0, d_jobs(1),
-                 d_first(1), nj[1]);
-    if (nj[2])
-      RCG_LAUNCH(ctx, "build_batch", (k_build_batch<kFromImage, kOutPair>), (unsigned)ctas[2], kPyrThreads, 0, d_jobs(2), d_first(2),
-                 nj[2]);
+    auto build = [&](int k, auto big, auto little) {
+      if (nj[k])
+        RCG_LAUNCH(ctx, "build_batch", (small[k] ? little : big), (unsigned)ctas[k], kPyrThreads, 0, d_jobs(k), d_first(k),
+                   nj[k]);
+    };
+    build(0, &k_build_batch<kFromImage, kOutRef, kPyrT>, &k_build_batch<kFromImage, kOutRef, kPyrTSmall>);
+    if (decoded)
+      build(1, &k_build_batch<kFromPlanes, kOutDiff, kPyrT>, &k_build_batch<kFromPlanes, kOutDiff, kPyrTSmall>);
+    else
+      build(1, &k_build_batch<kFromImage, kOutDiff, kPyrT>, &k_build_batch<kFromImage, kOutDiff, kPyrTSmall>);
+    build(2, &k_build_batch<kFromImage, kOutPair, kPyrT>, &k_build_batch<kFromImage, kOutPair, kPyrTSmall>);
     RCG_LAUNCH(ctx, "ssim2_tiles_batch", k_ssim2_tiles_batch, tile_grid(tiles), kTileThreads, tile_smem(kRefNone), d_segs,
                d_seg0, nseg);
     RCG_LAUNCH(ctx, "ssim2_reduce_batch", k_ssim2_reduce_batch, dim3(max_scales, kScoreSums, n), 256, 0, d_items,
