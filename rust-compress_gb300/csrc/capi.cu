@@ -1271,7 +1271,7 @@ struct SearchRun {
 };
 
 // Everything before the step loop, queued on the context's stream: the buffers, the quality-independent work (the
-// reference image's linear pyramid for SSIMULACRA2, colour planes, FDCTs) and the initial bisection state.
+// reference image's pyramids for SSIMULACRA2, the FDCTs) and the initial bisection state.
 static int search_prepare(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int metric, double target,
                           int max_q, int subsampling, int trellis_on, SearchRun* run) {
   int rc;

@@ -239,7 +239,7 @@ __device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) 
 // pass.
 // What bounds it: instruction issue (79% active, the FP32 pipes 62%). Measured per 12 MP score, against a kernel that
 // read both linear pyramids and converted every halo sample to XYB itself (1.5 conversions per pixel and half of its
-// instructions): reading form 538 -> 276 us, storing 597 -> 354; plain 4K score 397 -> 238. Of that, the planes of XYB
+// instructions): reading form 538 -> 277 us, storing 597 -> 361; plain 4K score 397 -> 239. Of that, the planes of XYB
 // alone gave 420; loads by quads with the next channel's in registers beside the passes, and the maps without their edge
 // cases inside the image, 349; eight outputs per thread in both passes with the halo copied asynchronously into one
 // buffer 276 (387 with two buffers of converted pairs, which left room for 16 warps per SM). CTAs per SM: 6 reading (5
