@@ -1076,9 +1076,58 @@ void host_requant_tables(StepDesc* st, int quality, int trellis, int tq_out[3], 
   std::memset(st->hist, 0, sizeof st->hist);
 }
 
+// The AC symbols of one block, eight coefficients at a time: `sizes` their 4-bit sizes, the nonzero ones found by their
+// bits (a loop over the block's nonzero coefficients instead of a branch per coefficient). Quantization keeps the branches:
+// its values arrive a coefficient at a time from 64 rows, and this form measured 14.2 against 12.2 us at 0.8 MP, 31.8
+// against 29.7 at 12 MP.
+__device__ __forceinline__ void hist_group(uint32_t sizes, int g, int& last, unsigned* hs) {
+  while (sizes) {
+    const int j = (__ffs(sizes) - 1) >> 2, k = g * 8 + j;
+    const unsigned size = (sizes >> (4 * j)) & 15u;
+    sizes &= ~(15u << (4 * j));
+    unsigned run = (unsigned)(k - last - 1);
+    last = k;
+    while (run >= 16) {
+      atomicAdd(&hs[0xF0], 1u);
+      run -= 16;
+    }
+    atomicAdd(&hs[(run << 4) | size], 1u);
+  }
+}
+
+// Adds the CTA's symbols to the candidate's. cls: the class of this thread's block if its last coefficients are zero (an
+// end-of-block symbol), else -1. Every thread of the CTA calls it.
+__device__ __forceinline__ void hist_finish(StepDesc* st, unsigned (&sh)[2][256], int cls) {
+  const unsigned n0 = __popc(__ballot_sync(0xffffffffu, cls == 0)), n1 = __popc(__ballot_sync(0xffffffffu, cls == 1));
+  if ((threadIdx.x & 31) == 0) {
+    if (n0) atomicAdd(&sh[0][0], n0);
+    if (n1) atomicAdd(&sh[1][0], n1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    const unsigned v = (&sh[0][0])[i];
+    if (v) atomicAdd(&(&st->hist[0][0])[i], v);
+  }
+}
+
+__device__ __forceinline__ int4 pack8(const int (&v)[8]) {
+  return make_int4((v[0] & 0xFFFF) | (v[1] << 16), (v[2] & 0xFFFF) | (v[3] << 16), (v[4] & 0xFFFF) | (v[5] << 16),
+                   (v[6] & 0xFFFF) | (v[7] << 16));
+}
+
+// 4-bit sizes of eight coefficients (at most 2047 in magnitude: sizes to 11).
+__device__ __forceinline__ uint32_t sizes8(const int (&v)[8]) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) w |= (uint32_t)bitlen((unsigned)abs(v[j])) << (4 * j);
+  return w;
+}
+
 // Plain requantization (jpeg/src/encode.rs:132-138): round_f32(coef * old/new) clamped to +-2047, every position.
 // When the trellis pass follows, also the AC symbol histogram of the result over the blocks of the MCU grid
 // (ac_code_lengths, :155 -> :223-227, :376-398).
+// What bounds it: the latency of its row loads between the histogram's serial steps; 28.6 -> 22.9 us per 6 MP candidate
+// with hist_group and the end-of-block symbols counted per warp.
 __global__ void __launch_bounds__(128) k_requant_plain(StepDesc* __restrict__ st) {
   grid_chain();
   __shared__ unsigned int sh[2][256];
@@ -1089,62 +1138,38 @@ __global__ void __launch_bounds__(128) k_requant_plain(StepDesc* __restrict__ st
     __syncthreads();
   }
   const long long gb = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int eob = -1;
   if (gb < st->nblocks) {
     const int c = comp_of(st, gb);
     const CompDesc& cd = st->comp[c];
     const float* ratio = st->ratio[c];
     const int4* src = reinterpret_cast<const int4*>(st->coef_src + gb * 64);
-    int v[64];
+    int4* out = reinterpret_cast<int4*>(st->coefs + gb * 64);
+    uint32_t sizes[8];
 #pragma unroll
     for (int g = 0; g < 8; g++) {
-      int4 pk = __ldg(src + g);
-      int w4[4] = {pk.x, pk.y, pk.z, pk.w};
+      const int4 pk = __ldg(src + g);
+      const int w4[4] = {pk.x, pk.y, pk.z, pk.w};
+      int v[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        int k = g * 8 + j;
-        int x = (int)(short)((w4[j >> 1] >> (16 * (j & 1))) & 0xFFFF);
-        v[k] = clampi(round_f32(fmul((float)x, ratio[k])), -2047, 2047);
+        const int x = (int)(short)((w4[j >> 1] >> (16 * (j & 1))) & 0xFFFF);
+        v[j] = clampi(round_f32(fmul((float)x, ratio[g * 8 + j])), -2047, 2047);
       }
-    }
-    int16_t* out = st->coefs + gb * 64;
-#pragma unroll
-    for (int g = 0; g < 8; g++) {
-      int4 pk;
-      pk.x = (v[g * 8 + 0] & 0xFFFF) | (v[g * 8 + 1] << 16);
-      pk.y = (v[g * 8 + 2] & 0xFFFF) | (v[g * 8 + 3] << 16);
-      pk.z = (v[g * 8 + 4] & 0xFFFF) | (v[g * 8 + 5] << 16);
-      pk.w = (v[g * 8 + 6] & 0xFFFF) | (v[g * 8 + 7] << 16);
-      reinterpret_cast<int4*>(out)[g] = pk;
+      out[g] = pack8(v);
+      sizes[g] = sizes8(v);
     }
     const long long lb = gb - cd.blk0;
     const int by = (int)(lb / cd.bw), bx = (int)(lb % cd.bw);
     if (hist && bx < st->mcus_x * cd.h && by < st->mcus_y * cd.v) {
-      unsigned* hs = sh[cd.cls];
-      unsigned run = 0;
+      sizes[0] &= ~15u;  // the DC
+      int last = 0;
 #pragma unroll
-      for (int k = 1; k < 64; k++) {
-        if (v[k] == 0) {
-          run++;
-          continue;
-        }
-        while (run >= 16) {
-          atomicAdd(&hs[0xF0], 1u);
-          run -= 16;
-        }
-        unsigned size = (unsigned)bitlen((unsigned)abs(v[k]));
-        atomicAdd(&hs[(run << 4) | size], 1u);
-        run = 0;
-      }
-      if (run > 0) atomicAdd(&hs[0], 1u);
+      for (int g = 0; g < 8; g++) hist_group(sizes[g], g, last, sh[cd.cls]);
+      if (last < 63) eob = cd.cls;
     }
   }
-  if (hist) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-      unsigned x = (&sh[0][0])[i];
-      if (x) atomicAdd(&(&st->hist[0][0])[i], x);
-    }
-  }
+  if (hist) hist_finish(st, sh, eob);
 }
 
 int requantize_plain(rcg_ctx* ctx, StepDesc* d_step, long long max_blocks) {
