@@ -61,19 +61,20 @@ __device__ __forceinline__ void planes_quad(const StepDesc* __restrict__ st, con
     for (int k = 0; k < 4; k++) l[0][k] = l[1][k] = l[2][k] = lut[(q >> (8 * k)) & 0xFF];
     return;
   }
+  // Each chroma component has a stride of its own: a caller's block grids need only cover the MCU grid.
   int up[2][4];
-  const int cstride = st->comp[1].bw * 8;
   if (st->hmax == 1) {
 #pragma unroll
     for (int c = 0; c < 2; c++) {
-      const uint32_t v =
-          *reinterpret_cast<const uint32_t*>(planes + st->comp[1 + c].plane_off + (size_t)y * cstride + x0);
+      const CompDesc& cd = st->comp[1 + c];
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(planes + cd.plane_off + (size_t)y * (cd.bw * 8) + x0);
 #pragma unroll
       for (int k = 0; k < 4; k++) up[c][k] = (v >> (8 * k)) & 0xFF;
     }
   } else if (st->vmax == 1) {
 #pragma unroll
     for (int c = 0; c < 2; c++) {
+      const int cstride = st->comp[1 + c].bw * 8;
       const uint32_t v = chroma4(planes + st->comp[1 + c].plane_off + (size_t)y * cstride, x0 / 2, (w + 1) / 2, cstride);
       const int b0 = v & 0xFF, b1 = (v >> 8) & 0xFF, b2 = (v >> 16) & 0xFF, b3 = v >> 24;
       up[c][0] = (3 * b1 + b0 + 1) >> 2;
@@ -86,6 +87,7 @@ __device__ __forceinline__ void planes_quad(const StepDesc* __restrict__ st, con
     const int far = (y & 1) ? min(j + 1, ch - 1) : max(j - 1, 0);
 #pragma unroll
     for (int c = 0; c < 2; c++) {
+      const int cstride = st->comp[1 + c].bw * 8;
       const uint8_t* p = planes + st->comp[1 + c].plane_off;
       chroma_up(chroma4(p + (size_t)j * cstride, x0 / 2, cw, cstride),
                 chroma4(p + (size_t)far * cstride, x0 / 2, cw, cstride), up[c]);
