@@ -382,14 +382,14 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
   __syncthreads();
   const float lambda = st->lambda[comp];
   // rate(run, v) = zrl * len[0xF0] + len[((run % 16) << 4) | size] + size, for size = bit length of v.
-  for (int i = t; i < 64 * 16; i += blockDim.x) {
-    int run = i / 16, size = i % 16;
+  for (int i = t; i < 64 * kRateSizes; i += blockDim.x) {
+    int run = i / kRateSizes, size = i % kRateSizes;
     float rate = fadd(fadd(fmul((float)(run / 16), len[0xF0]), len[((run % 16) << 4) | size]), (float)size);
     st->lr[comp][i] = fmul(lambda, rate);
   }
   // Per size, the least entry over all runs (the trellis's scan bound): 16 lanes of 4 runs each per size. The products
   // are those of the table and rounding is monotone, so the minimum is one of its entries.
-  if (t < 256) {
+  {
     const int size = t >> 4;
     float least = 3.0e38f;
     for (int run = t & 15; run < 64; run += 16) {
@@ -398,7 +398,7 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
     }
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, off));
-    if ((t & 15) == 0) st->lrmin[comp][size] = least;
+    if ((t & 15) == 0 && size < kRateSizes) st->lrmin[comp][size] = least;
   }
   if (t == 0) st->eob[comp] = fmul(lambda, len[0]);
 }
@@ -451,13 +451,13 @@ template <bool kWeighted>
 __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const CacheSet& cs, long long bx) {
   // The per-position tables of every component and the lambda*rate tables of the components this CTA's blocks
   // belong to (usually one), staged in shared memory: the DP reads them at every position.
-  __shared__ float lr[3][64 * 16];
+  __shared__ float lr[3][64 * kRateSizes];
   __shared__ float4 s_tab[3][64];  // per position: (scale, step, weight, -)
   if (!st->active || !st->use_trellis) return;
   const bool requant = st->requant != 0;
   const long long blk0 = bx * blockDim.x;
   const int c_lo = comp_of(st, blk0), c_hi = comp_of(st, min(blk0 + (long long)blockDim.x, st->nblocks) - 1);
-  for (int i = threadIdx.x; i < (c_hi - c_lo + 1) * 64 * 16; i += blockDim.x)
+  for (int i = threadIdx.x; i < (c_hi - c_lo + 1) * 64 * kRateSizes; i += blockDim.x)
     (&lr[c_lo][0])[i] = (&st->lr[c_lo][0])[i];
   for (int i = threadIdx.x; i < 3 * 64; i += blockDim.x) {
     const int c = i / 64, k = i % 64;
@@ -483,12 +483,12 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
   float4 nodes[126];
   // The newest kWin nodes, newest first (cost infinity: none yet), and the bound for the nodes older than they.
   float wcost[kWin], wzd[kWin];
-  int wrow[kWin];  // (position + 1) * 16: the rate row of position i is i * 16 - wrow
+  int wrow[kWin];  // (position + 1) * kRateSizes: the rate row of position i is i * kRateSizes - wrow
 #pragma unroll
   for (int n = 0; n < kWin; n++) {
     wcost[n] = __int_as_float(0x7f800000);
     wzd[n] = 0.0f;
-    wrow[n] = 16;
+    wrow[n] = kRateSizes;
   }
   float pm_all = __int_as_float(0x7f800000), pm_old = pm_all;
   bool prune = true;
@@ -553,12 +553,12 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
         float e_hi = fmul(fsub(m, (float)v0), q);
         float dnz_hi = fmul(fmul(e_hi, e_hi), w);
         int s_lo = bitlen(lo), s_hi = bitlen(v0);
-        float best_lo = fadd(fadd(zprev, lrc[(i - 1) * 16 + s_lo]), dnz_lo);
-        float best_hi = fadd(fadd(zprev, lrc[(i - 1) * 16 + s_hi]), dnz_hi);
+        float best_lo = fadd(fadd(zprev, lrc[(i - 1) * kRateSizes + s_lo]), dnz_lo);
+        float best_hi = fadd(fadd(zprev, lrc[(i - 1) * kRateSizes + s_hi]), dnz_hi);
         int prev_lo = -1, prev_hi = -1;
         auto offer = [&](float cost, float zd, int row, int ni) {
           const float base = fadd(cost, fsub(zprev, zd));
-          const float* lrow = lrc + (i * 16 - row);
+          const float* lrow = lrc + (i * kRateSizes - row);
           const float c_lo = fadd(fadd(base, lrow[s_lo]), dnz_lo);
           const float c_hi = fadd(fadd(base, lrow[s_hi]), dnz_hi);
           if (c_lo < best_lo || (c_lo == best_lo && prev_lo >= 0)) {
@@ -582,7 +582,7 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
           for (int ni = nn - 1 - kWin; ni >= 0; ni--) {
             const float4 nd = nodes[ni];
             if (settled(nd.z)) break;
-            offer(nd.x, nd.y, ((__float_as_int(nd.w) & 63) + 1) * 16, ni);
+            offer(nd.x, nd.y, ((__float_as_int(nd.w) & 63) + 1) * kRateSizes, ni);
           }
         }
         best[0] = best_lo;
@@ -610,7 +610,7 @@ __device__ __forceinline__ void trellis_body(StepDesc* __restrict__ st, const Ca
           }
           wcost[0] = best[n];
           wzd[0] = zcur;
-          wrow[0] = (i + 1) * 16;
+          wrow[0] = (i + 1) * kRateSizes;
         }
       }
       zprev = zcur;

@@ -62,6 +62,10 @@ struct CompDesc {
   long long plane_off;   // byte offset of the decoded component plane (stride bw*8) in the plane buffer
 };
 
+// Sizes of a value in the rate model: an encoder's values have at most 11 bits, those of a requantized source up to 16
+// (-32768, where its table entry is not raised).
+constexpr int kRateSizes = 17;
+
 // Everything the per-candidate kernels need; lives in device memory. Written by the host for single calls and by
 // the device-side search for each bisection step.
 struct StepDesc {
@@ -82,8 +86,8 @@ struct StepDesc {
   float rw[3][64];       // distortion weight per zigzag position
   float lambda[3];
   float eob[3];          // lambda * len[0x00]
-  float lr[3][64 * 16];  // lambda * rate(run, v) for run 0..63, size 0..15 (index run*16 + size)
-  float lrmin[3][16];    // least lr over the runs, per size
+  float lr[3][64 * kRateSizes];  // lambda * rate(run, v) for run 0..63, by the size of v (index run*kRateSizes + size)
+  float lrmin[3][kRateSizes];    // least lr over the runs, per size
   unsigned int hist[2][256];  // AC symbol histogram of the plain pass, per class (jpeg/src/encode.rs:223-227)
   // Requantization of existing coefficients (jpeg/src/encode.rs:107-172)
   int requant;           // 1: the candidate requantizes coef_src instead of quantizing the FDCT cache
