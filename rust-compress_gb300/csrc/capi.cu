@@ -1636,16 +1636,18 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
   // then the remaining steps run for all images (the finished ones skip).
   for (;;) {
     int from = max_steps;
+    bool paused = false;
     for (int i = 0; i < n; i++) {
       if (hs[(size_t)i].done != 2) continue;
+      paused = true;
       const SearchRun& r = runs[(size_t)i];
       if ((rc = exact_candidate(ctx, r.sc, r.d_st, r.planes, r.w, r.h, d_exact)) != RCG_OK) return rc;
       search_resume(ctx, r.d_ss, d_exact);
       ctx->tie_rescores++;
       from = std::min(from, hs[(size_t)i].step + 1);
     }
-    if (from == max_steps) break;
-    for (int s = from; s < max_steps; s++) issue_step(s, s == from);
+    if (!paused) break;
+    for (int s = from; s < max_steps; s++) issue_step(s, s == from);  // none after a tie at the last step
     if ((rc = read_states()) != RCG_OK) return rc;
   }
   // Results, each through its image's context (the step loop is complete: the states were read after it), in
