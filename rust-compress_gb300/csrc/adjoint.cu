@@ -626,17 +626,17 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
     k[i] /= sum;
     k32[i] = (float)k[i];
   }
-  // pageable sources: each upload has read its source when the call returns
-  cudaMemcpyToSymbolAsync(c_k64, k, sizeof k, 0, cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyToSymbolAsync(c_k32, k32, sizeof k32, 0, cudaMemcpyHostToDevice, ctx->stream);
-  double lin8[256], dlin8[256];
+  double lin8[256], dlin8[256], hs[kMaxScales * 18];
+  CopiesDone done(ctx);
+  symbol_to_device(ctx, c_k64, k, sizeof k);
+  symbol_to_device(ctx, c_k32, k32, sizeof k32);
   for (int i = 0; i < 256; i++) {
     const double v = (double)i / 255.0;
     lin8[i] = v <= 0.04045 ? v / 12.92 : std::pow((v + 0.055) / 1.055, 2.4);
     dlin8[i] = v <= 0.04045 ? 1.0 / (12.92 * 255.0) : 2.4 * std::pow((v + 0.055) / 1.055, 1.4) / (1.055 * 255.0);
   }
-  cudaMemcpyToSymbolAsync(c_lin8, lin8, sizeof lin8, 0, cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyToSymbolAsync(c_dlin8, dlin8, sizeof dlin8, 0, cudaMemcpyHostToDevice, ctx->stream);
+  symbol_to_device(ctx, c_lin8, lin8, sizeof lin8);
+  symbol_to_device(ctx, c_dlin8, dlin8, sizeof dlin8);
   // pyramid of both images (linear)
   struct Sc {
     int w, h;
@@ -731,9 +731,9 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
     RCG_LAUNCH(ctx, "adj_maps", k_maps<T>, grid(jobs), 256, 0, jobs, mom, xa, xb, parts);
     RCG_LAUNCH(ctx, "adj_sum_parts", k_sum_parts, (unsigned)g.size(), 192, 0, jobs, to, parts, sums);
   }
-  double hs[kMaxScales * 18];
-  cudaMemcpyAsync(hs, sums, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  int rc = read_back(ctx, hs, sums, sizeof hs);
+  if (rc != RCG_OK) return rc;
+  cudaError_t e = wait_stream(ctx);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "ssimulacra2 gradient");
   // final mapping (:491-511) and d score / d stat
   double st[kMaxScales][3][6], wst[kMaxScales][3][6];

@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -43,7 +44,10 @@ void* workspace(rcg_ctx* ctx, const char* name, size_t bytes, bool in_graphs) {
     b.bytes = 0;
   }
   size_t sz = std::max<size_t>(bytes, 256);
-  if (cudaMalloc(&b.ptr, sz) != cudaSuccess) {
+  size_t held = 0;
+  if (ctx->workspace_limit)
+    for (const auto& kv : ctx->bufs) held += kv.second.bytes;
+  if ((ctx->workspace_limit && held + sz > ctx->workspace_limit) || cudaMalloc(&b.ptr, sz) != cudaSuccess) {
     cudaGetLastError();
     b.ptr = nullptr;
     fail(ctx, RCG_NO_MEMORY, std::string("device allocation of ") + std::to_string(sz) + " bytes for " + name);
@@ -224,16 +228,29 @@ static void* grow_pinned(void** buf, size_t* cap, size_t bytes) {
 // Straight from the caller's memory, whatever its kind and thread: the GPU reads a Grace host's pageable pages at the
 // link's rate (18 MB: 121 us pageable, 101 pinned), where one core's copy into a pinned buffer takes 900.
 int copy_to_device(rcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  ctx->host_traffic = true;
   cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
   return e == cudaSuccess ? RCG_OK : cuda_fail(ctx, e, "host to device copy");
+}
+
+int read_back(rcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  ctx->host_traffic = true;
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+  return e == cudaSuccess ? RCG_OK : cuda_fail(ctx, e, "device to host copy");
+}
+
+cudaError_t wait_stream(rcg_ctx* ctx) {
+  ctx->host_traffic = false;
+  return cudaStreamSynchronize(ctx->stream);
 }
 
 // The other way too, but not from several threads at once into memory that was never touched, as results usually are:
 // the GPU's page faults then queue up (64 images of 166 MP: 566 ms, through a pinned buffer per worker 81).
 int copy_to_host(rcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
   void* st = ctx->stage_results && !is_pinned(dst) ? grow_pinned(&ctx->pinned_out, &ctx->pinned_out_bytes, bytes) : nullptr;
-  cudaError_t e = cudaMemcpyAsync(st ? st : dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  const int rc = read_back(ctx, st ? st : dst, src, bytes);
+  if (rc != RCG_OK) return rc;
+  const cudaError_t e = wait_stream(ctx);
   if (e == cudaSuccess && st) std::memcpy(dst, st, bytes);
   return e == cudaSuccess ? RCG_OK : cuda_fail(ctx, e, "device to host copy");
 }
@@ -275,8 +292,8 @@ static int ensure_init(rcg_ctx* ctx) {
 
 static int finish(rcg_ctx* ctx, const char* what) {
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-  e = cudaStreamSynchronize(ctx->stream);
+  const cudaError_t waited = wait_stream(ctx);  // after a failed launch too: copies may be queued
+  if (e == cudaSuccess) e = waited;
   if (e != cudaSuccess) return cuda_fail(ctx, e, what);
   if (ctx->profiling) collect_times(ctx);
   ctx->last_error.clear();
@@ -438,6 +455,11 @@ static void qtables_out(const int tq[3], const uint8_t slot_qt[4][64], const int
 using namespace rcg;
 
 extern "C" {
+
+// Not part of the library's interface: bounds a context's workspace for tests (rcg_ctx::workspace_limit).
+void rcg_internal_limit_workspace(rcg_ctx* ctx, uint64_t bytes) {
+  if (ctx) ctx->workspace_limit = (size_t)bytes;
+}
 
 int rcg_ctx_create(int device, rcg_ctx** out) {
   if (!out) return RCG_INVALID;
@@ -616,7 +638,8 @@ static int score_device_images(rcg_ctx* ctx, const uint8_t* d_ref, const uint8_t
   if ((rc = build_pair(ctx, pd, d_ref, d_dist, channels, depth, ref_pyr, dist_pyr)) != RCG_OK) return rc;
   score_pyramids(ctx, pd, ref_pyr, dist_pyr, d_score, nullptr, nullptr);
   double s = 0.0;
-  cudaMemcpyAsync(&s, d_score, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+  CopiesDone done(ctx);
+  if ((rc = read_back(ctx, &s, d_score, sizeof(double))) != RCG_OK) return rc;
   if ((rc = finish(ctx, "ssimulacra2")) != RCG_OK) return rc;
   if (!std::isfinite(s)) return fail(ctx, RCG_INVALID, "SSIMULACRA 2 produced a non-finite score");
   *score = s;
@@ -636,6 +659,7 @@ int rcg_ssimulacra2(rcg_ctx* ctx, const uint8_t* reference, const uint8_t* disto
   uint8_t* d_a = (uint8_t*)workspace(ctx, "img_a", bytes);
   uint8_t* d_b = (uint8_t*)workspace(ctx, "img_b", bytes);
   if (!d_a || !d_b) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   int rc;
   if ((rc = copy_to_device(ctx, d_a, reference, bytes)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_b, distorted, bytes)) != RCG_OK) return rc;
@@ -658,14 +682,15 @@ int rcg_ssimulacra2_exact(rcg_ctx* ctx, const uint8_t* reference, const uint8_t*
   float* lin = (float*)workspace(ctx, "x_lin", 2 * np * sizeof(float), false);
   double* d_score = (double*)workspace(ctx, "x_score", sizeof(double), false);
   if (!d_a || !d_b || !lin || !d_score) return RCG_NO_MEMORY;
+  double s = 0.0;
+  CopiesDone done(ctx);
   int rc;
   if ((rc = copy_to_device(ctx, d_a, reference, bytes)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_b, distorted, bytes)) != RCG_OK) return rc;
   if ((rc = to_linear(ctx, d_a, w, h, w, channels, depth, lin)) != RCG_OK) return rc;
   if ((rc = to_linear(ctx, d_b, w, h, w, channels, depth, lin + np)) != RCG_OK) return rc;
   if ((rc = exact_score(ctx, lin, lin + np, w, h, d_score)) != RCG_OK) return rc;
-  double s = 0.0;
-  cudaMemcpyAsync(&s, d_score, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+  if ((rc = read_back(ctx, &s, d_score, sizeof(double))) != RCG_OK) return rc;
   if ((rc = finish(ctx, "ssimulacra2_exact")) != RCG_OK) return rc;
   if (!std::isfinite(s)) return fail(ctx, RCG_INVALID, "SSIMULACRA 2 produced a non-finite score");
   *score = s;
@@ -718,6 +743,7 @@ int rcg_ssimulacra2_batch_device(rcg_ctx* ctx, int n, const uint8_t* const* d_re
   for (int i = 0; i < n; i++)
     if (!d_references[i] || !d_distorted[i]) return fail(ctx, RCG_INVALID, "null pointer");
   cudaSetDevice(ctx->device);
+  CopiesDone done(ctx);
   double* d_scores = nullptr;
   if ((rc = score_batch(ctx, n, d_references, d_distorted, widths, heights, channels, depths, &d_scores)) != RCG_OK)
     return rc;
@@ -755,6 +781,7 @@ int rcg_ssimulacra2_batch(rcg_ctx* ctx, int n, const uint8_t* const* references,
   }
   uint8_t* d_imgs = (uint8_t*)workspace(ctx, "batch_imgs", total);
   if (!d_imgs) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   std::vector<const uint8_t*> d_ref((size_t)n), d_dist((size_t)n);
   std::vector<char> sent(total / 256 + 1, 0);
   for (int i = 0; i < n; i++) {
@@ -829,12 +856,11 @@ static int sweep_group(rcg_ctx* ctx, int n, const uint8_t* const* images, const 
   for (int i = 0; i < n; i++)
     for (int k = 0; k < nq; k++)  // a chunk's candidates side by side, the next chunk after it in stream order
       st[(size_t)i * nq + k].coefs = d_coefs + (k % chunk[(size_t)i]) * max_coefs[(size_t)i];
-  // Host copies first: a pageable copy waits for the stream, so they go before any kernel of the group.
+  CopiesDone done(ctx);
+  // Host copies first: a pageable copy may wait for the stream, so they go before any kernel of the group.
   for (int i = 0; i < n; i++)
     if ((rc = copy_to_device(ctx, d_imgs + img_off[(size_t)i], images[i], img_bytes[(size_t)i])) != RCG_OK) return rc;
-  cudaError_t e = cudaMemcpyAsync(d_sts, st.data(), sizeof(StepDesc) * st.size(), cudaMemcpyHostToDevice,
-                                  ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep tables upload");
+  if ((rc = copy_to_device(ctx, d_sts, st.data(), sizeof(StepDesc) * st.size())) != RCG_OK) return rc;
   std::vector<const uint8_t*> refs(st.size());
   std::vector<Decoded> decoded(st.size());
   std::vector<uint32_t> ws(st.size()), hs(st.size());
@@ -921,7 +947,8 @@ static int metric_on_device(rcg_ctx* ctx, int metric, const uint8_t* d_a, const 
     double* d = (double*)workspace(ctx, "metric_score", sizeof(double) * 8);
     if (!d) return RCG_NO_MEMORY;
     if ((rc = ssim_score(ctx, d_a, d_b, w, h, ch, d, nullptr, nullptr)) != RCG_OK) return rc;
-    cudaMemcpyAsync(score, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    CopiesDone done(ctx);
+    if ((rc = read_back(ctx, score, d, sizeof(double))) != RCG_OK) return rc;
     return finish(ctx, "ssim");
   }
   if (metric == RCG_METRIC_PSNR) {
@@ -931,7 +958,8 @@ static int metric_on_device(rcg_ctx* ctx, int metric, const uint8_t* d_a, const 
     const size_t n = (size_t)w * h * ch;
     squared_error(ctx, d_a, d_b, n, d);
     unsigned long long se = 0;
-    cudaMemcpyAsync(&se, d, sizeof se, cudaMemcpyDeviceToHost, ctx->stream);
+    CopiesDone done(ctx);
+    if ((rc = read_back(ctx, &se, d, sizeof se)) != RCG_OK) return rc;
     if ((rc = finish(ctx, "psnr")) != RCG_OK) return rc;
     const double mse = (double)se / (double)std::max<size_t>(n, 1);
     *score = mse == 0.0 ? INFINITY : 10.0 * std::log10(255.0 * 255.0 / mse);
@@ -962,7 +990,8 @@ static int metric_on_device(rcg_ctx* ctx, int metric, const uint8_t* d_a, const 
       }
     }
     double s[5];
-    cudaMemcpyAsync(s, d, sizeof s, cudaMemcpyDeviceToHost, ctx->stream);
+    CopiesDone done(ctx);
+    if ((rc = read_back(ctx, s, d, sizeof s)) != RCG_OK) return rc;
     if ((rc = finish(ctx, "ms_ssim")) != RCG_OK) return rc;
     double out = 1.0;
     for (int i = 0; i < 5; i++) out *= std::pow(std::max(s[i], 1e-9), kW[i]);
@@ -983,6 +1012,7 @@ int rcg_metric_score(rcg_ctx* ctx, int metric, const uint8_t* reference, const u
   uint8_t* d_a = (uint8_t*)workspace(ctx, "img_a", bytes);
   uint8_t* d_b = (uint8_t*)workspace(ctx, "img_b", bytes);
   if (!d_a || !d_b) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   int rc;
   if ((rc = copy_to_device(ctx, d_a, reference, bytes)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_b, candidate, bytes)) != RCG_OK) return rc;
@@ -1012,50 +1042,38 @@ static int build_coefs_impl(rcg_ctx* ctx, const uint8_t* src, uint32_t width, ui
   if ((rc = check_opts(ctx, opts, true)) != RCG_OK) return rc;
   if (!src || !coefs) return fail(ctx, RCG_INVALID, "null pointer");
   int w = (int)width, h = (int)height;
-  StepDesc* st = new StepDesc;
-  host_step_tables(st, opts->quality, opts->subsampling, channels, opts->trellis, w, h);
+  std::unique_ptr<StepDesc> st(new StepDesc);
+  host_step_tables(st.get(), opts->quality, opts->subsampling, channels, opts->trellis, w, h);
   long long ncoefs = st->nblocks * 64;
-  if ((long long)coefs_len < ncoefs) {
-    delete st;
-    return fail(ctx, RCG_INVALID, "coefficient buffer too short");
-  }
-  if (weights && (long long)weights_len != ncoefs) {
-    delete st;
+  if ((long long)coefs_len < ncoefs) return fail(ctx, RCG_INVALID, "coefficient buffer too short");
+  if (weights && (long long)weights_len != ncoefs)
     return fail(ctx, RCG_INVALID, "weights do not match the coefficient layout");
-  }
   cudaSetDevice(ctx->device);
   size_t bytes = (size_t)w * h * channels;
   uint8_t* d_src = (uint8_t*)workspace(ctx, "img_a", bytes);
   int16_t* d_coefs = (int16_t*)workspace(ctx, "coefs_single", (size_t)ncoefs * 2);
   StepDesc* d_st = (StepDesc*)workspace(ctx, "step_single", sizeof(StepDesc));
   float* d_w = weights ? (float*)workspace(ctx, "weights_single", (size_t)ncoefs * sizeof(float)) : nullptr;
-  if (!d_src || !d_coefs || !d_st || (weights && !d_w)) {
-    delete st;
-    return RCG_NO_MEMORY;
-  }
+  if (!d_src || !d_coefs || !d_st || (weights && !d_w)) return RCG_NO_MEMORY;
   st->coefs = d_coefs;
   st->pweights = d_w;
-  if (weights) cudaMemcpyAsync(d_w, weights, (size_t)ncoefs * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyAsync(d_src, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  CopiesDone done(ctx);
+  if (weights && (rc = copy_to_device(ctx, d_w, weights, (size_t)ncoefs * sizeof(float))) != RCG_OK) return rc;
+  if ((rc = copy_to_device(ctx, d_src, src, bytes)) != RCG_OK) return rc;
+  if ((rc = copy_to_device(ctx, d_st, st.get(), sizeof(StepDesc))) != RCG_OK) return rc;
   EncoderSetup es;
   // Only this quality's layout is needed: pin Auto to what it resolves to.
   int sub = opts->subsampling;
   if (channels == 3 && sub == RCG_SUB_AUTO) sub = opts->quality < 90 ? RCG_SUB_420 : RCG_SUB_444;
-  if ((rc = setup_encoder(ctx, d_src, w, h, channels, sub, &es)) != RCG_OK) {
-    delete st;
-    return rc;
-  }
+  if ((rc = setup_encoder(ctx, d_src, w, h, channels, sub, &es)) != RCG_OK) return rc;
   quantize(ctx, d_st, es.caches, st->nblocks);
   rate_tables(ctx, d_st);
   trellis(ctx, d_st, es.caches, st->nblocks, weights != nullptr);
-  cudaMemcpyAsync(coefs, d_coefs, (size_t)ncoefs * 2, cudaMemcpyDeviceToHost, ctx->stream);
+  if ((rc = read_back(ctx, coefs, d_coefs, (size_t)ncoefs * 2)) != RCG_OK) return rc;
   if (qtables) {
     std::memcpy(qtables, st->qt[0], 64);
     std::memcpy(qtables + 64, st->qt[1], 64);
   }
-  cudaStreamSynchronize(ctx->stream);  // the host StepDesc must outlive the async upload
-  delete st;
   return finish(ctx, "build_coefs");
 }
 
@@ -1075,30 +1093,25 @@ int rcg_build_coefs_weighted(rcg_ctx* ctx, const uint8_t* src, uint32_t width, u
 // ---- decoder
 
 // reconstruct (jpeg/src/decode.rs:334-389) with the multipliers already in `st` (owned; deleted here).
-static int reconstruct_with(rcg_ctx* ctx, StepDesc* st, int w, int h, const int16_t* coefs, uint8_t* out,
+static int reconstruct_with(rcg_ctx* ctx, StepDesc* st_owned, int w, int h, const int16_t* coefs, uint8_t* out,
                             size_t out_len) {
+  const std::unique_ptr<StepDesc> st(st_owned);
   const int nc = st->ncomp;
-  long long blk = st->nblocks, poff = plane_bytes(st);
-  if (out_len < (size_t)w * h * nc) {
-    delete st;
-    return fail(ctx, RCG_INVALID, "output buffer too short");
-  }
+  long long blk = st->nblocks, poff = plane_bytes(st.get());
+  if (out_len < (size_t)w * h * nc) return fail(ctx, RCG_INVALID, "output buffer too short");
   cudaSetDevice(ctx->device);
   int16_t* d_coefs = (int16_t*)workspace(ctx, "coefs_single", (size_t)blk * 64 * 2);
   uint8_t* d_planes = (uint8_t*)workspace(ctx, "dec_planes_single", (size_t)poff);
   uint8_t* d_out = (uint8_t*)workspace(ctx, "img_b", (size_t)w * h * nc);
   StepDesc* d_st = (StepDesc*)workspace(ctx, "step_single", sizeof(StepDesc));
-  if (!d_coefs || !d_planes || !d_out || !d_st) {
-    delete st;
-    return RCG_NO_MEMORY;
-  }
-  cudaMemcpyAsync(d_coefs, coefs, (size_t)blk * 64 * 2, cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  if (!d_coefs || !d_planes || !d_out || !d_st) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
+  int rc;
+  if ((rc = copy_to_device(ctx, d_coefs, coefs, (size_t)blk * 64 * 2)) != RCG_OK) return rc;
+  if ((rc = copy_to_device(ctx, d_st, st.get(), sizeof(StepDesc))) != RCG_OK) return rc;
   dequant_idct(ctx, d_st, d_coefs, d_planes, blk);
   upsample_color(ctx, d_st, d_planes, w, h, d_out, nullptr);
-  cudaMemcpyAsync(out, d_out, (size_t)w * h * nc, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaStreamSynchronize(ctx->stream);
-  delete st;
+  if ((rc = read_back(ctx, out, d_out, (size_t)w * h * nc)) != RCG_OK) return rc;
   return finish(ctx, "reconstruct");
 }
 
@@ -1227,9 +1240,9 @@ static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st,
                           (size_t)s0.pitch * sizeof(float), (size_t)w * sizeof(float), (size_t)h, cudaMemcpyDeviceToDevice,
                           ctx->stream);
   static const int kActive = 1;  // the later steps' tables cleared it; the next step's set it again
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&d_st->active, &kActive, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "near-tie rescore");
+  int rc = copy_to_device(ctx, &d_st->active, &kActive, sizeof(int));
+  if (rc != RCG_OK) return rc;
   upsample_color(ctx, d_st, planes, w, h, nullptr, lin + 3 * np, w);
   return exact_score(ctx, lin, lin + 3 * np, w, h, d_exact);
 }
@@ -1252,7 +1265,7 @@ static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, 
     search_resume(ctx, d_ss, d_exact);
     ctx->tie_rescores++;
     for (int s = hs->step + 1; s < max_steps; s++) issue_step(s, s == hs->step + 1);
-    cudaMemcpyAsync(hs, d_ss, sizeof *hs, cudaMemcpyDeviceToHost, ctx->stream);
+    if ((rc = read_back(ctx, hs, d_ss, sizeof *hs)) != RCG_OK) return rc;
     if ((rc = finish(ctx, "search after a near tie")) != RCG_OK) return rc;
   }
   return RCG_OK;
@@ -1268,9 +1281,11 @@ struct SearchRun {
   StepDesc* d_st = nullptr;
   int16_t* slots = nullptr;
   uint8_t* planes = nullptr;
+  SearchState begin;  // the initial state's host copy: its upload may still read it when search_prepare returns
 };
 
-// Everything before the step loop, queued on the context's stream: the buffers, the quality-independent work (the
+// Everything before the step loop, queued on the context's stream (`run` stays in place until it has been waited for): the
+// buffers, the quality-independent work (the
 // reference image's pyramids for SSIMULACRA2, the FDCTs) and the initial bisection state.
 static int search_prepare(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int channels, int metric, double target,
                           int max_q, int subsampling, int trellis_on, SearchRun* run) {
@@ -1297,7 +1312,7 @@ static int search_prepare(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int 
   run->slots = (int16_t*)workspace(ctx, "coef_slots", (size_t)run->es.max_coefs * 2 * run->max_steps);
   run->planes = (uint8_t*)workspace(ctx, "dec_planes", (size_t)run->es.max_plane_bytes);
   if (!run->slots || !run->planes) return RCG_NO_MEMORY;
-  SearchState hs;
+  SearchState& hs = run->begin;
   std::memset(&hs, 0, sizeof hs);
   hs.lo = 1;
   hs.hi = max_q;
@@ -1310,10 +1325,7 @@ static int search_prepare(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int 
   hs.channels = channels;
   hs.best_q = max_q;
   hs.tie_band = metric == RCG_METRIC_SSIMULACRA2 ? ctx->tie_band : 0.0;
-  // A copy from pageable memory returns once the source is staged, so `hs` may go out of scope.
-  cudaError_t e = cudaMemcpyAsync(run->d_ss, &hs, sizeof hs, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "search state upload");
-  return RCG_OK;
+  return copy_to_device(ctx, run->d_ss, &hs, sizeof hs);
 }
 
 // The result of a finished search: Found, and the chosen coefficients and tables to device or host buffers.
@@ -1342,9 +1354,10 @@ static int search_collect(rcg_ctx* ctx, const SearchRun& run, const SearchState&
     }
   }
   uint8_t qt[128];
+  CopiesDone done(ctx);
   qtables_for(hs.best_q, qt);
   if (h_qt_out) std::memcpy(h_qt_out, qt, 128);
-  if (d_qt_out) cudaMemcpyAsync(d_qt_out, qt, 128, cudaMemcpyHostToDevice, ctx->stream);
+  if (d_qt_out && (rc = copy_to_device(ctx, d_qt_out, qt, 128)) != RCG_OK) return rc;
   return finish(ctx, "search output");
 }
 
@@ -1355,6 +1368,8 @@ static int search_impl(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int cha
                        size_t coefs_len, uint8_t* d_qt_out, int16_t* h_coefs_out, uint8_t* h_qt_out,
                        const float* d_weights = nullptr, int step_limit = 0) {
   SearchRun run;
+  SearchState hs;
+  CopiesDone done(ctx);
   int rc = search_prepare(ctx, d_src, w, h, channels, metric, target, max_q, subsampling, trellis_on, &run);
   if (rc != RCG_OK) return rc;
   const EncoderSetup& es = run.es;
@@ -1378,8 +1393,7 @@ static int search_impl(rcg_ctx* ctx, const uint8_t* d_src, int w, int h, int cha
     for (int s = 0; s < nsteps; s++) issue_step(s, s == 0);
   });
   if (rc != RCG_OK) return rc;
-  SearchState hs;
-  cudaMemcpyAsync(&hs, d_ss, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
+  if ((rc = read_back(ctx, &hs, d_ss, sizeof hs)) != RCG_OK) return rc;
   if ((rc = finish(ctx, "search")) != RCG_OK) return rc;
   if ((rc = settle_ties(ctx, sc, d_ss, &hs, d_st, run.planes, nsteps, w, h, issue_step)) != RCG_OK) return rc;
   if (nsteps < run.max_steps && !hs.done) {
@@ -1422,6 +1436,7 @@ int rcg_search_metric(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint32_t
   size_t bytes = (size_t)width * height * channels;
   uint8_t* d_src = (uint8_t*)workspace(ctx, "img_src", bytes);
   if (!d_src) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   if ((rc = copy_to_device(ctx, d_src, src, bytes)) != RCG_OK) return rc;
   return search_impl(ctx, d_src, (int)width, (int)height, channels, metric, target, max_q, opts->subsampling,
                      opts->trellis, found, nullptr, coefs_len, nullptr, coefs, qtables);
@@ -1479,6 +1494,7 @@ int rcg_search_batch(rcg_ctx* ctx, int n, const uint8_t* const* srcs, const uint
   std::vector<uint64_t> ties0;
   for (int t = 0; t < p; t++) {
     ctx->workers[t]->tie_band = ctx->tie_band;
+    ctx->workers[t]->workspace_limit = ctx->workspace_limit;
     ties0.push_back(ctx->workers[t]->tie_rescores);
   }
   std::atomic<int> next(0);
@@ -1532,9 +1548,12 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     sub->stage_results = true;
     ctx->lock_subs.push_back(sub);
   }
-  // Per image, on its own context's stream (the images' set-ups overlap one another): upload, colour planes, FDCTs,
-  // the reference's pyramid, the initial bisection state. Host threads share the images. Then the caller's stream waits for all of them.
+  // Per image, on its own context's stream (the images' set-ups overlap one another): upload, FDCTs, the reference's
+  // pyramids, the initial bisection state. Host threads share the images. Then the caller's stream waits for all of them.
   std::vector<SearchRun> runs((size_t)n);
+  std::vector<LockItem> items((size_t)n);
+  std::vector<SearchState> hs((size_t)n);
+  CopiesDone done(ctx, &ctx->lock_subs);  // one image's failure leaves the others' uploads queued
   std::vector<int> status((size_t)n, RCG_OK);
   const int nthreads = std::max(1, std::min(n, kLockThreads));
   auto for_images = [&](const std::function<void(int)>& fn) {
@@ -1553,6 +1572,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     sub->tie_band = ctx->tie_band;
     sub->band_chunks = ctx->band_chunks;
     sub->ref_cache = ctx->ref_cache;
+    sub->workspace_limit = ctx->workspace_limit;
     const size_t bytes = (size_t)widths[i] * heights[i] * channels[i];
     uint8_t* d_src = (uint8_t*)workspace(sub, "img_src", bytes);
     int r = d_src ? RCG_OK : RCG_NO_MEMORY;
@@ -1574,7 +1594,6 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     cudaStreamWaitEvent(ctx->stream, ctx->lock_subs[(size_t)i]->switch_event, 0);
   }
   // The work-lists: per image its StepDesc, search state, buffers and first CTA in each stage's grid.
-  std::vector<LockItem> items((size_t)n);
   long long q_total = 0, p_total = 0, t_total = 0;
   int max_scales = 1, max_steps = 1;
   for (int i = 0; i < n; i++) {
@@ -1613,7 +1632,7 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
   LockItem* d_items = (LockItem*)workspace(ctx, "lock_items", sizeof(LockItem) * (size_t)n);
   double* d_exact = (double*)workspace(ctx, "x_score", sizeof(double), false);
   if (!d_items || !d_exact) return RCG_NO_MEMORY;
-  cudaMemcpyAsync(d_items, items.data(), sizeof(LockItem) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
+  if ((rc = copy_to_device(ctx, d_items, items.data(), sizeof(LockItem) * (size_t)n)) != RCG_OK) return rc;
   auto issue_step = [&](int s, bool first) {
     lock_step_codec(ctx, d_items, n, q_total, first);
     lock_step_score(ctx, d_items, n, p_total, t_total, max_scales,
@@ -1625,10 +1644,11 @@ int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, c
     for (int s = 0; s < max_steps; s++) issue_step(s, s == 0);
   });
   if (rc != RCG_OK) return rc;
-  std::vector<SearchState> hs((size_t)n);
   auto read_states = [&]() -> int {
-    for (int i = 0; i < n; i++)
-      cudaMemcpyAsync(&hs[(size_t)i], runs[(size_t)i].d_ss, sizeof(SearchState), cudaMemcpyDeviceToHost, ctx->stream);
+    for (int i = 0; i < n; i++) {
+      const int r = read_back(ctx, &hs[(size_t)i], runs[(size_t)i].d_ss, sizeof(SearchState));
+      if (r != RCG_OK) return r;
+    }
     return finish(ctx, "lockstep batch");
   };
   if ((rc = read_states()) != RCG_OK) return rc;
@@ -1674,39 +1694,32 @@ int rcg_requantize(rcg_ctx* ctx, uint32_t width, uint32_t height, const rcg_coef
   if (layout->ncomp != 1 && layout->ncomp != 3)
     return fail(ctx, RCG_UNSUPPORTED, "requantization takes 1 or 3 components");
   if (quality < 1 || quality > 100) return fail(ctx, RCG_INVALID, "quality must be 1..=100");
-  StepDesc* st = new StepDesc;
-  int rc = layout_step(ctx, st, (int)width, (int)height, layout);
-  if (rc == RCG_OK) rc = requant_inputs(ctx, in, st);
+  const std::unique_ptr<StepDesc> st(new StepDesc);
+  int rc = layout_step(ctx, st.get(), (int)width, (int)height, layout);
+  if (rc == RCG_OK) rc = requant_inputs(ctx, in, st.get());
   if (rc == RCG_OK && (long long)coefs_len < st->nblocks * 64) rc = fail(ctx, RCG_INVALID, "coefficient buffer too short");
-  if (rc != RCG_OK) {
-    delete st;
-    return rc;
-  }
+  if (rc != RCG_OK) return rc;
   cudaSetDevice(ctx->device);
   const size_t cbytes = (size_t)st->nblocks * 64 * 2;
   int16_t* d_src = (int16_t*)workspace(ctx, "rq_src", cbytes);
   int16_t* d_out = (int16_t*)workspace(ctx, "coefs_single", cbytes);
   StepDesc* d_st = (StepDesc*)workspace(ctx, "step_single", sizeof(StepDesc));
-  if (!d_src || !d_out || !d_st) {
-    delete st;
-    return RCG_NO_MEMORY;
-  }
+  if (!d_src || !d_out || !d_st) return RCG_NO_MEMORY;
   int tq[3];
   uint8_t slot_qt[4][64];
   int present[4];
-  host_requant_tables(st, quality, trellis, tq, slot_qt, present);
+  host_requant_tables(st.get(), quality, trellis, tq, slot_qt, present);
   st->coef_src = d_src;
   st->coefs = d_out;
-  copy_to_device(ctx, d_src, coefs_in, cbytes);
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  CopiesDone done(ctx);
+  if ((rc = copy_to_device(ctx, d_src, coefs_in, cbytes)) != RCG_OK) return rc;
+  if ((rc = copy_to_device(ctx, d_st, st.get(), sizeof(StepDesc))) != RCG_OK) return rc;
   const float* no_caches[9] = {nullptr};
   requantize_plain(ctx, d_st, st->nblocks);
   rate_tables(ctx, d_st);
   rcg::trellis(ctx, d_st, no_caches, st->nblocks);
   rc = copy_to_host(ctx, coefs_out, d_out, cbytes);
-  cudaStreamSynchronize(ctx->stream);
   qtables_out(tq, slot_qt, present, st->ncomp, out);
-  delete st;
   if (rc != RCG_OK) return rc;
   return finish(ctx, "requantize");
 }
@@ -1727,13 +1740,13 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
     return fail(ctx, RCG_UNSUPPORTED, "requantization takes 1 or 3 components");
   const int w = (int)width, h = (int)height;
   const int max_q = std::max(1, std::min(max_quality, 100));
-  StepDesc* st = new StepDesc;
+  const std::unique_ptr<StepDesc> owned(new StepDesc);
+  StepDesc* const st = owned.get();
+  SearchState hs;
+  CopiesDone done(ctx);
   int rc = layout_step(ctx, st, w, h, layout);
   if (rc == RCG_OK) rc = requant_inputs(ctx, in, st);
-  if (rc != RCG_OK) {
-    delete st;
-    return rc;
-  }
+  if (rc != RCG_OK) return rc;
   cudaSetDevice(ctx->device);
   const long long nblocks = st->nblocks;
   const size_t cbytes = (size_t)nblocks * 64 * 2;
@@ -1749,22 +1762,17 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   SearchState* d_ss = (SearchState*)workspace(ctx, "search_state", sizeof(SearchState));
   StepDesc* d_st = (StepDesc*)workspace(ctx, "step_search", sizeof(StepDesc));
   if (!d_src || !slots || !planes || !d_ss || !d_st || (metric == RCG_METRIC_SSIM && !ref_px) ||
-      scorer_setup(ctx, metric, w, h, channels, &sc) != RCG_OK) {
-    delete st;
+      scorer_setup(ctx, metric, w, h, channels, &sc) != RCG_OK)
     return RCG_NO_MEMORY;
-  }
   sc.ref_px = ref_px;
-  if (!on_device && (rc = copy_to_device(ctx, d_src, coefs_in, cbytes)) != RCG_OK) {
-    delete st;
-    return rc;
-  }
+  if (!on_device && (rc = copy_to_device(ctx, d_src, coefs_in, cbytes)) != RCG_OK) return rc;
   // The reference image: the source reconstructed with its own tables (cli/src/pipeline.rs:372).
   for (int c = 0; c < st->ncomp; c++)
     for (int n = 0; n < 64; n++) st->mult[c][n] = mult_entry_host(st->src_qt[c], n);
   st->coef_src = d_src;
   st->coefs = d_src;
   st->requant = 1;
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  if ((rc = copy_to_device(ctx, d_st, st, sizeof(StepDesc))) != RCG_OK) return rc;
   dequant_idct(ctx, d_st, d_src, planes, nblocks);
   // A requantized candidate keeps the source's block layout.
   sc.direct = layout_direct(st);
@@ -1772,7 +1780,6 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
     upsample_color(ctx, d_st, planes, w, h, ref_px, nullptr);
   else
     build_decoded(ctx, sc.pd, d_st, planes, sc.direct, sc.ref_pyr, sc.ref_xyb, nullptr);
-  SearchState hs;
   std::memset(&hs, 0, sizeof hs);
   hs.lo = 1;
   hs.hi = max_q;
@@ -1783,7 +1790,7 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   hs.channels = channels;
   hs.best_q = max_q;
   hs.tie_band = metric == RCG_METRIC_SSIMULACRA2 ? ctx->tie_band : 0.0;
-  cudaMemcpyAsync(d_ss, &hs, sizeof hs, cudaMemcpyHostToDevice, ctx->stream);
+  if ((rc = copy_to_device(ctx, d_ss, &hs, sizeof hs)) != RCG_OK) return rc;
   const float* no_caches[9] = {nullptr};
   std::vector<long long> key = {2, (long long)(uintptr_t)d_src, w, h, st->ncomp, metric, trellis, max_steps,
                                 st->hmax, st->vmax, nblocks};
@@ -1802,20 +1809,12 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   rc = run_step_loop(ctx, key, [&]() {
     for (int s = 0; s < max_steps; s++) issue_step(s, s == 0);
   });
-  if (rc != RCG_OK) {
-    delete st;
-    return rc;
-  }
-  cudaMemcpyAsync(&hs, d_ss, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream);
+  if (rc != RCG_OK) return rc;
+  if ((rc = read_back(ctx, &hs, d_ss, sizeof hs)) != RCG_OK) return rc;
   if ((rc = finish(ctx, "search_requantize")) != RCG_OK ||
-      (rc = settle_ties(ctx, sc, d_ss, &hs, d_st, planes, max_steps, w, h, issue_step)) != RCG_OK) {
-    delete st;
+      (rc = settle_ties(ctx, sc, d_ss, &hs, d_st, planes, max_steps, w, h, issue_step)) != RCG_OK)
     return rc;
-  }
-  if (!hs.done) {
-    delete st;
-    return fail(ctx, RCG_TIMEOUT, "bisection did not finish within the step budget");
-  }
+  if (!hs.done) return fail(ctx, RCG_TIMEOUT, "bisection did not finish within the step budget");
   found->quality = hs.best_q;
   found->score = hs.best_score;
   found->nsteps = 0;
@@ -1825,15 +1824,11 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
     found->nsteps = s + 1;
   }
   if (coefs_out) {
-    if (coefs_len < (size_t)nblocks * 64) {
-      delete st;
-      return fail(ctx, RCG_INVALID, "coefficient buffer too short");
-    }
+    if (coefs_len < (size_t)nblocks * 64) return fail(ctx, RCG_INVALID, "coefficient buffer too short");
     const int16_t* best = slots + (size_t)hs.best_step * nblocks * 64;
     if (on_device) {
       cudaMemcpyAsync(coefs_out, best, cbytes, cudaMemcpyDeviceToDevice, ctx->stream);
     } else if ((rc = copy_to_host(ctx, coefs_out, best, cbytes)) != RCG_OK) {
-      delete st;
       return rc;
     }
   }
@@ -1842,7 +1837,6 @@ static int search_requantize_impl(rcg_ctx* ctx, uint32_t width, uint32_t height,
   int present[4];
   host_requant_tables(st, hs.best_q, trellis, tq, slot_qt, present);
   qtables_out(tq, slot_qt, present, st->ncomp, out);
-  delete st;
   return finish(ctx, "search_requantize output");
 }
 
@@ -1878,6 +1872,7 @@ static int plan_common(rcg_ctx* ctx, uint32_t width, uint32_t height, const rcg_
     return rc;
   }
   cudaSetDevice(ctx->device);
+  CopiesDone done(ctx);
   const int16_t* d = coefs;
   if (!on_device) {
     int16_t* buf = (int16_t*)workspace(ctx, "plan_coefs", (size_t)st->nblocks * 128);
@@ -1932,6 +1927,7 @@ int rcg_ssimulacra2_grad_device(rcg_ctx* ctx, const uint8_t* d_reference, const 
   if (width < (uint32_t)kMinSide || height < (uint32_t)kMinSide)
     return fail(ctx, RCG_INVALID, "SSIMULACRA 2 needs at least 8x8 pixels");
   cudaSetDevice(ctx->device);
+  CopiesDone done(ctx);
   int rc = ssim2_grad_device(ctx, d_reference, d_distorted, (int)width, (int)height, score, d_grad);
   if (rc != RCG_OK) return rc;
   return finish(ctx, "ssimulacra2 gradient");
@@ -1949,6 +1945,7 @@ int rcg_ssimulacra2_grad(rcg_ctx* ctx, const uint8_t* reference, const float* di
   float* d_dist = (float*)workspace(ctx, "grad_dist", n * sizeof(float));
   double* d_grad = (double*)workspace(ctx, "grad_out", n * sizeof(double));
   if (!d_ref || !d_dist || !d_grad) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   int rc;
   if ((rc = copy_to_device(ctx, d_ref, reference, n)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_dist, distorted, n * sizeof(float))) != RCG_OK) return rc;
@@ -2053,6 +2050,7 @@ int rcg_coef_gradient(rcg_ctx* ctx, const uint8_t* reference, const uint8_t* dec
                       int channels, const rcg_coef_layout* layout, double* score, double* grad, size_t grad_len) {
   if (!ctx) return RCG_INVALID;
   if (!score) return fail(ctx, RCG_INVALID, "null pointer");
+  CopiesDone done(ctx);
   StepDesc* st = nullptr;
   const uint8_t *d_ref = nullptr, *d_dec = nullptr;
   int rc = pullback_inputs(ctx, reference, decoded, width, height, channels, layout, grad, grad_len, &st, &d_ref,
@@ -2077,6 +2075,7 @@ int rcg_perceptual_weights(rcg_ctx* ctx, const uint8_t* reference, const uint8_t
   PerceptualParams p;
   int rc = check_popts(ctx, popts, &p);
   if (rc != RCG_OK) return rc;
+  CopiesDone done(ctx);
   StepDesc* st = nullptr;
   const uint8_t *d_ref = nullptr, *d_dec = nullptr;
   rc = pullback_inputs(ctx, reference, decoded, width, height, channels, layout, weights, weights_len, &st, &d_ref,
@@ -2126,6 +2125,7 @@ int rcg_search_weighted(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint32
   uint8_t* d_src = (uint8_t*)workspace(ctx, "img_src", bytes);
   float* d_w = (float*)workspace(ctx, "perc_weights", (size_t)ncoefs * sizeof(float));
   if (!d_src || !d_w) return RCG_NO_MEMORY;
+  CopiesDone done(ctx);
   if ((rc = copy_to_device(ctx, d_src, src, bytes)) != RCG_OK) return rc;
   if ((rc = copy_to_device(ctx, d_w, weights, (size_t)ncoefs * sizeof(float))) != RCG_OK) return rc;
   return search_impl(ctx, d_src, (int)width, (int)height, channels, RCG_METRIC_SSIMULACRA2, target, max_q,
@@ -2171,6 +2171,9 @@ int rcg_search_perceptual(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint
   uint8_t* d_dec = (uint8_t*)workspace(ctx, "perc_dec", npx * channels);
   StepDesc* d_st = (StepDesc*)workspace(ctx, "perc_step", sizeof(StepDesc));
   if (!d_src || !d_plain || !d_perc || !d_w || !d_dec || !d_st) return RCG_NO_MEMORY;
+  const std::unique_ptr<StepDesc> owned(new StepDesc);
+  StepDesc* const st = owned.get();
+  CopiesDone done(ctx);
   if ((rc = copy_to_device(ctx, d_src, src, npx * channels)) != RCG_OK) return rc;
   // 1. the plain search
   rc = search_impl(ctx, d_src, w, h, channels, RCG_METRIC_SSIMULACRA2, target, max_q, opts->subsampling,
@@ -2178,19 +2181,14 @@ int rcg_search_perceptual(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint
   if (rc != RCG_OK) return rc;
   // 2. its decoded image, and the weights from the gradient there
   p.strength = rcg_perceptual_strength(popts, plain->quality);
-  StepDesc* st = new StepDesc;
   host_step_tables(st, plain->quality, opts->subsampling, channels, opts->trellis, w, h);
   uint8_t* planes = (uint8_t*)workspace(ctx, "perc_planes", (size_t)plane_bytes(st));
-  if (!planes) {
-    delete st;
-    return RCG_NO_MEMORY;
-  }
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  if (!planes) return RCG_NO_MEMORY;
+  if ((rc = copy_to_device(ctx, d_st, st, sizeof(StepDesc))) != RCG_OK) return rc;
   dequant_idct(ctx, d_st, d_plain, planes, st->nblocks);
   upsample_color(ctx, d_st, planes, w, h, d_dec, nullptr);
   double gscore = 0.0;
   rc = perceptual_impl(ctx, d_src, d_dec, w, h, channels, st, p, &gscore, nullptr, d_w);
-  cudaStreamSynchronize(ctx->stream);  // the host StepDesc must outlive its upload
   // 3. the weighted search
   rcg_found perc;
   if (rc == RCG_OK)
@@ -2200,7 +2198,6 @@ int rcg_search_perceptual(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint
   uint64_t sz[2] = {0, 0};
   if (rc == RCG_OK) rc = planned_bytes(ctx, st, w, h, d_plain, &sz[0]);
   if (rc == RCG_OK) rc = planned_bytes(ctx, st, w, h, d_perc, &sz[1]);
-  delete st;
   if (rc != RCG_OK) return rc;
   const bool use_perc = !popts->keep_smaller || sz[1] <= sz[0];
   *found = use_perc ? perc : *plain;
@@ -2239,6 +2236,9 @@ int rcg_search_perceptual_fast(rcg_ctx* ctx, const uint8_t* src, uint32_t width,
   uint8_t* d_dec = (uint8_t*)workspace(ctx, "perc_dec", npx * channels);
   StepDesc* d_st = (StepDesc*)workspace(ctx, "perc_step", sizeof(StepDesc));
   if (!d_src || !d_probe || !d_perc || !d_w || !d_dec || !d_st) return RCG_NO_MEMORY;
+  const std::unique_ptr<StepDesc> owned(new StepDesc);
+  StepDesc* const st = owned.get();
+  CopiesDone done(ctx);
   if ((rc = copy_to_device(ctx, d_src, src, npx * channels)) != RCG_OK) return rc;
   // 1. the plain bisection's first kPerceptualProbeSteps candidates; the one scoring closest to the target stands in
   //    for the result (which lies within the 6 qualities the bisection has left after four steps from 1..100)
@@ -2250,20 +2250,14 @@ int rcg_search_perceptual_fast(rcg_ctx* ctx, const uint8_t* src, uint32_t width,
   if (probe) *probe = pr;
   // 2. the gradient at that candidate's decode, the weights with the strength its quality selects
   p.strength = rcg_perceptual_strength(popts, pr.quality);
-  StepDesc* st = new StepDesc;
   host_step_tables(st, pr.quality, opts->subsampling, channels, opts->trellis, w, h);
   uint8_t* planes = (uint8_t*)workspace(ctx, "perc_planes", (size_t)plane_bytes(st));
-  if (!planes) {
-    delete st;
-    return RCG_NO_MEMORY;
-  }
-  cudaMemcpyAsync(d_st, st, sizeof(StepDesc), cudaMemcpyHostToDevice, ctx->stream);
+  if (!planes) return RCG_NO_MEMORY;
+  if ((rc = copy_to_device(ctx, d_st, st, sizeof(StepDesc))) != RCG_OK) return rc;
   dequant_idct(ctx, d_st, d_probe, planes, st->nblocks);
   upsample_color(ctx, d_st, planes, w, h, d_dec, nullptr);
   double gscore = 0.0;
   rc = perceptual_impl(ctx, d_src, d_dec, w, h, channels, st, p, &gscore, nullptr, d_w);
-  cudaStreamSynchronize(ctx->stream);  // the host StepDesc must outlive its upload
-  delete st;
   if (rc != RCG_OK) return rc;
   // 3. one weighted search
   rc = search_impl(ctx, d_src, w, h, channels, RCG_METRIC_SSIMULACRA2, target, max_q, opts->subsampling,

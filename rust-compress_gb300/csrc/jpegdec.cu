@@ -1238,6 +1238,8 @@ int parse_jpeg(rcg_ctx* ctx, const uint8_t* d, size_t len, Parsed& P) {
 int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* info, rcg_coef_layout* layout,
                 rcg_qtables* tables, int16_t* coefs, size_t coefs_len, bool coefs_on_device) {
   Parsed P;
+  int h_changed[kMaxRounds], h_err = 0;
+  CopiesDone done(ctx);
   int rc = parse_jpeg(ctx, data, len, P);
   if (rc != RCG_OK) return rc;
   const int nc = (int)P.comps.size();
@@ -1311,9 +1313,10 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
       return RCG_NO_MEMORY;
     if (!sc.bytes.empty() && (rc = copy_to_device(ctx, d_bytes, sc.bytes.data(), sc.bytes.size())) != RCG_OK)
       return rc;
-    cudaMemcpyAsync(d_segs, sc.segs.data(), sizeof(Segment) * sc.segs.size(), cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemcpyAsync(d_sd, &sc.sd, sizeof(ScanDesc), cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemcpyAsync(d_tab, &sc.tables, sizeof(Tables), cudaMemcpyHostToDevice, ctx->stream);
+    if ((rc = copy_to_device(ctx, d_segs, sc.segs.data(), sizeof(Segment) * sc.segs.size())) != RCG_OK ||
+        (rc = copy_to_device(ctx, d_sd, &sc.sd, sizeof(ScanDesc))) != RCG_OK ||
+        (rc = copy_to_device(ctx, d_tab, &sc.tables, sizeof(Tables))) != RCG_OK)
+      return rc;
     if (sc.sd.kind == kDcRefine) {
       long long nb = 0;
       for (const Segment& g : sc.segs) nb = std::max(nb, g.block0 + g.nblocks);
@@ -1327,8 +1330,8 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
                  kRefineThreads, 0, d_sd, d_tab, d_segs, d_bytes, d_out, d_err);
       continue;
     }
-    cudaMemcpyAsync(d_seq, &sc.seq, offsetof(SeqTables, t) + sizeof(SeqHuff) * (size_t)sc.seq.n, cudaMemcpyHostToDevice,
-                    ctx->stream);
+    if ((rc = copy_to_device(ctx, d_seq, &sc.seq, offsetof(SeqTables, t) + sizeof(SeqHuff) * (size_t)sc.seq.n)) != RCG_OK)
+      return rc;
     cudaMemsetAsync(d_changed, 0, sizeof(int) * kMaxRounds, ctx->stream);
     const unsigned grid = (unsigned)((nsub + kDecThreads - 1) / kDecThreads);
     SubState* edge_cur = d_edges;
@@ -1349,9 +1352,8 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
         round = 1;
         break;
       }
-      int h_changed[kMaxRounds];
-      cudaMemcpyAsync(h_changed, d_changed, sizeof(int) * (size_t)launched, cudaMemcpyDeviceToHost, ctx->stream);
-      cudaError_t e = cudaStreamSynchronize(ctx->stream);
+      if ((rc = read_back(ctx, h_changed, d_changed, sizeof(int) * (size_t)launched)) != RCG_OK) return rc;
+      cudaError_t e = wait_stream(ctx);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "JPEG decode");
       for (; round < launched && !settled; round++) settled = h_changed[round] == 0;
     }
@@ -1368,10 +1370,9 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
     RCG_LAUNCH(ctx, "seq_write", k_seq_write, grid, kDecThreads, 0, d_sd, d_seq, d_segs, d_bytes, d_piece, d_cnt,
                d_base, d_out, d_err);
   }
-  int h_err = 0;
-  cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+  if ((rc = read_back(ctx, &h_err, d_err, sizeof(int))) != RCG_OK) return rc;
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess) e = wait_stream(ctx);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "JPEG decode");
   if (h_err) return fail(ctx, RCG_INVALID, h_err == 1 ? "bad JPEG entropy-coded data" : "JPEG decode lost its place");
   if (info) info->sync_rounds = fell_back ? -1 : rounds_max;

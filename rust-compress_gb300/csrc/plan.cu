@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "huffman.cuh"
@@ -641,7 +642,10 @@ int plan_scans(rcg_ctx* ctx, const StepDesc* lay, int w, int h, const int16_t* d
     return fail(ctx, RCG_INVALID, "device coefficients must be 16-byte aligned");
   std::vector<std::vector<HostScan>> scripts = candidate_scripts(nc);
   std::vector<HostScan> distinct;
-  PlanDesc* pd = new PlanDesc;
+  const std::unique_ptr<PlanDesc> owned(new PlanDesc);
+  PlanDesc* const pd = owned.get();
+  PlanOut host_out;
+  CopiesDone done(ctx);
   std::memset(pd, 0, sizeof *pd);
   pd->ncomp = nc;
   pd->nscripts = (int)scripts.size();
@@ -705,10 +709,8 @@ int plan_scans(rcg_ctx* ctx, const StepDesc* lay, int w, int h, const int16_t* d
     }
   }
   pd->nchunks = chunks;
-  if (mcu_pos >= (1ll << 31) || chunks >= (1ll << 31)) {
-    delete pd;
+  if (mcu_pos >= (1ll << 31) || chunks >= (1ll << 31))
     return fail(ctx, RCG_UNSUPPORTED, "image too large for scan planning");
-  }
   const int ns = pd->nscans;
   PlanDesc* d_pd = (PlanDesc*)workspace(ctx, "plan_desc", sizeof(PlanDesc));
   ScanStats* d_stats = (ScanStats*)workspace(ctx, "plan_stats", sizeof(ScanStats) * kMaxScans);
@@ -724,11 +726,10 @@ int plan_scans(rcg_ctx* ctx, const StepDesc* lay, int w, int h, const int16_t* d
   int* d_dht = (int*)workspace(ctx, "plan_dht", 4 * 4 * kMaxScans);
   PlanOut* d_out = (PlanOut*)workspace(ctx, "plan_out", sizeof(PlanOut));
   if (!d_pd || !d_stats || !d_flags || !d_prev || !d_P || !d_chunk_last || !d_chunk_pend || !d_chunk_prev ||
-      !d_chunk_pbase || !d_prev_end || !d_tbits || !d_dht || !d_out) {
-    delete pd;
+      !d_chunk_pbase || !d_prev_end || !d_tbits || !d_dht || !d_out)
     return RCG_NO_MEMORY;
-  }
-  cudaMemcpyAsync(d_pd, pd, sizeof(PlanDesc), cudaMemcpyHostToDevice, ctx->stream);
+  int rc = copy_to_device(ctx, d_pd, pd, sizeof(PlanDesc));
+  if (rc != RCG_OK) return rc;
   cudaMemsetAsync(d_stats, 0, sizeof(ScanStats) * ns, ctx->stream);
   RCG_LAUNCH(ctx, "plan_blocks", k_plan_blocks, (unsigned)chunks, kThreads, 0, d_pd, d_coefs, d_stats, d_flags,
              d_chunk_last, d_chunk_pend);
@@ -740,14 +741,10 @@ int plan_scans(rcg_ctx* ctx, const StepDesc* lay, int w, int h, const int16_t* d
              d_prev_end, d_stats);
   RCG_LAUNCH(ctx, "plan_tables", k_plan_tables, dim3(ns, 4), 288, 0, d_pd, d_stats, d_tbits, d_dht);
   RCG_LAUNCH(ctx, "plan_choose", k_plan_choose, 1, 256, 0, d_pd, d_stats, d_tbits, d_dht, d_out);
-  PlanOut host_out;
-  cudaMemcpyAsync(&host_out, d_out, sizeof(PlanOut), cudaMemcpyDeviceToHost, ctx->stream);
+  if ((rc = read_back(ctx, &host_out, d_out, sizeof(PlanOut))) != RCG_OK) return rc;
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) {
-    delete pd;
-    return cuda_fail(ctx, e, "scan planning");
-  }
+  if (e == cudaSuccess) e = wait_stream(ctx);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "scan planning");
   std::memset(res, 0, sizeof *res);
   res->progressive_bytes = host_out.prog;
   res->baseline_bytes = host_out.cost[ns - 1];
@@ -760,7 +757,6 @@ int plan_scans(rcg_ctx* ctx, const StepDesc* lay, int w, int h, const int16_t* d
     to_abi(distinct[i], &res->distinct[i]);
     res->distinct_bytes[i] = host_out.cost[i];
   }
-  delete pd;
   return RCG_OK;
 }
 

@@ -241,6 +241,9 @@ struct rcg_ctx {
   float* lut16 = nullptr;  // 65536-entry sRGB->linear table for 16-bit samples (allocated on first use)
   std::vector<rcg_ctx*> workers;  // sub-contexts of rcg_search_batch (own streams and workspaces)
   std::vector<rcg_ctx*> lock_subs;  // per-image sub-contexts of rcg_search_batch_lockstep (buffers, set-up streams)
+  // Copies to or from host memory have been queued since the stream was last waited for (CopiesDone).
+  bool host_traffic = false;
+  std::vector<unsigned char> work_list;  // the work-list scorer's upload: lives until the next one
   // Pinned buffer for results on their way to the caller's memory (grow-only), on batch contexts only (copy_to_host).
   bool stage_results = false;
   void* pinned_out = nullptr;
@@ -269,6 +272,9 @@ struct rcg_ctx {
   int band_chunks = 0;
   // The searches' reference moments (kRefWrite at the first candidate, kRefRead after): on by default.
   bool ref_cache = true;
+  // Workspace that would take the context past this many bytes fails as on a device without room; 0: no limit
+  // (rcg_internal_limit_workspace, for tests of what a call does then).
+  size_t workspace_limit = 0;
 };
 
 namespace rcg {
@@ -282,10 +288,33 @@ int cuda_fail(rcg_ctx* ctx, cudaError_t e, const char* what);
 // scorer's) move without making the graphs stale.
 void* workspace(rcg_ctx* ctx, const char* name, size_t bytes, bool in_graphs = true);
 
-// Host<->device copies of caller buffers. copy_to_device is asynchronous on the context stream (the source may be reused
-// as soon as it returns); copy_to_host synchronizes the stream.
+// Host<->device copies, asynchronous on the context stream whatever the memory's kind: the GPU may read a source or write
+// a destination, pageable ones too, until wait_stream. copy_to_host waits.
 int copy_to_device(rcg_ctx* ctx, void* dst, const void* src, size_t bytes);
+int read_back(rcg_ctx* ctx, void* dst, const void* src, size_t bytes);
 int copy_to_host(rcg_ctx* ctx, void* dst, const void* src, size_t bytes);
+cudaError_t wait_stream(rcg_ctx* ctx);
+
+// Keeps a function from returning (or throwing), with whatever status, while queued copies can still reach the caller's
+// memory or the function's own, which is declared before it. Nothing to wait for where the call has already waited.
+class CopiesDone {
+ public:
+  explicit CopiesDone(rcg_ctx* ctx, const std::vector<rcg_ctx*>* subs = nullptr) : ctx_(ctx), subs_(subs) {}
+  CopiesDone(const CopiesDone&) = delete;
+  CopiesDone& operator=(const CopiesDone&) = delete;
+  ~CopiesDone() {
+    settle(ctx_);
+    if (subs_)
+      for (rcg_ctx* sub : *subs_) settle(sub);
+  }
+
+ private:
+  static void settle(rcg_ctx* c) {
+    if (c->host_traffic && wait_stream(c) != cudaSuccess) cudaGetLastError();  // the call has its own status
+  }
+  rcg_ctx* ctx_;
+  const std::vector<rcg_ctx*>* subs_;  // contexts of a batch, their streams
+};
 
 // Kernel launch bookkeeping: counts launches and, when profiling, brackets them with events.
 void launch_begin(rcg_ctx* ctx, const char* name, cudaEvent_t* a, cudaEvent_t* b);
@@ -300,6 +329,13 @@ void collect_times(rcg_ctx* ctx);
 int run_step_loop(rcg_ctx* ctx, const std::vector<long long>& key, const std::function<void()>& issue);
 // Release the context's stored graphs.
 void drop_graphs(rcg_ctx* ctx);
+
+// A copy to a __constant__ or __device__ array, as copy_to_device.
+template <class T>
+void symbol_to_device(rcg_ctx* ctx, const T& symbol, const void* src, size_t bytes) {
+  ctx->host_traffic = true;
+  cudaMemcpyToSymbolAsync(symbol, src, bytes, 0, cudaMemcpyHostToDevice, ctx->stream);
+}
 
 // Kernels of one stream are launched as a chain: the next one's blocks may be placed as the running one's last blocks
 // leave, before its completion has been flushed and signalled, and wait in grid_chain() until it has completed and its

@@ -1792,7 +1792,9 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   }
   unsigned char* d_list = (unsigned char*)workspace(ctx, "batch_items", list_bytes);
   if (!d_list) return RCG_NO_MEMORY;
-  std::vector<unsigned char> list(list_bytes);
+  // The context keeps the list: its copy may still read it when this returns, and every call waits for its stream.
+  std::vector<unsigned char>& list = ctx->work_list;
+  list.assign(list_bytes, 0);
   std::memcpy(list.data() + o_items, items.data(), (size_t)n * sizeof(ScoreItem));
   for (int k = 0; k < kLists; k++) {
     if (jobs[k].empty()) continue;
@@ -1820,8 +1822,8 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
       seg0[gseg] = it.tile0 + sd.tile0;
     }
   }
-  cudaError_t e = cudaMemcpyAsync(d_list, list.data(), list_bytes, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "batch work-list upload");
+  int rc = copy_to_device(ctx, d_list, list.data(), list_bytes);
+  if (rc != RCG_OK) return rc;
   const ScoreItem* d_items = (const ScoreItem*)(d_list + o_items);
   const TileSeg* d_segs = (const TileSeg*)(d_list + o_seg);
   const long long* d_seg0 = (const long long*)(d_list + o_seg0);
@@ -1834,7 +1836,7 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
   const std::vector<long long> key = {3,     n,     nseg,    tiles,   max_scales, nj[0],
                                       nj[1], nj[2], ctas[0], ctas[1], ctas[2], decoded != nullptr,
                                       small[0], small[1], small[2]};
-  int rc = run_step_loop(ctx, key, [&]() {
+  rc = run_step_loop(ctx, key, [&]() {
     auto build = [&](int k, auto big, auto little) {
       if (nj[k])
         RCG_LAUNCH(ctx, "build_batch", (small[k] ? little : big), (unsigned)ctas[k], kPyrThreads, 0, d_jobs(k), d_first(k),
