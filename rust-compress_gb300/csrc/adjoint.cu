@@ -606,7 +606,8 @@ unsigned grid_of(long long n) {
 }
 
 // Moments of planes blurred together: their two buffers of five planes each stay within this (320 bytes a pixel in FP64:
-// images of up to 80 MP go as one group, in FP32 of up to 160 MP).
+// images of up to 80 MP go as one group, in FP32 of up to 160 MP) and within what can be allocated. Beside them the pass
+// holds 24 planes (192 bytes a pixel in FP64); at the least, a plane of scale 0 at a time, 272 bytes a pixel in all.
 constexpr long long kAdjBudgetBytes = 24ll << 30;
 
 // The whole pass in real type T; workspace buffers are named per type.
@@ -659,25 +660,27 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
     int s, c;
   };
   std::vector<std::vector<Plane>> groups;
-  const long long budget = std::max<long long>(5 * n0, kAdjBudgetBytes / (2 * (long long)sizeof(T)));
-  long long used = 0, most = 0;
-  for (int s = 0; s < ns; s++)
-    for (int c = 0; c < 3; c++) {
-      if (groups.empty() || used + 5 * sc[s].n > budget) {
-        groups.emplace_back();
-        used = 0;
+  long long most = 0, half = 0;
+  auto group_by = [&](long long budget) {
+    groups.clear();
+    long long used = 0;
+    most = 0;
+    for (int s = 0; s < ns; s++)
+      for (int c = 0; c < 3; c++) {
+        if (groups.empty() || used + 5 * sc[s].n > budget) {
+          groups.emplace_back();
+          used = 0;
+        }
+        groups.back().push_back({s, c});
+        used += 5 * sc[s].n;
+        most = std::max(most, used);
       }
-      groups.back().push_back({s, c});
-      used += 5 * sc[s].n;
-      most = std::max(most, used);
-    }
-  const bool keep = groups.size() == 1;
+    half = (most + 31) / 32 * 32;  // the second buffer starts as aligned as the first
+  };
   T* pa = ws("pa", total);
   T* pb = ws("pb", total);
   T* xa = ws("xa", total);
   T* xb = ws("xb", total);
-  T* hb5 = ws("hb5", most);  // row-blurred products; the gradients of the moments
-  T* mom = ws("mom", most);  // moments; the gradients through the transposed column blur
   T* gx = ws("gx", total);   // d score / d xb
   T* gl = ws("gl", total);   // d score / d linear
   // The jobs of a group with `ctas` CTAs each (by plane size).
@@ -702,11 +705,23 @@ int grad_impl(rcg_ctx* ctx, const uint8_t* d_ref, const float* d_dist, int w, in
     return [rows](const AdjJob& j) { return ((long long)((j.h + rows - 1) / rows) * j.w + 255) / 256; };
   };
   auto by_grid = [](const AdjJob& j) { return (long long)grid_of(j.n); };
-  size_t max_parts = 0;
-  for (const auto& g : groups) max_parts = std::max<size_t>(max_parts, grid(jobs_of(g, by_grid)));
   double* sums = (double*)workspace(ctx, (pfx + "sums").c_str(), sizeof(double) * kMaxScales * 18);
-  double* parts = (double*)workspace(ctx, (pfx + "parts").c_str(), sizeof(double) * 6 * max_parts);
-  if (!pa || !pb || !xa || !xb || !hb5 || !mom || !gx || !gl || !sums || !parts) return RCG_NO_MEMORY;
+  if (!pa || !pb || !xa || !xb || !gx || !gl || !sums) return RCG_NO_MEMORY;
+  // Row-blurred products, later the gradients of the moments; the moments, later those through the transposed column
+  // blur. One buffer, last: where it cannot be had, smaller groups, down to a plane at a time.
+  T* hb5 = nullptr;
+  double* parts = nullptr;
+  for (long long budget = kAdjBudgetBytes / (2 * (long long)sizeof(T));; budget = most / 2) {
+    group_by(budget);
+    size_t max_parts = 0;
+    for (const auto& g : groups) max_parts = std::max<size_t>(max_parts, grid(jobs_of(g, by_grid)));
+    parts = (double*)workspace(ctx, (pfx + "parts").c_str(), sizeof(double) * 6 * max_parts);
+    if (!parts) return RCG_NO_MEMORY;
+    if ((hb5 = ws("moments", 2 * half))) break;
+    if (most <= 5 * n0) return RCG_NO_MEMORY;
+  }
+  T* const mom = hb5 + half;
+  const bool keep = groups.size() == 1;
   RCG_LAUNCH(ctx, "adj_lin", k_lin<T>, grid_of(n0), 256, 0, d_ref, d_dist, n0, pa, pb);
   for (int s = 1; s < ns; s++)
     RCG_LAUNCH(ctx, "adj_down", k_down<T>, grid_rows(sc[s].w, sc[s].h, 6), 256, 0, pa + sc[s - 1].off,
