@@ -689,7 +689,7 @@ int rcg_ssimulacra2_exact(rcg_ctx* ctx, const uint8_t* reference, const uint8_t*
   if ((rc = copy_to_device(ctx, d_b, distorted, bytes)) != RCG_OK) return rc;
   if ((rc = to_linear(ctx, d_a, w, h, w, channels, depth, lin)) != RCG_OK) return rc;
   if ((rc = to_linear(ctx, d_b, w, h, w, channels, depth, lin + np)) != RCG_OK) return rc;
-  if ((rc = exact_score(ctx, lin, lin + np, w, h, d_score)) != RCG_OK) return rc;
+  if ((rc = exact_score(ctx, lin, lin + np, w, h, w, np / 3, d_score)) != RCG_OK) return rc;
   if ((rc = read_back(ctx, &s, d_score, sizeof(double))) != RCG_OK) return rc;
   if ((rc = finish(ctx, "ssimulacra2_exact")) != RCG_OK) return rc;
   if (!std::isfinite(s)) return fail(ctx, RCG_INVALID, "SSIMULACRA 2 produced a non-finite score");
@@ -1225,26 +1225,18 @@ static void score_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st
 }
 
 // The reference-order FP64 score of a paused search's candidate to d_exact. Its planes are still the paused candidate's
-// (every later step was inactive), so its linear samples are made again from them, and the reference's are copied out
-// of its pyramid: both in rows without padding, as exact_score reads them.
+// (every later step was inactive), so its linear samples are made again from them, in the place of its differences, which
+// the next candidate's replace; the reference's lie in its pyramid, in rows of the same pitch.
 static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st, const uint8_t* planes, int w, int h,
                            double* d_exact) {
-  const size_t np = (size_t)w * h;
-  float* lin = (float*)workspace(ctx, "x_lin", 6 * np * sizeof(float), false);
-  if (!lin) return RCG_NO_MEMORY;
   const ScaleDesc& s0 = sc.pd.s[0];
-  cudaError_t e = cudaSuccess;
-  for (int c = 0; c < 3 && e == cudaSuccess; c++)  // a gray reference's one plane three times
-    e = cudaMemcpy2DAsync(lin + c * np, (size_t)w * sizeof(float),
-                          sc.ref_pyr + s0.off + (s0.planes == 3 ? c : 0) * (size_t)s0.pitch * h,
-                          (size_t)s0.pitch * sizeof(float), (size_t)w * sizeof(float), (size_t)h, cudaMemcpyDeviceToDevice,
-                          ctx->stream);
+  const size_t plane = s0.planes == 3 ? (size_t)s0.pitch * h : 0;
   static const int kActive = 1;  // the later steps' tables cleared it; the next step's set it again
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "near-tie rescore");
   int rc = copy_to_device(ctx, &d_st->active, &kActive, sizeof(int));
   if (rc != RCG_OK) return rc;
-  upsample_color(ctx, d_st, planes, w, h, nullptr, lin + 3 * np, w);
-  return exact_score(ctx, lin, lin + 3 * np, w, h, d_exact);
+  float* lin = sc.dist_pyr + s0.off;
+  upsample_color(ctx, d_st, planes, w, h, nullptr, lin, s0.pitch, plane);
+  return exact_score(ctx, sc.ref_pyr + s0.off, lin, w, h, s0.pitch, plane, d_exact);
 }
 
 // Near ties. jpeg/src/target.rs:48 accepts a candidate on s >= target; the fast scorer is within about 1e-6 of the

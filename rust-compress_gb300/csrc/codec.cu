@@ -826,13 +826,14 @@ __device__ __forceinline__ int up_sample(const uint8_t* p, int stride, int cw, i
 
 // Decoder::finish for an 8-bit YCbCr or Gray CoefImage (jpeg/src/decode.rs:1404-1444): upsample every component to
 // full resolution, then the fixed-point YCbCr->RGB of :1438-1441. Writes interleaved pixels and/or the linear-light
-// planes the scorer starts from (core/src/ssimulacra2.rs:192-203: Gray is replicated to three channels).
+// planes the scorer starts from (core/src/ssimulacra2.rs:192-203: Gray is replicated to three channels), np samples apart
+// (0: Gray, one plane).
 // 10 CTAs per SM (48 registers) instead of 7: the kernel waits on loads, so more warps hide more of it
 // (51 -> 47 us per 12 MP candidate).
 __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__ st,
                                                     const uint8_t* __restrict__ planes, int w, int h,
                                                     uint8_t* __restrict__ rgb, float* __restrict__ lin,
-                                                    const int pitch, const unsigned bx, const unsigned by, const unsigned gy) {
+                                                    const int pitch, const size_t np, const unsigned bx, const unsigned by, const unsigned gy) {
   if (!st->active) return;
   const int ncomp = st->ncomp, hmax = st->hmax, vmax = st->vmax;
   const CompDesc c0 = st->comp[0];
@@ -843,7 +844,6 @@ __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__
   // Four consecutive pixels of one row per thread, so each thread moves enough bytes per request.
   const int x0 = 4 * (bx * blockDim.x + threadIdx.x);
   if (x0 >= w) return;
-  const size_t np = (size_t)pitch * h;  // a plane of lin
   const bool vec_out = pitch % 4 == 0;    // whole quads: the last one may run into the row's padding
   for (int y = by; y < h; y += gy) {
     int yv[4], cbv[4], crv[4];
@@ -935,16 +935,17 @@ __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__
 __global__ void __launch_bounds__(128, 10) k_upsample_color(const StepDesc* __restrict__ st,
                                                              const uint8_t* __restrict__ planes, int w, int h,
                                                              uint8_t* __restrict__ rgb, float* __restrict__ lin,
-                                                             int pitch) {
+                                                             int pitch, size_t np) {
   grid_chain();
-  upsample_color_body(st, planes, w, h, rgb, lin, pitch, blockIdx.x, blockIdx.y, gridDim.y);
+  upsample_color_body(st, planes, w, h, rgb, lin, pitch, np, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, uint8_t* d_rgb,
-                   float* d_lin, int pitch) {
+                   float* d_lin, int pitch, size_t plane) {
   // A CTA takes every (h + 1) / 8-th row, eight in all, so that it fills its shared-memory table once for them.
   dim3 grid(((w + 3) / 4 + 127) / 128, std::min(((h + 1) / 2 + 3) / 4, 65535));
-  RCG_LAUNCH(ctx, "upsample_color", k_upsample_color, grid, 128, 0, d_step, d_planes, w, h, d_rgb, d_lin, pitch);
+  RCG_LAUNCH(ctx, "upsample_color", k_upsample_color, grid, 128, 0, d_step, d_planes, w, h, d_rgb, d_lin, pitch,
+             plane);
   return RCG_OK;
 }
 

@@ -44,8 +44,8 @@ constexpr double kXM20 = 0.243422689245478200, kXM21 = 0.204767444244968200, kXM
 constexpr double kXBias = 0.0037930732552754493;
 constexpr double kXC2 = 0.0009;
 
-// downsample (:223-247): one output sample of channel blockIdx.y.
-__global__ void __launch_bounds__(256) k_x_down(const float* __restrict__ src, int w, int h,
+// downsample (:223-247): one output sample of channel blockIdx.y. Source rows are `pitch` samples apart, its planes `plane`.
+__global__ void __launch_bounds__(256) k_x_down(const float* __restrict__ src, int w, int h, int pitch, size_t plane,
                                                 float* __restrict__ dst, int ow, int oh) {
   grid_chain();
   const long long n = (long long)ow * oh;
@@ -53,11 +53,11 @@ __global__ void __launch_bounds__(256) k_x_down(const float* __restrict__ src, i
   if (i >= n) return;
   const int c = blockIdx.y;
   const int oy = (int)(i / ow), ox = (int)(i - (long long)oy * ow);
-  const float* p = src + (size_t)c * w * h;
+  const float* p = src + (size_t)c * plane;
   const int y0 = oy * 2, y1 = min(oy * 2 + 2, h), x0 = ox * 2, x1 = min(ox * 2 + 2, w);
   double sum = 0.0;
   for (int y = y0; y < y1; y++)
-    for (int x = x0; x < x1; x++) sum += (double)p[(size_t)y * w + x];
+    for (int x = x0; x < x1; x++) sum += (double)p[(size_t)y * pitch + x];
   dst[(size_t)c * n + i] = (float)(sum / (double)((y1 - y0) * (x1 - x0)));
 }
 
@@ -74,14 +74,16 @@ __device__ __forceinline__ void xyb_ref(double r, double g, double b, double out
   out[2] = (m2 - y) + 0.55;
 }
 
-// XYB of rows [lo, lo + rows) of both images (:353-367): planes [3][rows][w] each.
-__global__ void __launch_bounds__(256) k_x_xyb(const float* __restrict__ a, const float* __restrict__ b, int w, int h,
-                                               int lo, int rows, double* __restrict__ xa, double* __restrict__ xb) {
+// XYB of rows [lo, lo + rows) of both images (:353-367), laid out as k_x_down's source: planes [3][rows][w] each.
+__global__ void __launch_bounds__(256) k_x_xyb(const float* __restrict__ a, const float* __restrict__ b, int w, int pitch,
+                                               size_t plane, int lo, int rows, double* __restrict__ xa,
+                                               double* __restrict__ xb) {
   grid_chain();
   const long long n = (long long)rows * w;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const size_t np = (size_t)w * h, g = (size_t)lo * w + (size_t)i;
+  const int y = (int)(i / w), x = (int)(i - (long long)y * w);
+  const size_t np = plane, g = (size_t)(lo + y) * pitch + x;
   double pa[3], pb[3];
   xyb_ref((double)a[g], (double)a[np + g], (double)a[2 * np + g], pa);
   xyb_ref((double)b[g], (double)b[np + g], (double)b[2 * np + g], pb);
@@ -299,7 +301,8 @@ static size_t group_bytes(int w, int orows, int rows) {
 
 constexpr size_t kExactGroupBudget = (size_t)4 << 30;
 
-int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, int h, double* d_score) {
+int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, int h, int pitch0, size_t plane0,
+                double* d_score) {
   cudaError_t e = exact_constants(ctx->device);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "exact scorer constant tables");
   // Scales (:480-490): at most 6, while both sides are >= 8.
@@ -335,7 +338,8 @@ int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, 
   const float* b = d_dist0;
   float* next = pyr;
   for (int s = 0; s < ns; s++) {
-    const int W = sw[s], H = shh[s];
+    const int W = sw[s], H = shh[s], pitch = s == 0 ? pitch0 : W;
+    const size_t plane = s == 0 ? plane0 : (size_t)W * H;
     const int nst = (H + kStripe - 1) / kStripe;
     for (int j0 = 0; j0 < nst; j0 += gstripes) {
       const int j1 = std::min(nst, j0 + gstripes);
@@ -348,7 +352,7 @@ int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, 
       double* h5 = xb + 3 * n;
       double* maps = h5 + 5 * n;
       const unsigned gi = (unsigned)((n + 255) / 256), go = (unsigned)((no + 255) / 256);
-      RCG_LAUNCH(ctx, "x_xyb", k_x_xyb, gi, 256, 0, a, b, W, H, lo, rows, xa, xb);
+      RCG_LAUNCH(ctx, "x_xyb", k_x_xyb, gi, 256, 0, a, b, W, pitch, plane, lo, rows, xa, xb);
       for (int c = 0; c < 3; c++) {
         RCG_LAUNCH(ctx, "x_hblur", k_x_hblur, gi, 256, 0, xa + c * n, xb + c * n, W, rows, h5);
         RCG_LAUNCH(ctx, "x_vmaps", k_x_vmaps, go, 256, 0, h5, xa + c * n, xb + c * n, W, H, lo, rows, y0, y1,
@@ -365,8 +369,8 @@ int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, 
       float* nb = next + np;
       next += 2 * np;
       const dim3 g((unsigned)(((long long)ow * oh + 255) / 256), 3);
-      RCG_LAUNCH(ctx, "x_down", k_x_down, g, 256, 0, a, W, H, na, ow, oh);
-      RCG_LAUNCH(ctx, "x_down", k_x_down, g, 256, 0, b, W, H, nb, ow, oh);
+      RCG_LAUNCH(ctx, "x_down", k_x_down, g, 256, 0, a, W, H, pitch, plane, na, ow, oh);
+      RCG_LAUNCH(ctx, "x_down", k_x_down, g, 256, 0, b, W, H, pitch, plane, nb, ow, oh);
       a = na;
       b = nb;
     }

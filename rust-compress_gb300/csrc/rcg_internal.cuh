@@ -407,9 +407,11 @@ constexpr int kRefNone = 0, kRefWrite = 1, kRefRead = 2;
 int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_xyb, const float* d_diff, double* d_score,
                    SearchState* search, StepDesc* step, float2* refm = nullptr, int ref_mode = kRefNone,
                    const NextStep& next = NextStep());
-// The reference-order FP64 score (exact.cu) of two images given as scale-0 linear planes ([3][h][w] f32, as
-// to_linear writes them): to d_score (NaN for the reference's non-finite Err), queued on the context stream.
-int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, int h, double* d_score);
+// The reference-order FP64 score (exact.cu) of two images given as scale-0 linear planes, rows `pitch` and planes `plane`
+// samples apart (plane 0: gray, one plane for all three): to d_score (NaN for the reference's non-finite Err), queued on
+// the context stream.
+int exact_score(rcg_ctx* ctx, const float* d_ref0, const float* d_dist0, int w, int h, int pitch, size_t plane,
+                double* d_score);
 // Record the exact score of a paused search's candidate (search_record without the pause) and let it go on.
 int search_resume(rcg_ctx* ctx, SearchState* d_ss, const double* d_score);
 // The scorer's CTA layout for a pyramid: 32-column bands of `nch0` chunks of 32 rows at the scales with at least
@@ -465,9 +467,9 @@ int trellis_decode(rcg_ctx* ctx, StepDesc* d_step, const float* const* d_caches,
 int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t* d_planes, long long max_blocks,
                  int count = 1, long long planes_stride = 0);
 // Upsample + YCbCr->RGB (jpeg/src/decode.rs:1404-1444). Writes interleaved 8-bit pixels to d_rgb (nullable)
-// and/or linear planes [3][h][pitch] to d_lin (nullable).
+// and/or linear planes to d_lin (nullable), rows `pitch` and planes `plane` samples apart (plane 0: Gray, one plane).
 int upsample_color(rcg_ctx* ctx, StepDesc* d_step, const uint8_t* d_planes, int w, int h, uint8_t* d_rgb,
-                   float* d_lin, int pitch = 0);
+                   float* d_lin, int pitch = 0, size_t plane = 0);
 // Host-side table setup of one quality into a host StepDesc (no device work).
 void host_step_tables(StepDesc* st, int quality, int subsampling, int channels, int trellis, int w, int h);
 // core/src/metrics.rs on device images: ssim (score to d_score; with ss, one bisection step; gated by st), the

@@ -1413,7 +1413,8 @@ int build_decoded(rcg_ctx* ctx, const PyramidDesc& pd, StepDesc* d_step, const u
   g.ref = d_ref;
   g.planes = d_planes;
   g.st = d_step;
-  if (!direct) upsample_color(ctx, d_step, d_planes, pd.s[0].w, pd.s[0].h, nullptr, d_out, pd.s[0].pitch);
+  if (!direct) upsample_color(ctx, d_step, d_planes, pd.s[0].w, pd.s[0].h, nullptr, d_out, pd.s[0].pitch,
+                               (size_t)pd.s[0].pitch * pd.s[0].h);
   const char* name = d_ref ? "build_diff" : "build_reference";
   cudaEvent_t ea, eb;
   launch_begin(ctx, name, &ea, &eb);
