@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "rcg_internal.cuh"
+#include "curve_power.cuh"
 
 namespace rcg {
 
@@ -55,46 +56,12 @@ template <> __device__ __forceinline__ float tap<float>(int t) { return c_k32[t]
 __device__ __forceinline__ double cbrt_t(double x) { return cbrt(x); }
 __device__ __forceinline__ float cbrt_t(float x) { return cbrtf(x); }
 
-// x^0.4 = y + lo for x > 0, the fifth root of x^2 = a + ea: r = a^(-1/5) from an f32 seed by two steps of Newton's
-// iteration for the inverse root (r <- r (6 - a r^5) / 5; an error e becomes 3 e^2, 1e-6 -> 3e-12 -> 3e-23), then y = a
-// r^4 and one Newton step on y^5 = a + ea whose residual carries the rounding errors of a, y^2 and y^4, kept apart as lo.
-// About 30 FP64 operations where pow takes some two hundred; products formed with y and lo round once more, so the curve
-// below is within an ulp, as pow is. False for values outside the f32 range (those go to pow).
-__device__ __forceinline__ bool pow04(double x, double& a, double& ea, double& y, double& lo) {
-  a = x * x;
-  ea = fma(x, x, -a);
-  if (!(a > 1e-30 && a < 1e30)) return false;
-  const float l2 = log2f((float)a);
-  double r = (double)exp2f(-0.2f * l2);
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const double r2 = r * r, r5 = r2 * r2 * r;
-    r = r * fma(-0.2 * a, r5, 1.2);
-  }
-  const double r2 = r * r, r4 = r2 * r2;
-  y = a * r4;
-  const double y2 = y * y, e2 = fma(y, y, -y2);
-  const double y4 = y2 * y2, e4 = fma(2.0 * y2, e2, fma(y2, y2, -y4));
-  lo = (fma(-y4, y, a) + fma(-e4, y, ea)) * 0.2 * r4;  // y = 1 / r, so 1 / (5 y^4) = r^4 / 5
-  // The curve's exponents 2.4 and 1.4 are f64 values, both 8.88e-17 below the decimals: x^-8.88e-17 = 1 - 8.88e-17 ln x.
-  lo = fma(y, -8.881784197001252e-17 * 0.34657359027997264 * (double)l2, lo);
-  return true;
-}
-
 __device__ __forceinline__ double srgb64(double v) {
-  if (v <= 0.04045) return v / 12.92;
-  const double x = (v + 0.055) / 1.055;
-  double a, ea, y, lo;
-  if (!pow04(x, a, ea, y, lo)) return pow(x, 2.4);
-  return fma(a, y, fma(a, lo, ea * y));
+  return v <= 0.04045 ? v / 12.92 : pow24((v + 0.055) / 1.055);
 }
 __device__ __forceinline__ double srgb64_deriv(double v255) {
   const double v = v255 / 255.0;
-  if (v <= 0.04045) return 1.0 / (12.92 * 255.0);
-  const double x = (v + 0.055) / 1.055;
-  double a, ea, y, lo;
-  const double p = pow04(x, a, ea, y, lo) ? fma(x, y, x * lo) : pow(x, 1.4);
-  return 2.4 * p / (1.055 * 255.0);
+  return v <= 0.04045 ? 1.0 / (12.92 * 255.0) : 2.4 * pow14((v + 0.055) / 1.055) / (1.055 * 255.0);
 }
 
 __device__ __forceinline__ long long tid1() { return (long long)blockIdx.x * blockDim.x + threadIdx.x; }
