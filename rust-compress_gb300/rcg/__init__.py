@@ -204,7 +204,7 @@ class CoefImage:
         end = None
         for a in arrs:
             if not (isinstance(a, np.ndarray) and a.dtype == np.int16 and a.ndim == 1 and a.flags.c_contiguous
-                    and (end is None or a.ctypes.data == end)):
+                    and a.flags.aligned and (end is None or a.ctypes.data == end)):
                 break
             end = a.ctypes.data + a.nbytes
         else:
