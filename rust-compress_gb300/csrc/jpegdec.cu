@@ -193,52 +193,26 @@ __device__ __forceinline__ void add_count(SubCount& a, const SubCount& b) {
   for (int q = 0; q < 4; q++) a.dc[q] += b.dc[q];
 }
 
-// Bit reader over a segment's unstuffed bytes: reads past the segment's end give zeros (decode.rs:30-60). Bytes
-// inside a shared-memory window (the CTA's slice of the buffer, loaded once, coalesced) come from there; the rest
-// from global memory.
+// Bit reader over a segment's unstuffed bytes, of AC refinement scans: reads past the segment's end give zeros
+// (decode.rs:30-60).
 struct Reader {
-  const uint8_t* p;       // segment start in global memory
-  const uint8_t* win;     // shared-memory copy of global bytes [win_lo, win_hi) of the scan buffer
-  long long seg_at;       // scan-buffer offset of the segment start
-  long long win_lo, win_hi;
+  const uint8_t* p;  // segment start
   long long len, next;
   uint64_t buf;
   int n;
-  long long bit;
-  __device__ void init(const uint8_t* data, long long seg_byte0, long long nbytes, long long at,
-                       const uint8_t* window = nullptr, long long lo = 0, long long hi = 0) {
+  __device__ void init(const uint8_t* data, long long seg_byte0, long long nbytes) {
     p = data + seg_byte0;
-    seg_at = seg_byte0;
-    win = window;
-    win_lo = lo;
-    win_hi = hi;
     len = nbytes;
-    next = at >> 3;
+    next = 0;
     buf = 0;
     n = 0;
-    bit = at;
     refill();
-    skip((int)(at & 7));
-    bit = at;
   }
-  __device__ __forceinline__ uint64_t byte_at(long long j) const {
-    if (j >= len) return 0;
-    const long long g = seg_at + j;
-    if (g >= win_lo && g < win_hi) return win[g - win_lo];
-    return p[j];
-  }
+  __device__ __forceinline__ uint64_t byte_at(long long j) const { return j < len ? p[j] : 0; }
   __device__ __forceinline__ void refill() {
-    // Four bytes at a time (whole window hits take no per-byte checks); keeps at least 32 bits buffered.
-    while (n <= 32) {
-      const long long g = seg_at + next;
-      uint32_t w;
-      if (next + 4 <= len && g >= win_lo && g + 4 <= win_hi) {
-        const uint8_t* q = win + (g - win_lo);
-        w = ((uint32_t)q[0] << 24) | ((uint32_t)q[1] << 16) | ((uint32_t)q[2] << 8) | q[3];
-      } else {
-        w = (uint32_t)((byte_at(next) << 24) | (byte_at(next + 1) << 16) | (byte_at(next + 2) << 8) |
-                       byte_at(next + 3));
-      }
+    while (n <= 32) {  // four bytes at a time: at least 32 bits buffered
+      const uint32_t w = (uint32_t)((byte_at(next) << 24) | (byte_at(next + 1) << 16) | (byte_at(next + 2) << 8) |
+                                    byte_at(next + 3));
       buf |= (uint64_t)w << (32 - n);
       next += 4;
       n += 32;
@@ -251,7 +225,6 @@ struct Reader {
   __device__ __forceinline__ void skip(int k) {
     buf <<= k;
     n -= k;
-    bit += k;
   }
   __device__ __forceinline__ uint32_t bits(int k) {
     if (k == 0) return 0;
@@ -876,7 +849,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_ac_refine(const ScanDesc* __
     const Segment& sg = segs[s];
     const DevHuff& ac = tb.ac[sd.ac[0]];
     Reader r;
-    r.init(data, sg.byte0, sg.nbytes, 0);
+    r.init(data, sg.byte0, sg.nbytes);
     uint32_t eobrun = 0;
     int4 nxt[8];
     if (sg.nblocks > 0) {
@@ -1314,8 +1287,7 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
     if (!sc.bytes.empty() && (rc = copy_to_device(ctx, d_bytes, sc.bytes.data(), sc.bytes.size())) != RCG_OK)
       return rc;
     if ((rc = copy_to_device(ctx, d_segs, sc.segs.data(), sizeof(Segment) * sc.segs.size())) != RCG_OK ||
-        (rc = copy_to_device(ctx, d_sd, &sc.sd, sizeof(ScanDesc))) != RCG_OK ||
-        (rc = copy_to_device(ctx, d_tab, &sc.tables, sizeof(Tables))) != RCG_OK)
+        (rc = copy_to_device(ctx, d_sd, &sc.sd, sizeof(ScanDesc))) != RCG_OK)
       return rc;
     if (sc.sd.kind == kDcRefine) {
       long long nb = 0;
@@ -1326,6 +1298,7 @@ int jpeg_decode(rcg_ctx* ctx, const uint8_t* data, size_t len, rcg_jpeg_info* in
       continue;
     }
     if (sc.sd.kind == kAcRefine) {
+      if ((rc = copy_to_device(ctx, d_tab, &sc.tables, sizeof(Tables))) != RCG_OK) return rc;
       RCG_LAUNCH(ctx, "ac_refine", k_ac_refine, (unsigned)((sc.sd.nseg + kRefineThreads - 1) / kRefineThreads),
                  kRefineThreads, 0, d_sd, d_tab, d_segs, d_bytes, d_out, d_err);
       continue;
