@@ -340,12 +340,12 @@ int rcg_search_batch(rcg_ctx* ctx, int n, const uint8_t* const* srcs, const uint
                      const size_t* coefs_len, uint8_t* const* qtables);
 
 /* The same many searches in lockstep: every bisection step of every image is one launch per stage over a work-list
- * of all the images' CTAs (step tables, quantization, rate tables, trellis, dequantization + IDCT, upsampling,
- * pyramid, scorer tiles, reductions), the step loop captured as one CUDA graph per batch composition (the images'
- * sizes) and replayed for later batches of the same composition. Each image's set-up (upload, FDCTs,
- * the reference pyramid) runs on its own stream first. Results are exactly those of rcg_search on each image (the
+ * of all the images' CTAs (quantization, rate tables, trellis, dequantization + IDCT, pyramids from the decoded planes,
+ * scorer tiles, reductions, which also fill the next step's tables), the step loop captured as one CUDA graph per batch
+ * composition (the images' sizes) and replayed for later batches of the same composition. Each image's set-up (upload,
+ * FDCTs, the reference's pyramids) runs on its own stream first. Results are exactly those of rcg_search on each image (the
  * same kernels per image), near ties included; arguments as rcg_search_batch without `parallel`. All images' buffers
- * are resident at once (about 70 bytes per pixel). Like rcg_search_batch, no single reference function corresponds to
+ * are resident at once (colour at 4:2:0 with the reference moments stored: about 115 bytes per pixel). Like rcg_search_batch, no single reference function corresponds to
  * it: the cli runs find_quality_with per file (jpeg/src/target.rs:29-56) across rayon workers (cli/src/main.rs:57-60).
  */
 int rcg_search_batch_lockstep(rcg_ctx* ctx, int n, const uint8_t* const* srcs, const uint32_t* widths,
@@ -418,8 +418,8 @@ int rcg_search_perceptual(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint
 /* The perceptual search in one full search: the plain bisection's first four candidates only (the maximum quality,
  * then three bisection steps; `probe`, nullable, receives their trace and, as quality and score, the one scoring closest
  * to the target), the weights from the gradient at that candidate's decoded image (strength by its quality when
- * popts->strength_by_quality), then the weighted search, whose result `found`, `coefs` and `qtables` receive. No plain search to compare with and no
- * plans: the result is the weighted search's whatever its size (popts->keep_smaller does not apply). 12 candidates
+ * popts->strength_by_quality), then the weighted search, whose result `found`, `coefs` and `qtables` receive. No plain
+ * search to compare with and no plans: the result is the weighted search's whatever its size (popts->keep_smaller does not apply). 12 candidates
  * against rcg_search_perceptual's 16. */
 int rcg_search_perceptual_fast(rcg_ctx* ctx, const uint8_t* src, uint32_t width, uint32_t height, int channels,
                                double target, int max_quality, const rcg_encode_options* opts,

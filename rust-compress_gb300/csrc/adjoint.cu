@@ -569,7 +569,7 @@ __global__ void k_grad_out(const T* __restrict__ g_lin, const float* __restrict_
 }
 
 unsigned grid_of(long long n) {
-  return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152 * 32));
+  return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, kSms * 32));
 }
 
 // Moments of planes blurred together: their two buffers of five planes each stay within this (320 bytes a pixel in FP64:

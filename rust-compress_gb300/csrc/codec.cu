@@ -403,7 +403,10 @@ __device__ __forceinline__ void rate_tables_body(StepDesc* __restrict__ st, cons
   if (t == 0) st->eob[comp] = fmul(lambda, len[0]);
 }
 
-__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) { grid_chain(); rate_tables_body(st + blockIdx.y, blockIdx.x); }
+__global__ void __launch_bounds__(288) k_rate_tables(StepDesc* __restrict__ st) {
+  grid_chain();
+  rate_tables_body(st + blockIdx.y, blockIdx.x);
+}
 
 int rate_tables(rcg_ctx* ctx, StepDesc* d_step, int count) {
   RCG_LAUNCH(ctx, "rate_tables", k_rate_tables, dim3(3, (unsigned)count), 288, 0, d_step);
@@ -767,7 +770,7 @@ int dequant_idct(rcg_ctx* ctx, StepDesc* d_step, const int16_t* d_coefs, uint8_t
 // four CTAs per SM instead of seven, so the line lies at one wave of those. Measured per search, apart / together: 17 CTAs
 // (240x180) 551 / 542 us, 408 (0.8 MP) 1082 / 1076, 474 (3.9 MP gray) 1280 / 1265; 1107 (6 MP, requantizing) 4877 / 5015.
 constexpr int kDecodeCtas = 4;
-constexpr long long kTrellisDecodeCtas = kDecodeCtas * 152;
+constexpr long long kTrellisDecodeCtas = kDecodeCtas * kSms;
 
 template <bool kWeighted>
 __global__ void __launch_bounds__(128, kDecodeCtas) k_trellis_decode(StepDesc* __restrict__ st, CacheSet cs,
@@ -833,7 +836,8 @@ __device__ __forceinline__ int up_sample(const uint8_t* p, int stride, int cw, i
 __device__ __forceinline__ void upsample_color_body(const StepDesc* __restrict__ st,
                                                     const uint8_t* __restrict__ planes, int w, int h,
                                                     uint8_t* __restrict__ rgb, float* __restrict__ lin,
-                                                    const int pitch, const size_t np, const unsigned bx, const unsigned by, const unsigned gy) {
+                                                    const int pitch, const size_t np, const unsigned bx,
+                                                    const unsigned by, const unsigned gy) {
   if (!st->active) return;
   const int ncomp = st->ncomp, hmax = st->hmax, vmax = st->vmax;
   const CompDesc c0 = st->comp[0];

@@ -56,7 +56,7 @@ __device__ __forceinline__ void huff_merge(T* W, HuffScratch& s, int n) {
 
 
 // freq: 257 counts in shared memory (freq[256] = 1); lens: 257 code lengths out (0 = unused), shared memory.
-// Every thread of the CTA calls it; the CTA has at least 257 threads.
+// Every thread of the CTA calls it; the CTA has at least 260 threads (one per count and padding of the last quad).
 //
 // The two-queue merge is the one sequential step: one thread, with the head of each queue and the element behind it
 // held in registers so that a pick does not wait for a shared-memory load. The depth pass, the per-length counts

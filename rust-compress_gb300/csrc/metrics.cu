@@ -186,7 +186,7 @@ __global__ void k_down2(const uint8_t* __restrict__ in, int w, int nw, int nh, u
 }
 
 int grid_for(size_t n, int threads) {
-  return (int)std::min<size_t>((n + threads - 1) / threads, (size_t)152 * 16);
+  return (int)std::min<size_t>((n + threads - 1) / threads, (size_t)kSms * 16);
 }
 
 }  // namespace

@@ -252,7 +252,7 @@ int upload_tables(rcg_ctx* ctx) {
 }  // namespace
 
 int expand_rgb(rcg_ctx* ctx, const uint8_t* d_src, int channels, size_t npx, uint8_t* d_rgb8, float* d_rgbf) {
-  const unsigned grid = (unsigned)std::min<size_t>((npx + 255) / 256, 152 * 16);
+  const unsigned grid = (unsigned)std::min<size_t>((npx + 255) / 256, (size_t)kSms * 16);
   RCG_LAUNCH(ctx, "expand_rgb", k_expand_rgb, grid, 256, 0, d_src, channels, npx, d_rgb8, d_rgbf);
   return RCG_OK;
 }

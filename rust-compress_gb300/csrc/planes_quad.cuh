@@ -50,8 +50,8 @@ __device__ __forceinline__ void ycc_linear(uint32_t q, const int (&cb4)[4], cons
 }
 
 // Linear-light values of four columns (x0 .. x0+3, x0 % 4 == 0) of output row y, for the layouts of an encoder's own
-// candidates (layout_direct in capi.cu): Gray, 4:4:4, 4:2:2 and 4:2:0 with luma at full resolution (jpeg/src/decode.rs:1768-1828,
-// :1438-1441).
+// candidates (layout_direct in capi.cu): Gray, 4:4:4, 4:2:2 and 4:2:0 with luma at full resolution
+// (jpeg/src/decode.rs:1768-1828, :1438-1441).
 __device__ __forceinline__ void planes_quad(const StepDesc* __restrict__ st, const uint8_t* __restrict__ planes, int w,
                                             int h, const float* lut, int x0, int y, float (&l)[3][4]) {
   const CompDesc& c0 = st->comp[0];

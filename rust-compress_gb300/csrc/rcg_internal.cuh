@@ -26,6 +26,7 @@ constexpr int kRadius = 5;
 constexpr int kTileW = 32;
 constexpr int kTileH = 32;
 constexpr int kTileThreads = 128;
+constexpr int kSms = 152;  // of the GPU, where a grid's size or a rule's line follows from it
 constexpr int kTileCtas = 4, kTileCtasRead = 6;  // per SM: the scorer's form with five blurred moments, with three
 
 // ------------------------------------------------------------------------------------------------ descriptors

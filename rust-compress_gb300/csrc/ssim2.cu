@@ -1,8 +1,9 @@
 // SSIMULACRA2 scorer kernels (K8-K10): the reference's core/src/ssimulacra2.rs on one GPU.
 //
-// Pipeline per score: linear-light planes (f32, channel-planar) -> 2x2 pyramid (scales 1..5) -> one launch that
-// covers every tile of every scale (XYB, five moments, 11-tap blur, error maps, six partial sums per channel) ->
-// a deterministic f64 reduction and the final 108-weight mapping.
+// Pipeline per score: one launch that takes both images (or a decoded candidate and a reference's linear pyramid) to the
+// reference's XYB and the two images' XYB differences at every scale (f32, channel-planar; the 2x2 pyramid, scales 1..5,
+// in shared memory) -> one launch that covers every tile of every scale (five moments, 11-tap blur, error maps, six
+// partial sums per channel) -> a deterministic f64 reduction and the final 108-weight mapping.
 //
 // Arithmetic. The reference holds the planes in f32 and computes XYB, the blur, the maps and the sums in f64
 // (:18, :345-346, :361). GB300's FP64 rate is a small fraction of its FP32 rate, so here:
@@ -10,7 +11,7 @@
 //     reference's f64 sum nearly always);
 //   * XYB, blur and maps: f32, arranged so that nothing cancels catastrophically. Each pixel carries the reference
 //     image's XYB and the XYB *difference* of the two images, both computed from cube-root difference identities
-//     (see pix()); both are offset by their value at the tile centre, so the five blurred moments (mu_a, mu_(a-b),
+//     (see dsq2()); both are offset by their value at the tile centre, so the five blurred moments (mu_a, mu_(a-b),
 //     E[a^2], E[b^2], E[(a-b)^2]) are small where the image is smooth. The variances and mu1 - mu2 are recovered
 //     exactly from them (the offsets cancel wherever the blur taps sum to 1 and are corrected with the in-image tap
 //     sum within 5 columns of the zero left/right border, :34-40). The SSIM term is evaluated as
@@ -18,9 +19,11 @@
 //     that equal the reference's expressions algebraically but keep full relative precision for similar images;
 //   * cube roots: 2^(log2(x) / 3) from the hardware's approximate log2 and exp2 (relative error a few 1e-7; the
 //     differences between the two images never go through them, only through the identity below);
-//   * sums: f32 over the 4 pixels of a thread (in registers, then added to the thread's running sums of its band),
+//   * sums: f32 over the 8 pixels of a thread (in registers, then added to the thread's running sums of its band),
 //     f32 across a warp, f64 from there on, in a fixed order (bit-reproducible from run to run, as the reference's
-//     test :630 requires).
+//     test :630 requires). What they round does not show in a score: against the FP64 scorer, over 25 pairs (flat, ramps,
+//     photographs at four noise levels and four qualities, noise, gray; 23 of 9.4 MP), the error is 1.22e-6 on average and
+//     8.3e-6 at most with bands of 1, 8 or 64 chunks; with half the pixels per thread and warp 1.24e-6 and 8.2e-6.
 // Identical images give exactly 100: every difference term is exactly 0, so every map value is exactly 0.
 #include <type_traits>
 #include <cuda_runtime.h>
@@ -71,7 +74,7 @@ __device__ __forceinline__ float fdiv_ftz(float a, float b) {
   return r;
 }
 
-// x^2 + x*y + y^2 = D(x, y): cbrt(u) - cbrt(v) = (u - v) / D(cbrt(u), cbrt(v)).
+// x^2 + x*y + y^2 = D(x, y) (dsq2): cbrt(u) - cbrt(v) = (u - v) / D(cbrt(u), cbrt(v)).
 // Per pixel the scorer needs the reference image's XYB without its constants (`a`, core/src/ssimulacra2.rs:249-258 less
 // kXyb0*) and XYB(reference) - XYB(distorted) (`d`). Every quantity that is a small difference of nearly equal cube
 // roots is formed from the identity above, so it keeps its relative precision in f32: X - 0.42 = 7 (c0 - c1), B - 0.55 =
@@ -223,7 +226,7 @@ __device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) 
 }
 
 // One CTA = one band of 32 output columns and nch chunks of 32 output rows of one scale, walked top to bottom, from the
-// reference's XYB planes (Pix::a) and the XYB differences (Pix::d). Per chunk and channel: the halo's samples are copied
+// reference's XYB planes (`a`) and the XYB differences (`d`). Per chunk and channel: the halo's samples are copied
 // to shared memory asynchronously, the horizontal pass takes off the chunk's offsets and blurs the 42 halo rows, the
 // vertical pass blurs the columns and evaluates the error maps while the next halo is on its way. The blurs run the
 // moment pairs that share a tap weight as packed two-lane f32 FMAs, each lane exactly fmaf.
@@ -248,8 +251,8 @@ __device__ __forceinline__ void tap_one(float& s, float k, float v, bool first) 
 // chunk's channels measured 278, the maps of two rows as packed operations 273 but 242 plain: neither was kept.
 template <int kRef>
 __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, const int one,
-                                           const float* __restrict__ xa, const float* __restrict__ xd, double* __restrict__ out,
-                                           const size_t stride, float2* __restrict__ refm) {
+                                           const float* __restrict__ xa, const float* __restrict__ xd,
+                                           double* __restrict__ out, const size_t stride, float2* __restrict__ refm) {
   extern __shared__ float4 smem4[];
   float* const xs = reinterpret_cast<float*>(smem4);  // the channel's a, then its d
   // Horizontally blurred moments, [kIH][kTileW]: one plane of pairs (reading form) or two, then one of singles.
@@ -478,63 +481,63 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
       auto maps = [&](auto inside) {
         constexpr bool kInside = decltype(inside)::value;
 #pragma unroll
-      for (int o = 0; o < kVy; o++) {
-        int ry = rg * kVy + o;
-        int gy = y0 + ry;
-        if (kInside || (gx < w && gy < h)) {
-          // Blurred primed moments -> sigma_1^2, sigma_2^2, sigma_(a-b)^2, mu1 - mu2 (exactly, given K).
-          float m1, dmp, e11, e22, edd;
-          if constexpr (kRef == kRefRead) {
-            m1 = rm[o].x;
-            e11 = rm[o].y;
-            dmp = s4[o];
-            e22 = s1[o].x;
-            edd = s1[o].y;
-          } else {
-            m1 = s0[o].x;
-            dmp = s0[o].y;
-            e11 = s1[o].x;
-            edd = s1[o].y;
-            e22 = s4[o];
+        for (int o = 0; o < kVy; o++) {
+          int ry = rg * kVy + o;
+          int gy = y0 + ry;
+          if (kInside || (gx < w && gy < h)) {
+            // Blurred primed moments -> sigma_1^2, sigma_2^2, sigma_(a-b)^2, mu1 - mu2 (exactly, given K).
+            float m1, dmp, e11, e22, edd;
+            if constexpr (kRef == kRefRead) {
+              m1 = rm[o].x;
+              e11 = rm[o].y;
+              dmp = s4[o];
+              e22 = s1[o].x;
+              edd = s1[o].y;
+            } else {
+              m1 = s0[o].x;
+              dmp = s0[o].y;
+              e11 = s1[o].x;
+              edd = s1[o].y;
+              e22 = s4[o];
+            }
+            const float m2 = m1 - dmp;
+            float v1 = fmaf(-m1, m1, e11);
+            float v2 = fmaf(-m2, m2, e22);
+            float vd = fmaf(-dmp, dmp, edd);
+            float dmu;
+            if (!kInside && edge) {
+              v1 = fmaf(omk * ca, fmaf(ca, K, 2.0f * m1), v1);
+              v2 = fmaf(omk * cbv, fmaf(cbv, K, 2.0f * m2), v2);
+              vd = fmaf(omk * cd, fmaf(cd, K, 2.0f * dmp), vd);
+              dmu = fmaf(cd, K, dmp);
+            } else {
+              dmu = dmp + cd;
+            }
+            // SSIM error (core/src/ssimulacra2.rs:427-430) as (sigma_(a-b)^2 + dmu^2 num_s) / denom_s, which equals
+            // 1 - (1 - dmu^2) num_s / denom_s since num_s = denom_s - sigma_(a-b)^2.
+            float den = (v1 + v2) + 0.0009f;
+            float num_s = den - vd;
+            float d = fmaxf(fdiv_ftz(fmaf(dmu * dmu, num_s, vd), den), 0.0f);
+            // Edge maps (:431-433): d1 = (|r2| - |r1|) / (1 + |r1|) with r1 = a - mu1, r2 = b - mu2 = r1 - rd.
+            float r1 = ca0[o] - m1, rd = cd0[o] - dmp;
+            if (!kInside && edge) {
+              r1 = fmaf(ca, omk, r1);
+              rd = fmaf(cd, omk, rd);
+            }
+            // t is 0 (then so is the numerator) or far above the subnormal range: the residuals are differences of
+            // f32 values of order 1e-3..1 and their blurs, so the flush-to-zero division sees a normal divisor.
+            float t = fabsf(r1 - rd) + fabsf(r1);
+            float d1 = t > 0.0f ? fdiv_ftz(-rd * (2.0f * r1 - rd), t * (1.0f + fabsf(r1))) : 0.0f;
+            float art = fmaxf(d1, 0.0f), det = fmaxf(-d1, 0.0f);
+            float d2 = d * d, a2 = art * art, e2 = det * det;
+            acc[0] += d;
+            acc[1] += d2 * d2;
+            acc[2] += art;
+            acc[3] += a2 * a2;
+            acc[4] += det;
+            acc[5] += e2 * e2;
           }
-          const float m2 = m1 - dmp;
-          float v1 = fmaf(-m1, m1, e11);
-          float v2 = fmaf(-m2, m2, e22);
-          float vd = fmaf(-dmp, dmp, edd);
-          float dmu;
-          if (!kInside && edge) {
-            v1 = fmaf(omk * ca, fmaf(ca, K, 2.0f * m1), v1);
-            v2 = fmaf(omk * cbv, fmaf(cbv, K, 2.0f * m2), v2);
-            vd = fmaf(omk * cd, fmaf(cd, K, 2.0f * dmp), vd);
-            dmu = fmaf(cd, K, dmp);
-          } else {
-            dmu = dmp + cd;
-          }
-          // SSIM error (core/src/ssimulacra2.rs:427-430) as (sigma_(a-b)^2 + dmu^2 num_s) / denom_s, which equals
-          // 1 - (1 - dmu^2) num_s / denom_s since num_s = denom_s - sigma_(a-b)^2.
-          float den = (v1 + v2) + 0.0009f;
-          float num_s = den - vd;
-          float d = fmaxf(fdiv_ftz(fmaf(dmu * dmu, num_s, vd), den), 0.0f);
-          // Edge maps (:431-433): d1 = (|r2| - |r1|) / (1 + |r1|) with r1 = a - mu1, r2 = b - mu2 = r1 - rd.
-          float r1 = ca0[o] - m1, rd = cd0[o] - dmp;
-          if (!kInside && edge) {
-            r1 = fmaf(ca, omk, r1);
-            rd = fmaf(cd, omk, rd);
-          }
-          // t is 0 (then so is the numerator) or far above the subnormal range: the residuals are differences of
-          // f32 values of order 1e-3..1 and their blurs, so the flush-to-zero division sees a normal divisor.
-          float t = fabsf(r1 - rd) + fabsf(r1);
-          float d1 = t > 0.0f ? fdiv_ftz(-rd * (2.0f * r1 - rd), t * (1.0f + fabsf(r1))) : 0.0f;
-          float art = fmaxf(d1, 0.0f), det = fmaxf(-d1, 0.0f);
-          float d2 = d * d, a2 = art * art, e2 = det * det;
-          acc[0] += d;
-          acc[1] += d2 * d2;
-          acc[2] += art;
-          acc[3] += a2 * a2;
-          acc[4] += det;
-          acc[5] += e2 * e2;
         }
-      }
       };
       if (inner) maps(std::true_type());
       else maps(std::false_type());
@@ -544,8 +547,8 @@ __device__ __forceinline__ void ssim2_band(const ScaleDesc sd, const int local, 
       od = nod;
     }
   }
-  // Warp sums (f32, 32 threads x kVy pixels per chunk), then the warps in f64 in a fixed order. Sums 0..15 by a reduce-scatter
-  // butterfly: at each exchange (lane distance 16, 8, 4, 2) a lane keeps half of the values it carries and adds its
+  // Warp sums (f32, 32 threads x kVy pixels per chunk), then the warps in f64 in a fixed order. Sums 0..15 by a
+  // reduce-scatter butterfly: at each exchange (lane distance 16, 8, 4, 2) a lane keeps half of the values it carries and adds its
   // partner's copy of that half, then distance 1 adds the pair; lane l ends with sum l >> 1. The additions are those
   // of a full butterfly per sum, so every sum has the same bits, in 16 shuffles instead of 80. Sums 16 and 17 by full
   // butterflies.
@@ -928,7 +931,8 @@ __device__ __forceinline__ void emit_quad(const BuildArgs& g, const ScaleDesc& s
       r[c][3] = rq[c].w;
     }
 #pragma unroll
-    for (int k = 0; k < 2; k++) pix_diff2(at(r, 0, k), at(r, 1, k), at(r, 2, k), at(l, 0, k), at(l, 1, k), at(l, 2, k), o[k]);
+    for (int k = 0; k < 2; k++)
+      pix_diff2(at(r, 0, k), at(r, 1, k), at(r, 2, k), at(l, 0, k), at(l, 1, k), at(l, 2, k), o[k]);
     put4(g.out + i, np, o);
   } else {
 #pragma unroll
@@ -1136,7 +1140,7 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOut)) k_build(const _
 // CTA, where a 64 block takes four and two, one after the other. The same samples either way. Measured, 64 / 32: 12 blocks
 // (240x180) 16.6 / 10.7 us, 64 (512x512, a pair) 22.8 / 14.9, 294 (0.8 MP) 24.4 / 26.4, 442 (1.7 MP) 30.8 / 35.0: most
 // threads of a 32 block idle while the levels above 0 are converted.
-constexpr int kSmallBuild = 152;
+constexpr int kSmallBuild = kSms;
 
 // Queue one builder launch (st: the step that gates it, nullable). Samples that come as linear planes are never gray
 // ones: a gray layout is always read directly.
@@ -1266,7 +1270,8 @@ __global__ void __launch_bounds__(kPyrThreads, build_ctas(kOutDiff)) k_build_loc
 }
 
 template <int kRef>
-__global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_lock(const LockItem* __restrict__ items, int n) {
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef))
+    k_ssim2_tiles_lock(const LockItem* __restrict__ items, int n) {
   grid_chain();
   const int i = lock_find<&LockItem::t0>(items, n, blockIdx.x);
   const LockItem& it = items[i];
@@ -1275,8 +1280,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(kRef)) k_ssim2_tiles_l
   int s = 0;
   while (s + 1 < it.pd.nscales && blk >= it.pd.s[s + 1].tile0) s++;
   const ScaleDesc sd = it.pd.s[s];
-  ssim2_band<kRef>(sd, blk - sd.tile0, channel_of_cta(), it.ref_xyb, it.dist_pyr, it.partials + blk, (size_t)it.pd.total_tiles,
-                   it.refm);
+  ssim2_band<kRef>(sd, blk - sd.tile0, channel_of_cta(), it.ref_xyb, it.dist_pyr, it.partials + blk,
+                   (size_t)it.pd.total_tiles, it.refm);
 }
 
 __global__ void __launch_bounds__(256) k_ssim2_reduce_lock(const LockItem* __restrict__ items) {
@@ -1483,7 +1488,7 @@ int scorer_init(rcg_ctx* ctx) {
 
 // Bands pay off where a scale has enough tiles to keep every SM busy with long CTAs; smaller scales (and whole
 // images below kBandMinTiles0 scale-0 tiles, which are never tuned) keep 32x32 tiles.
-constexpr int kBandMinTiles = 3 * 152;
+constexpr int kBandMinTiles = 3 * kSms;
 constexpr int kBandMinTiles0 = 1024;
 constexpr int kBandCandidates[] = {1, 2, 4, 8};
 
@@ -1506,8 +1511,8 @@ PyramidDesc banded(const PyramidDesc& pd, int nch0, int min_tiles) {
   return b;
 }
 
-// Deterministic stand-in content for the tuning runs (linear values in [0, 1), the second image a perturbed copy);
-// the kernel's time does not depend on the values.
+// Deterministic stand-in content for the tuning runs, in place of the reference's XYB and of the differences (values in
+// [0, 1], the second half like the first); the kernel's time does not depend on the values.
 __global__ void k_tune_fill(float* __restrict__ p, long long n) {
   grid_chain();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -1539,7 +1544,7 @@ static int tune_bands(rcg_ctx* ctx, const PyramidDesc& pd) {
     if (pyr) cudaFree(pyr);
     return 1;  // no room to tune: tiles
   }
-  k_tune_fill<<<4 * 152, 256, 0, ctx->stream>>>(pyr, n);
+  k_tune_fill<<<4 * kSms, 256, 0, ctx->stream>>>(pyr, n);
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
@@ -1603,14 +1608,14 @@ int score_pyramids(rcg_ctx* ctx, const PyramidDesc& pd, const float* d_ref, cons
   unsigned* counter = (unsigned*)ctx->bufs["score_counter"].ptr;
   const PyramidDesc pb = plan_bands(ctx, pd);
   if (!refm || ref_mode == kRefNone)
-    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefNone), pb, d_ref, d_dist,
-               partials, step, nullptr);
+    RCG_LAUNCH(ctx, "ssim2_tiles", k_ssim2_tiles<kRefNone>, tile_grid(pb.total_tiles), kTileThreads,
+               tile_smem(kRefNone), pb, d_ref, d_dist, partials, step, nullptr);
   else if (ref_mode == kRefWrite)
-    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefWrite), pb, d_ref,
-               d_dist, partials, step, refm);
+    RCG_LAUNCH(ctx, "ssim2_tiles_store", k_ssim2_tiles<kRefWrite>, tile_grid(pb.total_tiles), kTileThreads,
+               tile_smem(kRefWrite), pb, d_ref, d_dist, partials, step, refm);
   else
-    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, tile_grid(pb.total_tiles), kTileThreads, tile_smem(kRefRead), pb, d_ref,
-               d_dist, partials, step, refm);
+    RCG_LAUNCH(ctx, "ssim2_tiles_cached", k_ssim2_tiles<kRefRead>, tile_grid(pb.total_tiles), kTileThreads,
+               tile_smem(kRefRead), pb, d_ref, d_dist, partials, step, refm);
   dim3 rg(pb.nscales, kScoreSums);
   RCG_LAUNCH(ctx, "ssim2_reduce", k_ssim2_reduce, rg, 256, 0, pb, partials, scale_sums, counter, d_score, search,
              step, next);
@@ -1809,8 +1814,8 @@ int score_batch(rcg_ctx* ctx, int n, const uint8_t* const* d_refs, const uint8_t
 
 namespace rcg {
 
-// Fixed scratch of rcg_ssimulacra2_device_noalloc: the reference's XYB pyramid and the differences, the per-tile partial sums, the
-// per-scale sums and the reduction's completion counter. Sized for images of at most kNoAllocMaxPixels pixels. CUDA
+// Fixed scratch of rcg_ssimulacra2_device_noalloc: the reference's XYB pyramid and the differences, the per-tile partial
+// sums, the per-scale sums and the reduction's completion counter. Sized for images of at most kNoAllocMaxPixels pixels. CUDA
 // places a module's device arrays on a device when the module is first used there, so every device where any scorer
 // call has run holds it (about 10 MB) until the process exits. The per-device set-up below is cached for the life of
 // the process; a cudaDeviceReset invalidates it and is not supported.
@@ -1887,10 +1892,10 @@ extern "C" int rcg_ssimulacra2_device_noalloc(const uint8_t* d_reference, const 
   g.xyb = pyr_ref;
   g.out = pyr_dist;
   launch_build<kFromImage, kOutPair>(pd, g, nullptr, s);
-  launch_chained(tile_grid(pd.total_tiles), kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref, pyr_dist,
-                 partials, nullptr, nullptr);
+  launch_chained(tile_grid(pd.total_tiles), kTileThreads, tile_smem(kRefNone), s, k_ssim2_tiles<kRefNone>, pd, pyr_ref,
+                 pyr_dist, partials, nullptr, nullptr);
   launch_chained(dim3(pd.nscales, kScoreSums), 256, 0, s, k_ssim2_reduce, pd, partials, sums, counter, d_score, nullptr,
-                                                              nullptr, NextStep());
+                 nullptr, NextStep());
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? RCG_OK : RCG_CUDA_ERROR;
 }

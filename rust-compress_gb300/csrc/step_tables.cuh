@@ -108,7 +108,9 @@ __host__ __device__ inline float mult_entry(const uint8_t* q, int n) { return mu
 //   fdct divisor for zigzag position k: fdct_divisors stores 1 / (q[v*8+u] * AAN[u] * AAN[v] * 8) at [u*8+v]
 //   (jpeg/src/encode.rs:174-183) and quantize_plane reads it at ZZ_T[k] = (n%8)*8 + n/8 (:202), i.e. u = n%8,
 //   v = n/8, q[v*8+u] = q[n]
-__host__ __device__ inline float divz_entry(const uint8_t* q, int k) { return fdiv(1.0f, fmul(mult_entry(q, zigzag(k)), 8.0f)); }
+__host__ __device__ inline float divz_entry(const uint8_t* q, int k) {
+  return fdiv(1.0f, fmul(mult_entry(q, zigzag(k)), 8.0f));
+}
 
 // Block layout of a candidate (jpeg/src/encode.rs:428-443, :511-517).
 __host__ __device__ inline void fill_layout(StepDesc* st, int quality, int subsampling, int channels, int trellis,
