@@ -315,8 +315,8 @@ static void layout_of(int w, int h, int channels, int quality, int subsampling, 
   delete st;
 }
 
-// Encoder front half shared by build_coefs and the search: colour planes and the FDCT caches of every sampling
-// layout the options can produce (two for Subsampling::Auto, whose layout depends on the quality).
+// Encoder front half shared by build_coefs and the search: the FDCT caches of every sampling layout the options can
+// produce (two for Subsampling::Auto, whose layout depends on the quality).
 struct EncoderSetup {
   const float* caches[9] = {nullptr};
   long long max_blocks = 0;
@@ -802,8 +802,9 @@ int rcg_ssimulacra2_batch(rcg_ctx* ctx, int n, const uint8_t* const* references,
 
 // ---- rate-quality sweep
 
-// Device bytes one image of a sweep holds until its group is scored: the image and its candidates' planes (8-bit), and both
-// sides' pyramids in the scorer (3 channels, 4/3 for the coarser scales, 4-byte floats: 16 B per pixel).
+// Device bytes one image of a sweep holds until its group is scored, about: the image and its candidates' planes (8-bit), and
+// a pyramid in the scorer for each of them (3 channels, 4/3 for the coarser scales, 4-byte floats: 16 B per pixel). The
+// image's second pyramid (linear light beside XYB) is not counted.
 static size_t sweep_bytes(uint32_t w, uint32_t h, int channels, int nq) {
   const size_t px = (size_t)w * h;
   return (px * channels + 16 * px) * (size_t)(nq + 1);
@@ -1210,8 +1211,7 @@ static int scorer_setup(rcg_ctx* ctx, int metric, int w, int h, int channels, Se
 }
 
 // Decoded planes of one candidate -> score -> one bisection step and the next one's tables (SSIMULACRA2), all gated by the
-// step's `active`. Step `s` of the
-// loop: the first candidate of a search (s = 0, always active) stores the reference moments, later ones read them.
+// step's `active`. Step `s` of the loop: the first candidate of a search (s = 0, always active) stores the reference moments, later ones read them.
 static void score_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st, const uint8_t* planes, int w,
                             int h, int channels, SearchState* d_ss, int s, const NextStep& next) {
   if (sc.metric == RCG_METRIC_SSIM) {
@@ -1241,10 +1241,10 @@ static int exact_candidate(rcg_ctx* ctx, const SearchScorer& sc, StepDesc* d_st,
 
 // Near ties. jpeg/src/target.rs:48 accepts a candidate on s >= target; the fast scorer is within about 1e-6 of the
 // reference, so a candidate scored within ctx->tie_band of the target paused the device bisection (search_record,
-// done = 2) with its decoded planes still in place (every later step was
-// inactive). Here it is rescored in the reference's f64 arithmetic and order on the GPU (exact_candidate), the bisection
-// records that score and goes on, and the remaining steps run as plain launches; repeated while a later candidate
-// pauses again. `issue_step(s, first)` issues step s's kernels; `first`: its tables too, which no step before it fills.
+// done = 2) with its decoded planes still in place (every later step was inactive). Here it is rescored in the reference's
+// f64 arithmetic and order on the GPU (exact_candidate), the bisection records that score and goes on, and the remaining
+// steps run as plain launches; repeated while a later candidate pauses again. `issue_step(s, first)` issues step s's
+// kernels; `first`: its tables too, which no step before it fills.
 static int settle_ties(rcg_ctx* ctx, const SearchScorer& sc, SearchState* d_ss, SearchState* hs, StepDesc* d_st,
                        const uint8_t* planes, int max_steps, int w, int h,
                        const std::function<void(int, bool)>& issue_step) {
